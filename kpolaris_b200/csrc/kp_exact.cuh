@@ -1,0 +1,66 @@
+// kp_exact.cuh -- correctly rounded FP64 quotients and square roots without
+// the range checks and the out-of-line path of the compiler's own, for
+// operands known to lie well inside the range.  Several quotients by one
+// divisor share its reciprocal, and nothing branches between independent
+// ones, so they overlap: the compiler's division takes a lone warp 127
+// cycles, one after the other, and the Kerr-Schild connection has twenty.
+//
+// Method: P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34 (1990) 111-119 (also Muller et
+// al., Handbook of Floating-Point Arithmetic, ch. 4).  With fused
+// multiply-adds, a reciprocal y of b within one ulp becomes the correctly
+// rounded one by y + y (1 - b y) (but for a divisor whose significand is all
+// ones); with it, a quotient q of a / b within one ulp becomes the correctly
+// rounded one by q - y (b q - a).  The residuals are formed as b q - a so that
+// a zero numerator keeps its sign.  A square root g of v within one ulp
+// becomes the rounded one by g + (v - g g) h with h = 1 / (2 sqrt(v)).  The
+// starting values are the hardware's approximate reciprocal and reciprocal
+// square root, taken to one ulp by a third-order Newton step.
+#pragma once
+
+#include "kp_common.cuh"
+
+namespace kp {
+
+#ifdef __CUDACC__
+
+struct ExactRecip {
+    double b, y;
+};
+
+// The correctly rounded reciprocal of b, 1e-150 < |b| < 1e150.
+__device__ __forceinline__ ExactRecip exact_recip(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    double e = __fma_rn(-b, y, 1.0);
+    y = __fma_rn(y, __fma_rn(e, e, e), y);
+    e = __fma_rn(-b, y, 1.0);
+    return ExactRecip{b, __fma_rn(y, e, y)};
+}
+
+// RN(a / b) for a zero or 1e-200 < |a| < 1e150 with 1e-250 < |a / b| < 1e150.
+__device__ __forceinline__ double exact_quot(double a, const ExactRecip& r) {
+    double q = __dmul_rn(a, r.y);
+    q = __fma_rn(-__fma_rn(r.b, q, -a), r.y, q);
+    return __fma_rn(-__fma_rn(r.b, q, -a), r.y, q);
+}
+
+// RN(sqrt(v)), 1e-290 < v < 1e290.
+__device__ __forceinline__ double exact_sqrt(double v) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+    const double e = __fma_rn(-__dmul_rn(v, y), y, 1.0);
+    y = __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
+    const double h = __dmul_rn(0.5, y);
+    double g = __dmul_rn(v, y);
+    g = __fma_rn(__fma_rn(-g, g, v), h, g);
+    return __fma_rn(__fma_rn(-g, g, v), h, g);
+}
+
+// A numerator's factor for which products of a few of its like stay clear of
+// underflow.
+__device__ __forceinline__ bool exact_factor(double v) { return abs_val(v) > 1e-50 || v == 0.0; }
+
+#endif
+
+}  // namespace kp

@@ -10,6 +10,7 @@
 #pragma once
 
 #include "kp_common.cuh"
+#include "kp_exact.cuh"
 
 namespace kp {
 
@@ -37,7 +38,14 @@ KP_HD double ks_radius(double spin, const D4& X) {
     const double a2 = spin * spin;
     const double radius2 = x * x + y * y + z * z;
     const double sqsum = radius2 - a2;
-    const double discr = sqrt(sqsum * sqsum + 4.0 * a2 * z * z);
+    const double v = sqsum * sqsum + 4.0 * a2 * z * z;
+#ifdef __CUDA_ARCH__
+    if (v > 1e-200 && v < 1e200) {
+        const double r2x = 0.5 * (sqsum + exact_sqrt(v));
+        if (r2x > 1e-200) return exact_sqrt(r2x);
+    }
+#endif
+    const double discr = sqrt(v);
     const double r2 = 0.5 * (sqsum + discr);
     return sqrt(max_val(r2, kTiny));
 }
@@ -118,7 +126,7 @@ struct KSConn {
     double dl[4][4];
 };
 
-KP_HD KSConn ks_conn(double mass, double spin, const D4& X) {
+KP_HD KSConn ks_conn_plain(double mass, double spin, const D4& X) {
     const double x = X.v[1], y = X.v[2], z = X.v[3];
     const double a = spin;
     const double a2 = spin * spin;
@@ -158,6 +166,78 @@ KP_HD KSConn ks_conn(double mass, double spin, const D4& X) {
     c.dl[2][3] = (y * dr3 * r2pa2 - 2.0 * r * py * dr3) / r2pa2_2;
     c.dl[3][3] = (r - z * dr3) / r2;
     return c;
+}
+
+#ifdef __CUDACC__
+// The same with the exact quotients and roots of kp_exact.cuh: every result
+// has ks_conn_plain's bits.  A point for which an operand could leave their
+// range (never one of a ray that is still traced in earnest) takes the plain
+// form.  7 reciprocals and 19 quotients: 3225 -> KP_RHS_CYCLES cycles per
+// right-hand side of a lone ray.
+static __device__ __noinline__ void ks_conn_far_out(double mass, double spin, const D4& X, KSConn& c) {
+    c = ks_conn_plain(mass, spin, X);
+}
+
+__device__ __forceinline__ KSConn ks_conn_exact(double mass, double spin, const D4& X) {
+    const double x = X.v[1], y = X.v[2], z = X.v[3];
+    const double a = spin;
+    const double a2 = spin * spin;
+    const double radius2 = x * x + y * y + z * z;
+    const double sqsum = radius2 - a2;
+    const double v = sqsum * sqsum + 4.0 * a2 * z * z;
+    const double discr = exact_sqrt(v);
+    const double r2 = 0.5 * (sqsum + discr);
+    if (!(v > 1e-16 && r2 > 1e-16 && radius2 < 1e16 && exact_factor(x) && exact_factor(y) && exact_factor(z))) {
+        KSConn plain;
+        ks_conn_far_out(mass, spin, X, plain);
+        return plain;
+    }
+    KSConn c;
+    const double r = exact_sqrt(r2);
+    const double denom = r2 * r2 + a2 * z * z;
+    const double r2pa2 = r2 + a2;
+    const double r2pa2_2 = r2pa2 * r2pa2;
+    const ExactRecip i_discr = exact_recip(discr), i_r = exact_recip(r), i_r2 = exact_recip(r2);
+    const ExactRecip i_denom = exact_recip(denom), i_denom2 = exact_recip(denom * denom);
+    const ExactRecip i_rp = exact_recip(r2pa2), i_rp2 = exact_recip(r2pa2_2);
+    const double amp = exact_quot(2.0 * mass * r2 * r, i_denom);
+    const double amp_r = exact_quot(-2.0 * mass * r2 * (r2 * r2 - 3.0 * a2 * z * z), i_denom2);
+    c.amp = amp;
+    c.l[0] = 1.0;
+    c.l[1] = exact_quot(r * x + a * y, i_rp);
+    c.l[2] = exact_quot(r * y - a * x, i_rp);
+    c.l[3] = exact_quot(z, i_r);
+    const double inv_2r = exact_quot(0.5, i_r);
+    const double dr1 = (x + exact_quot(sqsum * x, i_discr)) * inv_2r;
+    const double dr2 = (y + exact_quot(sqsum * y, i_discr)) * inv_2r;
+    const double dr3 = (z + exact_quot(sqsum * z + 2.0 * a2 * z, i_discr)) * inv_2r;
+    c.damp[0] = 0.0;
+    c.damp[1] = amp_r * dr1;
+    c.damp[2] = amp_r * dr2;
+    c.damp[3] = exact_quot(6.0 * mass * r2 * dr3, i_denom) -
+                exact_quot(amp, i_denom) * (4.0 * r * r2 * dr3 + 2.0 * a2 * z);
+    const double px = r * x + a * y;
+    const double py = r * y - a * x;
+    c.dl[1][1] = exact_quot((r + x * dr1) * r2pa2 - 2.0 * r * px * dr1, i_rp2);
+    c.dl[2][1] = exact_quot((-a + y * dr1) * r2pa2 - 2.0 * r * py * dr1, i_rp2);
+    const double mz = exact_quot(-z, i_r2);
+    c.dl[3][1] = mz * dr1;
+    c.dl[1][2] = exact_quot((a + x * dr2) * r2pa2 - 2.0 * r * px * dr2, i_rp2);
+    c.dl[2][2] = exact_quot((r + y * dr2) * r2pa2 - 2.0 * r * py * dr2, i_rp2);
+    c.dl[3][2] = mz * dr2;
+    c.dl[1][3] = exact_quot(x * dr3 * r2pa2 - 2.0 * r * px * dr3, i_rp2);
+    c.dl[2][3] = exact_quot(y * dr3 * r2pa2 - 2.0 * r * py * dr3, i_rp2);
+    c.dl[3][3] = exact_quot(r - z * dr3, i_r2);
+    return c;
+}
+#endif
+
+KP_HD KSConn ks_conn(double mass, double spin, const D4& X) {
+#ifdef __CUDA_ARCH__
+    return ks_conn_exact(mass, spin, X);
+#else
+    return ks_conn_plain(mass, spin, X);
+#endif
 }
 
 // Gamma^mu_{ab} p^a q^b without forming Gamma (ks_connection_contract, :302-327).

@@ -612,7 +612,7 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
     }
     if (opt.threads_per_block != 0)
         return set_error(KP_ERR_INVALID, "threads_per_block is fixed by the wavefront kernels (%d far, %d near): pass 0",
-                         kFarThreads, kNearThreads);
+                         kFarThreads, kNearBThreads);
     const bool mixed = family == kFamilyRiafMixed;
     int blocks[kPhases];
     for (int phase = 0; phase < kPhases; ++phase) {
@@ -631,7 +631,7 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
             if (per_sm <= 0) per_sm = 1;
         }
         blocks[phase] = dev->sms * per_sm;
-        const long long needed = (total + wave_threads(phase) - 1) / wave_threads(phase);
+        const long long needed = wave_blocks_needed(phase, total);
         if (blocks[phase] > needed) blocks[phase] = int(needed);
     }
     WaveCtrl* ctrl = dev->d_ctrl;
@@ -768,7 +768,7 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         stats->rays = total;
         stats->launches = launches;
         stats->blocks = blocks[kPhaseNearB];
-        stats->threads_per_block = kNearThreads;
+        stats->threads_per_block = kNearBThreads;
     }
     e = cudaEventSynchronize(dev->ev1);
     if (e != cudaSuccess) return cuda_error(e, "wavefront kernels");
@@ -952,7 +952,7 @@ static int image_riaf_impl(const kp_pass_a_params* params, const kp_riaf_model* 
         dptr = carve_outputs(buf, npix, nfreq);
     }
     const auto t0 = std::chrono::steady_clock::now();
-    cudaError_t e = launch_image_fp64(c, dptr, stream);
+    cudaError_t e = launch_image_fp64(c, dptr, dev->sms, stream);
     if (e != cudaSuccess) return cuda_error(e, "image kernel launch");
     if (opt.timing) {
         e = cudaStreamSynchronize(stream);

@@ -46,15 +46,16 @@ enum Mode : int {
 struct PolicyFP64 {
     static constexpr bool kMixed = false;
 };
-// Mixed policy: FP32 connection contraction in the far-phase kernel (rays
-// beyond ImageConsts::fp32_radius), FP64 inside; FP64 state, stage
-// combination and step control everywhere; FP32 radiative transfer.
+// Mixed policy: FP64 state, connection (in factored, fused form), step control
+// and Stokes transfer; many far-field steps taken at once (kp_quad.cuh); FP32
+// transfer coefficients.
 struct PolicyMixed {
     static constexpr bool kMixed = true;
 };
 
 // Radiation side of a policy and scene: FP64 (the reference's arithmetic) or
-// FP32 with the per-frequency 2^E emission scale (kp_radiation_f32.cuh).
+// FP32 coefficients with the per-frequency 2^E emission scale
+// (kp_radiation_f32.cuh).
 template<class P, class S = SceneRiaf>
 struct RadTraits;
 
@@ -84,10 +85,10 @@ struct RadTraits<PolicyFP64, SceneRiaf> {
 
 template<>
 struct RadTraits<PolicyMixed, SceneRiaf> {
-    using Stokes = StokesF;
+    using Stokes = StokesM;
     using Co = CoeffsF;
     using Sample = RiafSampleF;
-    __device__ static void zero(Stokes& s) { s = StokesF{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}; }
+    __device__ static void zero(Stokes& s) { s = StokesM{0.0, 0.0, 0.0, 0.0}; }
     __device__ static Sample sample(const ImageConsts& c, const Ray& r) { return riaf_sample_f(c, r); }
     __device__ static Sample none() {
         Sample s;
@@ -101,14 +102,20 @@ struct RadTraits<PolicyMixed, SceneRiaf> {
         return riaf_coefficients_f(c, p, float(c.ctl_freq[g] * 1e-9), c.ctl_emission_scale_pow2[g]);
     }
     __device__ static void step(Stokes& s, const Co& co, double h, const ImageConsts& c, int f) {
-        stokes_step_f(s, co, float(abs_val(h) * c.dlambda_scale[f]));
+        stokes_step_m(s, co, abs_val(h) * c.dlambda_scale[f]);
     }
     __device__ static Stokes4<double> result(const Stokes& s, const ImageConsts& c, int f) {
         const double inv = c.inv_emission_scale_pow2[f];
-        return Stokes4<double>{(double(s.I) + double(s.cI)) * inv, (double(s.Q) + double(s.cQ)) * inv,
-                               (double(s.U) + double(s.cU)) * inv, (double(s.V) + double(s.cV)) * inv};
+        return Stokes4<double>{s.I * inv, s.Q * inv, s.U * inv, s.V * inv};
     }
 };
+
+// Depths per dl of FP32 coefficients: their norms carry the coefficients'
+// own single precision.
+__device__ __forceinline__ RadDepths radiation_depths(const CoeffsF& co, double dls) {
+    return RadDepths{double(fabsf(co.aI) + sqrtf(co.aQ * co.aQ + co.aU * co.aU + co.aV * co.aV)),
+                     double(sqrtf(co.rQ * co.rQ + co.rU * co.rU + float(co.rV) * float(co.rV))), abs_val(dls)};
+}
 
 // GRMHD grid plasma, FP64 throughout.
 template<>
@@ -137,9 +144,8 @@ struct RadTraits<PolicyFP64, SceneGrmhd> {
 
 // GRMHD grid plasma under the mixed policy: the grid gather, the fluid and
 // field four-vectors and the screen angle stay FP64 (grmhd_sample, the
-// reference's fluid_state); the thermal fit per frequency and the Stokes
-// update run in FP32 with the 2^E emission scale and compensated sums, the
-// same code as the mixed RIAF scene.
+// reference's fluid_state); the thermal fit per frequency runs in FP32 with
+// the 2^E emission scale, the same code as the mixed RIAF scene.
 __device__ __forceinline__ RiafSampleF grmhd_sample_to_f(const ImageConsts& c, const GrmhdSample& p) {
     RiafSampleF o;
     o.emitting = p.emitting;
@@ -155,7 +161,7 @@ __device__ __forceinline__ RiafSampleF grmhd_sample_to_f(const ImageConsts& c, c
     o.theta = 0.0f;
     o.cos2chi = float(p.cos2chi);
     o.sin2chi = float(p.sin2chi);
-    riaf_sample_thermal_f(c, o);
+    riaf_sample_thermal_f(c, o, p.ne, p.thetae, p.b, p.ct, p.st, p.nu_scale);
     return o;
 }
 
@@ -186,7 +192,7 @@ struct RadTraits<PolicyMixed, SceneGrmhdSlow> : RadTraits<PolicyMixed, SceneRiaf
 
 // The RIAF in Boyer-Lindquist coordinates: the same plasma model, sampled
 // in the ray's own BL components (riaf_sample_t<true>); under the mixed
-// policy the FP64 sample feeds the FP32 fits and transfer.
+// policy the FP64 sample feeds the FP32 fits.
 template<>
 struct RadTraits<PolicyFP64, SceneRiafBL> : RadTraits<PolicyFP64, SceneRiaf> {
     __device__ static Sample sample(const ImageConsts& c, const Ray& r) { return riaf_sample_t<true>(c, r); }
@@ -207,7 +213,7 @@ __device__ __forceinline__ RiafSampleF riaf_sample_to_f(const ImageConsts& c, co
     o.theta = float(p.theta);
     o.cos2chi = float(p.cos2chi);
     o.sin2chi = float(p.sin2chi);
-    riaf_sample_thermal_f(c, o);
+    riaf_sample_thermal_f(c, o, p.ne, p.thetae, p.b, p.cos_theta, p.sin_theta, p.nu_fluid);
     return o;
 }
 
@@ -223,13 +229,12 @@ struct RadTraits<PolicyMixed, SceneRiafBL> : RadTraits<PolicyMixed, SceneRiaf> {
 template<class P, class B>
 struct RadTraits<P, SceneFarCks<B>> : RadTraits<P, B> {};
 
-// The scene's transport RHS under a policy; FP32 is a compile-time choice of
-// the calling kernel, so each kernel holds one contraction body.  The FP64
-// policy keeps the reference's operation order; the mixed policy uses the
-// factored form (kp_geometry_f32.cuh).
-template<class P, bool FP32, class S>
+// The scene's transport RHS under a policy.  The FP64 policy keeps the
+// reference's operation order; the mixed policy uses the factored form
+// (kp_geometry_f32.cuh).
+template<class P, class S>
 __device__ __forceinline__ Ray policy_rhs(const ImageConsts& c, const Ray& X) {
-    return S::template rhs<P::kMixed, FP32>(c, X);
+    return S::template rhs<P::kMixed>(c, X);
 }
 
 // ---------------------------------------------------------------- RK jobs
@@ -237,39 +242,39 @@ __device__ __forceinline__ Ray policy_rhs(const ImageConsts& c, const Ray& X) {
 // (sample point: the first half step for SD, the endpoint otherwise) and err
 // (SD / CK only).  The stage arithmetic is the reference's (see file header).
 // Cash-Karp attempt with the reference's stage coefficients (rk4.hpp:171-228).
-template<class P, bool FP32, class SC>
+template<class P, class SC>
 __device__ __noinline__ void ck_job(const ImageConsts& c, const Ray& S, double h, Ray& next,
                                     Ray& mid, double& err) {
     {
-        const Ray k1 = policy_rhs<P, FP32, SC>(c, S);
+        const Ray k1 = policy_rhs<P, SC>(c, S);
         Ray t;
         ray_axpy(t, S, h * 1.0 / 5.0, k1);
-        const Ray k2 = policy_rhs<P, FP32, SC>(c, t);
+        const Ray k2 = policy_rhs<P, SC>(c, t);
         {
             const Ray* const kk[2] = {&k1, &k2};
             const double cc[2] = {3.0 / 40.0, 9.0 / 40.0};
             ray_lincomb<2>(t, S, h, kk, cc);
         }
-        const Ray k3 = policy_rhs<P, FP32, SC>(c, t);
+        const Ray k3 = policy_rhs<P, SC>(c, t);
         {
             const Ray* const kk[3] = {&k1, &k2, &k3};
             const double cc[3] = {3.0 / 10.0, -9.0 / 10.0, 6.0 / 5.0};
             ray_lincomb<3>(t, S, h, kk, cc);
         }
-        const Ray k4 = policy_rhs<P, FP32, SC>(c, t);
+        const Ray k4 = policy_rhs<P, SC>(c, t);
         {
             const Ray* const kk[4] = {&k1, &k2, &k3, &k4};
             const double cc[4] = {-11.0 / 54.0, 5.0 / 2.0, -70.0 / 27.0, 35.0 / 27.0};
             ray_lincomb<4>(t, S, h, kk, cc);
         }
-        const Ray k5 = policy_rhs<P, FP32, SC>(c, t);
+        const Ray k5 = policy_rhs<P, SC>(c, t);
         {
             const Ray* const kk[5] = {&k1, &k2, &k3, &k4, &k5};
             const double cc[5] = {1631.0 / 55296.0, 175.0 / 512.0, 575.0 / 13824.0, 44275.0 / 110592.0,
                                   253.0 / 4096.0};
             ray_lincomb<5>(t, S, h, kk, cc);
         }
-        const Ray k6 = policy_rhs<P, FP32, SC>(c, t);
+        const Ray k6 = policy_rhs<P, SC>(c, t);
         {
             const Ray* const kk[4] = {&k1, &k3, &k4, &k6};
             const double cc[4] = {37.0 / 378.0, 250.0 / 621.0, 125.0 / 594.0, 512.0 / 1771.0};
@@ -287,179 +292,15 @@ __device__ __noinline__ void ck_job(const ImageConsts& c, const Ray& S, double h
     }
 }
 
-// Far-field RK chains of the mixed policy (Kerr-Schild scene).  Beyond the
-// radiating sphere the transports change the ray by ~M/r^2 per unit step, so
-// their FP32 rounding is far below the step-doubling tolerance; the state,
-// the position derivative (= k) and every chain endpoint stay FP64.  What
-// only feeds the FP32 contraction or sums FP32 derivatives is carried in
-// FP32: the stage inputs x, k, e1, e2 (formed from the chain base's FP32
-// copy) and the accumulator of dk, de1, de2.  Per stage that leaves four
-// FP32->FP64 conversions and eight FP64 FMAs (k of the next stage input, the
-// position accumulator) around the contraction, where converting FP64 stage
-// states took 28 conversions and 48 FP64 operations.  Stage order,
-// coefficients and the k1 reuse of step doubling are the reference's
-// (rk4.hpp:37-59, 108-161).
-struct ChainF {
-    float x[3];      // x^1..x^3 of the stage input
-    float q[3][4];   // k, e1, e2 of the stage input
-};
-
-__device__ __forceinline__ void chain_base_f(const Ray& B, ChainF& b) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) b.x[i] = float(B.x.v[i + 1]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        b.q[0][i] = float(B.k.v[i]);
-        b.q[1][i] = float(B.e1.v[i]);
-        b.q[2][i] = float(B.e2.v[i]);
-    }
-}
-
-// State of one RK4 chain between its stages: the next stage input (FP32,
-// with its k in FP64 as the position derivative) and the accumulators.
-struct ChainAcc {
-    ChainF X;      // stage input
-    D4 Xk;         // k of the stage input, FP64: the position derivative
-    D4 Ax;         // position accumulator, FP64
-    float Aq[3][4];
-};
-
-// Folds stage st's derivative kq into the chain of step hc from B (base b):
-// acc = ((k1 + 2 k2) + 2 k3) + k4, then the next stage input
-// B + cc * (this stage's derivative).
-__device__ __forceinline__ void chain_stage_f(ChainAcc& C, const ChainF& b, const Ray& B, double hc, int st,
-                                              const float (&kq)[3][4]) {
-    if (st == 0) {
-        C.Ax = C.Xk;
-#pragma unroll
-        for (int w = 0; w < 3; ++w)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) C.Aq[w][i] = kq[w][i];
-    } else {
-        const double wd = st == 3 ? 1.0 : 2.0;
-        const float wf = st == 3 ? 1.0f : 2.0f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) C.Ax.v[i] = C.Ax.v[i] + C.Xk.v[i] * wd;
-#pragma unroll
-        for (int w = 0; w < 3; ++w)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) C.Aq[w][i] = C.Aq[w][i] + kq[w][i] * wf;
-    }
-    if (st < 3) {
-        const double cc = st < 2 ? 0.5 * hc : hc;
-        const float cf = float(cc);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) C.X.x[i] = b.x[i] + C.X.q[0][i + 1] * cf;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) C.Xk.v[i] = B.k.v[i] + double(kq[0][i]) * cc;
-#pragma unroll
-        for (int w = 0; w < 3; ++w)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) C.X.q[w][i] = b.q[w][i] + kq[w][i] * cf;
-    }
-}
-
-__device__ __forceinline__ void chain_end_f(const ChainAcc& C, const Ray& B, double hc, Ray& end) {
-    const double h6 = hc / 6.0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        end.x.v[i] = B.x.v[i] + C.Ax.v[i] * h6;
-        end.k.v[i] = B.k.v[i] + double(C.Aq[0][i]) * h6;
-        end.e1.v[i] = B.e1.v[i] + double(C.Aq[1][i]) * h6;
-        end.e2.v[i] = B.e2.v[i] + double(C.Aq[2][i]) * h6;
-    }
-}
-
-// One RK4 chain of step hc from B.
-__device__ __forceinline__ void far_chain_f(const ImageConsts& c, const Ray& B, double hc, Ray& end) {
-    const float M = float(c.mass), a = float(c.spin);
-    ChainF b;
-    chain_base_f(B, b);
-    ChainAcc C;
-    C.X = b;
-    C.Xk = B.k;
-#pragma unroll 1
-    for (int st = 0; st < 4; ++st) {
-        float kq[3][4];
-        ks_transport_factored<float>(M, a, C.X.x[0], C.X.x[1], C.X.x[2], C.X.q, kq);
-        chain_stage_f(C, b, B, hc, st, kq);
-    }
-    chain_end_f(C, B, hc, end);
-}
-
-// Step-doubling attempt from far_chain_f pieces.  The full-step chain starts
-// from S like the first half chain and reuses its first derivative, so the
-// two run interleaved, stage by stage: their contractions are independent,
-// which gives the scheduler two dependency chains per lane.  Then the
-// second half chain from the half-step state.  Each chain's arithmetic is
-// the sequential chain's (same operations in the same order).
-__device__ __forceinline__ void far_sd_f(const ImageConsts& c, const Ray& S, double h, Ray& next, Ray& mid,
-                                         double& err) {
-    const float M = float(c.mass), a = float(c.spin);
-    ChainF b;
-    chain_base_f(S, b);
-    const double hh = 0.5 * h;
-    ChainAcc H, F;
-    H.X = b;
-    H.Xk = S.k;
-    F.X = b;
-    F.Xk = S.k;
-    Ray full;
-    {
-        float kq[3][4];
-        ks_transport_factored<float>(M, a, b.x[0], b.x[1], b.x[2], b.q, kq);
-        chain_stage_f(H, b, S, hh, 0, kq);
-        chain_stage_f(F, b, S, h, 0, kq);
-    }
-#pragma unroll 1
-    for (int st = 1; st < 4; ++st) {
-        float kh[3][4], kf[3][4];
-        ks_transport_factored<float>(M, a, H.X.x[0], H.X.x[1], H.X.x[2], H.X.q, kh);
-        ks_transport_factored<float>(M, a, F.X.x[0], F.X.x[1], F.X.x[2], F.X.q, kf);
-        chain_stage_f(H, b, S, hh, st, kh);
-        chain_stage_f(F, b, S, h, st, kf);
-    }
-    chain_end_f(H, S, hh, mid);
-    chain_end_f(F, S, h, full);
-    far_chain_f(c, mid, hh, next);
-    err = control_error(full, next, max_val(c.tolerance, kTolFloor));
-}
-
-// Step-doubling attempt, RK4 step or composed RK4 pair from the FP32
-// chains; outputs as rk_job's.
-__device__ __forceinline__ void far_job_f(int kind, const ImageConsts& c, const Ray& S, double h, Ray& next,
-                                          Ray& mid, double& err) {
-    err = 0.0;
-    if (kind == kRkSD) {
-        far_sd_f(c, S, h, next, mid, err);
-        return;
-    }
-    if (kind == kRkRK4) {
-        far_chain_f(c, S, h, next);
-        mid = next;
-        return;
-    }
-    Ray R2;
-    far_chain_f(c, S, 0.5 * h, R2);
-    far_chain_f(c, R2, 0.5 * h, next);
-    mid = next;
-}
-
 // Step-doubling attempt, RK4 step or composed RK4 pair as a stage loop around
 // one RHS site.  Out of line: the caller's control state is saved once per
 // job and the stage loop has the register file to itself.
-template<class P, bool FP32, class SC>
+template<class P, class SC>
 __device__ __noinline__ void rk_job(int kind, const ImageConsts& c, const Ray& S, double h,
                                     Ray& next, Ray& mid, double& err) {
     if (kind == kRkCK) {
-        ck_job<P, FP32, SC>(c, S, h, next, mid, err);
+        ck_job<P, SC>(c, S, h, next, mid, err);
         return;
-    }
-    if constexpr (FP32 && SC::kCksRhs) {
-        if (SC::chart_active(c)) {
-            far_job_f(kind, c, S, h, next, mid, err);
-            return;
-        }
     }
     // Stage schedule (see file header): SD = half chain (4), second half
     // chain (4), full chain (3); RK4 = 4; RK4x2 = 4 + 4.
@@ -475,7 +316,7 @@ __device__ __noinline__ void rk_job(int kind, const ImageConsts& c, const Ray& S
     Ray R2;      // SD / RK4x2: the first chain's endpoint (half step)
 #pragma unroll 1
     for (int st = 0; st < nstage; ++st) {
-        const Ray k = policy_rhs<P, FP32, SC>(c, X);
+        const Ray k = policy_rhs<P, SC>(c, X);
         // position of this stage inside its 4-stage RK4 chain
         const int cs = st < 4 ? st : (st < 8 ? st - 4 : st - 7);
         const bool full_chain = kind == kRkSD && st >= 8;

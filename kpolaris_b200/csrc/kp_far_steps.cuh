@@ -1,0 +1,66 @@
+// kp_far_steps.cuh -- how many steps of the step control the mixed policy's
+// far phase bridges at once (quad_macro_step in kp_quad.cuh).
+#pragma once
+
+#include "kp_common.cuh"
+
+namespace kp {
+
+// A run of accepted steps: their number, the affine distance they cover and
+// the size of the step after them (all positive; count 0: none).
+struct MacroRun {
+    int count;
+    double length, next_h;
+};
+
+// The run of steps the step control would take from a ray at radius r whose
+// next step has size h (at most `cap`, the step's own size for fixed steps),
+// with every one of them provably accepted:
+// * The step-doubling error of a step of size h at radius r is below
+//   (16 + r / 4) M h^5 / r^6 beyond the sphere (k, e1 and e2 in the first
+//   term; the position, whose components near zero are measured absolutely,
+//   in the second) plus rounding: tests/native/far_steps.cpp finds at most
+//   0.6 of it.  At tol / 64 or less the control doubles a step below the cap,
+//   at tol / 4 or less a step at the cap stays there, so the run's sizes are
+//   known: h, 2h, 4h, ... cap, cap, ...
+// * No step of the run starts in the near phase, reaches the camera's radius
+//   or, in pass A, the turning point.  xk is x.k (spatial), v the spatial
+//   speed |dx/dlambda|, dir the sign of the step; over a run the speed and the
+//   direction change by a few M / r, which the margins cover.
+// * The run covers at most a fifth of the radius, where quad_macro_step's
+//   error is below 1e-13.
+KP_HD MacroRun macro_run(const ImageConsts& c, double r, double xk, double v, double h, double cap, double dir,
+                         bool pass_a, int left) {
+    MacroRun none = {0, 0.0, 0.0};
+    const double rmin = 0.8 * r;
+    const double r2 = rmin * rmin, c2 = cap * cap;
+    const double bound = (16.0 + 0.25 * rmin) * c.mass * c2 * c2 * cap / (r2 * r2 * r2) + 1e-14;
+    const double tol = max_val(c.tolerance, kTolFloor) * (h < cap ? 1.0 / 64.0 : 0.25);
+    if (!(bound <= (c.adaptive ? tol : 1e-11))) return none;
+    double reach = 0.2 * r;
+    const double along = dir * xk;  // > 0: outward
+    if (pass_a) {
+        if (along >= 0.0) return none;
+        reach = min_val(reach, 0.8 * (-along / v) - 16.0 * c.mass);
+    } else {
+        reach = min_val(reach, abs_val(r - c.cam_radius) - 1.1 * v * cap);
+    }
+    if (!(along > 0.1 * r * v)) reach = min_val(reach, r - c.fp32_radius - 0.1 * v * cap);
+    const double span = reach / (v * (1.0 + 4.0 * c.mass / rmin));
+    if (!(span >= h) || !(span < 1e300) || left < 1) return none;
+    MacroRun run = {0, 0.0, h};
+    while (run.next_h < cap && run.count < left && run.length + run.next_h <= span) {
+        run.length += run.next_h;
+        run.next_h = min_val(cap, 2.0 * run.next_h);
+        ++run.count;
+    }
+    if (run.next_h >= cap) {
+        const double m = (span - run.length) / cap;
+        const int more = m < double(left - run.count) ? int(m) : left - run.count;
+        run.length += cap * double(more);
+        run.count += more;
+    }
+    return run;
+}
+
+}  // namespace kp

@@ -205,9 +205,22 @@ KP_HD SksConn sks_conn(double mass, double a, double r, double th) {
 // with p = k fixed, and the second-derivative terms of theta(x1, x2) carry
 // the result back (transport_rhs, kerr_fmks.hpp:455-479; fixed-p contraction,
 // kerr_schild_spherical.hpp:288-323).
-KP_HD Ray fmks_rhs(const FmksParams& m, const Ray& s) {
-    const FmksTheta t = fmks_theta(m, s.x.v[1], s.x.v[2]);
-    const SksConn c = sks_conn(m.mass, m.spin, t.r, t.th);
+struct FmksConn {
+    FmksTheta t;
+    SksConn c;
+};
+
+KP_HD FmksConn fmks_conn(const FmksParams& m, const D4& x) {
+    FmksConn o;
+    o.t = fmks_theta(m, x.v[1], x.v[2]);
+    o.c = sks_conn(m.mass, m.spin, o.t.r, o.t.th);
+    return o;
+}
+
+// -Gamma(k, q) at a point.
+KP_HD D4 fmks_contract(const FmksConn& w, const D4& kn, const D4& qn) {
+    const FmksTheta& t = w.t;
+    const SksConn& c = w.c;
     auto to_sph = [&](const D4& v) {
         D4 o;
         o.v[0] = v.v[0];
@@ -216,7 +229,7 @@ KP_HD Ray fmks_rhs(const FmksParams& m, const Ray& s) {
         o.v[3] = v.v[3];
         return o;
     };
-    const D4 ks = to_sph(s.k);
+    const D4 ks = to_sph(kn);
     double rowk_r[4], rowk_t[4];
     for (int nu = 0; nu < 4; ++nu) {
         double a = 0.0, b = 0.0;
@@ -227,50 +240,52 @@ KP_HD Ray fmks_rhs(const FmksParams& m, const Ray& s) {
         rowk_r[nu] = a;
         rowk_t[nu] = b;
     }
-    auto contract = [&](const D4& qn) {
-        const D4 q = to_sph(qn);
-        double rr[4], rt[4];
-        double d1 = 0.0, d2 = 0.0;
-        for (int nu = 0; nu < 4; ++nu) {
-            double a = 0.0, b = 0.0;
-            for (int w = 0; w < 4; ++w) {
-                a += c.dgr[nu][w] * q.v[w];
-                b += c.dgth[nu][w] * q.v[w];
-            }
-            rr[nu] = a;
-            rt[nu] = b;
-            d1 += ks.v[nu] * a;
-            d2 += ks.v[nu] * b;
+    const D4 q = to_sph(qn);
+    double rr[4], rt[4];
+    double d1 = 0.0, d2 = 0.0;
+    for (int nu = 0; nu < 4; ++nu) {
+        double a = 0.0, b = 0.0;
+        for (int v = 0; v < 4; ++v) {
+            a += c.dgr[nu][v] * q.v[v];
+            b += c.dgth[nu][v] * q.v[v];
         }
-        double tt[4];
-        for (int nu = 0; nu < 4; ++nu) {
-            double term = ks.v[1] * rr[nu] + q.v[1] * rowk_r[nu] + ks.v[2] * rt[nu] + q.v[2] * rowk_t[nu];
-            if (nu == 1) term -= d1;
-            else if (nu == 2) term -= d2;
-            tt[nu] = term;
-        }
-        double hs[4];
-        for (int mu = 0; mu < 4; ++mu) {
-            double comp = 0.0;
-            for (int nu = 0; nu < 4; ++nu) comp += c.gcon[mu][nu] * tt[nu];
-            hs[mu] = 0.5 * comp;
-        }
-        // back to native components (fmks_from_spherical_connection_contract, :414-431)
-        hs[1] += t.r * s.k.v[1] * qn.v[1];
-        hs[2] += t.d2th11 * s.k.v[1] * qn.v[1] + t.d2th12 * (s.k.v[1] * qn.v[2] + s.k.v[2] * qn.v[1]) +
-                 t.d2th22 * s.k.v[2] * qn.v[2];
-        D4 out;
-        out.v[0] = -hs[0];
-        out.v[1] = -(hs[1] / t.r);
-        out.v[2] = -((hs[2] - t.dth1 * hs[1] / t.r) / t.dth2);
-        out.v[3] = -hs[3];
-        return out;
-    };
+        rr[nu] = a;
+        rt[nu] = b;
+        d1 += ks.v[nu] * a;
+        d2 += ks.v[nu] * b;
+    }
+    double tt[4];
+    for (int nu = 0; nu < 4; ++nu) {
+        double term = ks.v[1] * rr[nu] + q.v[1] * rowk_r[nu] + ks.v[2] * rt[nu] + q.v[2] * rowk_t[nu];
+        if (nu == 1) term -= d1;
+        else if (nu == 2) term -= d2;
+        tt[nu] = term;
+    }
+    double hs[4];
+    for (int mu = 0; mu < 4; ++mu) {
+        double comp = 0.0;
+        for (int nu = 0; nu < 4; ++nu) comp += c.gcon[mu][nu] * tt[nu];
+        hs[mu] = 0.5 * comp;
+    }
+    // back to native components (fmks_from_spherical_connection_contract, :414-431)
+    hs[1] += t.r * kn.v[1] * qn.v[1];
+    hs[2] += t.d2th11 * kn.v[1] * qn.v[1] + t.d2th12 * (kn.v[1] * qn.v[2] + kn.v[2] * qn.v[1]) +
+             t.d2th22 * kn.v[2] * qn.v[2];
+    D4 out;
+    out.v[0] = -hs[0];
+    out.v[1] = -(hs[1] / t.r);
+    out.v[2] = -((hs[2] - t.dth1 * hs[1] / t.r) / t.dth2);
+    out.v[3] = -hs[3];
+    return out;
+}
+
+KP_HD Ray fmks_rhs(const FmksParams& m, const Ray& s) {
+    const FmksConn w = fmks_conn(m, s.x);
     Ray d;
     d.x = s.k;
-    d.k = contract(s.k);
-    d.e1 = contract(s.e1);
-    d.e2 = contract(s.e2);
+    d.k = fmks_contract(w, s.k, s.k);
+    d.e1 = fmks_contract(w, s.k, s.e1);
+    d.e2 = fmks_contract(w, s.k, s.e2);
     return d;
 }
 
@@ -280,8 +295,14 @@ KP_HD Ray fmks_rhs(const FmksParams& m, const Ray& s) {
 // d/dtheta g likewise with two different (0,3)/(1,3) entries), the inverse
 // metric five, and the three divisions by rho^2, r and dtheta/dx2 become
 // reciprocals.  Same algebra as fmks_rhs, regrouped: agrees to rounding.
-KP_HD Ray fmks_rhs_factored(const FmksParams& m, const Ray& s) {
-    const FmksTheta t = fmks_theta(m, s.x.v[1], s.x.v[2]);
+struct FmksFactored {
+    double r, inv_r, inv_dth2, dth1, dth2, d2th11, d2th12, d2th22;
+    double G00, G01, G11, G13, G22, G33;      // inverse spherical metric: g22 and g33 last
+    double A, B, C, Dr, E, F0, F1, Gt, Ht;    // d/dr g and d/dtheta g
+};
+
+KP_HD FmksFactored fmks_factored_conn(const FmksParams& m, const D4& x) {
+    const FmksTheta t = fmks_theta(m, x.v[1], x.v[2]);
     const double a = m.spin, M = m.mass, r = t.r;
     double sn, cs;
     sincos(t.th, &sn, &cs);
@@ -291,62 +312,81 @@ KP_HD Ray fmks_rhs_factored(const FmksParams& m, const Ray& s) {
     const double inv_rho4 = inv_rho2 * inv_rho2;
     const double f = 2.0 * M * r * inv_rho2;
     const double delta = r * r - 2.0 * M * r + a2;
-    // inverse metric: g00, g01 = g10, g11, g13 = g31, g22, g33
-    const double G00 = -(1.0 + f), G01 = f, G11 = delta * inv_rho2, G13 = a * inv_rho2, G22 = inv_rho2;
-    const double G33 = inv_rho2 / safe_s2;
-    // d/dr g and d/dtheta g
+    FmksFactored o;
+    o.r = r;
+    o.inv_r = 1.0 / r;
+    o.inv_dth2 = 1.0 / t.dth2;
+    o.dth1 = t.dth1;
+    o.dth2 = t.dth2;
+    o.d2th11 = t.d2th11;
+    o.d2th12 = t.d2th12;
+    o.d2th22 = t.d2th22;
+    o.G00 = -(1.0 + f);
+    o.G01 = f;
+    o.G11 = delta * inv_rho2;
+    o.G13 = a * inv_rho2;
+    o.G22 = inv_rho2;
+    o.G33 = inv_rho2 / safe_s2;
     const double drho_dth = -2.0 * a2 * sn * cs, ds2_dth = 2.0 * sn * cs;
     const double df_dr = 2.0 * M * (rho2 - 2.0 * r * r) * inv_rho4;
     const double df_dth = -2.0 * M * r * drho_dth * inv_rho4;
-    const double A = df_dr, B = -a * s2 * df_dr, C = 2.0 * r;
-    const double Dr = s2 * (2.0 * r + a2 * s2 * df_dr);
-    const double E = df_dth, F0 = -a * (s2 * df_dth + ds2_dth * f), F1 = -a * (ds2_dth * (1.0 + f) + s2 * df_dth);
-    const double Gt = drho_dth;
+    o.A = df_dr;
+    o.B = -a * s2 * df_dr;
+    o.C = 2.0 * r;
+    o.Dr = s2 * (2.0 * r + a2 * s2 * df_dr);
+    o.E = df_dth;
+    o.F0 = -a * (s2 * df_dth + ds2_dth * f);
+    o.F1 = -a * (ds2_dth * (1.0 + f) + s2 * df_dth);
+    o.Gt = drho_dth;
     const double bracket = rho2 + a2 * s2 * (1.0 + f);
-    const double Ht = ds2_dth * bracket + s2 * (drho_dth + a2 * (ds2_dth * (1.0 + f) + s2 * df_dth));
-    const double inv_r = 1.0 / r, inv_dth2 = 1.0 / t.dth2;
+    o.Ht = ds2_dth * bracket + s2 * (drho_dth + a2 * (ds2_dth * (1.0 + f) + s2 * df_dth));
+    return o;
+}
+
+// -Gamma(k, q) at a point.
+KP_HD D4 fmks_factored_contract(const FmksFactored& w, const D4& kn, const D4& qn) {
     struct V {
         double v0, v1, v2, v3;
     };
-    auto to_sph = [&](const D4& q) { return V{q.v[0], r * q.v[1], t.dth1 * q.v[1] + t.dth2 * q.v[2], q.v[3]}; };
+    auto to_sph = [&](const D4& q) { return V{q.v[0], w.r * q.v[1], w.dth1 * q.v[1] + w.dth2 * q.v[2], q.v[3]}; };
     auto drow = [&](const V& q, V& rr, V& rt) {
         const double sig = q.v0 + q.v1;
-        rr = V{A * sig + B * q.v3, A * sig + B * q.v3, C * q.v2, B * sig + Dr * q.v3};
-        rt = V{E * sig + F0 * q.v3, E * sig + F1 * q.v3, Gt * q.v2, F0 * q.v0 + F1 * q.v1 + Ht * q.v3};
+        rr = V{w.A * sig + w.B * q.v3, w.A * sig + w.B * q.v3, w.C * q.v2, w.B * sig + w.Dr * q.v3};
+        rt = V{w.E * sig + w.F0 * q.v3, w.E * sig + w.F1 * q.v3, w.Gt * q.v2, w.F0 * q.v0 + w.F1 * q.v1 + w.Ht * q.v3};
     };
-    const V ks = to_sph(s.k);
-    V rk, tk;
+    const V ks = to_sph(kn), q = to_sph(qn);
+    V rk, tk, rr, rt;
     drow(ks, rk, tk);
-    auto contract = [&](const D4& qn) {
-        const V q = to_sph(qn);
-        V rr, rt;
-        drow(q, rr, rt);
-        const double d1 = ks.v0 * rr.v0 + ks.v1 * rr.v1 + ks.v2 * rr.v2 + ks.v3 * rr.v3;
-        const double d2 = ks.v0 * rt.v0 + ks.v1 * rt.v1 + ks.v2 * rt.v2 + ks.v3 * rt.v3;
-        const double t0 = ks.v1 * rr.v0 + q.v1 * rk.v0 + ks.v2 * rt.v0 + q.v2 * tk.v0;
-        const double t1 = ks.v1 * rr.v1 + q.v1 * rk.v1 + ks.v2 * rt.v1 + q.v2 * tk.v1 - d1;
-        const double t2 = ks.v1 * rr.v2 + q.v1 * rk.v2 + ks.v2 * rt.v2 + q.v2 * tk.v2 - d2;
-        const double t3 = ks.v1 * rr.v3 + q.v1 * rk.v3 + ks.v2 * rt.v3 + q.v2 * tk.v3;
-        const double h0 = 0.5 * (G00 * t0 + G01 * t1);
-        double h1 = 0.5 * (G01 * t0 + G11 * t1 + G13 * t3);
-        double h2 = 0.5 * (G22 * t2);
-        const double h3 = 0.5 * (G13 * t1 + G33 * t3);
-        h1 += r * s.k.v[1] * qn.v[1];
-        h2 += t.d2th11 * s.k.v[1] * qn.v[1] + t.d2th12 * (s.k.v[1] * qn.v[2] + s.k.v[2] * qn.v[1]) +
-              t.d2th22 * s.k.v[2] * qn.v[2];
-        const double h1r = h1 * inv_r;
-        D4 out;
-        out.v[0] = -h0;
-        out.v[1] = -h1r;
-        out.v[2] = -((h2 - t.dth1 * h1r) * inv_dth2);
-        out.v[3] = -h3;
-        return out;
-    };
+    drow(q, rr, rt);
+    const double d1 = ks.v0 * rr.v0 + ks.v1 * rr.v1 + ks.v2 * rr.v2 + ks.v3 * rr.v3;
+    const double d2 = ks.v0 * rt.v0 + ks.v1 * rt.v1 + ks.v2 * rt.v2 + ks.v3 * rt.v3;
+    const double t0 = ks.v1 * rr.v0 + q.v1 * rk.v0 + ks.v2 * rt.v0 + q.v2 * tk.v0;
+    const double t1 = ks.v1 * rr.v1 + q.v1 * rk.v1 + ks.v2 * rt.v1 + q.v2 * tk.v1 - d1;
+    const double t2 = ks.v1 * rr.v2 + q.v1 * rk.v2 + ks.v2 * rt.v2 + q.v2 * tk.v2 - d2;
+    const double t3 = ks.v1 * rr.v3 + q.v1 * rk.v3 + ks.v2 * rt.v3 + q.v2 * tk.v3;
+    const double h0 = 0.5 * (w.G00 * t0 + w.G01 * t1);
+    double h1 = 0.5 * (w.G01 * t0 + w.G11 * t1 + w.G13 * t3);
+    double h2 = 0.5 * (w.G22 * t2);
+    const double h3 = 0.5 * (w.G13 * t1 + w.G33 * t3);
+    h1 += w.r * kn.v[1] * qn.v[1];
+    h2 += w.d2th11 * kn.v[1] * qn.v[1] + w.d2th12 * (kn.v[1] * qn.v[2] + kn.v[2] * qn.v[1]) +
+          w.d2th22 * kn.v[2] * qn.v[2];
+    const double h1r = h1 * w.inv_r;
+    D4 out;
+    out.v[0] = -h0;
+    out.v[1] = -h1r;
+    out.v[2] = -((h2 - w.dth1 * h1r) * w.inv_dth2);
+    out.v[3] = -h3;
+    return out;
+}
+
+KP_HD Ray fmks_rhs_factored(const FmksParams& m, const Ray& s) {
+    const FmksFactored w = fmks_factored_conn(m, s.x);
     Ray d;
     d.x = s.k;
-    d.k = contract(s.k);
-    d.e1 = contract(s.e1);
-    d.e2 = contract(s.e2);
+    d.k = fmks_factored_contract(w, s.k, s.k);
+    d.e1 = fmks_factored_contract(w, s.k, s.e1);
+    d.e2 = fmks_factored_contract(w, s.k, s.e2);
     return d;
 }
 

@@ -3,30 +3,28 @@
 #include <cuda_runtime.h>
 
 #include "kp_launch.h"
-#include "kp_persistent.cuh"
+#include "kp_quad.cuh"
 
 namespace kp {
 
 template<int NF>
 __global__ void __launch_bounds__(kFarThreads, 2) wave_bl_far(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseFar, SceneRiafBL>(W);
+    far_body<PolicyFP64, NF, SceneRiafBL>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, 1) wave_bl_near_a(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseNearA, SceneRiafBL>(W);
+__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_bl_near_a(const WaveDesc W) {
+    quad_body<PolicyFP64, kPhaseNearA, SceneRiafBL>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, 1) wave_bl_near_b(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseNearB, SceneRiafBL>(W);
+__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_bl_near_b(const WaveDesc W) {
+    quad_body<PolicyFP64, kPhaseNearB, SceneRiafBL>(W);
 }
 
 template<int NF>
 static const void* wave_bl_kernel(int phase) {
     if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_bl_far<NF>);
-    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_bl_near_a<NF>);
-    return reinterpret_cast<const void*>(wave_bl_near_b<NF>);
+    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_bl_near_a);
+    return reinterpret_cast<const void*>(wave_bl_near_b);
 }
 
 cudaError_t launch_wave_bl(int phase, const WaveDesc& W, int nf_max, int blocks, int threads, cudaStream_t stream) {

@@ -1,32 +1,30 @@
 // kp_kernels_bl_mixed.cu -- the RIAF in Boyer-Lindquist coordinates (SceneRiafBL)
-// on the wavefront engine with the mixed policy (FP64 BL geodesic, FP32 fits and compensated transfer), compiled with FMA contraction.
+// on the wavefront engine with the mixed policy (FP64 BL geodesic, FP32 fits, FP64 transfer), compiled with FMA contraction.
 #include <cuda_runtime.h>
 
 #include "kp_launch.h"
-#include "kp_persistent.cuh"
+#include "kp_quad.cuh"
 
 namespace kp {
 
 template<int NF>
 __global__ void __launch_bounds__(kFarThreads, 2) wave_bl_mixed_far(const WaveDesc W) {
-    persistent_body<PolicyMixed, NF, kPhaseFar, SceneRiafBL>(W);
+    far_body<PolicyMixed, NF, SceneRiafBL>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, 1) wave_bl_mixed_near_a(const WaveDesc W) {
-    persistent_body<PolicyMixed, NF, kPhaseNearA, SceneRiafBL>(W);
+__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_bl_mixed_near_a(const WaveDesc W) {
+    quad_body<PolicyMixed, kPhaseNearA, SceneRiafBL>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, 1) wave_bl_mixed_near_b(const WaveDesc W) {
-    persistent_body<PolicyMixed, NF, kPhaseNearB, SceneRiafBL>(W);
+__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_bl_mixed_near_b(const WaveDesc W) {
+    quad_body<PolicyMixed, kPhaseNearB, SceneRiafBL>(W);
 }
 
 template<int NF>
 static const void* wave_bl_mixed_kernel(int phase) {
     if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_bl_mixed_far<NF>);
-    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_bl_mixed_near_a<NF>);
-    return reinterpret_cast<const void*>(wave_bl_mixed_near_b<NF>);
+    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_bl_mixed_near_a);
+    return reinterpret_cast<const void*>(wave_bl_mixed_near_b);
 }
 
 cudaError_t launch_wave_bl_mixed(int phase, const WaveDesc& W, int nf_max, int blocks, int threads, cudaStream_t stream) {

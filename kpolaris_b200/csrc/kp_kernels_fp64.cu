@@ -3,52 +3,30 @@
 // reference's CPU code does: termination reasons and fixed-step counts are
 // bit-identical to it.
 //
-//  * image_fp64_per_pixel: the plain form -- one thread per pixel, one launch
-//    per image, the reference's per-pixel code structure.
+//  * image_fp64_per_pixel: the plain form -- one launch per image, one quad
+//    (kp_quad.cuh) per pixel from the camera to the end of its ray.
 //  * wave_far_fp64 / wave_near_fp64: the wavefront engine with the FP64
 //    policy; its arithmetic is the same, so its results equal the plain
 //    kernel's bit for bit whatever the batch composition.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "kp_analysis.cuh"
 #include "kp_bl.cuh"
 #include "kp_launch.h"
-#include "kp_persistent.cuh"
+#include "kp_quad.cuh"
 #include "kp_trace_fp64.cuh"
-
-// resident CTAs per SM the wavefront kernels are compiled for
-#ifndef KP_FAR_MIN_BLOCKS
-#define KP_FAR_MIN_BLOCKS 2
-#endif
-#ifndef KP_NEAR_MIN_BLOCKS
-#define KP_NEAR_MIN_BLOCKS 1
-#endif
 
 namespace kp {
 
-template<int NF>
-__global__ void __launch_bounds__(128) image_fp64_per_pixel(const ImageConsts c, const CameraFrame frame,
-                                                            const ImageOutPtrs out, int npix) {
-    const int pixel = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pixel >= npix) return;
-    const Ray cam = camera_ray(c, frame, pixel);
-    Ray state = cam;
-    PixelOut o;
-    int pa_reason = kMaxSteps;
-    const int valid = trace_pass_a(c, state, o.pass_a_steps, pa_reason);
-    Stokes4<double> stokes[NF];
-    o.steps = 0;
-    o.reason = pa_reason;
-    if (valid) {
-        trace_pass_b_fp64<NF>(c, state, stokes, o.steps, o.reason);
-    } else {
-#pragma unroll
-        for (int f = 0; f < NF; ++f) stokes[f] = Stokes4<double>{0.0, 0.0, 0.0, 0.0};
-    }
-    double obs[NF][4];
-    finish_ray<double, NF>(c, cam, state, valid, stokes, o, obs);
-    store_stokes<NF>(out, pixel, npix, obs);
-    store_diagnostics(out, pixel, o);
+__global__ void __launch_bounds__(kImageThreads, kImageBlocks) image_fp64_per_pixel(const __grid_constant__ JobDesc job,
+                                                                                   int per_warp) {
+    WaveDesc W = {};
+    W.jobs = &job;
+    W.njobs = 1;
+    W.fresh_end = job.npix;
+    quad_body<PolicyFP64, kPhaseAll>(W, per_warp);
 }
 
 // Analysis mode: the plain per-pixel form with the analysis pass B, one
@@ -173,18 +151,20 @@ void host_camera_frame(const ImageConsts& c, double frame[5][4]) {
     }
 }
 
-cudaError_t launch_image_fp64(const ImageConsts& c, const ImageOutPtrs& out, cudaStream_t stream) {
-    const CameraFrame frame = camera_frame(c);
-    const int npix = c.nx * c.ny;
-    const int block = 128;
-    const int grid = (npix + block - 1) / block;
-    switch (c.nfreq) {
-    case 1: image_fp64_per_pixel<1><<<grid, block, 0, stream>>>(c, frame, out, npix); break;
-    case 2: image_fp64_per_pixel<2><<<grid, block, 0, stream>>>(c, frame, out, npix); break;
-    case 3: image_fp64_per_pixel<3><<<grid, block, 0, stream>>>(c, frame, out, npix); break;
-    case 4: image_fp64_per_pixel<4><<<grid, block, 0, stream>>>(c, frame, out, npix); break;
-    default: return cudaErrorInvalidValue;
-    }
+cudaError_t launch_image_fp64(const ImageConsts& c, const ImageOutPtrs& out, int sms, cudaStream_t stream) {
+    if (c.nfreq < 1 || c.nfreq > kMaxFreq) return cudaErrorInvalidValue;
+    JobDesc job = {};
+    job.c = c;
+    job.frame = camera_frame(c);
+    job.out = out;
+    job.npix = c.nx * c.ny;
+    // As many warps as the SMs hold at once before a warp gets a second ray:
+    // a small image is as slow as its longest ray, and a warp's rays share
+    // its issue slots.
+    const long long warps = (long long)std::max(1, sms) * kImageBlocks * (kImageThreads / 32);
+    const int per_warp = int(std::min<long long>(8, std::max<long long>(1, (job.npix + warps - 1) / warps)));
+    const int per_block = per_warp * (kImageThreads / 32);
+    image_fp64_per_pixel<<<(job.npix + per_block - 1) / per_block, kImageThreads, 0, stream>>>(job, per_warp);
     return cudaGetLastError();
 }
 
@@ -193,25 +173,23 @@ cudaError_t launch_image_fp64(const ImageConsts& c, const ImageOutPtrs& out, cud
 // NF (the unit is compiled without FMA contraction), so every instantiation
 // traces a ray bit-identically to the plain kernel.
 template<int NF>
-__global__ void __launch_bounds__(kFarThreads, KP_FAR_MIN_BLOCKS) wave_far_fp64(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseFar>(W);
+__global__ void __launch_bounds__(kFarThreads, kFarBlocks) wave_far_fp64(const WaveDesc W) {
+    far_body<PolicyFP64, NF>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, KP_NEAR_MIN_BLOCKS) wave_near_a_fp64(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseNearA>(W);
+__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_fp64(const WaveDesc W) {
+    quad_body<PolicyFP64, kPhaseNearA>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, KP_NEAR_MIN_BLOCKS) wave_near_b_fp64(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseNearB>(W);
+__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_fp64(const WaveDesc W) {
+    quad_body<PolicyFP64, kPhaseNearB>(W);
 }
 
 template<int NF>
 static const void* wave_kernel_fp64(int phase) {
     if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_fp64<NF>);
-    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_fp64<NF>);
-    return reinterpret_cast<const void*>(wave_near_b_fp64<NF>);
+    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_fp64);
+    return reinterpret_cast<const void*>(wave_near_b_fp64);
 }
 
 cudaError_t launch_wave_fp64(int phase, const WaveDesc& W, int nf_max, int blocks, int threads,

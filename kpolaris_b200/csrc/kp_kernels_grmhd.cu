@@ -5,30 +5,28 @@
 #include <cuda_runtime.h>
 
 #include "kp_launch.h"
-#include "kp_persistent.cuh"
+#include "kp_quad.cuh"
 
 namespace kp {
 
 template<int NF>
 __global__ void __launch_bounds__(kFarThreads, 2) wave_far_grmhd(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseFar, SceneGrmhd>(W);
+    far_body<PolicyFP64, NF, SceneGrmhd>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, 1) wave_near_a_grmhd(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseNearA, SceneGrmhd>(W);
+__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_grmhd(const WaveDesc W) {
+    quad_body<PolicyFP64, kPhaseNearA, SceneGrmhd>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, 1) wave_near_b_grmhd(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseNearB, SceneGrmhd>(W);
+__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_grmhd(const WaveDesc W) {
+    quad_body<PolicyFP64, kPhaseNearB, SceneGrmhd>(W);
 }
 
 template<int NF>
 static const void* wave_kernel_grmhd(int phase) {
     if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_grmhd<NF>);
-    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_grmhd<NF>);
-    return reinterpret_cast<const void*>(wave_near_b_grmhd<NF>);
+    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_grmhd);
+    return reinterpret_cast<const void*>(wave_near_b_grmhd);
 }
 
 cudaError_t launch_wave_grmhd(int phase, const WaveDesc& W, int nf_max, int blocks, int threads,

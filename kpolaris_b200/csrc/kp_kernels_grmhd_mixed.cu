@@ -1,48 +1,44 @@
 // kp_kernels_grmhd_mixed.cu -- the GRMHD scene (FMKS metric, grid plasma) of
 // the wavefront engine with the mixed policy: FP64 geodesic and grid sample,
-// FP32 thermal fits and Stokes transfer with compensated accumulation.
+// FP32 thermal fits, FP64 Stokes transfer.
 // Compiled with FMA contraction (the mixed path is held to a flux/EVPA
 // budget, not to the reference's rounding).
 #include <cuda_runtime.h>
 
 #include "kp_launch.h"
-#include "kp_persistent.cuh"
+#include "kp_quad.cuh"
 
 namespace kp {
 
-template<int NF>
-__global__ void __launch_bounds__(kFarThreads, 2) wave_far_grmhd_mixed(const WaveDesc W) {
-    persistent_body<PolicyMixed, NF, kPhaseFar, SceneFarCks<SceneGrmhd>>(W);
+__global__ void __launch_bounds__(kFarThreads, kFarBlocks) wave_far_grmhd_mixed(const WaveDesc W) {
+    quad_body<PolicyMixed, kPhaseFar, SceneFarCks<SceneGrmhd>>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, 1) wave_near_a_grmhd_mixed(const WaveDesc W) {
-    persistent_body<PolicyMixed, NF, kPhaseNearA, SceneGrmhd>(W);
+__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_grmhd_mixed(const WaveDesc W) {
+    quad_body<PolicyMixed, kPhaseNearA, SceneGrmhd>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, 1) wave_near_b_grmhd_mixed(const WaveDesc W) {
-    persistent_body<PolicyMixed, NF, kPhaseNearB, SceneGrmhd>(W);
+__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_grmhd_mixed(const WaveDesc W) {
+    quad_body<PolicyMixed, kPhaseNearB, SceneGrmhd>(W);
 }
 
-template<int NF>
 static const void* wave_kernel_grmhd_mixed(int phase) {
-    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_grmhd_mixed<NF>);
-    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_grmhd_mixed<NF>);
-    return reinterpret_cast<const void*>(wave_near_b_grmhd_mixed<NF>);
+    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_grmhd_mixed);
+    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_grmhd_mixed);
+    return reinterpret_cast<const void*>(wave_near_b_grmhd_mixed);
 }
 
 cudaError_t launch_wave_grmhd_mixed(int phase, const WaveDesc& W, int nf_max, int blocks, int threads,
                                     cudaStream_t stream) {
     if (nf_max < 1 || nf_max > kMaxFreq || phase < 0 || phase >= kPhases) return cudaErrorInvalidValue;
-    const void* fn = nf_max == 1 ? wave_kernel_grmhd_mixed<1>(phase) : wave_kernel_grmhd_mixed<kMaxFreq>(phase);
+    const void* fn = wave_kernel_grmhd_mixed(phase);
     void* args[] = {const_cast<WaveDesc*>(&W)};
     return cudaLaunchKernel(fn, dim3(blocks), dim3(threads), args, 0, stream);
 }
 
 int wave_occupancy_grmhd_mixed(int phase, int nf_max, int threads) {
     if (phase < 0 || phase >= kPhases) return 0;
-    const void* fn = nf_max == 1 ? wave_kernel_grmhd_mixed<1>(phase) : wave_kernel_grmhd_mixed<kMaxFreq>(phase);
+    const void* fn = wave_kernel_grmhd_mixed(phase);
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, 0);
     return n;

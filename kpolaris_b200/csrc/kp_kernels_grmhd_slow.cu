@@ -4,30 +4,28 @@
 #include <cuda_runtime.h>
 
 #include "kp_launch.h"
-#include "kp_persistent.cuh"
+#include "kp_quad.cuh"
 
 namespace kp {
 
 template<int NF>
 __global__ void __launch_bounds__(kFarThreads, 2) wave_far_grmhd_slow(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseFar, SceneGrmhdSlow>(W);
+    far_body<PolicyFP64, NF, SceneGrmhdSlow>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, 1) wave_near_a_grmhd_slow(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseNearA, SceneGrmhdSlow>(W);
+__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_grmhd_slow(const WaveDesc W) {
+    quad_body<PolicyFP64, kPhaseNearA, SceneGrmhdSlow>(W);
 }
 
-template<int NF>
-__global__ void __launch_bounds__(kNearThreads, 1) wave_near_b_grmhd_slow(const WaveDesc W) {
-    persistent_body<PolicyFP64, NF, kPhaseNearB, SceneGrmhdSlow>(W);
+__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_grmhd_slow(const WaveDesc W) {
+    quad_body<PolicyFP64, kPhaseNearB, SceneGrmhdSlow>(W);
 }
 
 template<int NF>
 static const void* wave_kernel_grmhd_slow(int phase) {
     if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_grmhd_slow<NF>);
-    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_grmhd_slow<NF>);
-    return reinterpret_cast<const void*>(wave_near_b_grmhd_slow<NF>);
+    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_grmhd_slow);
+    return reinterpret_cast<const void*>(wave_near_b_grmhd_slow);
 }
 
 cudaError_t launch_wave_grmhd_slow(int phase, const WaveDesc& W, int nf_max, int blocks, int threads,

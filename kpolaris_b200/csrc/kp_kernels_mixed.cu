@@ -1,34 +1,23 @@
-// kp_kernels_mixed.cu -- the mixed-precision wavefront kernels.  FP64 ray
-// state, stage combination and step control everywhere; the far kernel
-// (rays beyond ImageConsts::fp32_radius) contracts the connection in FP32,
-// the near kernels in FP64; radiative transfer (near-B) in FP32.  Compiled with FMA
-// contraction enabled.  Both always carry four frequency channels, so the
-// same compiled code traces a ray whatever the rest of the batch is.
+// kp_kernels_mixed.cu -- the mixed-precision wavefront kernels: FP64 ray
+// state, transport, step control and Stokes transfer, many far-field steps at
+// once, FP32 transfer coefficients.  Compiled with FMA contraction enabled.
 #include <cuda_runtime.h>
 
 #include "kp_launch.h"
-#include "kp_persistent.cuh"
-
-// resident CTAs per SM the wavefront kernels are compiled for
-#ifndef KP_FAR_MIN_BLOCKS
-#define KP_FAR_MIN_BLOCKS 3
-#endif
-#ifndef KP_NEAR_MIN_BLOCKS
-#define KP_NEAR_MIN_BLOCKS 1
-#endif
+#include "kp_quad.cuh"
 
 namespace kp {
 
-__global__ void __launch_bounds__(kFarThreads, KP_FAR_MIN_BLOCKS) wave_far_mixed(const WaveDesc W) {
-    persistent_body<PolicyMixed, kMaxFreq, kPhaseFar>(W);
+__global__ void __launch_bounds__(kFarThreads, kFarBlocks) wave_far_mixed(const WaveDesc W) {
+    quad_body<PolicyMixed, kPhaseFar>(W);
 }
 
-__global__ void __launch_bounds__(kNearThreads, KP_NEAR_MIN_BLOCKS) wave_near_a_mixed(const WaveDesc W) {
-    persistent_body<PolicyMixed, kMaxFreq, kPhaseNearA>(W);
+__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_mixed(const WaveDesc W) {
+    quad_body<PolicyMixed, kPhaseNearA>(W);
 }
 
-__global__ void __launch_bounds__(kNearThreads, KP_NEAR_MIN_BLOCKS) wave_near_b_mixed(const WaveDesc W) {
-    persistent_body<PolicyMixed, kMaxFreq, kPhaseNearB>(W);
+__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_mixed(const WaveDesc W) {
+    quad_body<PolicyMixed, kPhaseNearB>(W);
 }
 
 static const void* wave_kernel_mixed(int phase) {

@@ -8,8 +8,8 @@
 
 namespace kp {
 
-// Plain FP64 kernel, one thread per pixel, one image (kp_kernels_fp64.cu).
-cudaError_t launch_image_fp64(const ImageConsts& c, const ImageOutPtrs& out, cudaStream_t stream);
+// Plain FP64 kernel, one quad per pixel, one image (kp_kernels_fp64.cu).
+cudaError_t launch_image_fp64(const ImageConsts& c, const ImageOutPtrs& out, int sms, cudaStream_t stream);
 // Analysis mode: the per-pixel FP64 image with the line-of-sight
 // diagnostics (one frequency; radial_bins in 1..24).
 constexpr int kMaxRadialBins = 24;  // KPOLARIS_MAX_ANALYSIS_RADIAL_BINS
@@ -150,11 +150,22 @@ cudaError_t launch_grid_derived(const GridConsts& g, double* derived, int sms, c
 // rays grazing the radiating sphere a few more).
 constexpr int kMaxWaveCycles = 24;
 
-// Threads per CTA of each phase kernel (its __launch_bounds__): the far
-// kernel runs two CTAs of 128 per SM, the near kernels one CTA of 256, so
-// that every resident warp of an SM steps through the same code region.
-constexpr int kFarThreads = 128;
-constexpr int kNearThreads = 256;
-inline int wave_threads(int phase) { return phase == kPhaseFar ? kFarThreads : kNearThreads; }
+// Threads per CTA of each phase kernel and resident CTAs per SM they are
+// compiled for: 8 warps of 255 registers per SM.  Near-B's one large CTA keeps
+// all of them in step (8 x 256^2 mixed: 189 ms against 197 ms for two CTAs);
+// near-A and the far phase are faster in two (57 against 62 ms).  12 warps of
+// 168 registers spill: a 128^2 image at 60 degrees took 293 instead of 219 ms.
+constexpr int kFarThreads = 128, kFarBlocks = 2;
+constexpr int kNearAThreads = 128, kNearABlocks = 2;
+constexpr int kNearBThreads = 256, kNearBBlocks = 1;
+constexpr int kImageThreads = 32, kImageBlocks = 8;  // the plain FP64 kernel: a warp's slot is free when its own rays end
+inline int wave_threads(int phase) {
+    return phase == kPhaseFar ? kFarThreads : (phase == kPhaseNearA ? kNearAThreads : kNearBThreads);
+}
+// CTAs that give every ray a warp: more would only idle.
+inline long long wave_blocks_needed(int phase, long long rays) {
+    const int warps = wave_threads(phase) / 32;
+    return (rays + warps - 1) / warps;
+}
 
 }  // namespace kp

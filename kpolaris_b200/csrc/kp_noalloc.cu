@@ -92,7 +92,7 @@ extern "C" int kp_batch_riaf_noalloc(const kp_riaf_job* jobs, int njobs, const k
         return set_error(KP_ERR_INVALID, "unknown integrator %d", opt.integrator);
     if (opt.threads_per_block != 0)
         return set_error(KP_ERR_INVALID, "threads_per_block is fixed by the wavefront kernels (%d far, %d near): pass 0",
-                         kFarThreads, kNearThreads);
+                         kFarThreads, kNearBThreads);
     long long total = 0;
     int nf_max = 1;
     for (int i = 0; i < njobs; ++i) {
@@ -162,7 +162,7 @@ extern "C" int kp_batch_riaf_noalloc(const kp_riaf_job* jobs, int njobs, const k
             if (per_sm <= 0) per_sm = 1;
         }
         blocks[phase] = std::max(1, sms) * per_sm;
-        const long long needed = (total + wave_threads(phase) - 1) / wave_threads(phase);
+        const long long needed = wave_blocks_needed(phase, total);
         if (blocks[phase] > needed) blocks[phase] = int(needed);
     }
     for (int cycle = 0; cycle < kMaxWaveCycles; ++cycle) {

@@ -6,11 +6,13 @@
 // budget is set).  See kp_engine.cuh for the RK jobs.
 //
 // Three phases, one kernel each, so that the lanes of a warp run the same
-// code and each kernel's instruction working set stays small:
+// code and each kernel's instruction working set stays small (this file: what
+// they share, and the far phase with one ray per lane; kp_quad.cuh: four lanes
+// per ray):
 //   far     rays beyond ImageConsts::fp32_radius, pass A and pass B: pure
 //           transport (no surface lies within a step, no plasma is sampled);
 //   near-A  pass A inside: the surface-crossing search, no radiation;
-//   near-B  pass B inside: radiative transfer, Stokes vectors in registers.
+//   near-B  pass B inside: radiative transfer.
 //
 // Parking happens only at the top of the pass-A or pass-B loop, where the
 // whole state is the record: a ray resumed from its record takes exactly the
@@ -58,9 +60,8 @@ static_assert(sizeof(LaneState) <= sizeof(((RayRecord*)nullptr)->st), "LaneState
 static_assert(offsetof(LaneState, old_r) % 8 == 0 && offsetof(LaneState, lo) % 8 == 0, "parts are whole doubles");
 
 // Bytes of LaneState a phase kernel moves: near-B runs no pass-A step and
-// never holds a far chart, far runs no crossing search, and near-A's
-// crossing search works on the crossing part in the record itself (one
-// search per ray, a few iterations).
+// never holds a far chart, far runs no crossing search, and a search never
+// spans two launches.
 template<int PHASE>
 constexpr size_t kLaneStateBytes = PHASE == kPhaseNearB ? offsetof(LaneState, old_r) : offsetof(LaneState, lo);
 
@@ -75,14 +76,35 @@ __device__ __forceinline__ void begin_adaptive(LS& L, double requested, double m
     L.attempt = 0;
 }
 
+// x^0.2 for x > 0: pow under the FP64 policy (the reference's); under the
+// mixed policy Newton's iteration for y^5 = x from a single-precision
+// exponential, two steps from 1e-6 to a few ulp (pow and its division cost a
+// lone ray 900 cycles a step).  Out of range it is pow.
+template<bool MIXED>
+__device__ __forceinline__ double fifth_root(double x) {
+    if constexpr (MIXED) {
+        if (x > 1e-30 && x < 1e30) {
+            double y = double(exp2f(0.2f * __log2f(float(x))));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const double y2 = y * y, y4 = y2 * y2;
+                y = y - (y4 * y - x) * kp_recip<double>(5.0 * y4);
+            }
+            return y;
+        }
+    }
+    return pow(x, 0.2);
+}
+
 // Step growth after an accepted attempt (rk4.hpp:130-142).  With
 // tol >= 64 err the factor 0.9 (tol/err)^0.2 is at least 2.07 and clamps to
 // 2, so pow is evaluated only below that ratio (same result).
+template<bool MIXED = false>
 __device__ __forceinline__ double accepted_next_h(double h, double err, double tol, double min_step,
                                                   double max_step, double requested) {
     double factor = 2.0;
     if (err > 0.0 && !(tol >= 64.0 * err)) {
-        factor = 0.9 * pow(tol / err, 0.2);
+        factor = 0.9 * fifth_root<MIXED>(MIXED ? tol * kp_recip<double>(err) : tol / err);
         factor = min_val(2.0, max_val(0.2, factor));
     }
     double next_h = min_val(max_step, max_val(min_step, abs_val(h) * factor));
@@ -93,7 +115,7 @@ __device__ __forceinline__ double accepted_next_h(double h, double err, double t
 // A rejected attempt: shrink and retry, or give up (rk4.hpp:143-160).
 // Returns 1 when the sequence is exhausted; L.h_current then holds the
 // signed next_h of the failed sequence.
-template<class LS>
+template<bool MIXED = false, class LS>
 __device__ __forceinline__ int rejected_attempt(LS& L, double err, double tol) {
     L.attempt += 1;
     int exhausted = L.attempt >= 10;
@@ -211,13 +233,14 @@ struct RecordScene<SceneFarCks<B>> {
     using type = B;
 };
 
-template<class P, int NF, int PHASE, class SC = SceneRiaf>
-__device__ __forceinline__ void persistent_body(const WaveDesc& W) {
-    constexpr bool kFar = PHASE == kPhaseFar;
-    constexpr bool kPassA = PHASE != kPhaseNearB;   // pass-A steps run here
-    constexpr bool kPassB = PHASE != kPhaseNearA;   // pass-B steps run here
-    constexpr bool kCross = PHASE == kPhaseNearA;   // surface-crossing search
-    constexpr bool kRad = PHASE == kPhaseNearB;     // radiative transfer (Stokes in registers)
+// The far phase with one ray per lane, for the scenes and policies that take
+// its steps one by one (FP64, and Boyer-Lindquist under either policy).  Pure
+// transport: every lane runs the same instructions, and with tens of
+// thousands of rays a lane per ray needs half the operations of a quad
+// (kp_quad.cuh), which evaluates a point's connection four times.
+template<class P, int NF, class SC = SceneRiaf>
+__device__ __forceinline__ void far_body(const WaveDesc& W) {
+    constexpr int PHASE = kPhaseFar;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     using RT = RadTraits<P, SC>;
@@ -228,13 +251,6 @@ __device__ __forceinline__ void persistent_body(const WaveDesc& W) {
     Ray S;
     typename RT::Stokes stokes[NF];
     unsigned my_id = 0;
-    // the crossing search's best state (near-A) lives in the record's Stokes
-    // slot, which pass A leaves unused: it holds no registers between the
-    // search's iterations
-    auto best = [&]() -> Ray& { return *reinterpret_cast<Ray*>(W.pool[my_id].stokes); };
-    // ... and its bracket, the crossing part of the control state, in the record
-    auto cs = [&]() -> LaneState& { return *reinterpret_cast<LaneState*>(W.pool[my_id].st); };
-    static_assert(sizeof(((RayRecord*)nullptr)->stokes) >= sizeof(Ray), "the Stokes slot holds a ray");
     int exhausted = 0;
     long long lane_jobs = 0;
     const JobDesc* J = nullptr;
@@ -267,13 +283,6 @@ __device__ __forceinline__ void persistent_body(const WaveDesc& W) {
                     my_id = unsigned(id);
                     J = &W.jobs[lo];
                     start_ray<SC>(st, S, J, lo, int(id - J->ray_begin));
-                    if constexpr (SC::kFarChart) {
-                        if (SC::chart_active(J->c)) {
-                            st.x3_ref = S.x.v[3];
-                            S = SC::to_phase(J->c, S);
-                            st.chart = 1;
-                        }
-                    }
                 } else if (W.budget > 0 && lane_jobs >= W.budget) {
                     // past the budget: hand the id on untouched (below)
                     my_id = W.in_ids[k - nfresh];
@@ -285,15 +294,6 @@ __device__ __forceinline__ void persistent_body(const WaveDesc& W) {
                     S = rec.S;
                     memcpy(&st, rec.st, kLaneStateBytes<PHASE>);
                     J = &W.jobs[st.job];
-                    if constexpr (SC::kFarChart) {
-                        // a record parked for this phase already holds its chart
-                        if (!st.chart && SC::chart_active(J->c)) {
-                            st.x3_ref = S.x.v[3];
-                            S = SC::to_phase(J->c, S);
-                            st.chart = 1;
-                        }
-                    }
-                    if constexpr (kRad) memcpy(&stokes[0], rec.stokes, sizeof(stokes));
                 }
             }
         }
@@ -307,7 +307,7 @@ __device__ __forceinline__ void persistent_body(const WaveDesc& W) {
 
         // ---------------------------------------------- control before the job
         int dest = -1;  // phase the ray is handed to (PHASE itself: its next launch)
-        if constexpr (kPassA) {
+        {
             if (active && st.mode == kAStep && st.rk_kind < 0) {
                 const ImageConsts& c = J->c;
                 const double r_bl = SC::radius(c, S.x);
@@ -385,21 +385,8 @@ __device__ __forceinline__ void persistent_body(const WaveDesc& W) {
         const bool park = dest >= 0;
         if (park) {
             RayRecord& rec = W.pool[my_id];
-            if constexpr (SC::kFarChart) {
-                // leaving the phase: back to the records' chart; parked for
-                // this phase (a tick budget): kept as is, so the ray resumes
-                // bit for bit as if it had not been parked
-                if (st.chart && dest != PHASE) {
-                    rec.S = SC::to_record(J->c, S, st.x3_ref);
-                    st.chart = 0;
-                } else {
-                    rec.S = S;
-                }
-            } else {
-                rec.S = S;
-            }
+            rec.S = S;
             memcpy(rec.st, &st, kLaneStateBytes<PHASE>);
-            if constexpr (kRad) memcpy(rec.stokes, &stokes[0], sizeof(stokes));
         }
         // A lane past its budget keeps claiming and parks each claimed ray at
         // once, so every input ends the launch finished or in a queue.
@@ -408,21 +395,11 @@ __device__ __forceinline__ void persistent_body(const WaveDesc& W) {
         if (park) st.mode = kIdle;
 
         // ------------------------------------------------------------ RK job
-        const bool run = !park && (st.mode == kAStep || st.mode == kACrossHi || st.mode == kACrossTrial ||
-                                   st.mode == kBStep || st.mode == kBCamCross);
-        // Mixed policy: FP32 stage chains in the far phase only.  Inside the
-        // radiating sphere FP32 rounding in dk and de reaches the
-        // step-doubling error estimate and reshapes the accepted-step
-        // sequence the Faraday-thick transfer is sensitive to.  One RK call
-        // site: the crossing search's job differs only in kind and step.
-        constexpr bool fp32 = P::kMixed && kFar;
+        const bool run = !park && (st.mode == kAStep || st.mode == kBStep || st.mode == kBCamCross);
         Ray next, mid;
         double err = 0.0;
         if (run) {
-            const bool crossing = kCross && (st.mode == kACrossHi || st.mode == kACrossTrial);
-            const int kind = crossing ? (J->c.adaptive ? kRkRK4x2 : kRkRK4) : st.rk_kind;
-            const double hj = crossing ? (st.mode == kACrossHi ? cs().full_h : cs().full_h * cs().trial) : st.h_try;
-            rk_job<P, fp32, SC>(kind, J->c, S, hj, next, mid, err);
+            rk_job<P, SC>(st.rk_kind, J->c, S, st.h_try, next, mid, err);
             if (++lane_jobs > (1LL << 30)) {
                 st.reason = kInvalidState;
                 st.mode = kDone;
@@ -437,10 +414,9 @@ __device__ __forceinline__ void persistent_body(const WaveDesc& W) {
         __syncthreads();
 
         // ----------------------------------------------- control after the job
-        if (kPassA && run && st.mode == kAStep) {
+        if (run && st.mode == kAStep) {
             const ImageConsts& c = J->c;
             bool accepted = true;
-            double used_h = st.h_try;
             if (st.rk_kind != kRkRK4) {
                 const double tol = max_val(c.tolerance, kTolFloor);
                 if (err <= tol) {
@@ -480,26 +456,9 @@ __device__ __forceinline__ void persistent_body(const WaveDesc& W) {
                         crossing = kEscaped;
                     }
                     if (crossing != kNone) {
-                        if constexpr (kCross) {
-                            cs().cross_reason = crossing;
-                            cs().surf = crossing == kReachedInner ? c.inner_radius : c.outer_radius;
-                            cs().full_h = used_h;
-                            best() = S;
-                            cs().lo = 0.0;
-                            cs().hi = 1.0;
-                            cs().flo = SC::radius(c, S.x) - cs().surf;
-                            if (cs().flo == 0.0 || !finite_ray(next)) {
-                                st.pa_steps += 1;  // the event keeps the first state
-                                st.reason = crossing;
-                                st.mode = kEndA;
-                            } else {
-                                st.mode = kACrossHi;
-                            }
-                        } else {
-                            atomicExch(W.status, 3);  // surfaces lie inside the near phase
-                            st.reason = kInvalidState;
-                            st.mode = kDone;
-                        }
+                        atomicExch(W.status, 3);  // surfaces lie inside the near phase
+                        st.reason = kInvalidState;
+                        st.mode = kDone;
                     } else {
                         S = next;
                         st.pa_steps += 1;
@@ -508,64 +467,7 @@ __device__ __forceinline__ void persistent_body(const WaveDesc& W) {
                     }
                 }
             }
-        } else if (kCross && run && (st.mode == kACrossHi || st.mode == kACrossTrial)) {
-            const ImageConsts& c = J->c;
-            bool finish = false;
-            if (st.mode == kACrossHi) {
-                if (!finite_ray(next)) {
-                    finish = true;
-                } else {
-                    const double fhi = SC::radius(c, next.x) - cs().surf;
-                    if (!(fhi == fhi) || abs_val(fhi) >= kLarge) {
-                        finish = true;
-                    } else if (fhi == 0.0) {
-                        best() = next;
-                        finish = true;
-                    } else if ((cs().flo > 0.0) == (fhi > 0.0)) {
-                        finish = true;
-                    } else {
-                        cs().fhi = fhi;
-                        cs().iter = 0;
-                        cs().use_secant = 1;
-                    }
-                }
-            } else {
-                const double ft = finite_ray(next) ? SC::radius(c, next.x) - cs().surf : 0.0;
-                if (!finite_ray(next) || !(ft == ft) || abs_val(ft) >= kLarge) {
-                    cs().hi = cs().trial;
-                    cs().use_secant = 0;
-                } else if (ft == 0.0) {
-                    best() = next;
-                    finish = true;
-                } else if ((cs().flo > 0.0) == (ft > 0.0)) {
-                    cs().lo = cs().trial;
-                    cs().flo = ft;
-                    best() = next;
-                } else {
-                    cs().hi = cs().trial;
-                    cs().fhi = ft;
-                }
-                cs().iter += 1;
-            }
-            if (!finish && cs().iter >= 12) finish = true;
-            if (finish) {
-                S = best();
-                st.pa_steps += 1;
-                st.reason = cs().cross_reason;
-                st.mode = kEndA;
-            } else {
-                const double width = cs().hi - cs().lo;
-                double trial = (cs().lo + cs().hi) * 0.5;
-                const double denom = cs().flo - cs().fhi;
-                if (cs().use_secant && abs_val(denom) > kTiny) {
-                    const double secant = cs().lo + width * cs().flo / denom;
-                    const double g = width * 0.1;
-                    if (secant > cs().lo + g && secant < cs().hi - g) trial = secant;
-                }
-                cs().trial = trial;
-                st.mode = kACrossTrial;
-            }
-        } else if (kPassB && run && (st.mode == kBStep || st.mode == kBCamCross)) {
+        } else if (run && (st.mode == kBStep || st.mode == kBCamCross)) {
             const ImageConsts& c = J->c;
             const bool cam = st.mode == kBCamCross;
             bool proceed = true;
@@ -616,103 +518,23 @@ __device__ __forceinline__ void persistent_body(const WaveDesc& W) {
                         }
                     }
                 }
-                bool stopped = false;
                 if (proceed) {
-                    // radiation at the sample point (pass_b.hpp:1414-1496)
+                    // The sample lies outside the radiating sphere: every
+                    // coefficient is zero, the transfer step leaves the Stokes
+                    // vector unchanged and the step cap resolves to max_step
+                    // (pass_b.hpp:1414-1496).
                     const double sample_r = SC::radius(c, sample.x);
                     const double next_r = SC::radius(c, next.x);
-                    const double local_max_rs =
-                        (c.max_radiation_step > 0.0 &&
-                         (st.start_r <= c.outer_radius || sample_r <= c.outer_radius || next_r <= c.outer_radius))
-                            ? c.max_radiation_step : 0.0;
-                    if constexpr (kRad) {
-                        // The frequency loops stay rolled: one copy of the
-                        // coefficient and transfer code keeps the kernel's
-                        // instruction working set small.
-                        typename RT::Co co[NF];
-                        typename RT::Sample ps = RT::none();
-                        bool radiating = sample_r - c.inner_radius > 0.0 && sample_r < c.outer_radius;
-                        if constexpr (SC::kSlowLight) {
-                            // slow_light_driver.hpp:1295-1304: a radiating sample
-                            // needs its fluid time among the resident snapshots;
-                            // otherwise the ray ends where it stands
-                            radiating = sample_r >= c.inner_radius && sample_r < c.outer_radius;
-                            if (radiating && !SC::time_resident(c, sample)) {
-                                st.reason = kSlowLightTimeExhausted;
-                                st.mode = kDone;
-                                stopped = true;
-                            }
-                        }
-                        if (radiating && !stopped) ps = RT::sample(c, sample);
-                        if (!stopped) {
-                        const int nf = c.nfreq < NF ? c.nfreq : NF;
-#pragma unroll 1
-                        for (int f = 0; f < nf; ++f) {
-                            co[f] = RT::coeffs(c, ps, f);
-                            if (!c.faraday_rotation) co[f].rV = 0.0;
-                        }
-                        // Substep counts at h (required) and at h_current
-                        // (predictive) in one pass: neither test changes h or
-                        // h_current.  Over the image's frequencies, or over a
-                        // separate step-control list (pass_b.hpp:1787-1833).
-                        int required = 1, pred = 1;
-                        const bool fused = c.nctl == 0;
-#pragma unroll 1
-                        for (int g = 0; g < (fused ? nf : c.nctl); ++g) {
-                            typename RT::Co cg;
-                            double dls;
-                            if (fused) {
-                                cg = co[g];
-                                dls = c.dlambda_scale[g];
-                            } else {
-                                cg = RT::coeffs_ctl(c, ps, g);
-                                if (!c.faraday_rotation) cg.rV = 0.0;
-                                dls = c.ctl_dlambda_scale[g];
-                            }
-                            const int cand = radiation_substep_count(cg, h, dls, local_max_rs, c.max_radiation_depth,
-                                                                     c.max_absorption_depth, c.max_faraday_depth);
-                            required = cand > required ? cand : required;
-                            const int pc = radiation_substep_count(cg, st.h_current, dls, local_max_rs,
-                                                                   c.max_radiation_depth, c.max_absorption_depth,
-                                                                   c.max_faraday_depth);
-                            pred = pc > pred ? pc : pred;
-                        }
-                        if (required > 1 && h > c.min_step_abs * 1.0001) {
-                            st.h_current = max_val(c.min_step_abs, h / double(required));
-                            st.cap = st.h_current;
-                        } else {
-                            if (local_max_rs > 0.0 || c.max_radiation_depth > 0.0 || c.max_absorption_depth > 0.0 ||
-                                c.max_faraday_depth > 0.0) {
-                                st.cap = pred > 1 ? max_val(c.min_step_abs, st.h_current / double(pred)) : c.max_step;
-                            } else {
-                                st.cap = c.max_step;
-                            }
-                            if (h > 0.0) {
-#pragma unroll 1
-                                for (int f = 0; f < nf; ++f) RT::step(stokes[f], co[f], h, c, f);
-                            }
-                            S = next;
-                            st.steps += 1;
-                            if (crosses) st.reached = 1;
-                        }
-                        }  // !stopped
-                    } else {
-                        // Far phase: the sample lies outside the radiating
-                        // sphere, every coefficient is zero and the transfer
-                        // step leaves the Stokes vector unchanged; the step
-                        // cap resolves to max_step (pass_b.hpp:1482-1486).
-                        if (local_max_rs > 0.0 || (sample_r - c.inner_radius > 0.0 && sample_r < c.outer_radius)) {
-                            atomicExch(W.status, 3);
-                        }
-                        st.cap = c.max_step;
-                        S = next;
-                        st.steps += 1;
-                        if (crosses) st.reached = 1;
-                    }
-                    if (!stopped) {
-                        st.mode = kBStep;
-                        st.rk_kind = -1;
-                    }
+                    if ((c.max_radiation_step > 0.0 &&
+                         (st.start_r <= c.outer_radius || sample_r <= c.outer_radius || next_r <= c.outer_radius)) ||
+                        (sample_r - c.inner_radius > 0.0 && sample_r < c.outer_radius))
+                        atomicExch(W.status, 3);
+                    st.cap = c.max_step;
+                    S = next;
+                    st.steps += 1;
+                    if (crosses) st.reached = 1;
+                    st.mode = kBStep;
+                    st.rk_kind = -1;
                 }
             }
         }
@@ -735,19 +557,12 @@ __device__ __forceinline__ void persistent_body(const WaveDesc& W) {
             const Ray cam = SC::camera(c, J->frame, st.pixel);
             double obs[NF][4];
             Stokes4<double> sd[NF];
-            if constexpr (!kRad) {
-                // only the radiating phase carries the Stokes vector: it is in the record
-                if (st.in_b) memcpy(&stokes[0], W.pool[my_id].stokes, sizeof(stokes));
-            }
+            // only the radiating phase carries the Stokes vector: it is in the record
+            if (st.in_b) memcpy(&stokes[0], W.pool[my_id].stokes, sizeof(stokes));
 #pragma unroll
             for (int f = 0; f < NF; ++f)
                 sd[f] = st.in_b ? RT::result(stokes[f], c, f) : Stokes4<double>{0.0, 0.0, 0.0, 0.0};
-            if constexpr (SC::kFarChart) {
-                const Ray S_rec = st.chart ? SC::to_record(c, S, st.x3_ref) : S;
-                finish_ray_scene<typename RecordScene<SC>::type, NF>(c, cam, S_rec, st.in_b, sd, o, obs);
-            } else {
-                finish_ray_scene<SC, NF>(c, cam, S, st.in_b, sd, o, obs);
-            }
+            finish_ray_scene<SC, NF>(c, cam, S, st.in_b, sd, o, obs);
             store_stokes_n<NF>(J->out, st.pixel, J->npix, c.nfreq, obs);
             store_diagnostics(J->out, st.pixel, o);
             if constexpr (SC::kSlowLight) {

@@ -10,13 +10,13 @@
 //  * absorption a = j / B_nu is formed as j_phys * [c^2/(2h)] (e^x - 1) / nu^2
 //    with nu in GHz so every intermediate stays inside FP32 range;
 //  * the Bessel K ratios cancel the common e^-x / sqrt(x) factor;
-//  * the Stokes update is compensated (a running TwoSum error term per
-//    component).
+//  * the plasma's geometry, its profiles, the Faraday phase and the Stokes
+//    update are FP64.
 // Absorption and Faraday coefficients times the affine step are O(1) and
 // need no scaling.
 #pragma once
 
-#include "kp_geometry.cuh"
+#include "kp_geometry_f32.cuh"
 
 namespace kp {
 
@@ -41,16 +41,23 @@ constexpr float kC2Over2hGHz2 = float(kCL * kCL / (2.0 * kHPL) / 1e18);
 constexpr float kOmega0PerB = float(kEE / (kME * kCL));
 // wp^2 per n_e: 4 pi e^2 / m_e
 constexpr float kWp2PerNe = float(4.0 * 3.141592653589793 * kEE * kEE / kME);
-// Dexter: 3 e / (4 pi m_e c)
-constexpr float kDexNus = float(3.0 * kEE / (4.0 * 3.141592653589793 * kME * kCL));
+// Dexter: 3 e / (4 pi m_e c); Pandya: 2/9 of the cyclotron frequency
+constexpr double kDexNus = 3.0 * kEE / (4.0 * 3.141592653589793 * kME * kCL);
+constexpr double kPandyaNus = 2.0 / 9.0 * kEE / (2.0 * 3.141592653589793 * kME * kCL);
+// (x / Theta_e)^2 of the Faraday fits: sqrt(2) 1e3 omega0 / (2 pi nu) per gauss and 1 / nu
+constexpr double kFaradayX2 = 1.4142135623730951 * 1e3 * kEE / (kME * kCL) / (2.0 * 3.141592653589793);
 // Dexter prefactor e^2 / (2 sqrt(3) c)
 constexpr float kDexPref = float(kEE * kEE / (2.0 * 1.7320508075688772 * kCL));
 // Dexter jV prefactor 2 e^2 / (3 sqrt(3) c)
 constexpr float kDexPrefV = float(2.0 * kEE * kEE / (3.0 * 1.7320508075688772 * kCL));
+// rho_V nu = (4 pi e^2 / m_e) (e / (m_e c)) n_e B cos(theta) / (4 pi^2 c nu) x fit
+constexpr double kRhoV = (4.0 * 3.141592653589793 * kEE * kEE / kME) * (kEE / (kME * kCL)) /
+                         (4.0 * 3.141592653589793 * 3.141592653589793 * kCL);
 }  // namespace f32c
 
 struct CoeffsF {
-    float jI, jQ, jU, jV, aI, aQ, aU, aV, rQ, rU, rV;
+    float jI, jQ, jU, jV, aI, aQ, aU, aV, rQ, rU;
+    double rV;  // the phase of thousands of radians that Faraday-thick rays gather
 };
 
 KP_HD float kp_rsqrtf(float x) {
@@ -61,104 +68,77 @@ KP_HD float kp_rsqrtf(float x) {
 #endif
 }
 
-KP_HD void kp_sincosf(float x, float* s, float* c) {
-#ifdef __CUDA_ARCH__
-    sincosf(x, s, c);
-#else
-    *s = sinf(x);
-    *c = cosf(x);
-#endif
-}
-
-// sin and cos of an angle that is usually small: below |x| = 0.5 from their
-// Taylor series to the x^9 / x^8 terms (truncation < 1e-11, under FP32
-// rounding), keeping full relative accuracy where a hardware sine's absolute
-// error would not; above it the library (or hardware) form.
-KP_HD void kp_sincos_small(float x, float* s, float* c) {
-    if (fabsf(x) < 0.5f) {
-        const float x2 = x * x;
-        *s = x * (1.0f - x2 * (1.0f / 6.0f) * (1.0f - x2 * (1.0f / 20.0f) * (1.0f - x2 * (1.0f / 42.0f) *
-                                                                                     (1.0f - x2 * (1.0f / 72.0f)))));
-        *c = 1.0f - x2 * 0.5f * (1.0f - x2 * (1.0f / 12.0f) * (1.0f - x2 * (1.0f / 30.0f) * (1.0f - x2 * (1.0f / 56.0f))));
-        return;
-    }
-    kp_sincosf(x, s, c);
-}
-
-struct StokesF {
-    float I, Q, U, V;     // scaled by 2^E
-    float cI, cQ, cU, cV; // compensation terms
-};
-
 // K0/K2 and K1/K2 for x = 1/Theta_e with the polynomial fits of
 // thermal_synchrotron.hpp:108-158; for x > 2 the factor e^-x / sqrt(x) cancels.
-KP_HD void bessel_ratios_f(float x, float& r0, float& r1) {
-    float p, q;
-    if (x <= 2.0f) {
-        const float y = x * x * 0.25f;
-        float i0, i1;
-        {
-            const float t = (x / 3.75f) * (x / 3.75f);
-            float a = 0.0045813f;
-            a = 0.0360768f + t * a;
-            a = 0.2659732f + t * a;
-            a = 1.2067492f + t * a;
-            a = 3.0899424f + t * a;
-            a = 3.5156229f + t * a;
-            i0 = 1.0f + t * a;
-            float b = 0.00032411f;
-            b = 0.00301532f + t * b;
-            b = 0.02658733f + t * b;
-            b = 0.15084934f + t * b;
-            b = 0.51498869f + t * b;
-            b = 0.87890594f + t * b;
-            b = 0.5f + t * b;
-            i1 = x * b;
-        }
-        float a = 0.00000740f;
-        a = 0.00010750f + y * a;
-        a = 0.00262698f + y * a;
-        a = 0.03488590f + y * a;
-        a = 0.23069756f + y * a;
-        a = 0.42278420f + y * a;
-        a = -0.57721566f + y * a;
-        const float lg = logf(x * 0.5f);
-        p = -lg * i0 + a;
-        float b = -0.00004686f;
-        b = -0.00110404f + y * b;
-        b = -0.01919402f + y * b;
-        b = -0.18156897f + y * b;
-        b = -0.67278579f + y * b;
-        b = 0.15443144f + y * b;
-        b = 1.0f + y * b;
-        q = lg * i1 + b / x;
+template<class T>
+KP_HD void bessel_ratios(T x, T& r0, T& r1) {
+    T p, q;
+    if (x <= T(2)) {
+        const T y = x * x * T(0.25);
+        const T t = y * T(4.0 / (3.75 * 3.75));
+        T i0 = T(0.0045813);
+        i0 = T(0.0360768) + t * i0;
+        i0 = T(0.2659732) + t * i0;
+        i0 = T(1.2067492) + t * i0;
+        i0 = T(3.0899424) + t * i0;
+        i0 = T(3.5156229) + t * i0;
+        i0 = T(1) + t * i0;
+        T i1 = T(0.00032411);
+        i1 = T(0.00301532) + t * i1;
+        i1 = T(0.02658733) + t * i1;
+        i1 = T(0.15084934) + t * i1;
+        i1 = T(0.51498869) + t * i1;
+        i1 = T(0.87890594) + t * i1;
+        i1 = x * (T(0.5) + t * i1);
+        T a = T(0.00000740);
+        a = T(0.00010750) + y * a;
+        a = T(0.00262698) + y * a;
+        a = T(0.03488590) + y * a;
+        a = T(0.23069756) + y * a;
+        a = T(0.42278420) + y * a;
+        a = T(-0.57721566) + y * a;
+        const T lg = log(x * T(0.5));
+        p = a - lg * i0;
+        T b = T(-0.00004686);
+        b = T(-0.00110404) + y * b;
+        b = T(-0.01919402) + y * b;
+        b = T(-0.18156897) + y * b;
+        b = T(-0.67278579) + y * b;
+        b = T(0.15443144) + y * b;
+        b = T(1) + y * b;
+        q = lg * i1 + b * kp_recip<T>(x);
     } else {
-        const float y = 2.0f / x;
-        float a = 0.00053208f;
-        a = -0.00251540f + y * a;
-        a = 0.00587872f + y * a;
-        a = -0.01062446f + y * a;
-        a = 0.02189568f + y * a;
-        a = -0.07832358f + y * a;
-        a = 1.25331414f + y * a;
-        p = a;
-        float b = -0.00068245f;
-        b = 0.00325614f + y * b;
-        b = -0.00780353f + y * b;
-        b = 0.01504268f + y * b;
-        b = -0.03655620f + y * b;
-        b = 0.23498619f + y * b;
-        b = 1.25331414f + y * b;
-        q = b;
+        const T y = T(2) * kp_recip<T>(x);
+        T a = T(0.00053208);
+        a = T(-0.00251540) + y * a;
+        a = T(0.00587872) + y * a;
+        a = T(-0.01062446) + y * a;
+        a = T(0.02189568) + y * a;
+        a = T(-0.07832358) + y * a;
+        p = T(1.25331414) + y * a;
+        T b = T(-0.00068245);
+        b = T(0.00325614) + y * b;
+        b = T(-0.00780353) + y * b;
+        b = T(0.01504268) + y * b;
+        b = T(-0.03655620) + y * b;
+        b = T(0.23498619) + y * b;
+        q = T(1.25331414) + y * b;
     }
-    const float k2 = p + 2.0f * q / x;
-    r0 = k2 > 0.0f ? p / k2 : 1.0f;
-    r1 = k2 > 0.0f ? q / k2 : 1.0f;
+    const T k2 = p + T(2) * q * kp_recip<T>(x);
+    const T inv = k2 > T(0) ? kp_recip<T>(k2) : T(0);
+    r0 = k2 > T(0) ? p * inv : T(1);
+    r1 = k2 > T(0) ? q * inv : T(1);
 }
 
 // Plasma state at a sample point (FP32), with the frequency-independent
-// factors of the thermal fits (riaf_sample_thermal_f).
+// factors of the thermal fits (riaf_sample_thermal_f).  The Faraday rotation
+// adds up to hundreds of radians along a thick ray, where a single-precision
+// rounding of n_e B K0/K2 cos(theta), repeated at every step, becomes an
+// error of the polarisation: that factor is formed in FP64.
 struct RiafSampleF {
+    double rv0;     // rho_V nu at nu = nu_fluid hertz, without the fit's logarithm
+    double xf0;     // argument of the Faraday fits at nu = nu_fluid hertz (it falls as nu^-1/2)
+    double xs0;     // argument of the emission fit, over the frequency in hertz
     int emitting, on_axis, has_chi;
     float ne, thetae, b, nu_fluid, cos_theta, sin_theta, theta, cos2chi, sin2chi;
     float r0, r1;   // K0/K2, K1/K2 at 1/Theta_e (Faraday fits)
@@ -166,6 +146,20 @@ struct RiafSampleF {
     float vt1;      // (37 - 87 sin(theta - 0.45)) / (100 (T + 1)), Pandya jV
     float vt2a;     // T^0.6 / 25 + 0.7, Pandya jV
 };
+
+// Cube root of x > 0 to a few ulp: Newton's step in FP64 from a
+// single-precision start.  The fits take exp(-x^(1/3)): an error of the root
+// is multiplied by the root there.
+KP_HD double cube_root(double x) {
+    if (!(x > 1e-30 && x < 1e30)) return cbrt(x);
+#ifdef __CUDA_ARCH__
+    const double y = double(exp2f(__log2f(float(x)) * (1.0f / 3.0f)));
+#else
+    const double y = double(cbrtf(float(x)));
+#endif
+    const double y2 = y * y;
+    return y - (y2 * y - x) * kp_recip<double>(3.0 * y2);
+}
 
 // x^y for x > 0 as 2^(y log2 x): one LG2 shared by several powers of x.
 KP_HD float pow2_of(float y, float lg2x) {
@@ -179,9 +173,23 @@ KP_HD float pow2_of(float y, float lg2x) {
 // Frequency-independent factors of the thermal fits at one sample
 // (thermal_synchrotron.hpp:312-395, 462-506), evaluated once per sample
 // instead of once per frequency.
-KP_HD void riaf_sample_thermal_f(const ImageConsts& c, RiafSampleF& p) {
+KP_HD void riaf_sample_thermal_f(const ImageConsts& c, RiafSampleF& p, double ne, double thetae, double b,
+                                 double cos_theta, double sin_theta, double nu_fluid) {
+    double r0, r1;
+    bessel_ratios<double>(kp_recip<double>(thetae), r0, r1);
+    p.r0 = float(r0);
+    p.r1 = float(r1);
+    const double inv_nu = kp_recip<double>(nu_fluid), sth = max_val(sin_theta, c.min_sin_theta);
+    p.rv0 = f32c::kRhoV * ne * b * r0 * cos_theta * inv_nu;
+    {
+        double g, inv;
+        kp_sqrt_pair<double>(max_val(f32c::kFaradayX2 * sth * b * inv_nu, 1e-60), g, inv);
+        p.xf0 = thetae * g;
+    }
+    const double nus = c.fit == 4 ? f32c::kDexNus * b * sth * thetae * thetae + 1.0
+                                  : f32c::kPandyaNus * b * sth * thetae * thetae;
+    p.xs0 = nu_fluid * kp_recip<double>(max_val(nus, 1e-60));
     const float te = p.thetae;
-    bessel_ratios_f(1.0f / te, p.r0, p.r1);
     const float lt = log2f(te);
     const float t2425 = pow2_of(24.0f / 25.0f, lt);
     p.qterm = (7.0f * t2425 + 35.0f) / (10.0f * t2425 + 75.0f);
@@ -191,217 +199,183 @@ KP_HD void riaf_sample_thermal_f(const ImageConsts& c, RiafSampleF& p) {
     p.vt2a = pow2_of(0.6f, lt) / 25.0f + 0.7f;
 }
 
-KP_HD float dot_gf(const float g[4][4], const float* u, const float* v) {
-    float out = 0.0f;
-#pragma unroll
-    for (int mu = 0; mu < 4; ++mu)
-#pragma unroll
-        for (int nu = 0; nu < 4; ++nu) out += g[mu][nu] * u[mu] * v[nu];
-    return out;
+KP_HD void riaf_sample_thermal_f(const ImageConsts& c, RiafSampleF& p) {
+    riaf_sample_thermal_f(c, p, p.ne, p.thetae, p.b, p.cos_theta, p.sin_theta, p.nu_fluid);
 }
 
-KP_HD void bl_metric_f(float r, float sinth, float costh, float a, float gcov[4][4],
-                                            float gcon[4][4]) {
-    const float a2 = a * a;
-    const float sin2 = fmaxf(sinth * sinth, 1e-30f);
-    const float sigma = r * r + a2 * costh * costh;
-    const float delta = r * r - 2.0f * r + a2;
-#pragma unroll
-    for (int mu = 0; mu < 4; ++mu)
-#pragma unroll
-        for (int nu = 0; nu < 4; ++nu) {
-            gcov[mu][nu] = 0.0f;
-            gcon[mu][nu] = 0.0f;
-        }
-    gcov[0][0] = -(1.0f - 2.0f * r / sigma);
-    gcov[0][3] = gcov[3][0] = -2.0f * a * r * sin2 / sigma;
-    gcov[1][1] = sigma / fmaxf(delta, 1e-30f);
-    gcov[2][2] = sigma;
-    gcov[3][3] = (r * r + a2 + 2.0f * a2 * r * sin2 / sigma) * sin2;
-    const float inv_sd = 1.0f / fmaxf(sigma * delta, 1e-30f);
-    gcon[0][0] = -((r * r + a2) * (r * r + a2) - a2 * delta * sin2) * inv_sd;
-    gcon[0][3] = gcon[3][0] = -2.0f * a * r * inv_sd;
-    gcon[1][1] = delta / sigma;
-    gcon[2][2] = 1.0f / sigma;
-    gcon[3][3] = (delta - a2 * sin2) / fmaxf(sigma * delta * sin2, 1e-30f);
+// Boyer-Lindquist metric entries at (r, theta) with unit mass, FP64.
+struct BlEntries {
+    double tt, tp, pp, rr;      // covariant
+    double itt, itp, ipp, irr;  // contravariant
+};
+
+KP_HD BlEntries bl_entries(double r, double s2, double c2, double a) {
+    const double a2 = a * a, ra = r * r + a2;
+    const double sigma = r * r + a2 * c2, delta = ra - 2.0 * r;
+    const double i_s = kp_recip<double>(sigma), i_d = kp_recip<double>(max_val(delta, 1e-30));
+    const double f = 2.0 * r * i_s, i_sd = i_s * i_d;
+    BlEntries m;
+    m.tt = f - 1.0;
+    m.tp = -a * f * s2;
+    m.pp = (ra + a2 * f * s2) * s2;
+    m.rr = sigma * i_d;
+    m.itt = -(ra * ra - a2 * delta * s2) * i_sd;
+    m.itp = -2.0 * a * r * i_sd;
+    m.ipp = (delta - a2 * s2) * i_sd * kp_recip<double>(s2);
+    m.irr = delta * i_s;
+    return m;
 }
 
-KP_HD void bl_to_cks_f(float vt, float vr, float vphi, float r, float sinth, float costh,
-                                            float cphi, float sphi, float a, float* o) {
-    const float delta = fmaxf(r * r - 2.0f * r + a * a, 1e-30f);
-    const float vt_ks = vt + 2.0f * r / delta * vr;
-    const float vphi_ks = vphi + a / delta * vr;
-    o[0] = vt_ks;
-    o[1] = vr * cphi * sinth + vphi_ks * (-r * sphi - a * cphi) * sinth;
-    o[2] = vr * sphi * sinth + vphi_ks * (r * cphi - a * sphi) * sinth;
-    o[3] = vr * costh;
-}
-
-// riaf_sample (kp_radiation.cuh) in FP32.
+// riaf_sample (kp_radiation.cuh) for the mixed policy: geometry, flow and the
+// plasma's profiles in FP64 with refined reciprocals, the result in FP32.
+// With the Kerr-Schild vector l = (1, l1, l2, l3) at the point, g = eta + f l l,
+// so a dot product is eta(u, v) + f (l.u)(l.v) with l.u formed once per
+// vector; (l1, l2) = sin(theta) (cos phi, sin phi) gives the BL angles, and
+// the azimuthal vector is (0, -y, x, 0).
 KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
     RiafSampleF out;
     out.emitting = 0;
     out.on_axis = 0;
     out.has_chi = 0;
-    const float a = float(c.spin);
-    const float xx = float(s.x.v[1]), yy = float(s.x.v[2]), zz = float(s.x.v[3]);
-    const float a2 = a * a;
-    const float radius2 = xx * xx + yy * yy + zz * zz;
-    const float sqsum = radius2 - a2;
-    const float discr = sqrtf(sqsum * sqsum + 4.0f * a2 * zz * zz);
-    const float rc = sqrtf(fmaxf(0.5f * (sqsum + discr), 1e-30f));
-    const float cos_th = fminf(fmaxf(zz / fmaxf(rc, 1e-30f), -1.0f), 1.0f);
-    const float sin_th = sqrtf(fmaxf(0.0f, 1.0f - cos_th * cos_th));
-    const float sinth_f = fmaxf(sin_th, 1e-30f);
-    const float denom = fmaxf(sinth_f * (rc * rc + a2), 1e-30f);
-    float cphi = (rc * xx + a * yy) / denom;
-    float sphi = (rc * yy - a * xx) / denom;
-    const float inv_np = kp_rsqrtf(fmaxf(cphi * cphi + sphi * sphi, 1e-30f));
-    cphi *= inv_np;
-    sphi *= inv_np;
-    const float r_bl = fmaxf(rc, float(c.min_radius));
-    if (r_bl <= float(c.horizon + c.horizon_buffer) || r_bl < float(c.r_min) || r_bl > float(c.r_max)) return out;
-    float ne_norm;
+    const double a = c.spin, a2 = a * a;
+    const double x = s.x.v[1], y = s.x.v[2], z = s.x.v[3];
+    const double sqsum = x * x + y * y + z * z - a2;
+    double discr, inv_discr, r, inv_r;
+    kp_sqrt_pair<double>(sqsum * sqsum + 4.0 * a2 * z * z, discr, inv_discr);
+    kp_sqrt_pair<double>(max_val(0.5 * (sqsum + discr), 1e-30), r, inv_r);
+    const double r_bl = max_val(r, c.min_radius);
+    if (r_bl <= c.horizon + c.horizon_buffer || r_bl < c.r_min || r_bl > c.r_max) return out;
+    const double r2 = r * r, inv_rp = kp_recip<double>(r2 + a2);
+    const double l1 = (r * x + a * y) * inv_rp, l2 = (r * y - a * x) * inv_rp, l3 = z * inv_r;
+    const double c2 = min_val(l3 * l3, 1.0), s2 = max_val((x * x + y * y) * inv_rp, 1e-30);
+    const double amp = 2.0 * c.mass * r2 * r * kp_recip<double>(r2 * r2 + a2 * z * z);
+    // n_e, Theta_e and B (riaf.hpp:54-96)
+    double ne, thetae, b;
     {
-        const float zc = r_bl * cos_th;
-        const float rcyl = fmaxf(r_bl * sin_th, float(c.min_radius));
-        const float h = fmaxf(float(c.disk_h), 1e-6f);
-        const float vertical = expf(-(zc * zc) / (2.0f * rcyl * rcyl * h * h));
-        ne_norm = float(c.nth0) * vertical * powf(fmaxf(r_bl, float(c.min_radius)), float(c.pow_nth));
+        const double lr = log(r_bl);
+        const double h = max_val(c.disk_h, 1e-6);
+        const double rcyl2 = max_val(r_bl * r_bl * s2, c.min_radius * c.min_radius);
+        const double zc = r_bl * l3;
+        ne = c.nth0 * exp(c.pow_nth * lr - zc * zc * kp_recip<double>(2.0 * rcyl2 * h * h));
+        if (!(float(ne) > 0.0f)) return out;
+        ne *= c.ne_unit;
+        thetae = max_val(c.Te0 * exp(c.pow_T * lr) * c.thetae_unit, c.min_thetae);
+        const double kb = 8.0 * 3.141592653589793 * 0.1 * f32c::kMP * f32c::kCL * f32c::kCL / 6.0;
+        b = max_val(sqrt(max_val(kb * ne * kp_recip<double>(r_bl), 0.0)), 1e-12);
     }
-    if (!(ne_norm > 0.0f)) return out;
     out.emitting = 1;
-    out.ne = ne_norm * float(c.ne_unit);
-    out.thetae = fmaxf(float(c.Te0) * powf(fmaxf(r_bl, float(c.min_radius)), float(c.pow_T)) * float(c.thetae_unit),
-                       float(c.min_thetae));
+    out.ne = float(ne);
+    out.thetae = float(thetae);
+    out.b = float(b);
+    // fluid velocity (riaf.hpp:206-273): circular, with the plunge inside the ISCO
+    double vt = 1.0, vr = 0.0, vphi = 0.0;
     {
-        // B = sqrt(8 pi eps n_e m_p c^2 / (6 r)), eps = 0.1 (riaf.hpp:87-96)
-        const float k = float(8.0 * 3.141592653589793 * 0.1 * f32c::kMP * f32c::kCL * f32c::kCL / 6.0);
-        out.b = fmaxf(sqrtf(fmaxf(k * out.ne / fmaxf(r_bl, float(c.min_radius)), 0.0f)), 1e-12f);
-    }
-    // Kerr-Schild metric at the sample point
-    float g[4][4];
-    {
-        const float z = zz;
-        const float r2 = rc * rc;
-        const float dn = r2 * r2 + a2 * z * z;
-        const float amp = 2.0f * float(c.mass) * r2 * rc / dn;
-        const float r2pa2 = r2 + a2;
-        const float l[4] = {1.0f, (rc * xx + a * yy) / r2pa2, (rc * yy - a * xx) / r2pa2, z / rc};
-#pragma unroll
-        for (int mu = 0; mu < 4; ++mu)
-#pragma unroll
-            for (int nu = 0; nu < 4; ++nu) {
-                const float eta = mu != nu ? 0.0f : (mu == 0 ? -1.0f : 1.0f);
-                g[mu][nu] = eta + amp * l[mu] * l[nu];
-            }
-    }
-    float ucon[4];
-    {
-        const float r = r_bl;
-        float gcov[4][4], gcon[4][4];
-        bl_metric_f(r, sin_th, cos_th, a, gcov, gcon);
-        float vt = 1.0f, vr = 0.0f, vphi = 0.0f;
-        const float kf = float(c.keplerian_factor), inf = float(c.infall_factor);
-        if (r < float(c.horizon)) {
-            vt = kp_rsqrtf(fmaxf(-gcon[0][0], 1e-30f));
-        } else if (r < float(c.isco)) {
-            float gi[4][4], gci[4][4];
-            const float risco = float(c.isco);
-            bl_metric_f(risco, sin_th, cos_th, a, gi, gci);
-            const float omega_isco = 1.0f / (risco * sqrtf(risco) + a);
-            const float qi = gi[0][0] + 2.0f * omega_isco * gi[0][3] + omega_isco * omega_isco * gi[3][3];
-            const float ut_i = kp_rsqrtf(fmaxf(-qi, 1e-30f));
-            const float e = (gi[0][0] + gi[0][3] * omega_isco) * ut_i;
-            const float l = (gi[3][0] + gi[3][3] * omega_isco) * ut_i;
-            const float k_con = gcon[0][0] * e * e + 2.0f * gcon[0][3] * e * l + gcon[3][3] * l * l;
-            const float ur_cov = -sqrtf(fmaxf(-(1.0f + k_con) / fmaxf(gcon[1][1], 1e-30f), 0.0f));
-            const float vr_tmp = gcon[1][1] * ur_cov;
-            const float vt_tmp = gcon[0][0] * e + gcon[0][3] * l;
-            const float vphi_tmp = gcon[3][0] * e + gcon[3][3] * l;
-            const float omega_k = vphi_tmp / fmaxf(vt_tmp, 1e-30f);
-            const float g00 = gcon[0][0];
-            const float omega_ff = gcon[0][3] / (fabsf(g00) > 1e-30f ? g00 : (g00 < 0.0f ? -1e-30f : 1e-30f));
-            const float omega = omega_k + (1.0f - kf) * (omega_ff - omega_k);
-            const float ur_ff = -sqrtf(fmaxf(-(1.0f + gcon[0][0]) * gcon[1][1], 0.0f));
-            vr = vr_tmp + inf * (ur_ff - vr_tmp);
-            const float q = gcov[0][0] + 2.0f * omega * gcov[0][3] + omega * omega * gcov[3][3];
-            vt = sqrtf(fmaxf(-(1.0f + vr * vr * gcov[1][1]) / q, 0.0f));
-            vphi = omega * vt;
+        const double rr = r_bl;
+        const BlEntries m = bl_entries(rr, s2, c2, a);
+        const double kf = c.keplerian_factor, inf = c.infall_factor;
+        if (rr < c.horizon) {
+            vt = kp_recip<double>(sqrt(max_val(-m.itt, 1e-30)));
         } else {
-            const float r_eff = fmaxf(r, float(c.min_radius));
-            const float omega_k = 1.0f / (r_eff * sqrtf(r_eff) + a);
-            const float g00 = gcon[0][0];
-            const float omega_ff = gcon[0][3] / (fabsf(g00) > 1e-30f ? g00 : (g00 < 0.0f ? -1e-30f : 1e-30f));
-            const float omega = omega_k + (1.0f - kf) * (omega_ff - omega_k);
-            vr = inf * -sqrtf(fmaxf(-(1.0f + gcon[0][0]) * gcon[1][1], 0.0f));
-            const float q = gcov[0][0] + 2.0f * omega * gcov[0][3] + omega * omega * gcov[3][3];
-            vt = sqrtf(fmaxf(-(1.0f + vr * vr * gcov[1][1]) / q, 0.0f));
+            double omega;
+            const bool plunge = rr < c.isco;
+            if (plunge) {
+                const double ri = c.isco;
+                const BlEntries mi = bl_entries(ri, s2, c2, a);
+                const double oi = kp_recip<double>(ri * sqrt(ri) + a);
+                const double qi = mi.tt + 2.0 * oi * mi.tp + oi * oi * mi.pp;
+                const double ut = kp_recip<double>(sqrt(max_val(-qi, 1e-30)));
+                const double e = (mi.tt + mi.tp * oi) * ut, l = (mi.tp + mi.pp * oi) * ut;
+                const double kc = m.itt * e * e + 2.0 * m.itp * e * l + m.ipp * l * l;
+                vr = -m.irr * sqrt(max_val(-(1.0 + kc) * kp_recip<double>(max_val(m.irr, 1e-30)), 0.0));
+                omega = (m.itp * e + m.ipp * l) * kp_recip<double>(max_val(m.itt * e + m.itp * l, 1e-30));
+            } else {
+                double sr, isr;
+                kp_sqrt_pair<double>(rr, sr, isr);
+                omega = kp_recip<double>(rr * sr + a);
+            }
+            if (kf != 1.0) {
+                const double g = m.itt;
+                const double off = m.itp * kp_recip<double>(abs_val(g) > 1e-30 ? g : (g < 0.0 ? -1e-30 : 1e-30));
+                omega = omega + (1.0 - kf) * (off - omega);
+            }
+            if (inf != 0.0) {
+                const double ff = -sqrt(max_val(-(1.0 + m.itt) * m.irr, 0.0));
+                vr = plunge ? vr + inf * (ff - vr) : inf * ff;
+            }
+            const double q = m.tt + 2.0 * omega * m.tp + omega * omega * m.pp;
+            vt = sqrt(max_val(-(1.0 + vr * vr * m.rr) * kp_recip<double>(q), 0.0));
             vphi = omega * vt;
         }
-        bl_to_cks_f(vt, vr, vphi, r, sin_th, cos_th, cphi, sphi, a, ucon);
-        const float n2 = dot_gf(g, ucon, ucon);
-        if (n2 < 0.0f) {
-            const float sc = kp_rsqrtf(fmaxf(-n2, 1e-30f));
-            for (int i = 0; i < 4; ++i) ucon[i] *= sc;
-        }
+        const double i_d = kp_recip<double>(max_val(rr * rr - 2.0 * rr + a2, 1e-30));
+        vt += 2.0 * rr * i_d * vr;
+        vphi += a * i_d * vr;
     }
-    float k[4], e1[4], e2[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        k[i] = float(s.k.v[i]);
-        e1[i] = float(s.e1.v[i]);
-        e2[i] = float(s.e2.v[i]);
-    }
-    const float uk = dot_gf(g, ucon, k);
-    out.nu_fluid = fmaxf(fabsf(uk), float(c.min_frequency_scale));
-    // toroidal field unit vector at the raw radius
-    float bcon[4];
+    struct Vec {
+        double t, x, y, z, l;
+    };
+    auto vec = [&](double t, double vx, double vy, double vz) {
+        return Vec{t, vx, vy, vz, t + l1 * vx + l2 * vy + l3 * vz};
+    };
+    auto dot = [&](const Vec& u, const Vec& v) {
+        return u.x * v.x + u.y * v.y + u.z * v.z - u.t * v.t + amp * u.l * v.l;
+    };
+    Vec u = vec(vt, vr * l1 - vphi * y, vr * l2 + vphi * x, vr * l3);
     {
-        float bt[4];
-        bl_to_cks_f(0.0f, 0.0f, 1.0f, rc, sin_th, cos_th, cphi, sphi, a, bt);
-        float ub = dot_gf(g, ucon, bt);
-        for (int i = 0; i < 4; ++i) bcon[i] = bt[i] + ucon[i] * ub;
-        float bsq = dot_gf(g, bcon, bcon);
-        if (!(bsq > 1e-30f)) {
-            const float z4[4] = {0.0f, 0.0f, 0.0f, 1.0f};
-            ub = dot_gf(g, ucon, z4);
-            for (int i = 0; i < 4; ++i) bcon[i] = z4[i] + ucon[i] * ub;
-            bsq = dot_gf(g, bcon, bcon);
-        }
-        if (!(bsq > 1e-30f)) {
-            const float x4[4] = {0.0f, 1.0f, 0.0f, 0.0f};
-            ub = dot_gf(g, ucon, x4);
-            for (int i = 0; i < 4; ++i) bcon[i] = x4[i] + ucon[i] * ub;
-            bsq = dot_gf(g, bcon, bcon);
-        }
-        if (bsq > 1e-30f) {
-            const float sc = kp_rsqrtf(bsq);
-            for (int i = 0; i < 4; ++i) bcon[i] *= sc;
+        const double n2 = dot(u, u);
+        if (n2 < 0.0) {
+            double n, inv;
+            kp_sqrt_pair<double>(max_val(-n2, 1e-30), n, inv);
+            u = Vec{u.t * inv, u.x * inv, u.y * inv, u.z * inv, u.l * inv};
         }
     }
-    const float kdotb = dot_gf(g, k, bcon);
-    out.cos_theta = fminf(fmaxf(kdotb / fmaxf(out.nu_fluid, 1e-30f), -1.0f), 1.0f);
-    out.sin_theta = fmaxf(sqrtf(fmaxf(0.0f, 1.0f - out.cos_theta * out.cos_theta)), float(c.min_sin_theta));
+    const Vec k = vec(s.k.v[0], s.k.v[1], s.k.v[2], s.k.v[3]);
+    const double uk = dot(u, k);
+    const double nu_fluid = max_val(abs_val(uk), c.min_frequency_scale);
+    // toroidal field unit vector, normal to u
+    Vec bv;
+    double bsq;
+    auto project = [&](const Vec& t) {
+        const double ub = dot(u, t);
+        bv = Vec{t.t + u.t * ub, t.x + u.x * ub, t.y + u.y * ub, t.z + u.z * ub, t.l + u.l * ub};
+        bsq = dot(bv, bv);
+    };
+    project(vec(0.0, -y, x, 0.0));
+    if (!(bsq > 1e-30)) project(vec(0.0, 0.0, 0.0, 1.0));
+    if (!(bsq > 1e-30)) project(vec(0.0, 1.0, 0.0, 0.0));
+    if (bsq > 1e-30) {
+        double n, inv;
+        kp_sqrt_pair<double>(bsq, n, inv);
+        bv = Vec{bv.t * inv, bv.x * inv, bv.y * inv, bv.z * inv, bv.l * inv};
+    }
+    const double kb = dot(k, bv);
+    const double ct = min_val(max_val(kb * kp_recip<double>(max_val(nu_fluid, 1e-30)), -1.0), 1.0);
+    out.nu_fluid = float(nu_fluid);
+    out.cos_theta = float(ct);
+    const double st = max_val(sqrt(max_val(0.0, 1.0 - ct * ct)), c.min_sin_theta);
+    out.sin_theta = float(st);
     out.theta = acosf(out.cos_theta);
-    riaf_sample_thermal_f(c, out);
+    riaf_sample_thermal_f(c, out, ne, thetae, b, ct, st, nu_fluid);
     if (out.theta <= 0.0f || out.theta >= f32c::kPi) {
         out.on_axis = 1;
         return out;
     }
-    // screen projections of b (riaf.hpp:320-336)
-    const float eK_s = -1.0f / uk;
-    float eK[4];
-    for (int i = 0; i < 4; ++i) eK[i] = k[i] * eK_s - ucon[i];
-    const bool degenerate = fabsf(uk) <= 1e-30f;
-    const float ub_ = dot_gf(g, ucon, bcon), kb_ = dot_gf(g, eK, bcon);
-    const float b1 = dot_gf(g, e1, bcon) + (degenerate ? 0.0f : dot_gf(g, ucon, e1) * ub_ - dot_gf(g, eK, e1) * kb_);
-    const float b2 = dot_gf(g, e2, bcon) + (degenerate ? 0.0f : dot_gf(g, ucon, e2) * ub_ - dot_gf(g, eK, e2) * kb_);
-    const float bproj2 = b1 * b1 + b2 * b2;
-    if (bproj2 > 1e-30f) {
+    // screen projections of b (riaf.hpp:320-336) with eK = -k / (u.k) - u
+    const Vec e1 = vec(s.e1.v[0], s.e1.v[1], s.e1.v[2], s.e1.v[3]);
+    const Vec e2 = vec(s.e2.v[0], s.e2.v[1], s.e2.v[2], s.e2.v[3]);
+    double b1 = dot(e1, bv), b2 = dot(e2, bv);
+    if (abs_val(uk) > 1e-30) {
+        const double iu = -kp_recip<double>(uk);
+        const double ub = dot(u, bv), Kb = kb * iu - ub;
+        const double ue1 = dot(u, e1), ue2 = dot(u, e2);
+        b1 += ue1 * ub - (dot(k, e1) * iu - ue1) * Kb;
+        b2 += ue2 * ub - (dot(k, e2) * iu - ue2) * Kb;
+    }
+    const double bproj2 = b1 * b1 + b2 * b2;
+    if (bproj2 > 1e-30) {
+        const double inv = kp_recip<double>(bproj2);
         out.has_chi = 1;
-        out.cos2chi = (b2 * b2 - b1 * b1) / bproj2;
-        out.sin2chi = -2.0f * b1 * b2 / bproj2;
+        out.cos2chi = float((b2 * b2 - b1 * b1) * inv);
+        out.sin2chi = float(-2.0 * b1 * b2 * inv);
     }
     return out;
 }
@@ -416,25 +390,23 @@ KP_HD CoeffsF riaf_coefficients_f(const ImageConsts& c, const RiafSampleF& p, fl
     const float ne = p.ne, te = p.thetae, b = p.b;
     const float st = fmaxf(p.sin_theta, float(c.min_sin_theta));
     const float ct = p.cos_theta;
+    const double freq = double(freq_ghz) * 1e9;
     // Faraday rotation / conversion (symphony_rho_QV), invariant rho * nu
-    float rQ, rV;
+    float rQ;
+    double rV;
     {
         const float omega0 = f32c::kOmega0PerB * b;
         const float wp2 = f32c::kWp2PerNe * ne;
-        const float two_pi_nu = 2.0f * f32c::kPi * nu * 1e9f;
-        const float sst = p.on_axis ? fmaxf(sinf(p.theta), float(c.min_sin_theta)) : st;
-        const float x = fmaxf(te * sqrtf(fmaxf(0.0f, 1.41421356f * sst * (1e3f * omega0 / two_pi_nu))), 1e-12f);
-        const float inv_w = 1.0f / two_pi_nu;
-        // eps12 = wp2 omega0 / (2 pi nu)^3 ; rho_V = 2 pi nu / c * eps12 ; inv = rho_V * nu
-        const float shgm = 1.0f - 0.11f * logf(1.0f + 0.035f * x);
-        const float cosv = p.on_axis ? cosf(p.theta) : ct;
-        float e12 = wp2 * omega0 * inv_w;
-        e12 *= inv_w;
-        e12 *= inv_w;
-        e12 *= p.r0 * shgm * cosv;
-        rV = float(2.0 * 3.141592653589793 / f32c::kCL) * (nu * 1e9f) * e12 * (nu * 1e9f);
+        const float inv_w = 1.0f / (2.0f * f32c::kPi * nu * 1e9f);
+        double sf, isf;
+        kp_sqrt_pair<double>(freq, sf, isf);
+        const double xd = max_val(p.xf0 * isf, 1e-12);
+        // eps12 = wp2 omega0 / (2 pi nu)^3 K0/K2 fit cos(theta); rho_V = 2 pi nu / c eps12;
+        // the invariant is rho_V nu (on the axis cos(theta) is 1 or -1 to rounding)
+        rV = p.rv0 * (1.0 - 0.11 * log(1.0 + 0.035 * xd)) * (isf * isf);
+        const float x = float(xd);
         if (p.on_axis) {
-            o.rV = float(c.faraday_scale) * rV;
+            o.rV = c.faraday_scale * rV;
             return o;
         }
         // every power of x from one LG2; 0.5 + 0.5 tanh(z) = 1 / (1 + e^-2z)
@@ -457,10 +429,9 @@ KP_HD CoeffsF riaf_coefficients_f(const ImageConsts& c, const RiafSampleF& p, fl
     float jI, jQ, jV;
     const float inv_nu2 = escale / (nu * nu) * 1e-18f;  // 2^E / (nu_Hz^2)
     if (c.fit == 4) {
-        const float nus = f32c::kDexNus * b * st * te * te + 1.0f / 1e9f * 1e9f;  // + 1 Hz
-        const float xh = fmaxf(nu * 1e9f / fmaxf(nus, 1e-30f), 1e-30f);
-        const float xm13 = 1.0f / cbrtf(xh);
-        const float exps = expf(-1.8899f / xm13);
+        const double xd = max_val(p.xs0 * freq, 1e-30), root = cube_root(xd);
+        const float xh = float(xd), xm13 = float(kp_recip<double>(root));
+        const float exps = float(exp(-1.8899 * root));
         const float pref = f32c::kDexPref * ne * (nu * 1e9f) / (te * te);
         jI = pref * (2.5651f * (1.0f + 1.92f * xm13 + 0.9977f * xm13 * xm13) * exps) * inv_nu2;
         jQ = pref * (2.5651f * (1.0f + 0.93193f * xm13 + 0.499873f * xm13 * xm13) * exps) * inv_nu2;
@@ -471,13 +442,12 @@ KP_HD CoeffsF riaf_coefficients_f(const ImageConsts& c, const RiafSampleF& p, fl
         jV = f32c::kDexPrefV * ne * (nu * 1e9f) / (tan_theta * te * te * te) * iv * inv_nu2;
     } else {
         const float nu_c = f32c::kNuCPerB * b;
-        const float nu_s = 2.0f / 9.0f * nu_c * st * te * te;
-        const float x = fmaxf(nu * 1e9f / fmaxf(nu_s, 1e-30f), 1e-30f);
+        const double xd = max_val(p.xs0 * freq, 1e-30), root = cube_root(xd);
+        const float x = float(xd), x13 = float(root);
         const float pref = ne * f32c::kE2OverC * nu_c * f32c::kTerm1 * st;
         const float lx = log2f(x);
-        const float x13 = pow2_of(1.0f / 3.0f, lx);
         const float sqx = sqrtf(x), sqx13 = sqrtf(x13);
-        const float ex13 = expf(-x13);
+        const float ex13 = float(exp(-root));
         const float sh = sqx + 1.8877486253633869933f * sqx13;
         jI = pref * (sh * sh) * ex13 * inv_nu2;
         const float shq = sqx + p.qterm * 1.8877486253633869933f * sqx13;
@@ -510,7 +480,7 @@ KP_HD CoeffsF riaf_coefficients_f(const ImageConsts& c, const RiafSampleF& p, fl
     o.jV = es * jV;
     o.aI = as * aI;
     o.aV = as * aV;
-    o.rV = fs * rV;
+    o.rV = c.faraday_scale * rV;
     if (p.has_chi) {
         o.jQ = es * jQ * p.cos2chi;
         o.jU = es * jQ * p.sin2chi;
@@ -523,107 +493,123 @@ KP_HD CoeffsF riaf_coefficients_f(const ImageConsts& c, const RiafSampleF& p, fl
 }
 
 // ---- transfer -----------------------------------------------------------
-KP_HD float atten_f(float kappa, float dl) {
-    const float x = kappa * dl;
-    if (x > 87.0f) return 0.0f;
-    return expf(-x);
-}
+// The Strang step in FP64 on FP32 coefficients.  A Faraday-thick ray turns
+// its polarisation through thousands of radians and what is left of it is a
+// small difference of large contributions: rounding the Stokes vector, the
+// rotation or the attenuation to single precision at every step was the
+// largest error of the mixed policy (1e-6 of I, 1e-5 to 1e-3 of Q and U;
+// in FP64 6e-8 and 1e-6 to 1e-5, from the coefficients).
+struct StokesM {
+    double I, Q, U, V;  // scaled by 2^E
+};
 
-KP_HD float source_f(float kappa, float dl) {
-    const float x = kappa * dl;
-    if (fabsf(x) < 1e-3f) return dl * (1.0f - x * (0.5f - x * (1.0f / 6.0f - x * (1.0f / 24.0f))));
-    return -expm1f(-x) / kappa;
-}
-
-// s = a + b with the rounding error accumulated into c (TwoSum).
-KP_HD float two_sum_acc(float a, float b, float& c) {
-    const float s = a + b;
-    const float bb = s - a;
-    c += (a - (s - bb)) + (b - bb);
-    return s;
-}
-
-KP_HD void faraday_rotate_f(StokesF& s, const CoeffsF& c, float dl) {
-    const float rn = sqrtf(c.rQ * c.rQ + c.rU * c.rU + c.rV * c.rV);
-    if (rn == 0.0f || dl == 0.0f) return;
-    // fold the compensation in before rotating
-    const float px = s.Q + s.cQ, py = s.U + s.cU, pz = s.V + s.cV;
-    s.cQ = s.cU = s.cV = 0.0f;
-    const float theta = rn * dl;
-    float ox, oy, oz;
-    if (fabsf(theta) < 1e-4f) {
-        ox = px + (c.rU * pz - c.rV * py) * dl;
-        oy = py + (c.rV * px - c.rQ * pz) * dl;
-        oz = pz + (c.rQ * py - c.rU * px) * dl;
-    } else {
-        const float inv = 1.0f / rn;
-        const float nx = c.rQ * inv, ny = c.rU * inv, nz = c.rV * inv;
-        // half-angle forms: 1 - cos(theta) = 2 sin^2(theta/2) keeps its
-        // relative accuracy for small rotations
-        float sh, ch;
-        kp_sincos_small(0.5f * theta, &sh, &ch);
-        const float st = 2.0f * sh * ch;
-        const float omc = 2.0f * sh * sh;
-        const float ct = 1.0f - omc;
-        const float f = (nx * px + ny * py + nz * pz) * omc;
-        ox = px * ct + nx * f + (ny * pz - nz * py) * st;
-        oy = py * ct + ny * f + (nz * px - nx * pz) * st;
-        oz = pz * ct + nz * f + (nx * py - ny * px) * st;
-    }
-    s.Q = ox;
-    s.U = oy;
-    s.V = oz;
-}
-
-KP_HD void absorb_emit_f(StokesF& s, const CoeffsF& c, float dl) {
-    const float an = sqrtf(c.aQ * c.aQ + c.aU * c.aU + c.aV * c.aV);
-    const float I = s.I + s.cI, Q = s.Q + s.cQ, U = s.U + s.cU, V = s.V + s.cV;
-    if (an < 1e-30f) {
-        const float e = atten_f(c.aI, dl);
-        const float f = source_f(c.aI, dl);
-        float ci = 0.f, cq = 0.f, cu = 0.f, cv = 0.f;
-        s.I = two_sum_acc(e * I, f * c.jI, ci);
-        s.Q = two_sum_acc(e * Q, f * c.jQ, cq);
-        s.U = two_sum_acc(e * U, f * c.jU, cu);
-        s.V = two_sum_acc(e * V, f * c.jV, cv);
-        s.cI = ci;
-        s.cQ = cq;
-        s.cU = cu;
-        s.cV = cv;
+// e^-x - 1 and (1 - e^-x) / kappa for x = kappa dl.
+KP_HD void fade_and_source(double kappa, double dl, double& em1, double& src) {
+    const double x = kappa * dl;
+    if (fabs(x) < 0.0625) {
+        // (1 - e^-x) / x to the x^8 term
+        double p = -1.0 / 362880.0 * x + 1.0 / 40320.0;
+        p = 1.0 / 5040.0 - x * p;
+        p = 1.0 / 720.0 - x * p;
+        p = 1.0 / 120.0 - x * p;
+        p = 1.0 / 24.0 - x * p;
+        p = 1.0 / 6.0 - x * p;
+        p = 0.5 - x * p;
+        p = 1.0 - x * p;
+        src = dl * p;
+        em1 = -x * p;
         return;
     }
-    const float inv = 1.0f / an;
-    const float nx = c.aQ * inv, ny = c.aU * inv, nz = c.aV * inv;
-    const float p_par = nx * Q + ny * U + nz * V;
-    const float j_par = nx * c.jQ + ny * c.jU + nz * c.jV;
-    const float ppx = Q - nx * p_par, ppy = U - ny * p_par, ppz = V - nz * p_par;
-    const float jpx = c.jQ - nx * j_par, jpy = c.jU - ny * j_par, jpz = c.jV - nz * j_par;
-    const float kp = c.aI + an, km = c.aI - an;
-    float csp = 0.f, csm = 0.f;
-    const float sp = two_sum_acc(atten_f(kp, dl) * (I + p_par), source_f(kp, dl) * (c.jI + j_par), csp);
-    const float sm = two_sum_acc(atten_f(km, dl) * (I - p_par), source_f(km, dl) * (c.jI - j_par), csm);
-    const float ei = atten_f(c.aI, dl), fi = source_f(c.aI, dl);
-    float cx = 0.f, cy = 0.f, cz = 0.f;
-    const float ox = two_sum_acc(ppx * ei, jpx * fi, cx);
-    const float oy = two_sum_acc(ppy * ei, jpy * fi, cy);
-    const float oz = two_sum_acc(ppz * ei, jpz * fi, cz);
-    const float spc = sp + csp, smc = sm + csm;
-    s.I = 0.5f * (spc + smc);
-    const float par = 0.5f * (spc - smc);
-    float c2x = 0.f, c2y = 0.f, c2z = 0.f;
-    s.Q = two_sum_acc(nx * par, ox, c2x);
-    s.U = two_sum_acc(ny * par, oy, c2y);
-    s.V = two_sum_acc(nz * par, oz, c2z);
-    s.cI = 0.0f;
-    s.cQ = cx + c2x;
-    s.cU = cy + c2y;
-    s.cV = cz + c2z;
+    em1 = x > 700.0 ? -1.0 : expm1(-x);
+    src = -em1 / kappa;
 }
 
-KP_HD void stokes_step_f(StokesF& s, const CoeffsF& c, float dl) {
-    faraday_rotate_f(s, c, 0.5f * dl);
-    absorb_emit_f(s, c, dl);
-    faraday_rotate_f(s, c, 0.5f * dl);
+// The Faraday rotation of one half step: axis n, sin and 1 - cos of its
+// angle |rho| dl / 2, from the half angle reduced by its period pi.  Both half
+// steps of a Strang step are this rotation.
+struct RotationM {
+    double nx, ny, nz, st, omc;
+    int none;
+};
+
+KP_HD void kp_sincospi(double u, double* s, double* c) {
+#ifdef __CUDA_ARCH__
+    sincospi(u, s, c);
+#else
+    *s = sin(3.14159265358979323846 * u);
+    *c = cos(3.14159265358979323846 * u);
+#endif
+}
+
+KP_HD RotationM faraday_rotation(const CoeffsF& c, double dl) {
+    RotationM r;
+    const double rq = c.rQ, ru = c.rU, rv = c.rV;
+    const double n2 = rq * rq + ru * ru + rv * rv;
+    r.none = !(n2 > 0.0) || dl == 0.0;
+    if (r.none) return r;
+    double n, inv;
+    if (n2 > 1e-280 && n2 < 1e280) {
+        kp_sqrt_pair<double>(n2, n, inv);
+    } else {
+        n = sqrt(n2);
+        inv = 1.0 / n;
+    }
+    r.nx = rq * inv;
+    r.ny = ru * inv;
+    r.nz = rv * inv;
+    double sh, ch;
+    kp_sincospi(n * dl * (0.25 / 3.14159265358979323846), &sh, &ch);
+    r.st = 2.0 * sh * ch;
+    r.omc = 2.0 * sh * sh;
+    return r;
+}
+
+// P + (n x P) sin + (n (n.P) - P) (1 - cos)
+KP_HD void faraday_rotate(StokesM& s, const RotationM& r) {
+    if (r.none) return;
+    const double px = s.Q, py = s.U, pz = s.V;
+    const double f = r.nx * px + r.ny * py + r.nz * pz;
+    s.Q = px + ((r.ny * pz - r.nz * py) * r.st + (r.nx * f - px) * r.omc);
+    s.U = py + ((r.nz * px - r.nx * pz) * r.st + (r.ny * f - py) * r.omc);
+    s.V = pz + ((r.nx * py - r.ny * px) * r.st + (r.nz * f - pz) * r.omc);
+}
+
+KP_HD void absorb_emit(StokesM& s, const CoeffsF& c, double dl) {
+    const double aq = c.aQ, au = c.aU, av = c.aV, ai = c.aI;
+    const double jq = c.jQ, ju = c.jU, jv = c.jV, ji = c.jI;
+    const double n2 = aq * aq + au * au + av * av;
+    double em, src;
+    fade_and_source(ai, dl, em, src);
+    if (n2 < 1e-60) {
+        s.I = s.I + (em * s.I + src * ji);
+        s.Q = s.Q + (em * s.Q + src * jq);
+        s.U = s.U + (em * s.U + src * ju);
+        s.V = s.V + (em * s.V + src * jv);
+        return;
+    }
+    double an, inv;
+    kp_sqrt_pair<double>(n2, an, inv);
+    const double nx = aq * inv, ny = au * inv, nz = av * inv;
+    const double par = nx * s.Q + ny * s.U + nz * s.V;
+    const double jpar = nx * jq + ny * ju + nz * jv;
+    double emp, srcp, emm, srcm;
+    fade_and_source(ai + an, dl, emp, srcp);
+    fade_and_source(ai - an, dl, emm, srcm);
+    // changes of I + P_par, I - P_par and of the part of P across n
+    const double dp = emp * (s.I + par) + srcp * (ji + jpar);
+    const double dm = emm * (s.I - par) + srcm * (ji - jpar);
+    const double dpar = 0.5 * (dp - dm);
+    s.I += 0.5 * (dp + dm);
+    s.Q += nx * dpar + (em * (s.Q - nx * par) + src * (jq - nx * jpar));
+    s.U += ny * dpar + (em * (s.U - ny * par) + src * (ju - ny * jpar));
+    s.V += nz * dpar + (em * (s.V - nz * par) + src * (jv - nz * jpar));
+}
+
+KP_HD void stokes_step_m(StokesM& s, const CoeffsF& c, double dl) {
+    const RotationM r = faraday_rotation(c, dl);
+    faraday_rotate(s, r);
+    absorb_emit(s, c, dl);
+    faraday_rotate(s, r);
 }
 
 }  // namespace kp

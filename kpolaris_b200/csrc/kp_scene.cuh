@@ -22,13 +22,16 @@
 namespace kp {
 
 // Mixed policy marker types live in kp_engine.cuh; the scenes only need to
-// know whether FP32 contraction was requested.
-template<bool MIXED, bool FP32>
+// know whether the mixed policy's form was requested.
+template<bool MIXED>
 __device__ __forceinline__ Ray riaf_rhs(double mass, double spin, const Ray& X) {
-    if constexpr (MIXED && FP32) return ks_rhs_factored<float>(mass, spin, X);
-    else if constexpr (MIXED) return ks_rhs_factored<double>(mass, spin, X);
+    if constexpr (MIXED) return ks_rhs_factored<double>(mass, spin, X);
     else return ks_rhs(mass, spin, X);
 }
+
+struct KerrGeo {
+    double mass, spin;
+};
 
 struct SceneRiaf {
     static constexpr bool kSlowLight = false;
@@ -40,9 +43,33 @@ struct SceneRiaf {
         __device__ double dot(const D4& u, const D4& v) const { return ks_dot_at(w, u, v); }
     };
     __device__ static double radius(const ImageConsts& c, const D4& X) { return ks_radius(c.spin, X); }
-    template<bool MIXED, bool FP32>
+    // radius of a loop top: the same bits at every call site
+    template<bool MIXED>
+    __device__ static double top_radius(const ImageConsts& c, const D4& X) {
+        if constexpr (MIXED) return ks_radius_refined(c.spin, X);
+        else return ks_radius(c.spin, X);
+    }
+    template<bool MIXED>
     __device__ static Ray rhs(const ImageConsts& c, const Ray& X) {
-        return riaf_rhs<MIXED, FP32>(c.mass, c.spin, X);
+        return riaf_rhs<MIXED>(c.mass, c.spin, X);
+    }
+    // what a transport needs of the image, and one transport: -Gamma(k, q) at
+    // position x
+    using Geo = KerrGeo;
+    __device__ static Geo geo(const ImageConsts& c) { return KerrGeo{c.mass, c.spin}; }
+    template<bool MIXED>
+    __device__ static D4 transport(const Geo& c, const D4& x, const D4& k, const D4& q) {
+        if constexpr (MIXED) {
+            const KsFactored<double> w = ks_factored_conn<double>(c.mass, c.spin, x.v[1], x.v[2], x.v[3]);
+            const KsFactoredK<double> p = ks_factored_k<double>(w, k.v);
+            D4 d;
+            ks_factored_contract<double>(w, p, q.v, d.v);
+            return d;
+        } else {
+            const KSConn w = ks_conn(c.mass, c.spin, x);
+            const D4 g = ks_contract(w, k, q);
+            return d4(-g.v[0], -g.v[1], -g.v[2], -g.v[3]);
+        }
     }
     __device__ static Ray camera(const ImageConsts& c, const CameraFrame& f, int pixel) {
         return camera_ray(c, f, pixel);
@@ -99,9 +126,19 @@ struct SceneRiafBL {
         __device__ double dot(const D4& u, const D4& v) const { return bl_dot_at(p, u, v); }
     };
     __device__ static double radius(const ImageConsts&, const D4& X) { return X.v[1]; }
-    template<bool MIXED, bool FP32>
+    template<bool MIXED>
+    __device__ static double top_radius(const ImageConsts&, const D4& X) { return X.v[1]; }
+    template<bool MIXED>
     __device__ static Ray rhs(const ImageConsts& c, const Ray& X) {
         return bl_rhs(c.mass, c.spin, X);
+    }
+    using Geo = KerrGeo;
+    __device__ static Geo geo(const ImageConsts& c) { return KerrGeo{c.mass, c.spin}; }
+    template<bool MIXED>
+    __device__ static D4 transport(const Geo& c, const D4& x, const D4& k, const D4& q) {
+        const BLConnWork w = bl_conn_work(c.mass, c.spin, x);
+        const D4 g = bl_contract(w, k, q);
+        return d4(-g.v[0], -g.v[1], -g.v[2], -g.v[3]);
     }
     __device__ static Ray camera(const ImageConsts& c, const CameraFrame& f, int pixel) {
         return bl_camera_ray(c, f, pixel);
@@ -159,14 +196,26 @@ struct SceneGrmhd {
         __device__ double dot(const D4& u, const D4& v) const { return dot_gm(g, u, v); }
     };
     __device__ static double radius(const ImageConsts&, const D4& X) { return fmks_radius(X); }
+    template<bool MIXED>
+    __device__ static double top_radius(const ImageConsts&, const D4& X) { return fmks_radius(X); }
     // FP64 everywhere (an FP32 FMKS connection puts its rounding noise into
     // the step-doubling error norm); the mixed policy uses the factored form
-    template<bool MIXED, bool FP32>
+    template<bool MIXED>
     __device__ static Ray rhs(const ImageConsts& c, const Ray& X) {
         if constexpr (MIXED) {
             return fmks_rhs_factored(c.fmks, X);
         } else {
             return fmks_rhs(c.fmks, X);
+        }
+    }
+    using Geo = FmksParams;
+    __device__ static Geo geo(const ImageConsts& c) { return c.fmks; }
+    template<bool MIXED>
+    __device__ static D4 transport(const Geo& c, const D4& x, const D4& k, const D4& q) {
+        if constexpr (MIXED) {
+            return fmks_factored_contract(fmks_factored_conn(c, x), k, q);
+        } else {
+            return fmks_contract(fmks_conn(c, x), k, q);
         }
     }
     __device__ static Ray camera(const ImageConsts& c, const CameraFrame& f, int pixel) {
@@ -192,8 +241,8 @@ struct SceneGrmhdSlow : SceneGrmhd {
 
 // A GRMHD scene as the mixed policy's far kernel runs it: beyond the
 // radiating sphere no plasma is sampled, so the ray is integrated in
-// Cartesian Kerr-Schild (the RIAF scene's FP32 stage chains, with the
-// policy's step control) and converted at the phase boundary
+// Cartesian Kerr-Schild (the RIAF scene's far phase) and converted at the
+// phase boundary
 // (kp_chart.cuh).  Records, cameras and the end of a ray stay in FMKS:
 // to_phase converts a claimed ray, to_record converts it back before it is
 // parked or finished.  Phase decisions use the radius its record will hold.
@@ -211,10 +260,23 @@ struct SceneFarCks : Base {
     __device__ static double radius(const ImageConsts& c, const D4& X) {
         return chart_active(c) ? cks_record_radius(c.spin, X) : Base::radius(c, X);
     }
-    // reached only with the chart inactive (the active chart runs far_job_f)
-    template<bool MIXED, bool FP32>
-    __device__ static Ray rhs(const ImageConsts& c, const Ray& X) {
-        return Base::template rhs<MIXED, false>(c, X);
+    // records and near kernels hold exp(log r) as the radius: so does the chart
+    template<bool MIXED>
+    __device__ static double top_radius(const ImageConsts& c, const D4& X) {
+        return radius(c, X);
+    }
+    struct Geo {
+        KerrGeo kerr;
+        typename Base::Geo base;
+        int cks;
+    };
+    __device__ static Geo geo(const ImageConsts& c) {
+        return Geo{KerrGeo{c.mass, c.spin}, Base::geo(c), chart_active(c)};
+    }
+    template<bool MIXED>
+    __device__ static D4 transport(const Geo& c, const D4& x, const D4& k, const D4& q) {
+        if (c.cks) return SceneRiaf::template transport<MIXED>(c.kerr, x, k, q);
+        return Base::template transport<MIXED>(c.base, x, k, q);
     }
     // out of line: conversions happen a few times per ray, and inlined at
     // each claim, park and finish site they crowd the kernel's registers

@@ -149,6 +149,52 @@ __device__ __forceinline__ int radiation_substep_count(const C& co, double h, do
     return nsub;
 }
 
+#ifdef __CUDACC__
+// The same count in closed form: the depths of a unit dl, then for each limit
+// the smallest power of two n (at most 4096) with depth <= lim n.  For two
+// positive normal numbers n is the ratio of their binades, doubled if the
+// depth's significand is the larger; anything else takes the loop.
+struct RadDepths {
+    double a, r, dls;  // absorption and Faraday depth per dl; |dls|
+};
+
+__device__ __forceinline__ RadDepths radiation_depths(const Coeffs<double>& co, double dls) {
+    return RadDepths{abs_val(co.aI) + sqrt(co.aQ * co.aQ + co.aU * co.aU + co.aV * co.aV),
+                     sqrt(co.rQ * co.rQ + co.rU * co.rU + co.rV * co.rV), abs_val(dls)};
+}
+
+__device__ __forceinline__ int pow2_steps(double depth, double lim) {
+    if (!(depth > lim)) return 1;
+    const unsigned long long d = (unsigned long long)__double_as_longlong(depth);
+    const unsigned long long l = (unsigned long long)__double_as_longlong(lim);
+    const int ed = int(d >> 52), el = int(l >> 52);
+    if (el == 0) {
+        int n = 1;
+        while (depth > lim * double(n) && n < 4096) n *= 2;
+        return n;
+    }
+    const unsigned long long frac = (1ull << 52) - 1;
+    const int e = ed - el + ((d & frac) > (l & frac) ? 1 : 0);
+    return 1 << (e > 12 ? 12 : e);
+}
+
+__device__ __forceinline__ int substeps_for(const RadDepths& p, double h, double max_rad_step, const ImageConsts& c) {
+    const double abs_h = abs_val(h);
+    int n = max_rad_step > 0.0 ? pow2_steps(abs_h, max_rad_step) : 1;
+    const double dl = abs_h * p.dls;
+    const double alim = c.max_absorption_depth >= 0.0 ? c.max_absorption_depth : c.max_radiation_depth;
+    if (alim > 0.0) n = max(n, pow2_steps(p.a * dl, alim));
+    const double flim = c.max_faraday_depth >= 0.0 ? c.max_faraday_depth : c.max_radiation_depth;
+    if (flim > 0.0) n = max(n, pow2_steps(p.r * dl, flim));
+    return n;
+}
+
+// h / n for a power of two n <= 4096, as the exact product with 1 / n.
+__device__ __forceinline__ double over_pow2(double h, int n) {
+    return h * __longlong_as_double((long long)(1023 - (31 - __clz(n))) << 52);
+}
+#endif
+
 struct PixelOut {
     double r11, r12, r21, r22;
     double closure_x, closure_k, final_null, frame_error;

@@ -1,0 +1,166 @@
+// Host check of the far field's bridged runs of steps (macro_run in
+// kpolaris_b200/csrc/kp_far_steps.cuh) against the step control itself, in
+// FP64 with the reference's transport.  Rays of a pinhole camera at several
+// radii, seeded.  Prints
+//   the largest step-doubling error of a run's steps over the bound macro_run
+//   takes for it,
+//   the number of runs, and of runs that the step control does not take
+//   (another step size, a step from or into the near phase, past the camera
+//   or, in pass A, outward),
+//   the largest distance (over max(1, |.|)) between the extrapolated midpoint
+//   rule over a run and the steps themselves.
+#include <cmath>
+#include <cstdio>
+#include <cstring>
+#include <random>
+#define __host__
+#define __device__
+#define __forceinline__ inline
+#define __noinline__
+#include "kp_far_steps.cuh"
+#include "kp_geometry.cuh"
+
+using namespace kp;
+
+static Ray axpy(const Ray& y, double a, const Ray& x) {
+    Ray o;
+    const double* p = reinterpret_cast<const double*>(&y);
+    const double* q = reinterpret_cast<const double*>(&x);
+    double* r = reinterpret_cast<double*>(&o);
+    for (int i = 0; i < 16; ++i) r[i] = p[i] + a * q[i];
+    return o;
+}
+
+static Ray rk4(double M, double a, const Ray& s, double h) {
+    const Ray k1 = ks_rhs(M, a, s), k2 = ks_rhs(M, a, axpy(s, 0.5 * h, k1));
+    const Ray k3 = ks_rhs(M, a, axpy(s, 0.5 * h, k2)), k4 = ks_rhs(M, a, axpy(s, h, k3));
+    return axpy(axpy(axpy(axpy(s, h / 6.0, k1), h / 3.0, k2), h / 3.0, k3), h / 6.0, k4);
+}
+
+static double distance(const Ray& a, const Ray& b) {
+    const double* p = reinterpret_cast<const double*>(&a);
+    const double* q = reinterpret_cast<const double*>(&b);
+    double d = 0.0;
+    for (int i = 0; i < 16; ++i)
+        d = std::fmax(d, std::fabs(p[i] - q[i]) / std::fmax(1.0, std::fmax(std::fabs(p[i]), std::fabs(q[i]))));
+    return d;
+}
+
+// Gragg's midpoint rule with 2, 4, 6, 8 substeps, extrapolated.
+static Ray midpoint(double M, double a, const Ray& s, double H) {
+    const Ray f0 = ks_rhs(M, a, s);
+    Ray T[4], P[4];
+    for (int j = 0; j < 4; ++j) {
+        const int n = 2 * j + 2;
+        const double h = H / n;
+        Ray z0 = s, z1 = axpy(s, h, f0);
+        for (int i = 1; i < n; ++i) {
+            const Ray z2 = axpy(z0, 2.0 * h, ks_rhs(M, a, z1));
+            z0 = z1;
+            z1 = z2;
+        }
+        Ray t = axpy(axpy(axpy(z1, h, ks_rhs(M, a, z1)), 1.0, z0), 0.0, z0);
+        double* v = reinterpret_cast<double*>(&t);
+        for (int i = 0; i < 16; ++i) v[i] *= 0.5;
+        T[0] = t;
+        for (int k = 1; k <= j; ++k) {
+            const double q = double(n) / (2.0 * (j - k) + 2.0);
+            T[k] = axpy(axpy(T[k - 1], 1.0 / (q * q - 1.0), T[k - 1]), -1.0 / (q * q - 1.0), P[k - 1]);
+        }
+        for (int k = 0; k <= j; ++k) P[k] = T[k];
+    }
+    return P[3];
+}
+
+int main() {
+    std::mt19937_64 rng(20260101);
+    std::uniform_real_distribution<double> u(0.0, 1.0);
+    double worst_const = 0.0, worst_dist = 0.0;
+    int runs = 0, wrong = 0;
+    for (int ray = 0; ray < 400; ++ray) {
+        ImageConsts c;
+        std::memset(&c, 0, sizeof(c));
+        c.mass = 1.0;
+        c.spin = 0.99 * u(rng);
+        c.adaptive = ray % 4 != 3;
+        c.max_step = ray % 4 == 1 ? 0.7 : (ray % 4 == 2 ? 5.0 : 2.0);
+        c.step = ray % 4 == 3 ? 1.0 : 0.025;
+        c.tolerance = ray % 4 == 2 ? 1e-6 : 1e-8;
+        c.outer_radius = 50.0 + 65.0 * u(rng);
+        c.fp32_radius = c.outer_radius + 2.0 * std::fmax(c.max_step, c.step);
+        c.cam_radius = 200.0 + 1800.0 * u(rng);
+        // a ray through the camera's radius at some impact parameter, its
+        // wavevector null in the Kerr-Schild metric to first order
+        const double r = c.cam_radius, b = 400.0 * (u(rng) - 0.5), th = std::acos(2.0 * u(rng) - 1.0), ph = 6.28 * u(rng);
+        const double n[3] = {std::sin(th) * std::cos(ph), std::sin(th) * std::sin(ph), std::cos(th)};
+        double e[3] = {n[1], -n[0], 0.0};
+        const double en = std::sqrt(e[0] * e[0] + e[1] * e[1]) + 1e-300;
+        Ray s;
+        const double out = std::sqrt(r * r - b * b);
+        for (int i = 0; i < 3; ++i) {
+            s.x.v[i + 1] = out * n[i] + b * e[i] / en;
+            s.k.v[i + 1] = n[i];
+            s.e1.v[i + 1] = e[i] / en;
+        }
+        s.x.v[0] = 0.0;
+        s.k.v[0] = 1.0 + 2.0 / r;
+        s.e1.v[0] = s.e2.v[0] = 0.0;
+        for (int i = 0; i < 3; ++i) {
+            const int p = (i + 1) % 3, q = (i + 2) % 3;
+            s.e2.v[i + 1] = n[p] * s.e1.v[q + 1] - n[q] * s.e1.v[p + 1];
+        }
+        for (int pass = 0; pass < 2; ++pass) {
+            // pass A: backward from the camera; pass B: forward from where A stopped
+            const double dir = pass == 0 ? -1.0 : 1.0;
+            const double cap = c.adaptive ? c.max_step : c.step;
+            double h = c.step;
+            if (pass == 1) h = cap;
+            const double rr = ks_radius(c.spin, s.x);
+            if (pass == 1 && !(rr > c.fp32_radius)) break;
+            for (int guard = 0; guard < 60; ++guard) {
+                const double r0 = ks_radius(c.spin, s.x);
+                if (!(r0 > c.fp32_radius)) break;
+                double xk = 0.0, kk = 0.0;
+                for (int i = 1; i < 4; ++i) {
+                    xk += s.x.v[i] * s.k.v[i];
+                    kk += s.k.v[i] * s.k.v[i];
+                }
+                const MacroRun run = macro_run(c, r0, xk, std::sqrt(kk), h, cap, dir, pass == 0, 100000);
+                if (run.count < 3) break;
+                ++runs;
+                const Ray far = midpoint(c.mass, c.spin, s, dir * run.length);
+                double len = 0.0, hh = h, old = r0;
+                bool ok = true;
+                for (int k = 0; k < run.count; ++k) {
+                    const double rk = ks_radius(c.spin, s.x);
+                    ok = ok && rk > c.fp32_radius;
+                    const Ray full = rk4(c.mass, c.spin, s, dir * hh);
+                    const Ray half = rk4(c.mass, c.spin, s, 0.5 * dir * hh);
+                    const Ray two = rk4(c.mass, c.spin, half, 0.5 * dir * hh);
+                    const double err = distance(full, two);
+                    worst_const = std::fmax(
+                        worst_const, err / ((16.0 + 0.25 * rk) * std::pow(hh, 5) / std::pow(rk, 6) + 1e-14));
+                    s = c.adaptive ? two : full;
+                    len += hh;
+                    if (c.adaptive) {
+                        ok = ok && err <= c.tolerance;
+                        double f = err > 0.0 ? 0.9 * std::pow(c.tolerance / err, 0.2) : 2.0;
+                        f = std::fmin(2.0, std::fmax(0.2, f));
+                        hh = std::fmin(c.max_step, hh * f);
+                    }
+                    const double r1 = ks_radius(c.spin, s.x);
+                    if (pass == 0) ok = ok && r1 < old;
+                    if (pass == 1) ok = ok && (old - c.cam_radius) * (r1 - c.cam_radius) > 0.0;
+                    old = r1;
+                }
+                ok = ok && old > c.fp32_radius && std::fabs(len - run.length) <= 1e-9 * len &&
+                     std::fabs(hh - run.next_h) <= 1e-12 * hh;
+                if (!ok) ++wrong;
+                worst_dist = std::fmax(worst_dist, distance(far, s));
+                h = run.next_h;
+            }
+        }
+    }
+    std::printf("%.3f %d %d %.3e\n", worst_const, runs, wrong, worst_dist);
+    return 0;
+}

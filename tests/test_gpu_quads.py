@@ -1,0 +1,78 @@
+"""GPU tests of the quad engine (kpolaris_b200/csrc/kp_quad.cuh): the sizes
+and mixes at which four lanes per ray can go wrong.
+
+* Image sizes around the quads of a warp and the warps of a block, one to four
+  frequencies: the one-launch FP64 kernel's reasons and step counts are the
+  CPU oracle's, and all of its outputs the wavefront's, bit for bit (whose
+  Stokes vectors tests/test_gpu_parity.py holds to the oracle's, within the
+  conditioning of libm's last bits).
+* Many small images of different spins and frequency counts in one batch, so
+  that the quads of a warp trace different images: each is bit for bit the
+  image traced alone, in either precision.
+* The mixed policy's far field takes many steps at once and counts them: on
+  rays that miss the sphere, cameras near, inside the far boundary and far
+  out, and large and small step caps, its reasons are those of the FP64 policy
+  and so are its step counts, up to the rays that the fused arithmetic of the
+  near phases moves across a step's rounding (at most 1 in 200)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import kpolaris_b200 as kp
+import oracle
+from kpolaris_b200 import _abi, configs
+
+pytestmark = pytest.mark.gpu
+
+ALL_FIELDS = _abi.IMAGE_FIELDS + _abi.DIAG_FIELDS + _abi.INT_FIELDS
+
+
+def job(nx, ny, nf, *, spin=0.9375, inclination=50.0, adaptive=True, **camera):
+    p = (configs.config2 if adaptive else configs.config1)(nx, ny)[0]
+    p.spin = spin
+    p.inner_radius = configs.reference_horizon(spin) * 1.05
+    p.camera.inclination = configs.inclination_from_degrees(inclination)
+    for k, v in camera.items():
+        setattr(p.camera, k, v)
+    return p, configs.riaf_model(), configs.CONFIG2_FREQS[:nf]
+
+
+def assert_bitwise(a, b, what):
+    for key in ALL_FIELDS:
+        assert np.array_equal(a.arrays[key], b.arrays[key], equal_nan=True), (what, key)
+
+
+@pytest.mark.parametrize("nx,ny,nf,adaptive", [(1, 1, 1, True), (3, 1, 2, True), (7, 1, 3, False), (8, 1, 4, True),
+                                               (9, 1, 1, False), (11, 3, 4, True)])
+def test_small_sizes_match_the_oracle(nx, ny, nf, adaptive):
+    p, m, f = job(nx, ny, nf, adaptive=adaptive)
+    got = kp.image_riaf(p, m, f)
+    ref = oracle.image_riaf(p, m, f, kind="port", threads=0)
+    for key in _abi.INT_FIELDS:
+        assert np.array_equal(got.arrays[key], ref.arrays[key]), key
+    assert_bitwise(kp.image_riaf(p, m, f, schedule=_abi.SCHEDULE_PERSISTENT), got, "wavefront")
+
+
+@pytest.mark.parametrize("precision", [_abi.PRECISION_FP64, _abi.PRECISION_MIXED])
+def test_mixed_warps_match_images_alone(precision):
+    jobs = [job(5 + k, 3 + (k % 4), 1 + k % 4, spin=0.09 * k, inclination=15.0 + 14.0 * k, fov_y=0.16 + 0.05 * (k % 3))
+            for k in range(11)]
+    outs = kp.batch_riaf(jobs, precision=precision)
+    for k, (p, m, f) in enumerate(jobs):
+        alone = kp.image_riaf(p, m, f, precision=precision, schedule=_abi.SCHEDULE_PERSISTENT)
+        assert_bitwise(outs[k], alone, k)
+
+
+@pytest.mark.parametrize("radius,fov,max_step", [(1000.0, 0.5, 2.0), (300.0, 1.2, 2.0), (121.0, 0.6, 2.0),
+                                                 (1000.0, 0.3, 0.7), (5000.0, 0.1, 5.0)])
+def test_far_field_runs_keep_the_step_counts(radius, fov, max_step):
+    p, m, f = job(24, 20, 1, radius=radius, fov=fov, fov_y=fov)
+    p.max_step = max_step
+    p.max_radiation_step = max_step
+    mixed = kp.image_riaf(p, m, f, precision=_abi.PRECISION_MIXED)
+    fp64 = kp.image_riaf(p, m, f, schedule=_abi.SCHEDULE_PERSISTENT)
+    assert np.array_equal(mixed.reason, fp64.reason)
+    for key in ("pass_a_steps", "steps"):
+        d = mixed.arrays[key] != fp64.arrays[key]
+        assert np.mean(d) <= 0.005, (key, int(d.sum()))

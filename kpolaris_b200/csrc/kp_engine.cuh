@@ -294,9 +294,11 @@ __device__ __noinline__ void ck_job(const ImageConsts& c, const Ray& S, double h
 
 // Step-doubling attempt, RK4 step or composed RK4 pair as a stage loop around
 // one RHS site.  Out of line: the caller's control state is saved once per
-// job and the stage loop has the register file to itself.
+// job and the stage loop has the register file to itself.  `sure`: a
+// step-doubling attempt that is certain to be accepted with the growth of err
+// = 0 (certain_step) leaves its full chain out.
 template<class P, class SC>
-__device__ __noinline__ void rk_job(int kind, const ImageConsts& c, const Ray& S, double h,
+__device__ __noinline__ void rk_job(int kind, const ImageConsts& c, const Ray& S, double h, bool sure,
                                     Ray& next, Ray& mid, double& err) {
     if (kind == kRkCK) {
         ck_job<P, SC>(c, S, h, next, mid, err);
@@ -304,7 +306,7 @@ __device__ __noinline__ void rk_job(int kind, const ImageConsts& c, const Ray& S
     }
     // Stage schedule (see file header): SD = half chain (4), second half
     // chain (4), full chain (3); RK4 = 4; RK4x2 = 4 + 4.
-    const int nstage = kind == kRkSD ? 11 : (kind == kRkRK4 ? 4 : 8);
+    const int nstage = kind == kRkSD && !sure ? 11 : (kind == kRkRK4 ? 4 : 8);
     const double hs = kind == kRkSD ? h * 0.5 : (kind == kRkRK4x2 ? h * 0.5 : h);  // step of the first chain
     const double hh_s = 0.5 * hs;
     const double h6_s = hs / 6.0;
@@ -345,8 +347,9 @@ __device__ __noinline__ void rk_job(int kind, const ImageConsts& c, const Ray& S
                     X = R2;
                 }
             } else if (st == 7) {
-                if (kind == kRkRK4x2) {
+                if (kind == kRkRK4x2 || sure) {
                     ray_axpy(next, R2, h6, A);
+                    mid = R2;
                 } else {
                     // two_half = R2 + (hs/6) A; start the full chain from k1 of S
                     Ray two_half;
@@ -366,10 +369,8 @@ __device__ __noinline__ void rk_job(int kind, const ImageConsts& c, const Ray& S
             }
         }
     }
-    if (kind == kRkRK4 || kind == kRkRK4x2) {
-        mid = next;
-        err = 0.0;
-    }
+    if (kind == kRkRK4 || kind == kRkRK4x2) mid = next;
+    if (nstage < 11) err = 0.0;
 }
 
 }  // namespace kp

@@ -1,5 +1,6 @@
-// kp_far_steps.cuh -- how many steps of the step control the mixed policy's
-// far phase bridges at once (quad_macro_step in kp_quad.cuh).
+// kp_far_steps.cuh -- what the step control will do, known without asking it:
+// how many of its steps the mixed policy's far phase bridges at once
+// (quad_macro_step in kp_quad.cuh), and which steps need no error estimate.
 #pragma once
 
 #include "kp_common.cuh"
@@ -61,6 +62,21 @@ KP_HD MacroRun macro_run(const ImageConsts& c, double r, double xk, double v, do
         run.count += more;
     }
     return run;
+}
+
+// Whether the step-doubling error of a step of size h at radius r is certain
+// to be at most `lim`, from a bound on the Kerr-Schild transport: km the
+// largest |k^mu|, w the largest component of k, e1 and e2.  With `lim` a
+// quarter of the tolerance for a step at the cap and 1/64 of it otherwise the
+// step control accepts the step and the next one's size is known (the cap, or
+// twice the size): the attempt needs no full-step chain.  The error found by
+// tests/native/far_steps.cpp along camera rays past the hole, down to r = 2 M,
+// is at most 0.3 of the bound; its last term covers rounding.
+KP_HD bool certain_step(double mass, double r, double km, double w, double h, double lim) {
+    const double ah = abs_val(h), rl = r - 3.5 * ah * km;
+    if (!(rl > 2.0 * mass) || !(w < 1e4)) return false;
+    const double hk = ah * km, hk2 = hk * hk, r2 = rl * rl;
+    return (16.0 + 0.25 * rl) * mass * (hk2 * hk2 * ah * w) <= (lim - 1e-13 * max_val(1.0, w)) * (r2 * r2 * r2);
 }
 
 }  // namespace kp

@@ -23,6 +23,7 @@
 #include <cstddef>
 
 #include "kp_engine.cuh"
+#include "kp_far_steps.cuh"
 
 namespace kp {
 
@@ -399,7 +400,23 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
         Ray next, mid;
         double err = 0.0;
         if (run) {
-            rk_job<P, SC>(st.rk_kind, J->c, S, st.h_try, next, mid, err);
+            bool sure = false;
+            if constexpr (SC::kCksRhs) {
+                if (st.rk_kind == kRkSD) {
+                    double km = 0.0, w = 0.0, z = 0.0;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        km = max_val(km, abs_val(S.k.v[i]));
+                        w = max_val(w, max_val(abs_val(S.e1.v[i]), abs_val(S.e2.v[i])));
+                        z += S.k.v[i] + (S.e1.v[i] + S.e2.v[i]);
+                    }
+                    if (!(z - z == 0.0)) w = kLarge;  // a NaN or an infinity among them
+                    const double tol = max_val(J->c.tolerance, kTolFloor);
+                    sure = certain_step(J->c.mass, st.mode == kAStep ? st.old_r : st.start_r, km, max_val(km, w), st.h_try,
+                                        (abs_val(st.h_try) == st.ctl_max ? 0.25 : 1.0 / 64.0) * tol);
+                }
+            }
+            rk_job<P, SC>(st.rk_kind, J->c, S, st.h_try, sure, next, mid, err);
             if (++lane_jobs > (1LL << 30)) {
                 st.reason = kInvalidState;
                 st.mode = kDone;

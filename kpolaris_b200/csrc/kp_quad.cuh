@@ -253,10 +253,12 @@ __device__ __forceinline__ D4 quad_macro_step(const ImageConsts& c, const D4& S,
 // along on what they hold and their outputs mean nothing.  A step-doubling
 // attempt runs three chains of four stages (half step, second half step, full
 // step with its first derivative reused), a composed pair two, a single step
-// one.
+// one.  `sure`: the attempt is certain to be accepted with the growth of err =
+// 0 (certain_step); if the warp's other attempts are too, the full chain is
+// left out.
 template<class P, class SC, bool MACRO>
-__device__ __forceinline__ void quad_job(int kind, const ImageConsts& c, const D4& S, double h, int role, D4& next,
-                                         D4& mid, double& err) {
+__device__ __forceinline__ void quad_job(int kind, const ImageConsts& c, const D4& S, double h, int role, bool sure,
+                                         D4& next, D4& mid, double& err) {
     err = 0.0;
     const typename SC::Geo geo = SC::geo(c);
     const bool ck = kind == kRkCK;
@@ -280,7 +282,7 @@ __device__ __forceinline__ void quad_job(int kind, const ImageConsts& c, const D
         }
     }
     const bool sd = kind == kRkSD, single = kind == kRkRK4;
-    const int nchain = __any_sync(kFullWarp, sd) ? 3 : (__any_sync(kFullWarp, kind == kRkRK4x2) ? 2 : 1);
+    const int nchain = __any_sync(kFullWarp, sd && !sure) ? 3 : (__any_sync(kFullWarp, sd || kind == kRkRK4x2) ? 2 : 1);
     D4 B = S;             // chain base
     D4 K1, R2, end, A, X, k;
     double hc = single ? h : h * 0.5;
@@ -604,7 +606,20 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
                     hj = st.h_try < 0.0 ? -run_of.length : run_of.length;
                 }
             }
-            quad_job<P, SC, kMacro>(kind, c, V, hj, role, next, mid, err);
+            bool sure = false;
+            if constexpr (SC::kCksRhs) {
+                double m = 0.0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) m = max_val(m, abs_val(V.v[i]));
+                const double z = (V.v[0] + V.v[1]) + (V.v[2] + V.v[3]);
+                if (!(z - z == 0.0)) m = kLarge;  // a NaN or an infinity among them
+                const double km = quad_get(m, 1), w = quad_max(role == 0 ? 0.0 : m);
+                if (run && kind == kRkSD && SC::chart_active(c)) {
+                    const double tol = max_val(c.tolerance, kTolFloor);
+                    sure = certain_step(c.mass, r_top, km, w, hj, (abs_val(hj) == st.ctl_max ? 0.25 : 1.0 / 64.0) * tol);
+                }
+            }
+            quad_job<P, SC, kMacro>(kind, c, V, hj, role, sure, next, mid, err);
             next_r = SC::template top_radius<P::kMixed>(c, quad_get3(next, 0));
         }
         if (!kAll && run && ++quad_jobs > (1LL << 30)) {

@@ -8,7 +8,9 @@
 //   (another step size, a step from or into the near phase, past the camera
 //   or, in pass A, outward),
 //   the largest distance (over max(1, |.|)) between the extrapolated midpoint
-//   rule over a run and the steps themselves.
+//   rule over a run and the steps themselves,
+//   how many steps certain_step promised, and the largest error of one of
+//   them over the error it was promised to stay under.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -17,6 +19,7 @@
 #define __device__
 #define __forceinline__ inline
 #define __noinline__
+#include "kp_camera.cuh"
 #include "kp_far_steps.cuh"
 #include "kp_geometry.cuh"
 
@@ -161,6 +164,50 @@ int main() {
             }
         }
     }
-    std::printf("%.3f %d %d %.3e\n", worst_const, runs, wrong, worst_dist);
+    // certain_step: the error of a step against the bound it is promised by,
+    // along camera rays past the hole, backward and forward
+    double worst_certain = 0.0;
+    long certain = 0;
+    for (int ray = 0; ray < 150; ++ray) {
+        ImageConsts c;
+        std::memset(&c, 0, sizeof(c));
+        c.mass = 1.0;
+        c.spin = 0.99 * u(rng);
+        c.nx = c.ny = 64;
+        c.cam_radius = u(rng) < 0.5 ? 1000.0 : 50.0 + 1000.0 * u(rng);
+        const double inc = 0.1 + 2.9 * u(rng);
+        c.sin_inc = std::sin(inc);
+        c.cos_inc = std::cos(inc);
+        c.fov = c.fov_y = (u(rng) < 0.6 ? 24.0 : 160.0) / c.cam_radius;
+        const CameraFrame f = camera_frame(c);
+        Ray s = camera_ray(c, f, int(4096 * u(rng)));
+        const double rh = 1.0 + std::sqrt(1.0 - c.spin * c.spin);
+        double dir = -1.0;
+        for (int n = 0; n < 6000; ++n) {
+            const double r = ks_radius(c.spin, s.x);
+            if (dir < 0.0 ? (r < rh * 1.05 || (r > 1200.0 && n > 100)) : (r > 1100.0 || r < rh * 1.01)) {
+                if (dir > 0.0) break;
+                dir = 1.0;
+            }
+            double km = 0.0, w = 0.0;
+            for (int i = 0; i < 4; ++i) {
+                km = std::fmax(km, std::fabs(s.k.v[i]));
+                w = std::fmax(w, std::fmax(std::fabs(s.e1.v[i]), std::fabs(s.e2.v[i])));
+            }
+            w = std::fmax(km, w);
+            for (const double h : {4.0, 2.0, 0.7, 0.2, 0.03}) {
+                for (const double lim : {2.5e-9, 1e-8 / 64.0, 1e-6 / 64.0}) {
+                    if (!certain_step(c.mass, r, km, w, h, lim)) continue;
+                    ++certain;
+                    const Ray half = rk4(c.mass, c.spin, s, 0.5 * dir * h);
+                    const double err = distance(rk4(c.mass, c.spin, s, dir * h), rk4(c.mass, c.spin, half, 0.5 * dir * h));
+                    worst_certain = std::fmax(worst_certain, err / lim);
+                }
+            }
+            s = rk4(c.mass, c.spin, s, dir * (r > 130.0 ? 4.0 : std::fmin(2.0, 0.05 * r * (0.3 + u(rng)))));
+            if (!(std::fabs(s.x.v[1]) < 1e9)) break;
+        }
+    }
+    std::printf("%.3f %d %d %.3e %ld %.3f\n", worst_const, runs, wrong, worst_dist, certain, worst_certain);
     return 0;
 }

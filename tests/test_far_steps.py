@@ -1,4 +1,4 @@
-"""CPU test of the far field's bridged runs of steps
+"""CPU test of what the engine knows of the step control without asking it
 (kpolaris_b200/csrc/kp_far_steps.cuh, host build of tests/native/far_steps.cpp).
 
 * The step-doubling error of every step of a run stays under the bound that
@@ -10,7 +10,9 @@
   steps themselves drift from the geodesic by at most their summed
   step-doubling errors: up to 100 steps at a quarter of the tolerance 1e-6 of
   the coarsest rays would be 2.5e-5, but the bound holds at the run's inner
-  end only; 1e-7 is a tenth of one step's tolerance."""
+  end only; 1e-7 is a tenth of one step's tolerance.
+* Every step that certain_step promises to be accepted has a step-doubling
+  error under the promised one."""
 from __future__ import annotations
 
 import subprocess
@@ -29,3 +31,6 @@ def test_runs_are_the_step_controls(tmp_path):
     assert runs > 1000, runs
     assert wrong == 0, wrong
     assert dist <= 1e-7, dist
+    certain, worst = int(out[4]), float(out[5])
+    assert certain > 100000, certain
+    assert worst <= 1.0, worst

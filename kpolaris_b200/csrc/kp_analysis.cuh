@@ -566,11 +566,14 @@ __device__ __forceinline__ void trace_pass_b_analysis(const ImageConsts& c, cons
                 const double r = riaf_bl_coords(spin, sample.x).rc;
                 const int bin = analysis_radial_bin(k, r);
                 analysis_sample(c, sample, co, dlambda, r, bin, a);
-                Coeffs<double> propagation = co;
-                propagation.jI = propagation.jQ = propagation.jU = propagation.jV = 0.0;
                 if (resp) response_sample(c, *resp, sample, ps, stokes, co, dlambda, resp_data, pixel, npix);
+                // the sample emits into its own bin; the others only propagate
+                const StokesOp op = stokes_op(co, dlambda);
 #pragma unroll 1
-                for (int b = 0; b < k.radial_bins; ++b) stokes_step(a.radial[b], b == bin ? co : propagation, dlambda);
+                for (int b = 0; b < k.radial_bins; ++b) {
+                    stokes_apply(a.radial[b], op, b == bin ? co.jI : 0.0, b == bin ? co.jQ : 0.0,
+                                 b == bin ? co.jU : 0.0, b == bin ? co.jV : 0.0);
+                }
                 a.substeps += 1;
             }
             stokes_step(stokes, co, abs_val(h) * dls);

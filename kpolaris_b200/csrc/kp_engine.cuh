@@ -74,14 +74,23 @@ struct RadTraits<PolicyFP64, SceneRiaf> {
     __device__ static Co coeffs(const ImageConsts& c, const Sample& p, int f) {
         return riaf_coefficients(c, p, c.freq[f]);
     }
+    __device__ static RadDepths depths(const Co& co, double dls) { return radiation_depths(co, dls); }
     __device__ static Co coeffs_ctl(const ImageConsts& c, const Sample& p, int g) {
         return riaf_coefficients(c, p, c.ctl_freq[g]);
     }
     __device__ static void step(Stokes& s, const Co& co, double h, const ImageConsts& c, int f) {
-        stokes_step(s, co, abs_val(h) * c.dlambda_scale[f]);
+        stokes_apply(s, stokes_op(co, abs_val(h) * c.dlambda_scale[f]), co.jI, co.jQ, co.jU, co.jV);
     }
     __device__ static Stokes4<double> result(const Stokes& s, const ImageConsts&, int) { return s; }
 };
+
+__device__ __forceinline__ double norm_refined(double x, double y, double z) {
+    const double n2 = x * x + y * y + z * z;
+    if (!(n2 > 1e-280 && n2 < 1e280)) return sqrt(n2);
+    double n, inv;
+    kp_sqrt_pair<double>(n2, n, inv);
+    return n;
+}
 
 template<>
 struct RadTraits<PolicyMixed, SceneRiaf> {
@@ -133,11 +142,12 @@ struct RadTraits<PolicyFP64, SceneGrmhd> {
     __device__ static Co coeffs(const ImageConsts& c, const Sample& p, int f) {
         return grmhd_coefficients(c, p, c.freq[f]);
     }
+    __device__ static RadDepths depths(const Co& co, double dls) { return radiation_depths(co, dls); }
     __device__ static Co coeffs_ctl(const ImageConsts& c, const Sample& p, int g) {
         return grmhd_coefficients(c, p, c.ctl_freq[g]);
     }
     __device__ static void step(Stokes& s, const Co& co, double h, const ImageConsts& c, int f) {
-        stokes_step(s, co, abs_val(h) * c.dlambda_scale[f]);
+        stokes_apply(s, stokes_op(co, abs_val(h) * c.dlambda_scale[f]), co.jI, co.jQ, co.jU, co.jV);
     }
     __device__ static Stokes4<double> result(const Stokes& s, const ImageConsts&, int) { return s; }
 };

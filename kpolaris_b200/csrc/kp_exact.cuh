@@ -18,6 +18,8 @@
 // square root, taken to one ulp by a third-order Newton step.
 #pragma once
 
+#include <cmath>
+
 #include "kp_common.cuh"
 
 namespace kp {
@@ -60,6 +62,59 @@ __device__ __forceinline__ double exact_sqrt(double v) {
 // A numerator's factor for which products of a few of its like stay clear of
 // underflow.
 __device__ __forceinline__ bool exact_factor(double v) { return abs_val(v) > 1e-50 || v == 0.0; }
+
+// 2^-500 < |v| < 2^500 or zero: with a divisor between 2^-200 and 2^200 the
+// quotient and its residuals are normal numbers.
+__device__ __forceinline__ bool exact_numerator(double v) {
+    return (unsigned(__double2hiint(v) >> 20) & 0x7ffu) - 523u < 1000u || v == 0.0;
+}
+
+// 2^-200 < |b| < 2^200.
+__device__ __forceinline__ bool exact_divisor(double b) {
+    return (unsigned(__double2hiint(b) >> 20) & 0x7ffu) - 823u < 400u;
+}
+
+// The rare operands out of range.
+static __device__ __noinline__ double plain_quot(double a, double b) { return a / b; }
+
+// v[i] = RN(v[i] / b) for any operands: together where all of them are in
+// range, by the compiler's division otherwise.
+template<int N>
+__device__ __forceinline__ void exact_quots(double (&v)[N], double b) {
+    bool ok = exact_divisor(b);
+#pragma unroll
+    for (int i = 0; i < N; ++i) ok = ok && exact_numerator(v[i]);
+    if (ok) {
+        const ExactRecip r = exact_recip(b);
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] = exact_quot(v[i], r);
+    } else {
+#pragma unroll 1
+        for (int i = 0; i < N; ++i) v[i] = plain_quot(v[i], b);
+    }
+}
+
+// RN(a / b) for a constant b of ordinary size: `inv` is RN(1 / b), folded by
+// the compiler.
+__device__ __forceinline__ double exact_over(double a, double b, double inv) {
+    if (exact_numerator(a)) return exact_quot(a, ExactRecip{b, inv});
+    return plain_quot(a, b);
+}
+#define KP_OVER(a, b) exact_over((a), (b), 1.0 / (b))
+
+#else  // host builds of the device code: the compiler's own
+
+struct ExactRecip {
+    double b;
+};
+inline ExactRecip exact_recip(double b) { return ExactRecip{b}; }
+inline double exact_quot(double a, const ExactRecip& r) { return a / r.b; }
+inline double exact_sqrt(double v) { return sqrt(v); }
+template<int N>
+inline void exact_quots(double (&v)[N], double b) {
+    for (int i = 0; i < N; ++i) v[i] = v[i] / b;
+}
+#define KP_OVER(a, b) ((a) / (b))
 
 #endif
 

@@ -67,12 +67,23 @@ KP_HD KSMetricPoint ks_point(double mass, double spin, const D4& X) {
     const double r = sqrt(max_val(r2, kTiny));
     const double denom = r2 * r2 + a2 * z * z;
     KSMetricPoint p;
-    p.amp = 2.0 * mass * r2 * r / denom;
     const double r2pa2 = r2 + a2;
     p.l[0] = 1.0;
+#ifdef __CUDA_ARCH__
+    double amp[1] = {2.0 * mass * r2 * r}, l12[2] = {r * x + a * y, r * y - a * x}, l3[1] = {z};
+    exact_quots(amp, denom);
+    exact_quots(l12, r2pa2);
+    exact_quots(l3, r);
+    p.amp = amp[0];
+    p.l[1] = l12[0];
+    p.l[2] = l12[1];
+    p.l[3] = l3[0];
+#else
+    p.amp = 2.0 * mass * r2 * r / denom;
     p.l[1] = (r * x + a * y) / r2pa2;
     p.l[2] = (r * y - a * x) / r2pa2;
     p.l[3] = z / r;
+#endif
     return p;
 }
 

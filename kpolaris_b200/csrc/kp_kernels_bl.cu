@@ -2,6 +2,7 @@
 // on the wavefront engine with the FP64 policy, compiled without FMA contraction so the arithmetic stays closest to the reference's CPU rounding.
 #include <cuda_runtime.h>
 
+#define KP_MATH_CALLS 1  // kp_radiation.cuh
 #include "kp_launch.h"
 #include "kp_quad.cuh"
 

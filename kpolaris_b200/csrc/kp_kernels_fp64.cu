@@ -12,6 +12,7 @@
 
 #include <algorithm>
 
+#define KP_MATH_CALLS 1  // kp_radiation.cuh
 #include "kp_analysis.cuh"
 #include "kp_bl.cuh"
 #include "kp_launch.h"

@@ -3,6 +3,7 @@
 // the FP64 policy. Compiled without FMA contraction, as the fast-light GRMHD kernels.
 #include <cuda_runtime.h>
 
+#define KP_MATH_CALLS 1  // kp_radiation.cuh
 #include "kp_launch.h"
 #include "kp_quad.cuh"
 

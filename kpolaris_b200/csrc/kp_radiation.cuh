@@ -21,42 +21,107 @@ constexpr double kCL = 2.99792458e10;
 constexpr double kHPL = 6.62607015e-27;
 constexpr double kMP = 1.67262192369e-24;
 
+// The functions that the fits call up to seven times a sample.  With
+// KP_MATH_CALLS a unit holds one copy of each: inlined, a radiating step of
+// the FP64 quads walks through more code than the instruction caches hold
+// (near-B of a 256^2 image 790 -> 746 ms, the plain kernel at 64^2 34.6 ->
+// 33.2 ms).  The mixed kernels are faster with the functions inlined (near-B
+// of the same image 177 against 188 ms).
+#if defined(__CUDA_ARCH__) && defined(KP_MATH_CALLS)
+static __device__ __noinline__ double kp_exp(double x) { return exp(x); }
+static __device__ __noinline__ double kp_log(double x) { return log(x); }
+static __device__ __noinline__ double kp_pow(double x, double y) { return pow(x, y); }
+#else
+__host__ __device__ __forceinline__ double kp_exp(double x) { return exp(x); }
+__host__ __device__ __forceinline__ double kp_log(double x) { return log(x); }
+__host__ __device__ __forceinline__ double kp_pow(double x, double y) { return pow(x, y); }
+#endif
+
 // ---- transfer ----------------------------------------------------------
-__device__ __forceinline__ double stable_attenuation(double kappa, double dl) {
-    const double x = kappa * dl;
-    if (x > 700.0) return 0.0;
-    return exp(-x);
-}
-
-__device__ __forceinline__ double stable_source_factor(double kappa, double dl) {
-    const double x = kappa * dl;
-    if (abs_val(x) < 1e-6) return dl * (1.0 - x / 2.0 + x * x / 6.0 - x * x * x / 24.0);
-    return (1.0 - exp(-x)) / kappa;
-}
-
 // scaled Euclidean norm (src/common/vec.hpp:62-70)
 __device__ __forceinline__ double norm3(double x, double y, double z) {
     const double scale = max_val(abs_val(x), max_val(abs_val(y), abs_val(z)));
     if (scale == 0.0) return 0.0;
-    const double a = x / scale, b = y / scale, c = z / scale;
-    return scale * sqrt(a * a + b * b + c * c);
+    double v[3] = {x, y, z};
+    exact_quots(v, scale);
+    return scale * exact_sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);  // between 1 and 3
 }
 
-__device__ __forceinline__ void faraday_rotate(Stokes4<double>& s, const Coeffs<double>& c, double dl) {
-    const double px = s.Q, py = s.U, pz = s.V;
-    const double rho_norm = norm3(c.rQ, c.rU, c.rV);
-    if (rho_norm == 0.0 || dl == 0.0) return;
-    const double theta = rho_norm * dl;
-    double ox, oy, oz;
-    if (abs_val(theta) < 1e-8) {
-        ox = px + (c.rU * pz - c.rV * py) * dl;
-        oy = py + (c.rV * px - c.rQ * pz) * dl;
-        oz = pz + (c.rQ * py - c.rU * px) * dl;
+// The Strang step of one set of coefficients over dl, but for the emission
+// and the vector it acts on: both Faraday half steps are one rotation, the
+// attenuation and the source factor of an eigenvalue share an exponential, and
+// an analysis image applies one step to every radial bin.
+struct StokesOp {
+    int rot;                        // 0: none, 1: linear, 2: rotation
+    double rx, ry, rz, half, ct, st;
+    int pol;                        // polarised absorption
+    double nx, ny, nz, ap, sp, am, sm, e, f;
+};
+
+__device__ __forceinline__ void fade_source(double kappa, double dl, double& att, double& src) {
+    const double x = kappa * dl;
+    const double ex = kp_exp(-x);
+    att = x > 700.0 ? 0.0 : ex;
+    if (abs_val(x) < 1e-6) {
+        src = dl * (1.0 - x * 0.5 + KP_OVER(x * x, 6.0) - KP_OVER(x * x * x, 24.0));
     } else {
-        const double inv = 1.0 / rho_norm;
-        const double nx = c.rQ * inv, ny = c.rU * inv, nz = c.rV * inv;
-        double st, ct;
-        sincos(theta, &st, &ct);
+        double q[1] = {1.0 - ex};
+        exact_quots(q, kappa);
+        src = q[0];
+    }
+}
+
+__device__ __forceinline__ StokesOp stokes_op(const Coeffs<double>& c, double dl) {
+    StokesOp o;
+    const double half = 0.5 * dl;
+    const double rho_norm = norm3(c.rQ, c.rU, c.rV);
+    o.rx = c.rQ;
+    o.ry = c.rU;
+    o.rz = c.rV;
+    o.half = half;
+    o.ct = o.st = 0.0;
+    if (rho_norm == 0.0 || half == 0.0) {
+        o.rot = 0;
+    } else {
+        const double theta = rho_norm * half;
+        o.rot = abs_val(theta) < 1e-8 ? 1 : 2;
+        if (o.rot == 2) {
+            double q[1] = {1.0};
+            exact_quots(q, rho_norm);
+            const double inv = q[0];
+            o.rx = c.rQ * inv;
+            o.ry = c.rU * inv;
+            o.rz = c.rV * inv;
+            sincos(theta, &o.st, &o.ct);
+        }
+    }
+    const double an = norm3(c.aQ, c.aU, c.aV);
+    o.pol = !(an < kTiny);
+    fade_source(c.aI, dl, o.e, o.f);
+    o.nx = o.ny = o.nz = o.ap = o.sp = o.am = o.sm = 0.0;
+    if (o.pol) {
+        double q[1] = {1.0};
+        exact_quots(q, an);
+        const double inv = q[0];
+        o.nx = c.aQ * inv;
+        o.ny = c.aU * inv;
+        o.nz = c.aV * inv;
+        fade_source(c.aI + an, dl, o.ap, o.sp);
+        fade_source(c.aI - an, dl, o.am, o.sm);
+    }
+    return o;
+}
+
+__device__ __forceinline__ void faraday_rotate(Stokes4<double>& s, const StokesOp& o) {
+    if (o.rot == 0) return;
+    const double px = s.Q, py = s.U, pz = s.V;
+    double ox, oy, oz;
+    if (o.rot == 1) {
+        ox = px + (o.ry * pz - o.rz * py) * o.half;
+        oy = py + (o.rz * px - o.rx * pz) * o.half;
+        oz = pz + (o.rx * py - o.ry * px) * o.half;
+    } else {
+        const double nx = o.rx, ny = o.ry, nz = o.rz, ct = o.ct, st = o.st;
         const double f = (nx * px + ny * py + nz * pz) * (1.0 - ct);
         ox = px * ct + nx * f + (ny * pz - nz * py) * st;
         oy = py * ct + ny * f + (nz * px - nx * pz) * st;
@@ -67,54 +132,43 @@ __device__ __forceinline__ void faraday_rotate(Stokes4<double>& s, const Coeffs<
     s.V = oz;
 }
 
-__device__ __forceinline__ void absorb_emit(Stokes4<double>& s, const Coeffs<double>& c, double dl) {
-    const double an = norm3(c.aQ, c.aU, c.aV);
-    if (an < kTiny) {
-        const double e = stable_attenuation(c.aI, dl);
-        const double f = stable_source_factor(c.aI, dl);
-        s.I = e * s.I + f * c.jI;
-        s.Q = e * s.Q + f * c.jQ;
-        s.U = e * s.U + f * c.jU;
-        s.V = e * s.V + f * c.jV;
-        return;
+__device__ __forceinline__ void stokes_apply(Stokes4<double>& s, const StokesOp& o, double jI, double jQ, double jU,
+                                             double jV) {
+    faraday_rotate(s, o);
+    if (!o.pol) {
+        s.I = o.e * s.I + o.f * jI;
+        s.Q = o.e * s.Q + o.f * jQ;
+        s.U = o.e * s.U + o.f * jU;
+        s.V = o.e * s.V + o.f * jV;
+    } else {
+        const double nx = o.nx, ny = o.ny, nz = o.nz;
+        const double p_par = nx * s.Q + ny * s.U + nz * s.V;
+        const double ppx = s.Q - nx * p_par, ppy = s.U - ny * p_par, ppz = s.V - nz * p_par;
+        const double j_par = nx * jQ + ny * jU + nz * jV;
+        const double jpx = jQ - nx * j_par, jpy = jU - ny * j_par, jpz = jV - nz * j_par;
+        const double sp = o.ap * (s.I + p_par) + o.sp * (jI + j_par);
+        const double sm = o.am * (s.I - p_par) + o.sm * (jI - j_par);
+        const double ox = ppx * o.e + jpx * o.f;
+        const double oy = ppy * o.e + jpy * o.f;
+        const double oz = ppz * o.e + jpz * o.f;
+        const double par_out = 0.5 * (sp - sm);
+        s.I = 0.5 * (sp + sm);
+        s.Q = nx * par_out + ox;
+        s.U = ny * par_out + oy;
+        s.V = nz * par_out + oz;
     }
-    const double inv = 1.0 / an;
-    const double nx = c.aQ * inv, ny = c.aU * inv, nz = c.aV * inv;
-    const double p_par = nx * s.Q + ny * s.U + nz * s.V;
-    const double ppx = s.Q - nx * p_par, ppy = s.U - ny * p_par, ppz = s.V - nz * p_par;
-    const double j_par = nx * c.jQ + ny * c.jU + nz * c.jV;
-    const double jpx = c.jQ - nx * j_par, jpy = c.jU - ny * j_par, jpz = c.jV - nz * j_par;
-    const double s_plus = s.I + p_par;
-    const double s_minus = s.I - p_par;
-    const double j_plus = c.jI + j_par;
-    const double j_minus = c.jI - j_par;
-    const double k_plus = c.aI + an;
-    const double k_minus = c.aI - an;
-    const double sp = stable_attenuation(k_plus, dl) * s_plus + stable_source_factor(k_plus, dl) * j_plus;
-    const double sm = stable_attenuation(k_minus, dl) * s_minus + stable_source_factor(k_minus, dl) * j_minus;
-    const double e_i = stable_attenuation(c.aI, dl);
-    const double f_i = stable_source_factor(c.aI, dl);
-    const double ox = ppx * e_i + jpx * f_i;
-    const double oy = ppy * e_i + jpy * f_i;
-    const double oz = ppz * e_i + jpz * f_i;
-    const double i_out = 0.5 * (sp + sm);
-    const double par_out = 0.5 * (sp - sm);
-    s.I = i_out;
-    s.Q = nx * par_out + ox;
-    s.U = ny * par_out + oy;
-    s.V = nz * par_out + oz;
+    faraday_rotate(s, o);
 }
 
 static __device__ __noinline__ void stokes_step(Stokes4<double>& s, const Coeffs<double>& c, double dl) {
-    faraday_rotate(s, c, 0.5 * dl);
-    absorb_emit(s, c, dl);
-    faraday_rotate(s, c, 0.5 * dl);
+    const StokesOp o = stokes_op(c, dl);
+    stokes_apply(s, o, c.jI, c.jQ, c.jU, c.jV);
 }
 
 // ---- thermal synchrotron ------------------------------------------------
 __device__ __forceinline__ double bessel_i0(double ax) {
     if (ax < 3.75) {
-        double y = ax / 3.75;
+        double y = KP_OVER(ax, 3.75);
         y *= y;
         double p = 0.0045813;
         p = 0.0360768 + y * p;
@@ -134,12 +188,12 @@ __device__ __forceinline__ double bessel_i0(double ax) {
     p = 0.00225319 + y * p;
     p = 0.01328592 + y * p;
     p = 0.39894228 + y * p;
-    return exp(ax) / sqrt(ax) * p;
+    return kp_exp(ax) / sqrt(ax) * p;
 }
 
 __device__ __forceinline__ double bessel_i1(double ax) {
     if (ax < 3.75) {
-        double y = ax / 3.75;
+        double y = KP_OVER(ax, 3.75);
         y *= y;
         double p = 0.00032411;
         p = 0.00301532 + y * p;
@@ -160,7 +214,7 @@ __device__ __forceinline__ double bessel_i1(double ax) {
     p = -0.00362018 + y * p;
     p = -0.03988024 + y * p;
     p = 0.39894228 + y * p;
-    return exp(ax) / sqrt(ax) * p;
+    return kp_exp(ax) / sqrt(ax) * p;
 }
 
 // K0, K1 and K2 = max(K0 + 2 K1 / x, 1e-300) (thermal_synchrotron.hpp:108-229).
@@ -177,7 +231,7 @@ __device__ __forceinline__ void bessel_k012(double x, double& k0, double& k1, do
         p = 0.23069756 + y * p;
         p = 0.42278420 + y * p;
         p = -0.57721566 + y * p;
-        const double lg = log(x * 0.5);
+        const double lg = kp_log(x * 0.5);
         k0 = -lg * bessel_i0(x) + p;
         double q = -0.00004686;
         q = -0.00110404 + y * q;
@@ -186,7 +240,9 @@ __device__ __forceinline__ void bessel_k012(double x, double& k0, double& k1, do
         q = -0.67278579 + y * q;
         q = 0.15443144 + y * q;
         q = 1.0 + y * q;
-        k1 = lg * bessel_i1(x) + q / x;
+        double d[1] = {q};
+        exact_quots(d, x);
+        k1 = lg * bessel_i1(x) + d[0];
     } else {
         const double y = 2.0 / x;
         double p = 0.00053208;
@@ -196,7 +252,7 @@ __device__ __forceinline__ void bessel_k012(double x, double& k0, double& k1, do
         p = 0.02189568 + y * p;
         p = -0.07832358 + y * p;
         p = 1.25331414 + y * p;
-        const double ex = exp(-x) / sqrt(x);
+        const double ex = kp_exp(-x) / sqrt(x);
         k0 = ex * p;
         double q = -0.00068245;
         q = 0.00325614 + y * q;
@@ -207,52 +263,74 @@ __device__ __forceinline__ void bessel_k012(double x, double& k0, double& k1, do
         q = 1.25331414 + y * q;
         k1 = ex * q;
     }
-    k2 = max_val(k0 + 2.0 * k1 / max_val(x, 1e-300), 1e-300);
+    double d[1] = {2.0 * k1};
+    exact_quots(d, max_val(x, 1e-300));
+    k2 = max_val(k0 + d[0], 1e-300);
 }
 
 __device__ __forceinline__ double bnu_inv(double nu, double thetae) {
     if (!(thetae > 0.0)) return 0.0;
-    const double x = kHPL * nu / (kME * kCL * kCL * thetae);
-    if (x < 2e-3) {
-        const double denom = x / 24.0 * (24.0 + x * (12.0 + x * (4.0 + x)));
-        return (2.0 * kHPL / max_val(denom, kTiny)) / (kCL * kCL);
-    }
-    const double denom = exp(x) - 1.0;
-    return (2.0 * kHPL / max_val(denom, kTiny)) / (kCL * kCL);
+    double x[1] = {kHPL * nu};
+    exact_quots(x, kME * kCL * kCL * thetae);
+    const double denom = x[0] < 2e-3 ? KP_OVER(x[0], 24.0) * (24.0 + x[0] * (12.0 + x[0] * (4.0 + x[0])))
+                                     : kp_exp(x[0]) - 1.0;
+    double q[1] = {2.0 * kHPL};
+    exact_quots(q, max_val(denom, kTiny));
+    return KP_OVER(q[0], kCL * kCL);
 }
 
 // rho_Q and rho_V fits (symphony_rho_QV, thermal_synchrotron.hpp:462-506).
 __device__ __forceinline__ void rho_QV(double nu, double ne, double thetae, double b, double st,
                                        double ct, double& rhoQ, double& rhoV) {
-    const double omega0 = kEE * b / (kME * kCL);
-    const double wp2 = 4.0 * kPi * ne * kEE * kEE / kME;
+    const double omega0 = KP_OVER(kEE * b, kME * kCL);
+    const double wp2 = KP_OVER(4.0 * kPi * ne * kEE * kEE, kME);
     const double two_pi_nu = 2.0 * kPi * nu;
-    const double x = max_val(thetae * sqrt(max_val(0.0, sqrt(2.0) * st * (1e3 * omega0 / max_val(two_pi_nu, kTiny)))), 1e-12);
-    double k0, k1, k2;
-    bessel_k012(1.0 / thetae, k0, k1, k2);
-    const double exp_x_47 = exp(-x / 47.2);
-    const double extraterm = (0.011 * exp_x_47 - 369.69342869090815 * pow(x + 1e-16, -8.0 / 3.0)) *
-                             (0.5 + 0.5 * tanh((log(x) - 4.787491742782046) / 0.1));
-    const double jffunc = 2.011 * exp(-pow(x, 1.035) / 4.7) - cos(x / 2.0) * exp(-pow(x, 1.2) / 2.73) -
-                          0.011 * exp_x_47 + extraterm;
-    const double k1_ratio = k2 > 0.0 ? k1 / k2 : 1.0;
     const double safe = max_val(two_pi_nu, kTiny);
+    double t[1] = {1e3 * omega0};
+    exact_quots(t, safe);
+    const double x = max_val(thetae * sqrt(max_val(0.0, sqrt(2.0) * st * t[0])), 1e-12);
+    double k0, k1, k2;
+    {
+        double y[1] = {1.0};
+        exact_quots(y, thetae);
+        bessel_k012(y[0], k0, k1, k2);
+    }
+    const double exp_x_47 = kp_exp(-KP_OVER(x, 47.2));
+    const double extraterm = (0.011 * exp_x_47 - 369.69342869090815 * kp_pow(x + 1e-16, -8.0 / 3.0)) *
+                             (0.5 + 0.5 * tanh(KP_OVER(kp_log(x) - 4.787491742782046, 0.1)));
+    const double jffunc = 2.011 * kp_exp(-KP_OVER(kp_pow(x, 1.035), 4.7)) -
+                          cos(x / 2.0) * kp_exp(-KP_OVER(kp_pow(x, 1.2), 2.73)) - 0.011 * exp_x_47 + extraterm;
+    double kr[2] = {k0, k1};
+    exact_quots(kr, k2);  // k2 >= 1e-300 > 0
+    const double k0_ratio = kr[0], k1_ratio = kr[1];
     double e11 = jffunc * wp2 * omega0 * omega0;
-    e11 /= safe;
-    e11 /= safe;
-    e11 /= safe;
-    e11 /= safe;
-    e11 *= (k1_ratio + 6.0 * thetae) * st * st;
-    rhoQ = kPi * nu / kCL * e11;
-    const double shgm = 1.0 - 0.11 * log(1.0 + 0.035 * x);
-    const double k0_ratio = k2 > 0.0 ? k0 / k2 : 1.0;
-    const double fit_factor = k0_ratio * shgm;
+    const double shgm = 1.0 - 0.11 * kp_log(1.0 + 0.035 * x);
     double e12 = wp2 * omega0;
-    e12 /= safe;
-    e12 /= safe;
-    e12 /= safe;
+    // e11 / safe^4 and e12 / safe^3, one division at a time
+    if (safe > 1.0 && safe < 1e20 && (abs_val(e11) > 1e-100 || e11 == 0.0) && (e12 > 1e-100 || e12 == 0.0) &&
+        abs_val(e11) < 1e100 && e12 < 1e100) {
+        const ExactRecip r = exact_recip(safe);
+        e11 = exact_quot(e11, r);
+        e12 = exact_quot(e12, r);
+        e11 = exact_quot(e11, r);
+        e12 = exact_quot(e12, r);
+        e11 = exact_quot(e11, r);
+        e12 = exact_quot(e12, r);
+        e11 = exact_quot(e11, r);
+    } else {
+        e11 /= safe;
+        e11 /= safe;
+        e11 /= safe;
+        e11 /= safe;
+        e12 /= safe;
+        e12 /= safe;
+        e12 /= safe;
+    }
+    e11 *= (k1_ratio + 6.0 * thetae) * st * st;
+    rhoQ = KP_OVER(kPi * nu, kCL) * e11;
+    const double fit_factor = k0_ratio * shgm;
     e12 *= fit_factor * ct;
-    rhoV = 2.0 * kPi * nu / kCL * e12;
+    rhoV = KP_OVER(2.0 * kPi * nu, kCL) * e12;
 }
 
 // symphony_rho_V with theta on the field axis (thermal_synchrotron.hpp:433-460).
@@ -265,7 +343,7 @@ __device__ __forceinline__ double rho_V_axis(double nu, double ne, double thetae
     const double x = max_val(thetae * sqrt(max_val(0.0, sqrt(2.0) * st * (1e3 * omega0 / max_val(two_pi_nu, kTiny)))), 1e-12);
     double k0, k1, k2;
     bessel_k012(1.0 / thetae, k0, k1, k2);
-    const double shgm = 1.0 - 0.11 * log(1.0 + 0.035 * x);
+    const double shgm = 1.0 - 0.11 * kp_log(1.0 + 0.035 * x);
     const double k_ratio = k2 > 0.0 ? k0 / k2 : 1.0;
     const double fit_factor = k_ratio * shgm;
     const double safe = max_val(two_pi_nu, kTiny);
@@ -293,7 +371,7 @@ static __device__ __noinline__ Coeffs<double> thermal_coefficients(const Thermal
         const double nus = 3.0 * kEE * s.b * st / (4.0 * kPi * kME * kCL) * s.thetae * s.thetae + 1.0;
         const double x = max_val(nu / max_val(nus, kTiny), kTiny);
         const double xm13 = 1.0 / cbrt(x);
-        const double exp_shape = exp(-1.8899 / xm13);
+        const double exp_shape = kp_exp(-1.8899 / xm13);
         const double pref = s.ne * kEE * kEE * nu / (2.0 * sqrt(3.0) * kCL * s.thetae * s.thetae);
         const double i_val = 2.5651 * (1.0 + 1.92 * xm13 + 0.9977 * xm13 * xm13) * exp_shape;
         const double iq = 2.5651 * (1.0 + 0.93193 * xm13 + 0.499873 * xm13 * xm13) * exp_shape;
@@ -311,33 +389,44 @@ static __device__ __noinline__ Coeffs<double> thermal_coefficients(const Thermal
         if (!(s.thetae > 0.0) || !(s.ne > 0.0) || !(s.b > 0.0) || !(st > 0.0)) {
             jI = jQ = jV = 0.0;
         } else {
-            const double nu_c = kEE * s.b / (2.0 * kPi * kME * kCL);
+            const double nu_c = KP_OVER(kEE * s.b, 2.0 * kPi * kME * kCL);
             const double nu_s = 2.0 / 9.0 * nu_c * st * s.thetae * s.thetae;
-            const double x = max_val(nu / max_val(nu_s, kTiny), kTiny);
-            const double prefactor = s.ne * kEE * kEE * nu_c / kCL;
+            double xq[1] = {nu};
+            exact_quots(xq, max_val(nu_s, kTiny));
+            const double x = max_val(xq[0], kTiny);
+            const double prefactor = KP_OVER(s.ne * kEE * kEE * nu_c, kCL);
             const double term1 = sqrt(2.0) * kPi / 27.0 * st;
             const double x13 = cbrt(x);
             const double sqx = sqrt(x);
             const double sqx13 = sqrt(x13);
-            const double ex13 = exp(-x13);
+            const double ex13 = kp_exp(-x13);
             const double shape = sqx + 1.8877486253633869933 * sqx13;
             jI = prefactor * term1 * (shape * shape) * ex13;
-            const double t2425 = pow(s.thetae, 24.0 / 25.0);
-            const double term2 = (7.0 * t2425 + 35.0) / (10.0 * t2425 + 75.0);
+            const double t2425 = kp_pow(s.thetae, 24.0 / 25.0);
+            double tq[1] = {7.0 * t2425 + 35.0};
+            exact_quots(tq, 10.0 * t2425 + 75.0);
+            const double term2 = tq[0];
             const double shapeq = sqx + term2 * 1.8877486253633869933 * sqx13;
             jQ = prefactor * term1 * (shapeq * shapeq) * ex13;
             const double sin_shift = st * 0.4356824462767121 - s.ct * 0.9001004421765051;
-            const double vt1 = (37.0 - 87.0 * sin_shift) / (100.0 * (s.thetae + 1.0));
-            const double vt2 = pow(1.0 + (pow(s.thetae, 3.0 / 5.0) / 25.0 + 7.0 / 10.0) * pow(x, 9.0 / 25.0), 5.0 / 3.0);
+            double vq[1] = {37.0 - 87.0 * sin_shift};
+            exact_quots(vq, 100.0 * (s.thetae + 1.0));
+            const double vt1 = vq[0];
+            const double vt2 = kp_pow(1.0 + (KP_OVER(kp_pow(s.thetae, 3.0 / 5.0), 25.0) + 7.0 / 10.0) * kp_pow(x, 9.0 / 25.0), 5.0 / 3.0);
             jV = prefactor * vt1 * vt2 * ex13;
         }
     }
     const double nusq = nu * nu;
-    double jI_inv = jI / max_val(nusq, kTiny);
-    double jQ_inv = jQ / max_val(nusq, kTiny);
-    double jV_inv = jV / max_val(nusq, kTiny);
+    double jv[3] = {jI, jQ, jV};
+    exact_quots(jv, max_val(nusq, kTiny));
+    double jI_inv = jv[0], jQ_inv = jv[1], jV_inv = jv[2];
     const double jP_scale = max_val(abs_val(jQ_inv), abs_val(jV_inv));
-    const double jP = jP_scale > 0.0 ? jP_scale * sqrt(sq(jQ_inv / jP_scale) + sq(jV_inv / jP_scale)) : 0.0;
+    double jP = 0.0;
+    if (jP_scale > 0.0) {
+        double q[2] = {jQ_inv, jV_inv};
+        exact_quots(q, jP_scale);
+        jP = jP_scale * exact_sqrt(sq(q[0]) + sq(q[1]));  // between 1 and 2
+    }
     if (jI_inv > 0.0 && jP > 0.0 && jI_inv < jP / max_val(c.max_pol_frac, 1e-30)) {
         const double scale = jI_inv / jP * c.max_pol_frac;
         jQ_inv *= scale;
@@ -346,9 +435,11 @@ static __device__ __noinline__ Coeffs<double> thermal_coefficients(const Thermal
     double aI = 0.0, aQ = 0.0, aV = 0.0;
     const double b_inv = bnu_inv(nu, s.thetae);
     if (b_inv > 0.0) {
-        aI = jI_inv / b_inv;
-        aQ = jQ_inv / b_inv;
-        aV = jV_inv / b_inv;
+        double q[3] = {jI_inv, jQ_inv, jV_inv};
+        exact_quots(q, b_inv);
+        aI = q[0];
+        aQ = q[1];
+        aV = q[2];
     }
     double rQ = 0.0, rV = 0.0;
     rho_QV(nu, s.ne, s.thetae, s.b, st, s.ct, rQ, rV);
@@ -378,17 +469,26 @@ __device__ __forceinline__ void bl_metric(double r, double th, double spin, doub
             gcov[mu][nu] = 0.0;
             gcon[mu][nu] = 0.0;
         }
-    gcov[0][0] = -(1.0 - 2.0 * r / sigma);
-    gcov[0][3] = gcov[3][0] = -2.0 * a * r * sin2 / sigma;
-    gcov[1][1] = sigma / max_val(delta, kTiny);
+    const double ddelta = max_val(delta, kTiny);
+    double by_sigma[5] = {2.0 * r, -2.0 * a * r * sin2, 2.0 * a2 * r * sin2, delta, 1.0};
+    exact_quots(by_sigma, sigma);
+    double by_delta[1] = {sigma};
+    exact_quots(by_delta, ddelta);
+    gcov[0][0] = -(1.0 - by_sigma[0]);
+    gcov[0][3] = gcov[3][0] = by_sigma[1];
+    gcov[1][1] = by_delta[0];
     gcov[2][2] = sigma;
-    gcov[3][3] = (r * r + a2 + 2.0 * a2 * r * sin2 / sigma) * sin2;
-    const double inv_sd = 1.0 / max_val(sigma * delta, kTiny);
+    gcov[3][3] = (r * r + a2 + by_sigma[2]) * sin2;
+    double one[1] = {1.0};
+    exact_quots(one, max_val(sigma * delta, kTiny));
+    const double inv_sd = one[0];
     gcon[0][0] = -((r * r + a2) * (r * r + a2) - a2 * delta * sin2) * inv_sd;
     gcon[0][3] = gcon[3][0] = -2.0 * a * r * inv_sd;
-    gcon[1][1] = delta / sigma;
-    gcon[2][2] = 1.0 / sigma;
-    gcon[3][3] = (delta - a2 * sin2) / max_val(sigma * delta * sin2, kTiny);
+    gcon[1][1] = by_sigma[3];
+    gcon[2][2] = by_sigma[4];
+    double g33[1] = {delta - a2 * sin2};
+    exact_quots(g33, max_val(sigma * delta * sin2, kTiny));
+    gcon[3][3] = g33[0];
 }
 
 __device__ __forceinline__ double signed_nonzero(double x) {
@@ -401,8 +501,10 @@ __device__ __forceinline__ D4 bl_to_cks(double vt, double vr, double vth, double
                                         double spin) {
     const double a = spin;
     const double delta = max_val(r * r - 2.0 * r + a * a, kTiny);
-    const double vt_ks = vt + 2.0 * r / delta * vr;
-    const double vphi_ks = vphi + a / delta * vr;
+    double q[2] = {2.0 * r, a};
+    exact_quots(q, delta);
+    const double vt_ks = vt + q[0] * vr;
+    const double vphi_ks = vphi + q[1] * vr;
     const double dx_dr = cphi * sinth;
     const double dy_dr = sphi * sinth;
     const double dz_dr = costh;
@@ -482,11 +584,12 @@ __device__ __forceinline__ BlCoords riaf_bl_coords(double spin, const D4& x) {
     sincos(q.th, &q.sin_th, &q.cos_th);
     const double sinth_f = max_val(q.sin_th, 1e-30);
     const double denom = max_val(sinth_f * (q.rc * q.rc + a2), kTiny);
-    q.cphi = (q.rc * xx + spin * yy) / denom;
-    q.sphi = (q.rc * yy - spin * xx) / denom;
-    const double normp = sqrt(max_val(q.cphi * q.cphi + q.sphi * q.sphi, kTiny));
-    q.cphi /= normp;
-    q.sphi /= normp;
+    double cs[2] = {q.rc * xx + spin * yy, q.rc * yy - spin * xx};
+    exact_quots(cs, denom);
+    const double normp = sqrt(max_val(cs[0] * cs[0] + cs[1] * cs[1], kTiny));
+    exact_quots(cs, normp);
+    q.cphi = cs[0];
+    q.sphi = cs[1];
     return q;
 }
 
@@ -502,12 +605,12 @@ __device__ __forceinline__ int riaf_plasma(const ImageConsts& c, const BlCoords&
         const double zc = r_bl * q.cos_th;
         const double rcyl = max_val(r_bl * q.sin_th, c.min_radius);
         const double h = max_val(c.disk_h, 1e-6);
-        const double vertical = exp(-(zc * zc) / (2.0 * rcyl * rcyl * h * h));
-        ne_norm = c.nth0 * vertical * pow(max_val(r_bl, c.min_radius), c.pow_nth);
+        const double vertical = kp_exp(-(zc * zc) / (2.0 * rcyl * rcyl * h * h));
+        ne_norm = c.nth0 * vertical * kp_pow(max_val(r_bl, c.min_radius), c.pow_nth);
     }
     if (!(ne_norm > 0.0)) return 0;
     ne = ne_norm * c.ne_unit;
-    thetae = max_val(c.Te0 * pow(max_val(r_bl, c.min_radius), c.pow_T) * c.thetae_unit, c.min_thetae);
+    thetae = max_val(c.Te0 * kp_pow(max_val(r_bl, c.min_radius), c.pow_T) * c.thetae_unit, c.min_thetae);
     {
         const double bb = sqrt(max_val(8.0 * kPi * 0.1 * ne * kMP * kCL * kCL / (6.0 * max_val(r_bl, c.min_radius)), 0.0));
         b = max_val(bb, 1e-12);

@@ -290,156 +290,6 @@ __device__ __forceinline__ int trace_pass_a(const ImageConsts& c, Ray& state, in
     return entered && (pa_reason == kReachedInner || pa_reason == kEscaped);
 }
 
-// Pass B (pass_b.hpp:940-1114 / :1312-1501) with NF channels, FP64 transfer.
-template<int NF>
-__device__ __forceinline__ void trace_pass_b_fp64(const ImageConsts& c, Ray& state,
-                                                  Stokes4<double> (&stokes)[NF], int& steps,
-                                                  int& reason) {
-    const double mass = c.mass, spin = c.spin;
-    StepControl ctl;
-    ctl.tolerance = c.tolerance;
-    ctl.min_step = c.min_step_abs;
-    ctl.max_step = c.max_step;
-#pragma unroll
-    for (int f = 0; f < NF; ++f) stokes[f] = Stokes4<double>{0.0, 0.0, 0.0, 0.0};
-    int reached = 0;
-    steps = 0;
-    double h_current = c.step;
-    double cap = c.max_radiation_step > 0.0 ? c.max_radiation_step : c.max_step;
-    const double eff_min = c.min_step_abs;
-#pragma unroll 1
-    while (!reached && steps < c.max_steps) {
-        double h = h_current;
-        const Ray old = state;
-        const double start_r = ks_radius(spin, old.x);
-        if (start_r <= c.outer_radius && cap > 0.0) h = min_val(h, cap);
-        Ray next, sample;
-        if (c.adaptive) {
-            AdaptiveStep st;
-            adaptive_step(c.integrator, mass, spin, old, h, ctl, st);
-            if (!st.accepted) {
-                h_current = abs_val(st.next_h);
-                if (h_current <= eff_min * 1.0001) {
-                    reason = kAdaptiveUnderflow;
-                    break;
-                }
-                continue;
-            }
-            h = abs_val(st.used_h);
-            h_current = abs_val(st.next_h);
-            next = st.state;
-            sample = st.mid_state;
-        } else {
-            next = rk4_step(mass, spin, old, h);
-            sample = next;
-        }
-        const double old_r = start_r;
-        const double s0 = old_r - c.cam_radius;
-        const double s1 = ks_radius(spin, next.x) - c.cam_radius;
-        const int crosses = (s0 == 0.0 || s1 == 0.0) ? 1 : ((s0 < 0.0 && s1 > 0.0) || (s0 > 0.0 && s1 < 0.0));
-        if (crosses) {
-            const double denom = s0 - s1;
-            const double frac = abs_val(denom) <= kTiny ? 1.0 : min_val(1.0, max_val(0.0, s0 / denom));
-            const double h_cross = h * frac;
-            if (abs_val(h_cross) <= 1e-14) {
-                h = 0.0;
-                next = old;
-                sample = old;
-            } else if (frac < 0.999999999999) {
-                h = h_cross;
-                if (c.adaptive) {
-                    StepControl cc = ctl;
-                    cc.min_step = min_val(eff_min, abs_val(h));
-                    cc.max_step = max_val(cc.min_step, abs_val(h));
-                    AdaptiveStep cs;
-                    adaptive_step(c.integrator, mass, spin, old, h, cc, cs);
-                    if (!cs.accepted) {
-                        h_current = abs_val(cs.next_h);
-                        continue;
-                    }
-                    h = abs_val(cs.used_h);
-                    next = cs.state;
-                    sample = cs.mid_state;
-                } else {
-                    next = rk4_step(mass, spin, old, h);
-                    sample = next;
-                }
-            }
-        }
-        const double sample_r = ks_radius(spin, sample.x);
-        const double next_r = ks_radius(spin, next.x);
-        const double local_max_rs =
-            (c.max_radiation_step > 0.0 &&
-             (old_r <= c.outer_radius || sample_r <= c.outer_radius || next_r <= c.outer_radius))
-                ? c.max_radiation_step : 0.0;
-        Coeffs<double> co[NF];
-        const int inside = sample_r - c.inner_radius > 0.0 && sample_r < c.outer_radius;
-        RiafSample ps;
-        ps.emitting = 0;
-        if (inside) ps = riaf_sample(c, sample);
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            co[f] = riaf_coefficients(c, ps, c.freq[f]);
-            if (!c.faraday_rotation) co[f].rV = 0.0;
-        }
-        // Substep counts at h (required) and at h_current (predictive) in
-        // one pass: neither test changes h or h_current.  Over the image's
-        // frequencies, or over a separate step-control list
-        // (pass_b.hpp:1787-1833).
-        int required = 1, pred = 1;
-        if (c.nctl == 0) {
-#pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                const int cand = radiation_substep_count(co[f], h, c.dlambda_scale[f], local_max_rs,
-                                                         c.max_radiation_depth, c.max_absorption_depth,
-                                                         c.max_faraday_depth);
-                required = cand > required ? cand : required;
-                const int pc = radiation_substep_count(co[f], h_current, c.dlambda_scale[f], local_max_rs,
-                                                       c.max_radiation_depth, c.max_absorption_depth,
-                                                       c.max_faraday_depth);
-                pred = pc > pred ? pc : pred;
-            }
-        } else {
-#pragma unroll 1
-            for (int g = 0; g < c.nctl; ++g) {
-                Coeffs<double> cg = riaf_coefficients(c, ps, c.ctl_freq[g]);
-                if (!c.faraday_rotation) cg.rV = 0.0;
-                const int cand = radiation_substep_count(cg, h, c.ctl_dlambda_scale[g], local_max_rs,
-                                                         c.max_radiation_depth, c.max_absorption_depth,
-                                                         c.max_faraday_depth);
-                required = cand > required ? cand : required;
-                const int pc = radiation_substep_count(cg, h_current, c.ctl_dlambda_scale[g], local_max_rs,
-                                                       c.max_radiation_depth, c.max_absorption_depth,
-                                                       c.max_faraday_depth);
-                pred = pc > pred ? pc : pred;
-            }
-        }
-        if (required > 1 && h > eff_min * 1.0001) {
-            h_current = max_val(eff_min, h / double(required));
-            cap = h_current;
-            continue;
-        }
-        if (local_max_rs > 0.0 || c.max_radiation_depth > 0.0 || c.max_absorption_depth > 0.0 ||
-            c.max_faraday_depth > 0.0) {
-            cap = pred > 1 ? max_val(eff_min, h_current / double(pred)) : c.max_step;
-        } else {
-            cap = c.max_step;
-        }
-        if (h > 0.0) {
-#pragma unroll
-            for (int f = 0; f < NF; ++f) stokes_step(stokes[f], co[f], abs_val(h) * c.dlambda_scale[f]);
-        }
-        state = next;
-        steps += 1;
-        if (crosses) reached = 1;
-    }
-    if (reached) {
-        reason = kReachedCamera;
-    } else if (reason != kAdaptiveUnderflow) {
-        reason = kMaxSteps;
-    }
-}
-
 // Screen overlap, observer transform and closure diagnostics
 // (pass_b.hpp:87-98, :1096-1113; stokes_rotation.hpp:39-57).
 template<class R, int NF>

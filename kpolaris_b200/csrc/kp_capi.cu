@@ -417,6 +417,7 @@ ImageConsts make_consts(const kp_pass_a_params* p, const kp_riaf_model* m, const
     {
         const double kbol = 1.380649e-16, me = 9.1093837015e-28, cl = 2.99792458e10;
         c.thetae_unit = m->te_unit * kbol / (me * cl * cl);  // riaf.hpp:67-74
+        c.log_te0 = std::log(std::max(c.Te0 * c.thetae_unit, 1e-300));
     }
     c.isco = isco_radius(p->spin);
     // Boundary of the far phase: two of the longest steps either pass can

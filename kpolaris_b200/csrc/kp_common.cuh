@@ -111,6 +111,7 @@ struct ImageConsts {
     double keplerian_factor, infall_factor;
     double min_frequency_scale, min_sin_theta, min_thetae, min_radius;
     double thetae_unit;  // te_unit * k_B / (m_e c^2)
+    double log_te0;      // log(Te0 thetae_unit)
     double isco;         // isco_radius(spin), riaf.hpp:166-174
     // boundary of the far phase (FP32 contraction under the mixed policy):
     // outside the radiating sphere by two of the longest steps

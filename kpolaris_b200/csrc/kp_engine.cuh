@@ -47,14 +47,14 @@ struct PolicyFP64 {
     static constexpr bool kMixed = false;
 };
 // Mixed policy: FP64 state, connection (in factored, fused form), step control
-// and Stokes transfer; many far-field steps taken at once (kp_quad.cuh); FP32
-// transfer coefficients.
+// and radiation (factored, fused forms that round differently); many far-field
+// steps taken at once (kp_quad.cuh).
 struct PolicyMixed {
     static constexpr bool kMixed = true;
 };
 
 // Radiation side of a policy and scene: FP64 (the reference's arithmetic) or
-// FP32 coefficients with the per-frequency 2^E emission scale
+// the factored form with the per-frequency 2^E emission scale
 // (kp_radiation_f32.cuh).
 template<class P, class S = SceneRiaf>
 struct RadTraits;
@@ -105,10 +105,14 @@ struct RadTraits<PolicyMixed, SceneRiaf> {
         return s;
     }
     __device__ static Co coeffs(const ImageConsts& c, const Sample& p, int f) {
-        return riaf_coefficients_f(c, p, float(c.freq[f] * 1e-9), c.emission_scale_pow2[f]);
+        return riaf_coefficients_f(c, p, c.freq[f] * 1e-9, c.emission_scale_pow2[f]);
     }
     __device__ static Co coeffs_ctl(const ImageConsts& c, const Sample& p, int g) {
-        return riaf_coefficients_f(c, p, float(c.ctl_freq[g] * 1e-9), c.ctl_emission_scale_pow2[g]);
+        return riaf_coefficients_f(c, p, c.ctl_freq[g] * 1e-9, c.ctl_emission_scale_pow2[g]);
+    }
+    __device__ static RadDepths depths(const Co& co, double dls) {
+        return RadDepths{abs_val(co.aI) + norm_refined(co.aQ, co.aU, co.aV), norm_refined(co.rQ, co.rU, co.rV),
+                         abs_val(dls)};
     }
     __device__ static void step(Stokes& s, const Co& co, double h, const ImageConsts& c, int f) {
         stokes_step_m(s, co, abs_val(h) * c.dlambda_scale[f]);
@@ -118,13 +122,6 @@ struct RadTraits<PolicyMixed, SceneRiaf> {
         return Stokes4<double>{s.I * inv, s.Q * inv, s.U * inv, s.V * inv};
     }
 };
-
-// Depths per dl of FP32 coefficients: their norms carry the coefficients'
-// own single precision.
-__device__ __forceinline__ RadDepths radiation_depths(const CoeffsF& co, double dls) {
-    return RadDepths{double(fabsf(co.aI) + sqrtf(co.aQ * co.aQ + co.aU * co.aU + co.aV * co.aV)),
-                     double(sqrtf(co.rQ * co.rQ + co.rU * co.rU + float(co.rV) * float(co.rV))), abs_val(dls)};
-}
 
 // GRMHD grid plasma, FP64 throughout.
 template<>
@@ -154,24 +151,23 @@ struct RadTraits<PolicyFP64, SceneGrmhd> {
 
 // GRMHD grid plasma under the mixed policy: the grid gather, the fluid and
 // field four-vectors and the screen angle stay FP64 (grmhd_sample, the
-// reference's fluid_state); the thermal fit per frequency runs in FP32 with
-// the 2^E emission scale, the same code as the mixed RIAF scene.
+// reference's fluid_state); the thermal fit per frequency and the transfer
+// are the mixed RIAF scene's.
 __device__ __forceinline__ RiafSampleF grmhd_sample_to_f(const ImageConsts& c, const GrmhdSample& p) {
     RiafSampleF o;
-    o.emitting = p.emitting;
+    o.emitting = p.emitting && p.ne > 0.0;
     o.on_axis = 0;
     o.has_chi = p.has_chi;
-    if (!p.emitting) return o;
-    o.ne = float(p.ne);
-    o.thetae = float(p.thetae);
-    o.b = float(p.b);
-    o.nu_fluid = float(p.nu_scale);
-    o.cos_theta = float(p.ct);
-    o.sin_theta = float(p.st);
-    o.theta = 0.0f;
-    o.cos2chi = float(p.cos2chi);
-    o.sin2chi = float(p.sin2chi);
-    riaf_sample_thermal_f(c, o, p.ne, p.thetae, p.b, p.ct, p.st, p.nu_scale);
+    if (!o.emitting) return o;
+    o.ne = p.ne;
+    o.thetae = p.thetae;
+    o.b = p.b;
+    o.nu_fluid = p.nu_scale;
+    o.cos_theta = p.ct;
+    o.sin_theta = p.st;
+    o.cos2chi = p.cos2chi;
+    o.sin2chi = p.sin2chi;
+    riaf_sample_thermal_f(c, o);
     return o;
 }
 
@@ -202,7 +198,7 @@ struct RadTraits<PolicyMixed, SceneGrmhdSlow> : RadTraits<PolicyMixed, SceneRiaf
 
 // The RIAF in Boyer-Lindquist coordinates: the same plasma model, sampled
 // in the ray's own BL components (riaf_sample_t<true>); under the mixed
-// policy the FP64 sample feeds the FP32 fits.
+// policy its sample feeds the factored fits.
 template<>
 struct RadTraits<PolicyFP64, SceneRiafBL> : RadTraits<PolicyFP64, SceneRiaf> {
     __device__ static Sample sample(const ImageConsts& c, const Ray& r) { return riaf_sample_t<true>(c, r); }
@@ -214,16 +210,15 @@ __device__ __forceinline__ RiafSampleF riaf_sample_to_f(const ImageConsts& c, co
     o.on_axis = p.on_axis;
     o.has_chi = p.has_chi;
     if (!p.emitting) return o;
-    o.ne = float(p.ne);
-    o.thetae = float(p.thetae);
-    o.b = float(p.b);
-    o.nu_fluid = float(p.nu_fluid);
-    o.cos_theta = float(p.cos_theta);
-    o.sin_theta = float(p.sin_theta);
-    o.theta = float(p.theta);
-    o.cos2chi = float(p.cos2chi);
-    o.sin2chi = float(p.sin2chi);
-    riaf_sample_thermal_f(c, o, p.ne, p.thetae, p.b, p.cos_theta, p.sin_theta, p.nu_fluid);
+    o.ne = p.ne;
+    o.thetae = p.thetae;
+    o.b = p.b;
+    o.nu_fluid = p.nu_fluid;
+    o.cos_theta = p.cos_theta;
+    o.sin_theta = p.sin_theta;
+    o.cos2chi = p.cos2chi;
+    o.sin2chi = p.sin2chi;
+    riaf_sample_thermal_f(c, o);
     return o;
 }
 

@@ -882,7 +882,7 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
                                     if (!c.faraday_rotation) cg.rV = 0.0;
                                     dls = c.ctl_dlambda_scale[g];
                                 }
-                                const RadDepths depth = radiation_depths(cg, dls);
+                                const RadDepths depth = RT::depths(cg, dls);
                                 const int cand = substeps_for(depth, h, local_max_rs, c);
                                 required = cand > required ? cand : required;
                                 const int pc = substeps_for(depth, st.h_current, local_max_rs, c);

@@ -1,19 +1,21 @@
-// kp_radiation_f32.cuh -- FP32 radiation side of the mixed-precision path:
-// RIAF plasma state, thermal synchrotron coefficients and the Strang transfer
-// step, with the same formulas as kp_radiation.cuh (and the reference's
+// kp_radiation_f32.cuh -- the radiation side of the mixed policy: RIAF plasma
+// state, thermal synchrotron coefficients and the Strang transfer step, with
+// the formulas of kp_radiation.cuh (and the reference's
 // src/model/riaf.hpp:54-549, src/radiation/thermal_synchrotron.hpp:60-627,
-// src/radiation/semi_analytic.hpp:10-100) rearranged for FP32 range:
+// src/radiation/semi_analytic.hpp:10-100) factored for throughput: every power
+// of an argument from one logarithm, refined hardware reciprocals and square
+// roots, dot products through the Kerr-Schild vector, frequency-independent
+// factors once per sample, the Bessel K ratios without their common
+// e^-x / sqrt(x).
 //
-//  * invariant emissivities j ~ 1e-38..1e-48 underflow FP32, so emission and
-//    the Stokes vector carry a per-image, per-frequency factor 2^E (the
-//    transfer equation is linear in (j, S)); the image is unscaled in FP64;
-//  * absorption a = j / B_nu is formed as j_phys * [c^2/(2h)] (e^x - 1) / nu^2
-//    with nu in GHz so every intermediate stays inside FP32 range;
-//  * the Bessel K ratios cancel the common e^-x / sqrt(x) factor;
-//  * the plasma's geometry, its profiles, the Faraday phase and the Stokes
-//    update are FP64.
-// Absorption and Faraday coefficients times the affine step are O(1) and
-// need no scaling.
+// All of it is FP64.  A Faraday-thick ray turns its polarisation through
+// thousands of radians, and powers of two of its depths decide how its steps
+// are cut: coefficients in single precision put 1e-6 into Stokes I, up to 1e-3
+// into Q and U, and let one image in a few lose a pixel to a decision that
+// fell the other way.  On quads the difference in time is a tenth of near-B.
+//
+// Emission and the Stokes vector carry a per-image, per-frequency factor 2^E
+// (the transfer equation is linear in (j, S)); the image is unscaled at the end.
 #pragma once
 
 #include "kp_geometry_f32.cuh"
@@ -21,57 +23,39 @@
 namespace kp {
 
 namespace f32c {
-constexpr float kPi = 3.14159265358979323846f;
+constexpr double kPiD = 3.141592653589793;
 constexpr double kEE = 4.803204712570263e-10;
 constexpr double kME = 9.1093837015e-28;
 constexpr double kCL = 2.99792458e10;
 constexpr double kHPL = 6.62607015e-27;
 constexpr double kMP = 1.67262192369e-24;
-// nu_c = e B / (2 pi m_e c) per gauss
-constexpr float kNuCPerB = float(kEE / (2.0 * 3.141592653589793 * kME * kCL));
-// e^2 / c
-constexpr float kE2OverC = float(kEE * kEE / kCL);
-// sqrt(2) pi / 27
-constexpr float kTerm1 = float(1.4142135623730951 * 3.141592653589793 / 27.0);
-// h / (m_e c^2) * 1e9 : x = h nu / (m_e c^2 Theta_e) with nu in GHz
-constexpr float kHOverMc2GHz = float(kHPL / (kME * kCL * kCL) * 1e9);
-// c^2 / (2 h) / 1e18 : absorption factor with nu in GHz
-constexpr float kC2Over2hGHz2 = float(kCL * kCL / (2.0 * kHPL) / 1e18);
-// omega0 per gauss: e / (m_e c)
-constexpr float kOmega0PerB = float(kEE / (kME * kCL));
-// wp^2 per n_e: 4 pi e^2 / m_e
-constexpr float kWp2PerNe = float(4.0 * 3.141592653589793 * kEE * kEE / kME);
+// Pandya emission: e^2 / c times the cyclotron frequency per gauss; sqrt(2) pi / 27
+constexpr double kPandyaPref = kEE * kEE / kCL * (kEE / (2.0 * kPiD * kME * kCL));
+constexpr double kTerm1 = 1.4142135623730951 * kPiD / 27.0;
+// h / (m_e c^2) and c^2 / (2 h)
+constexpr double kHOverMc2 = kHPL / (kME * kCL * kCL);
+constexpr double kC2Over2h = kCL * kCL / (2.0 * kHPL);
 // Dexter: 3 e / (4 pi m_e c); Pandya: 2/9 of the cyclotron frequency
-constexpr double kDexNus = 3.0 * kEE / (4.0 * 3.141592653589793 * kME * kCL);
-constexpr double kPandyaNus = 2.0 / 9.0 * kEE / (2.0 * 3.141592653589793 * kME * kCL);
+constexpr double kDexNus = 3.0 * kEE / (4.0 * kPiD * kME * kCL);
+constexpr double kPandyaNus = 2.0 / 9.0 * kEE / (2.0 * kPiD * kME * kCL);
+// Dexter prefactors e^2 / (2 sqrt(3) c) and 2 e^2 / (3 sqrt(3) c)
+constexpr double kDexPref = kEE * kEE / (2.0 * 1.7320508075688772 * kCL);
+constexpr double kDexPrefV = 2.0 * kEE * kEE / (3.0 * 1.7320508075688772 * kCL);
 // (x / Theta_e)^2 of the Faraday fits: sqrt(2) 1e3 omega0 / (2 pi nu) per gauss and 1 / nu
-constexpr double kFaradayX2 = 1.4142135623730951 * 1e3 * kEE / (kME * kCL) / (2.0 * 3.141592653589793);
-// Dexter prefactor e^2 / (2 sqrt(3) c)
-constexpr float kDexPref = float(kEE * kEE / (2.0 * 1.7320508075688772 * kCL));
-// Dexter jV prefactor 2 e^2 / (3 sqrt(3) c)
-constexpr float kDexPrefV = float(2.0 * kEE * kEE / (3.0 * 1.7320508075688772 * kCL));
+constexpr double kFaradayX2 = 1.4142135623730951 * 1e3 * kEE / (kME * kCL) / (2.0 * kPiD);
 // rho_V nu = (4 pi e^2 / m_e) (e / (m_e c)) n_e B cos(theta) / (4 pi^2 c nu) x fit
-constexpr double kRhoV = (4.0 * 3.141592653589793 * kEE * kEE / kME) * (kEE / (kME * kCL)) /
-                         (4.0 * 3.141592653589793 * 3.141592653589793 * kCL);
+constexpr double kRhoV = (4.0 * kPiD * kEE * kEE / kME) * (kEE / (kME * kCL)) / (4.0 * kPiD * kPiD * kCL);
+// rho_Q nu = (4 pi e^2 / m_e) (e / (m_e c))^2 n_e B^2 sin^2(theta) / (2^4 pi^3 c nu^2) x fit
+constexpr double kRhoQ = (4.0 * kPiD * kEE * kEE / kME) * (kEE / (kME * kCL)) * (kEE / (kME * kCL)) * kPiD /
+                         (16.0 * kPiD * kPiD * kPiD * kPiD * kCL);
 }  // namespace f32c
 
-struct CoeffsF {
-    float jI, jQ, jU, jV, aI, aQ, aU, aV, rQ, rU;
-    double rV;  // the phase of thousands of radians that Faraday-thick rays gather
-};
-
-KP_HD float kp_rsqrtf(float x) {
-#ifdef __CUDA_ARCH__
-    return rsqrtf(x);
-#else
-    return 1.0f / sqrtf(x);
-#endif
-}
+using CoeffsF = Coeffs<double>;
 
 // K0/K2 and K1/K2 for x = 1/Theta_e with the polynomial fits of
 // thermal_synchrotron.hpp:108-158; for x > 2 the factor e^-x / sqrt(x) cancels.
 template<class T>
-KP_HD void bessel_ratios(T x, T& r0, T& r1) {
+KP_HD void bessel_ratios(T x, T lg, T& r0, T& r1) {  // lg = log(x / 2)
     T p, q;
     if (x <= T(2)) {
         const T y = x * x * T(0.25);
@@ -97,7 +81,6 @@ KP_HD void bessel_ratios(T x, T& r0, T& r1) {
         a = T(0.23069756) + y * a;
         a = T(0.42278420) + y * a;
         a = T(-0.57721566) + y * a;
-        const T lg = log(x * T(0.5));
         p = a - lg * i0;
         T b = T(-0.00004686);
         b = T(-0.00110404) + y * b;
@@ -130,21 +113,19 @@ KP_HD void bessel_ratios(T x, T& r0, T& r1) {
     r1 = k2 > T(0) ? q * inv : T(1);
 }
 
-// Plasma state at a sample point (FP32), with the frequency-independent
-// factors of the thermal fits (riaf_sample_thermal_f).  The Faraday rotation
-// adds up to hundreds of radians along a thick ray, where a single-precision
-// rounding of n_e B K0/K2 cos(theta), repeated at every step, becomes an
-// error of the polarisation: that factor is formed in FP64.
+// Plasma state at a sample point, with the frequency-independent factors of
+// the thermal fits (riaf_sample_thermal_f).
 struct RiafSampleF {
-    double rv0;     // rho_V nu at nu = nu_fluid hertz, without the fit's logarithm
-    double xf0;     // argument of the Faraday fits at nu = nu_fluid hertz (it falls as nu^-1/2)
+    double ne, thetae, b, nu_fluid, cos_theta, sin_theta, theta, cos2chi, sin2chi;
     double xs0;     // argument of the emission fit, over the frequency in hertz
+    double xf0;     // argument of the Faraday fits times the root of the frequency
+    double rv0;     // rho_V nu times the frequency, without the fit's logarithm
+    double rq0;     // rho_Q nu times the frequency squared, without the fit's function of x
+    double pref;    // emission prefactor
+    double qterm;   // (7 T^0.96 + 35) / (10 T^0.96 + 75), Pandya jQ
+    double vt1;     // (37 - 87 sin(theta - 0.45)) / (100 (T + 1)), Pandya jV
+    double vt2a;    // T^0.6 / 25 + 0.7, Pandya jV
     int emitting, on_axis, has_chi;
-    float ne, thetae, b, nu_fluid, cos_theta, sin_theta, theta, cos2chi, sin2chi;
-    float r0, r1;   // K0/K2, K1/K2 at 1/Theta_e (Faraday fits)
-    float qterm;    // (7 T^0.96 + 35) / (10 T^0.96 + 75), Pandya jQ
-    float vt1;      // (37 - 87 sin(theta - 0.45)) / (100 (T + 1)), Pandya jV
-    float vt2a;     // T^0.6 / 25 + 0.7, Pandya jV
 };
 
 // Cube root of x > 0 to a few ulp: Newton's step in FP64 from a
@@ -161,47 +142,37 @@ KP_HD double cube_root(double x) {
     return y - (y2 * y - x) * kp_recip<double>(3.0 * y2);
 }
 
-// x^y for x > 0 as 2^(y log2 x): one LG2 shared by several powers of x.
-KP_HD float pow2_of(float y, float lg2x) {
-#ifdef __CUDA_ARCH__
-    return exp2f(y * lg2x);
-#else
-    return std::exp2(y * lg2x);
-#endif
-}
-
 // Frequency-independent factors of the thermal fits at one sample
 // (thermal_synchrotron.hpp:312-395, 462-506), evaluated once per sample
-// instead of once per frequency.
-KP_HD void riaf_sample_thermal_f(const ImageConsts& c, RiafSampleF& p, double ne, double thetae, double b,
-                                 double cos_theta, double sin_theta, double nu_fluid) {
+// instead of once per frequency.  lt = log(Theta_e).
+KP_HD void riaf_sample_thermal_f(const ImageConsts& c, RiafSampleF& p, double lt) {
+    const double te = p.thetae, st = max_val(p.sin_theta, c.min_sin_theta);
+    const double inv_nu = kp_recip<double>(p.nu_fluid);
     double r0, r1;
-    bessel_ratios<double>(kp_recip<double>(thetae), r0, r1);
-    p.r0 = float(r0);
-    p.r1 = float(r1);
-    const double inv_nu = kp_recip<double>(nu_fluid), sth = max_val(sin_theta, c.min_sin_theta);
-    p.rv0 = f32c::kRhoV * ne * b * r0 * cos_theta * inv_nu;
+    bessel_ratios<double>(kp_recip<double>(te), -lt - 0.69314718055994530942, r0, r1);
+    p.rv0 = f32c::kRhoV * p.ne * p.b * r0 * p.cos_theta * inv_nu;
+    p.rq0 = f32c::kRhoQ * p.ne * (p.b * p.b) * (r1 + 6.0 * te) * (st * st) * (inv_nu * inv_nu);
     {
         double g, inv;
-        kp_sqrt_pair<double>(max_val(f32c::kFaradayX2 * sth * b * inv_nu, 1e-60), g, inv);
-        p.xf0 = thetae * g;
+        kp_sqrt_pair<double>(max_val(f32c::kFaradayX2 * st * p.b * inv_nu, 1e-200), g, inv);
+        p.xf0 = te * g;
     }
-    const double nus = c.fit == 4 ? f32c::kDexNus * b * sth * thetae * thetae + 1.0
-                                  : f32c::kPandyaNus * b * sth * thetae * thetae;
-    p.xs0 = nu_fluid * kp_recip<double>(max_val(nus, 1e-60));
-    const float te = p.thetae;
-    const float lt = log2f(te);
-    const float t2425 = pow2_of(24.0f / 25.0f, lt);
-    p.qterm = (7.0f * t2425 + 35.0f) / (10.0f * t2425 + 75.0f);
-    const float st = fmaxf(p.sin_theta, float(c.min_sin_theta));
-    const float sin_shift = st * 0.4356824462767121f - p.cos_theta * 0.9001004421765051f;
-    p.vt1 = (37.0f - 87.0f * sin_shift) / (100.0f * (te + 1.0f));
-    p.vt2a = pow2_of(0.6f, lt) / 25.0f + 0.7f;
+    const double nus = c.fit == 4 ? f32c::kDexNus * p.b * st * te * te + 1.0 : f32c::kPandyaNus * p.b * st * te * te;
+    p.xs0 = p.nu_fluid * kp_recip<double>(max_val(nus, 1e-200));
+    p.qterm = p.vt1 = p.vt2a = 0.0;
+    if (c.fit == 4) {
+        p.pref = p.ne * kp_recip<double>(te * te);
+        return;
+    }
+    p.pref = f32c::kPandyaPref * p.ne * p.b;
+    const double t2425 = exp(0.96 * lt);
+    p.qterm = (7.0 * t2425 + 35.0) * kp_recip<double>(10.0 * t2425 + 75.0);
+    const double sin_shift = st * 0.4356824462767121 - p.cos_theta * 0.9001004421765051;
+    p.vt1 = (37.0 - 87.0 * sin_shift) * kp_recip<double>(100.0 * (te + 1.0));
+    p.vt2a = exp(0.6 * lt) * 0.04 + 0.7;
 }
 
-KP_HD void riaf_sample_thermal_f(const ImageConsts& c, RiafSampleF& p) {
-    riaf_sample_thermal_f(c, p, p.ne, p.thetae, p.b, p.cos_theta, p.sin_theta, p.nu_fluid);
-}
+KP_HD void riaf_sample_thermal_f(const ImageConsts& c, RiafSampleF& p) { riaf_sample_thermal_f(c, p, log(p.thetae)); }
 
 // Boyer-Lindquist metric entries at (r, theta) with unit mass, FP64.
 struct BlEntries {
@@ -226,8 +197,7 @@ KP_HD BlEntries bl_entries(double r, double s2, double c2, double a) {
     return m;
 }
 
-// riaf_sample (kp_radiation.cuh) for the mixed policy: geometry, flow and the
-// plasma's profiles in FP64 with refined reciprocals, the result in FP32.
+// riaf_sample (kp_radiation.cuh) for the mixed policy.
 // With the Kerr-Schild vector l = (1, l1, l2, l3) at the point, g = eta + f l l,
 // so a dot product is eta(u, v) + f (l.u)(l.v) with l.u formed once per
 // vector; (l1, l2) = sin(theta) (cos phi, sin phi) gives the BL angles, and
@@ -250,23 +220,29 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
     const double c2 = min_val(l3 * l3, 1.0), s2 = max_val((x * x + y * y) * inv_rp, 1e-30);
     const double amp = 2.0 * c.mass * r2 * r * kp_recip<double>(r2 * r2 + a2 * z * z);
     // n_e, Theta_e and B (riaf.hpp:54-96)
-    double ne, thetae, b;
+    double ne, thetae, b, lt;
     {
         const double lr = log(r_bl);
         const double h = max_val(c.disk_h, 1e-6);
         const double rcyl2 = max_val(r_bl * r_bl * s2, c.min_radius * c.min_radius);
         const double zc = r_bl * l3;
         ne = c.nth0 * exp(c.pow_nth * lr - zc * zc * kp_recip<double>(2.0 * rcyl2 * h * h));
-        if (!(float(ne) > 0.0f)) return out;
+        if (!(ne > 0.0)) return out;
         ne *= c.ne_unit;
-        thetae = max_val(c.Te0 * exp(c.pow_T * lr) * c.thetae_unit, c.min_thetae);
+        lt = c.log_te0 + c.pow_T * lr;
+        thetae = exp(lt);
+        if (!(thetae > c.min_thetae)) {
+            thetae = c.min_thetae;
+            lt = log(thetae);
+        }
         const double kb = 8.0 * 3.141592653589793 * 0.1 * f32c::kMP * f32c::kCL * f32c::kCL / 6.0;
-        b = max_val(sqrt(max_val(kb * ne * kp_recip<double>(r_bl), 0.0)), 1e-12);
+        double inv;
+        kp_sqrt_pair<double>(max_val(kb * ne * kp_recip<double>(r_bl), 1e-24), b, inv);
     }
     out.emitting = 1;
-    out.ne = float(ne);
-    out.thetae = float(thetae);
-    out.b = float(b);
+    out.ne = ne;
+    out.thetae = thetae;
+    out.b = b;
     // fluid velocity (riaf.hpp:206-273): circular, with the plunge inside the ISCO
     double vt = 1.0, vr = 0.0, vphi = 0.0;
     {
@@ -303,7 +279,8 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
                 vr = plunge ? vr + inf * (ff - vr) : inf * ff;
             }
             const double q = m.tt + 2.0 * omega * m.tp + omega * omega * m.pp;
-            vt = sqrt(max_val(-(1.0 + vr * vr * m.rr) * kp_recip<double>(q), 0.0));
+            double inv;
+            kp_sqrt_pair<double>(max_val(-(1.0 + vr * vr * m.rr) * kp_recip<double>(q), 1e-60), vt, inv);
             vphi = omega * vt;
         }
         const double i_d = kp_recip<double>(max_val(rr * rr - 2.0 * rr + a2, 1e-30));
@@ -349,13 +326,15 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
     }
     const double kb = dot(k, bv);
     const double ct = min_val(max_val(kb * kp_recip<double>(max_val(nu_fluid, 1e-30)), -1.0), 1.0);
-    out.nu_fluid = float(nu_fluid);
-    out.cos_theta = float(ct);
-    const double st = max_val(sqrt(max_val(0.0, 1.0 - ct * ct)), c.min_sin_theta);
-    out.sin_theta = float(st);
-    out.theta = acosf(out.cos_theta);
-    riaf_sample_thermal_f(c, out, ne, thetae, b, ct, st, nu_fluid);
-    if (out.theta <= 0.0f || out.theta >= f32c::kPi) {
+    out.nu_fluid = nu_fluid;
+    out.cos_theta = ct;
+    {
+        double st, inv;
+        kp_sqrt_pair<double>(max_val(1.0 - ct * ct, 1e-60), st, inv);
+        out.sin_theta = max_val(st, c.min_sin_theta);
+    }
+    riaf_sample_thermal_f(c, out, lt);
+    if (ct >= 1.0 || ct <= -1.0) {
         out.on_axis = 1;
         return out;
     }
@@ -374,118 +353,93 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
     if (bproj2 > 1e-30) {
         const double inv = kp_recip<double>(bproj2);
         out.has_chi = 1;
-        out.cos2chi = float((b2 * b2 - b1 * b1) * inv);
-        out.sin2chi = float(-2.0 * b1 * b2 * inv);
+        out.cos2chi = (b2 * b2 - b1 * b1) * inv;
+        out.sin2chi = -2.0 * b1 * b2 * inv;
     }
     return out;
 }
 
-// Thermal coefficients at one frequency, FP32, emission scaled by 2^E
-// (`escale`).  nu_ghz = max(freq * nu_fluid, 1 Hz) in GHz.
-KP_HD CoeffsF riaf_coefficients_f(const ImageConsts& c, const RiafSampleF& p, float freq_ghz,
-                                                        float escale) {
+// Thermal coefficients at one frequency (in GHz), emission scaled by 2^E
+// (`escale`).
+KP_HD CoeffsF riaf_coefficients_f(const ImageConsts& c, const RiafSampleF& p, double freq_ghz, double escale) {
     CoeffsF o = {};
     if (!p.emitting) return o;
-    const float nu = fmaxf(freq_ghz * p.nu_fluid, 1e-9f);  // GHz
-    const float ne = p.ne, te = p.thetae, b = p.b;
-    const float st = fmaxf(p.sin_theta, float(c.min_sin_theta));
-    const float ct = p.cos_theta;
-    const double freq = double(freq_ghz) * 1e9;
-    // Faraday rotation / conversion (symphony_rho_QV), invariant rho * nu
-    float rQ;
-    double rV;
-    {
-        const float omega0 = f32c::kOmega0PerB * b;
-        const float wp2 = f32c::kWp2PerNe * ne;
-        const float inv_w = 1.0f / (2.0f * f32c::kPi * nu * 1e9f);
-        double sf, isf;
-        kp_sqrt_pair<double>(freq, sf, isf);
-        const double xd = max_val(p.xf0 * isf, 1e-12);
-        // eps12 = wp2 omega0 / (2 pi nu)^3 K0/K2 fit cos(theta); rho_V = 2 pi nu / c eps12;
-        // the invariant is rho_V nu (on the axis cos(theta) is 1 or -1 to rounding)
-        rV = p.rv0 * (1.0 - 0.11 * log(1.0 + 0.035 * xd)) * (isf * isf);
-        const float x = float(xd);
-        if (p.on_axis) {
-            o.rV = c.faraday_scale * rV;
-            return o;
-        }
-        // every power of x from one LG2; 0.5 + 0.5 tanh(z) = 1 / (1 + e^-2z)
-        const float lx = log2f(x);
-        const float exp_x_47 = expf(-x / 47.2f);
-        const float z = (lx * 0.6931471805599453f - 4.787491742782046f) / 0.1f;
-        const float sigm = 1.0f / (1.0f + expf(-2.0f * z));
-        const float extraterm = (0.011f * exp_x_47 - 369.69342869090815f * pow2_of(-8.0f / 3.0f, lx)) * sigm;
-        // the cosine term is below 1e-13 of the sum beyond x = 40
-        const float cterm = x < 40.0f ? cosf(x / 2.0f) * expf(-pow2_of(1.2f, lx) / 2.73f) : 0.0f;
-        const float jffunc = 2.011f * expf(-pow2_of(1.035f, lx) / 4.7f) - cterm - 0.011f * exp_x_47 + extraterm;
-        float e11 = jffunc * wp2 * omega0 * inv_w;
-        e11 *= omega0 * inv_w;
-        e11 *= inv_w;
-        e11 *= inv_w;
-        e11 *= (p.r1 + 6.0f * te) * st * st;
-        rQ = float(3.141592653589793 / f32c::kCL) * (nu * 1e9f) * e11 * (nu * 1e9f);
+    const double freq = freq_ghz * 1e9;
+    double sf, isf;
+    kp_sqrt_pair<double>(freq, sf, isf);
+    const double inv_freq = isf * isf;
+    // Faraday rotation and conversion (symphony_rho_QV), invariant rho nu
+    const double x = max_val(p.xf0 * isf, 1e-12);
+    const double rV = p.rv0 * (1.0 - 0.11 * log(1.0 + 0.035 * x)) * inv_freq;
+    if (p.on_axis) {
+        o.rV = c.faraday_scale * rV;
+        return o;
     }
-    // emissivities, scaled by 2^E / nu^2 (nu^2 in Hz^2)
-    float jI, jQ, jV;
-    const float inv_nu2 = escale / (nu * nu) * 1e-18f;  // 2^E / (nu_Hz^2)
+    double rQ;
+    {
+        const double lx = log(x);
+        double j = 2.011 * exp(exp(1.035 * lx) * (-1.0 / 4.7));
+        const double e12 = exp(1.2 * lx) * (-1.0 / 2.73);
+        if (e12 > -60.0) j -= cos(0.5 * x) * exp(e12);
+        const double e47 = 0.011 * exp(x * (-1.0 / 47.2));
+        j -= e47;
+        // 0.5 + 0.5 tanh(z) = 1 / (1 + e^-2z); below z = -20 it is under 1e-17
+        const double z2 = 20.0 * (lx - 4.787491742782046);
+        if (z2 > -40.0) j += (e47 - 369.69342869090815 * exp((-8.0 / 3.0) * lx)) * kp_recip<double>(1.0 + exp(-z2));
+        rQ = p.rq0 * j * (inv_freq * inv_freq);
+    }
+    // emissivities j / nu^2, scaled by 2^E
+    const double nu = max_val(freq * p.nu_fluid, 1.0);
+    const double inv_nu2 = escale * kp_recip<double>(nu * nu);
+    const double xs = max_val(p.xs0 * freq, 1e-200), root = cube_root(xs);
+    double jI, jQ, jV;
     if (c.fit == 4) {
-        const double xd = max_val(p.xs0 * freq, 1e-30), root = cube_root(xd);
-        const float xh = float(xd), xm13 = float(kp_recip<double>(root));
-        const float exps = float(exp(-1.8899 * root));
-        const float pref = f32c::kDexPref * ne * (nu * 1e9f) / (te * te);
-        jI = pref * (2.5651f * (1.0f + 1.92f * xm13 + 0.9977f * xm13 * xm13) * exps) * inv_nu2;
-        jQ = pref * (2.5651f * (1.0f + 0.93193f * xm13 + 0.499873f * xm13 * xm13) * exps) * inv_nu2;
-        const float iv = (1.81384f / xh + 3.42319f * xm13 * xm13 + 0.0292545f * kp_rsqrtf(xh) + 2.03773f * xm13) * exps;
-        float cft = ct;
-        if (fabsf(cft) < 1e-10f) cft = cft >= 0.0f ? 1e-10f : -1e-10f;
-        const float tan_theta = st / cft;
-        jV = f32c::kDexPrefV * ne * (nu * 1e9f) / (tan_theta * te * te * te) * iv * inv_nu2;
+        const double inv_root = kp_recip<double>(root), inv2 = inv_root * inv_root;
+        const double shape = exp(-1.8899 * root);
+        const double pref = f32c::kDexPref * p.pref * nu * shape * inv_nu2;
+        jI = pref * (2.5651 * (1.0 + 1.92 * inv_root + 0.9977 * inv2));
+        jQ = pref * (2.5651 * (1.0 + 0.93193 * inv_root + 0.499873 * inv2));
+        const double iv = 1.81384 * (inv2 * inv_root) + 3.42319 * inv2 + 0.0292545 * sqrt(inv2 * inv_root) + 2.03773 * inv_root;
+        double cft = p.cos_theta;
+        if (abs_val(cft) < 1e-10) cft = cft >= 0.0 ? 1e-10 : -1e-10;
+        const double st = max_val(p.sin_theta, c.min_sin_theta);
+        jV = f32c::kDexPrefV * p.pref * nu * cft * kp_recip<double>(st * p.thetae) * iv * shape * inv_nu2;
     } else {
-        const float nu_c = f32c::kNuCPerB * b;
-        const double xd = max_val(p.xs0 * freq, 1e-30), root = cube_root(xd);
-        const float x = float(xd), x13 = float(root);
-        const float pref = ne * f32c::kE2OverC * nu_c * f32c::kTerm1 * st;
-        const float lx = log2f(x);
-        const float sqx = sqrtf(x), sqx13 = sqrtf(x13);
-        const float ex13 = float(exp(-root));
-        const float sh = sqx + 1.8877486253633869933f * sqx13;
-        jI = pref * (sh * sh) * ex13 * inv_nu2;
-        const float shq = sqx + p.qterm * 1.8877486253633869933f * sqx13;
-        jQ = pref * (shq * shq) * ex13 * inv_nu2;
-        const float vt2 = pow2_of(5.0f / 3.0f, log2f(1.0f + p.vt2a * pow2_of(0.36f, lx)));
-        jV = ne * f32c::kE2OverC * nu_c * p.vt1 * vt2 * ex13 * inv_nu2;
+        double sx, isx, sr, isr;
+        kp_sqrt_pair<double>(xs, sx, isx);
+        kp_sqrt_pair<double>(root, sr, isr);
+        const double st = max_val(p.sin_theta, c.min_sin_theta);
+        const double pref = p.pref * exp(-root) * inv_nu2, lin = pref * f32c::kTerm1 * st;
+        const double bend = 1.8877486253633869933 * sr;
+        const double hi = sx + bend, hq = sx + p.qterm * bend;
+        jI = lin * (hi * hi);
+        jQ = lin * (hq * hq);
+        const double v = 1.0 + p.vt2a * exp(0.36 * log(xs)), rv = cube_root(v);
+        jV = pref * p.vt1 * (v * (rv * rv));
     }
     // polarisation cap (thermal_synchrotron.hpp:575-588)
-    const float jps = fmaxf(fabsf(jQ), fabsf(jV));
-    const float jP = jps > 0.0f ? jps * sqrtf((jQ / jps) * (jQ / jps) + (jV / jps) * (jV / jps)) : 0.0f;
-    const float mpf = float(c.max_pol_frac);
-    if (jI > 0.0f && jP > 0.0f && jI < jP / fmaxf(mpf, 1e-30f)) {
-        const float sc = jI / jP * mpf;
+    const double jp2 = jQ * jQ + jV * jV, mpf = max_val(c.max_pol_frac, 1e-30);
+    if (jI > 0.0 && jp2 > 0.0 && jI * jI * (mpf * mpf) < jp2) {
+        const double sc = jI * c.max_pol_frac / sqrt(jp2);
         jQ *= sc;
         jV *= sc;
     }
-    // Kirchhoff: a = j / B_nu, with B_nu = 2 h nu^3 / (c^2 (e^x - 1))
-    float aI = 0.0f, aQ = 0.0f, aV = 0.0f;
-    if (te > 0.0f) {
-        const float xb = f32c::kHOverMc2GHz * nu / te;
-        const float em1 = expm1f(xb);
-        // j_inv / bnu_inv = j_phys / nu^2 * c^2 (e^x - 1) / (2 h) ; j here carries 2^E / nu^2
-        const float fac = f32c::kC2Over2hGHz2 * em1 / escale * 1e18f;
-        aI = jI * fac;
-        aQ = jQ * fac;
-        aV = jV * fac;
-    }
-    const float es = float(c.emission_scale), as = float(c.absorption_scale), fs = float(c.faraday_scale);
+    // Kirchhoff: a = j / B_nu, with B_nu = 2 h nu^3 / (c^2 (e^x - 1)) and the
+    // reference's series for small x
+    const double xb = f32c::kHOverMc2 * nu * kp_recip<double>(p.thetae);
+    const double em1 = xb < 2e-3 ? xb * (1.0 / 24.0) * (24.0 + xb * (12.0 + xb * (4.0 + xb))) : exp(xb) - 1.0;
+    const double fac = f32c::kC2Over2h * em1 * kp_recip<double>(escale) * c.absorption_scale;
+    const double es = c.emission_scale, fs = c.faraday_scale;
     o.jI = es * jI;
     o.jV = es * jV;
-    o.aI = as * aI;
-    o.aV = as * aV;
-    o.rV = c.faraday_scale * rV;
+    o.aI = fac * jI;
+    o.aV = fac * jV;
+    o.rV = fs * rV;
     if (p.has_chi) {
         o.jQ = es * jQ * p.cos2chi;
         o.jU = es * jQ * p.sin2chi;
-        o.aQ = as * aQ * p.cos2chi;
-        o.aU = as * aQ * p.sin2chi;
+        o.aQ = fac * jQ * p.cos2chi;
+        o.aU = fac * jQ * p.sin2chi;
         o.rQ = fs * rQ * p.cos2chi;
         o.rU = fs * rQ * p.sin2chi;
     }
@@ -493,12 +447,6 @@ KP_HD CoeffsF riaf_coefficients_f(const ImageConsts& c, const RiafSampleF& p, fl
 }
 
 // ---- transfer -----------------------------------------------------------
-// The Strang step in FP64 on FP32 coefficients.  A Faraday-thick ray turns
-// its polarisation through thousands of radians and what is left of it is a
-// small difference of large contributions: rounding the Stokes vector, the
-// rotation or the attenuation to single precision at every step was the
-// largest error of the mixed policy (1e-6 of I, 1e-5 to 1e-3 of Q and U;
-// in FP64 6e-8 and 1e-6 to 1e-5, from the coefficients).
 struct StokesM {
     double I, Q, U, V;  // scaled by 2^E
 };

@@ -12,8 +12,39 @@
 #pragma once
 
 #include "kp_camera.cuh"
+#include "kp_exact.cuh"
+#include "kp_geometry_f32.cuh"
 
 namespace kp {
+
+// The quotients of the FP64 right-hand side.  It has seventeen divisions by
+// nine divisors; the compiler's, at 127 cycles each and one after the other,
+// were two thirds of its 3,000 cycles.  They are formed by shared reciprocals
+// (kp_exact.cuh, the same rounding) without a branch between them, and taken
+// again by the compiler's division in the rare case that an operand was out
+// of that method's range.
+struct FmksDivisor {
+    double b, y;
+};
+
+KP_HD FmksDivisor fmks_divisor(double b) {
+#ifdef __CUDA_ARCH__
+    return FmksDivisor{b, exact_recip(b).y};
+#else
+    return FmksDivisor{b, 0.0};
+#endif
+}
+
+template<bool EXACT>
+KP_HD double fmks_quot(double a, const FmksDivisor& d, bool& in_range) {
+#ifdef __CUDA_ARCH__
+    if constexpr (!EXACT) return plain_quot(a, d.b);
+    in_range = in_range && exact_numerator(a) && exact_divisor(d.b);
+    return exact_quot(a, ExactRecip{d.b, d.y});
+#else
+    return a / d.b;
+#endif
+}
 
 KP_HD double fmks_power(double x, double p) {
     const int n = int(p + 0.5);
@@ -33,11 +64,13 @@ struct FmksTheta {
     double r, th, dth1, dth2, d2th11, d2th12, d2th22;
 };
 
-KP_HD FmksTheta fmks_theta(const FmksParams& m, double x1, double x2) {
-    const double y = 2.0 * x2 - 1.0;
-    const double z = y / m.poly_xt;
-    const double expfac = exp(m.mks_smooth * (m.startx1 - x1));
-    double za, za1, za2;
+// The quotients of the map: za / (alpha + 1), dthJ's second term, d2thJ's
+// factor and its two terms.
+struct FmksMap {
+    double za_al, dj, cj, t1, t2;
+};
+
+KP_HD void fmks_powers(const FmksParams& m, double z, double& za, double& za1, double& za2) {
     if (abs_val(m.poly_alpha - 14.0) < 1e-12) {
         const double z2 = z * z;
         const double z4 = z2 * z2;
@@ -50,16 +83,58 @@ KP_HD FmksTheta fmks_theta(const FmksParams& m, double x1, double x2) {
         za1 = fmks_power(z, m.poly_alpha - 1.0);
         za2 = fmks_power(z, m.poly_alpha - 2.0);
     }
+}
+
+template<bool EXACT>
+KP_HD FmksMap fmks_map(const FmksParams& m, double y, bool& in_range) {
+    const double al1 = m.poly_alpha + 1.0;
+    const FmksDivisor xt = fmks_divisor(m.poly_xt), al = fmks_divisor(al1);
+    const double z = fmks_quot<EXACT>(y, xt, in_range);
+    double za, za1, za2;
+    fmks_powers(m, z, za, za1, za2);
+    FmksMap q;
+    q.za_al = fmks_quot<EXACT>(za, al, in_range);
+    q.cj = fmks_quot<EXACT>(4.0 * m.poly_norm * m.poly_alpha, al, in_range);
+    q.dj = fmks_quot<EXACT>(2.0 * m.poly_alpha * m.poly_norm * y * za1, fmks_divisor(al1 * m.poly_xt), in_range);
+    q.t1 = fmks_quot<EXACT>(2.0 * za1, xt, in_range);
+    q.t2 = fmks_quot<EXACT>(y * (m.poly_alpha - 1.0) * za2, fmks_divisor(m.poly_xt * m.poly_xt), in_range);
+    return q;
+}
+
+template<bool MIXED = false>
+KP_HD FmksTheta fmks_theta(const FmksParams& m, double x1, double x2) {
+    const double y = 2.0 * x2 - 1.0;
+    const double expfac = exp(m.mks_smooth * (m.startx1 - x1));
     double s2, c2;
-    sincos(2.0 * kPi * x2, &s2, &c2);
+    FmksMap q;
+    if constexpr (MIXED) {
+        // reciprocals of the map's constants, and its angle in half turns
+        const double inv_xt = kp_recip<double>(m.poly_xt);
+        const double inv_al1 = kp_recip<double>(m.poly_alpha + 1.0);
+        double za, za1, za2;
+        fmks_powers(m, y * inv_xt, za, za1, za2);
+        q.za_al = za * inv_al1;
+        q.dj = (2.0 * m.poly_alpha * m.poly_norm * y * za1) * (inv_al1 * inv_xt);
+        q.cj = 4.0 * m.poly_norm * m.poly_alpha * inv_al1;
+        q.t1 = 2.0 * za1 * inv_xt;
+        q.t2 = y * (m.poly_alpha - 1.0) * za2 * (inv_xt * inv_xt);
+#ifdef __CUDA_ARCH__
+        sincospi(2.0 * x2, &s2, &c2);
+#else
+        sincos(2.0 * kPi * x2, &s2, &c2);
+#endif
+    } else {
+        bool in_range = true;
+        q = fmks_map<true>(m, y, in_range);
+        if (!in_range) q = fmks_map<false>(m, y, in_range);
+        sincos(2.0 * kPi * x2, &s2, &c2);
+    }
     const double thG = kPi * x2 + ((1.0 - m.hslope) / 2.0) * s2;
-    const double thJ = m.poly_norm * y * (1.0 + za / (m.poly_alpha + 1.0)) + 0.5 * kPi;
+    const double thJ = m.poly_norm * y * (1.0 + q.za_al) + 0.5 * kPi;
     const double dthG = kPi + (1.0 - m.hslope) * kPi * c2;
-    const double dthJ = 2.0 * m.poly_norm * (1.0 + za / (m.poly_alpha + 1.0)) +
-                        (2.0 * m.poly_alpha * m.poly_norm * y * za1) / ((m.poly_alpha + 1.0) * m.poly_xt);
+    const double dthJ = 2.0 * m.poly_norm * (1.0 + q.za_al) + q.dj;
     const double d2thG = -2.0 * (1.0 - m.hslope) * kPi * kPi * s2;
-    const double d2thJ = 4.0 * m.poly_norm * m.poly_alpha / (m.poly_alpha + 1.0) *
-                         (2.0 * za1 / m.poly_xt + y * (m.poly_alpha - 1.0) * za2 / (m.poly_xt * m.poly_xt));
+    const double d2thJ = q.cj * (q.t1 + q.t2);
     FmksTheta t;
     t.r = exp(x1);
     t.th = thG + expfac * (thJ - thG);
@@ -154,49 +229,43 @@ KP_HD double dot_gm(const double g[4][4], const D4& u, const D4& v) {
 
 // Spherical Kerr-Schild connection work at (r, theta): g^{mu nu} and the
 // r- and theta-derivatives of g_{mu nu} (build_spherical_ks_connection_work,
-// kerr_schild_spherical.hpp:198-266).
+// kerr_schild_spherical.hpp:198-266), by their distinct nonzero entries: d/dr
+// g has (A A 0 B), (A A 0 B), (0 0 C 0), (B B 0 D) as its rows and d/dtheta g
+// (E E 0 F0), (E E 0 F1), (0 0 G 0), (F0 F1 0 H).
 struct SksConn {
-    double gcon[4][4], dgr[4][4], dgth[4][4];
+    double g00, g01, g11, g13, g22, g33;
+    double A, B, C, D, E, F0, F1, G, H;
 };
 
-KP_HD SksConn sks_conn(double mass, double a, double r, double th) {
+template<bool EXACT>
+KP_HD SksConn sks_conn(double mass, double a, double r, double s, double cc, bool& in_range) {
     SksConn c;
-    for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) c.gcon[i][j] = c.dgr[i][j] = c.dgth[i][j] = 0.0;
-    double s, cc;
-    sincos(th, &s, &cc);
     const double a2 = a * a, s2 = s * s, safe_s2 = max_val(s2, kTiny);
     const double rho2 = r * r + a2 * cc * cc, rho4 = rho2 * rho2;
-    const double f = 2.0 * mass * r / rho2;
     const double delta = r * r - 2.0 * mass * r + a2;
-    c.gcon[0][0] = -(1.0 + f);
-    c.gcon[0][1] = c.gcon[1][0] = f;
-    c.gcon[1][1] = delta / rho2;
-    c.gcon[1][3] = c.gcon[3][1] = a / rho2;
-    c.gcon[2][2] = 1.0 / rho2;
-    c.gcon[3][3] = 1.0 / (rho2 * safe_s2);
     const double drho_dr = 2.0 * r, drho_dth = -2.0 * a2 * s * cc, ds2_dth = 2.0 * s * cc;
-    const double df_dr = 2.0 * mass * (rho2 - r * drho_dr) / rho4;
-    const double df_dth = -2.0 * mass * r * drho_dth / rho4;
-    auto sr = [&](int m, int n, double v) { c.dgr[m][n] = v; c.dgr[n][m] = v; };
-    auto st = [&](int m, int n, double v) { c.dgth[m][n] = v; c.dgth[n][m] = v; };
-    sr(0, 0, df_dr);
-    st(0, 0, df_dth);
-    sr(0, 1, df_dr);
-    st(0, 1, df_dth);
-    sr(0, 3, -a * s2 * df_dr);
-    st(0, 3, -a * (s2 * df_dth + ds2_dth * f));
-    sr(1, 1, df_dr);
-    st(1, 1, df_dth);
-    sr(1, 3, -a * s2 * df_dr);
-    st(1, 3, -a * (ds2_dth * (1.0 + f) + s2 * df_dth));
-    sr(2, 2, drho_dr);
-    st(2, 2, drho_dth);
+    const FmksDivisor d2 = fmks_divisor(rho2), d4 = fmks_divisor(rho4);
+    const double f = fmks_quot<EXACT>(2.0 * mass * r, d2, in_range);
+    const double df_dr = fmks_quot<EXACT>(2.0 * mass * (rho2 - r * drho_dr), d4, in_range);
+    const double df_dth = fmks_quot<EXACT>(-2.0 * mass * r * drho_dth, d4, in_range);
+    c.g00 = -(1.0 + f);
+    c.g01 = f;
+    c.g11 = fmks_quot<EXACT>(delta, d2, in_range);
+    c.g13 = fmks_quot<EXACT>(a, d2, in_range);
+    c.g22 = fmks_quot<EXACT>(1.0, d2, in_range);
+    c.g33 = fmks_quot<EXACT>(1.0, fmks_divisor(rho2 * safe_s2), in_range);
+    c.A = df_dr;
+    c.B = -a * s2 * df_dr;
+    c.C = drho_dr;
+    c.E = df_dth;
+    c.F0 = -a * (s2 * df_dth + ds2_dth * f);
+    c.F1 = -a * (ds2_dth * (1.0 + f) + s2 * df_dth);
+    c.G = drho_dth;
     const double bracket = rho2 + a2 * s2 * (1.0 + f);
     const double dbr = drho_dr + a2 * s2 * df_dr;
     const double dbt = drho_dth + a2 * (ds2_dth * (1.0 + f) + s2 * df_dth);
-    sr(3, 3, s2 * dbr);
-    st(3, 3, ds2_dth * bracket + s2 * dbt);
+    c.D = s2 * dbr;
+    c.H = ds2_dth * bracket + s2 * dbt;
     return c;
 }
 
@@ -213,11 +282,16 @@ struct FmksConn {
 KP_HD FmksConn fmks_conn(const FmksParams& m, const D4& x) {
     FmksConn o;
     o.t = fmks_theta(m, x.v[1], x.v[2]);
-    o.c = sks_conn(m.mass, m.spin, o.t.r, o.t.th);
+    double s, c;
+    sincos(o.t.th, &s, &c);
+    bool in_range = true;
+    o.c = sks_conn<true>(m.mass, m.spin, o.t.r, s, c, in_range);
+    if (!in_range) o.c = sks_conn<false>(m.mass, m.spin, o.t.r, s, c, in_range);
     return o;
 }
 
-// -Gamma(k, q) at a point.
+// -Gamma(k, q) at a point: the reference's sums without their zero terms, in
+// its order.
 KP_HD D4 fmks_contract(const FmksConn& w, const D4& kn, const D4& qn) {
     const FmksTheta& t = w.t;
     const SksConn& c = w.c;
@@ -229,31 +303,22 @@ KP_HD D4 fmks_contract(const FmksConn& w, const D4& kn, const D4& qn) {
         o.v[3] = v.v[3];
         return o;
     };
-    const D4 ks = to_sph(kn);
-    double rowk_r[4], rowk_t[4];
-    for (int nu = 0; nu < 4; ++nu) {
-        double a = 0.0, b = 0.0;
-        for (int q = 0; q < 4; ++q) {
-            a += c.dgr[nu][q] * ks.v[q];
-            b += c.dgth[nu][q] * ks.v[q];
-        }
-        rowk_r[nu] = a;
-        rowk_t[nu] = b;
-    }
-    const D4 q = to_sph(qn);
-    double rr[4], rt[4];
-    double d1 = 0.0, d2 = 0.0;
-    for (int nu = 0; nu < 4; ++nu) {
-        double a = 0.0, b = 0.0;
-        for (int v = 0; v < 4; ++v) {
-            a += c.dgr[nu][v] * q.v[v];
-            b += c.dgth[nu][v] * q.v[v];
-        }
-        rr[nu] = a;
-        rt[nu] = b;
-        d1 += ks.v[nu] * a;
-        d2 += ks.v[nu] * b;
-    }
+    auto rows = [&](const D4& v, double (&r)[4], double (&h)[4]) {
+        r[0] = c.A * v.v[0] + c.A * v.v[1] + c.B * v.v[3];
+        r[1] = r[0];
+        r[2] = c.C * v.v[2];
+        r[3] = c.B * v.v[0] + c.B * v.v[1] + c.D * v.v[3];
+        h[0] = c.E * v.v[0] + c.E * v.v[1] + c.F0 * v.v[3];
+        h[1] = c.E * v.v[0] + c.E * v.v[1] + c.F1 * v.v[3];
+        h[2] = c.G * v.v[2];
+        h[3] = c.F0 * v.v[0] + c.F1 * v.v[1] + c.H * v.v[3];
+    };
+    const D4 ks = to_sph(kn), q = to_sph(qn);
+    double rowk_r[4], rowk_t[4], rr[4], rt[4];
+    rows(ks, rowk_r, rowk_t);
+    rows(q, rr, rt);
+    const double d1 = ks.v[0] * rr[0] + ks.v[1] * rr[1] + ks.v[2] * rr[2] + ks.v[3] * rr[3];
+    const double d2 = ks.v[0] * rt[0] + ks.v[1] * rt[1] + ks.v[2] * rt[2] + ks.v[3] * rt[3];
     double tt[4];
     for (int nu = 0; nu < 4; ++nu) {
         double term = ks.v[1] * rr[nu] + q.v[1] * rowk_r[nu] + ks.v[2] * rt[nu] + q.v[2] * rowk_t[nu];
@@ -262,19 +327,26 @@ KP_HD D4 fmks_contract(const FmksConn& w, const D4& kn, const D4& qn) {
         tt[nu] = term;
     }
     double hs[4];
-    for (int mu = 0; mu < 4; ++mu) {
-        double comp = 0.0;
-        for (int nu = 0; nu < 4; ++nu) comp += c.gcon[mu][nu] * tt[nu];
-        hs[mu] = 0.5 * comp;
-    }
+    hs[0] = 0.5 * (c.g00 * tt[0] + c.g01 * tt[1]);
+    hs[1] = 0.5 * (c.g01 * tt[0] + c.g11 * tt[1] + c.g13 * tt[3]);
+    hs[2] = 0.5 * (c.g22 * tt[2]);
+    hs[3] = 0.5 * (c.g13 * tt[1] + c.g33 * tt[3]);
     // back to native components (fmks_from_spherical_connection_contract, :414-431)
     hs[1] += t.r * kn.v[1] * qn.v[1];
     hs[2] += t.d2th11 * kn.v[1] * qn.v[1] + t.d2th12 * (kn.v[1] * qn.v[2] + kn.v[2] * qn.v[1]) +
              t.d2th22 * kn.v[2] * qn.v[2];
+    bool in_range = true;
+    const FmksDivisor dr = fmks_divisor(t.r), d2th = fmks_divisor(t.dth2);
+    double o1 = fmks_quot<true>(hs[1], dr, in_range);
+    double o2 = fmks_quot<true>(hs[2] - fmks_quot<true>(t.dth1 * hs[1], dr, in_range), d2th, in_range);
+    if (!in_range) {
+        o1 = fmks_quot<false>(hs[1], dr, in_range);
+        o2 = fmks_quot<false>(hs[2] - fmks_quot<false>(t.dth1 * hs[1], dr, in_range), d2th, in_range);
+    }
     D4 out;
     out.v[0] = -hs[0];
-    out.v[1] = -(hs[1] / t.r);
-    out.v[2] = -((hs[2] - t.dth1 * hs[1] / t.r) / t.dth2);
+    out.v[1] = -o1;
+    out.v[2] = -o2;
     out.v[3] = -hs[3];
     return out;
 }
@@ -302,20 +374,20 @@ struct FmksFactored {
 };
 
 KP_HD FmksFactored fmks_factored_conn(const FmksParams& m, const D4& x) {
-    const FmksTheta t = fmks_theta(m, x.v[1], x.v[2]);
+    const FmksTheta t = fmks_theta<true>(m, x.v[1], x.v[2]);
     const double a = m.spin, M = m.mass, r = t.r;
     double sn, cs;
     sincos(t.th, &sn, &cs);
     const double a2 = a * a, s2 = sn * sn, safe_s2 = max_val(s2, kTiny);
     const double rho2 = r * r + a2 * cs * cs;
-    const double inv_rho2 = 1.0 / rho2;
+    const double inv_rho2 = kp_recip<double>(rho2);
     const double inv_rho4 = inv_rho2 * inv_rho2;
     const double f = 2.0 * M * r * inv_rho2;
     const double delta = r * r - 2.0 * M * r + a2;
     FmksFactored o;
     o.r = r;
-    o.inv_r = 1.0 / r;
-    o.inv_dth2 = 1.0 / t.dth2;
+    o.inv_r = kp_recip<double>(r);
+    o.inv_dth2 = kp_recip<double>(t.dth2);
     o.dth1 = t.dth1;
     o.dth2 = t.dth2;
     o.d2th11 = t.d2th11;
@@ -326,7 +398,7 @@ KP_HD FmksFactored fmks_factored_conn(const FmksParams& m, const D4& x) {
     o.G11 = delta * inv_rho2;
     o.G13 = a * inv_rho2;
     o.G22 = inv_rho2;
-    o.G33 = inv_rho2 / safe_s2;
+    o.G33 = inv_rho2 * kp_recip<double>(safe_s2);
     const double drho_dth = -2.0 * a2 * sn * cs, ds2_dth = 2.0 * sn * cs;
     const double df_dr = 2.0 * M * (rho2 - 2.0 * r * r) * inv_rho4;
     const double df_dth = -2.0 * M * r * drho_dth * inv_rho4;

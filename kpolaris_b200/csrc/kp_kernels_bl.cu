@@ -10,7 +10,7 @@ namespace kp {
 
 template<int NF>
 __global__ void __launch_bounds__(kFarThreads, 2) wave_bl_far(const WaveDesc W) {
-    far_body<PolicyFP64, NF, SceneRiafBL>(W);
+    far_phase<PolicyFP64, NF, SceneRiafBL>(W);
 }
 
 __global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_bl_near_a(const WaveDesc W) {

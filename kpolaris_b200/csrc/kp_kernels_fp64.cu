@@ -175,7 +175,7 @@ cudaError_t launch_image_fp64(const ImageConsts& c, const ImageOutPtrs& out, int
 // traces a ray bit-identically to the plain kernel.
 template<int NF>
 __global__ void __launch_bounds__(kFarThreads, kFarBlocks) wave_far_fp64(const WaveDesc W) {
-    far_body<PolicyFP64, NF>(W);
+    far_phase<PolicyFP64, NF>(W);
 }
 
 __global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_fp64(const WaveDesc W) {

@@ -12,7 +12,7 @@ namespace kp {
 
 template<int NF>
 __global__ void __launch_bounds__(kFarThreads, 2) wave_far_grmhd(const WaveDesc W) {
-    far_body<PolicyFP64, NF, SceneGrmhd>(W);
+    far_phase<PolicyFP64, NF, SceneGrmhd>(W);
 }
 
 __global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_grmhd(const WaveDesc W) {

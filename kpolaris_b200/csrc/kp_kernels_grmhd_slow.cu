@@ -11,7 +11,7 @@ namespace kp {
 
 template<int NF>
 __global__ void __launch_bounds__(kFarThreads, 2) wave_far_grmhd_slow(const WaveDesc W) {
-    far_body<PolicyFP64, NF, SceneGrmhdSlow>(W);
+    far_phase<PolicyFP64, NF, SceneGrmhdSlow>(W);
 }
 
 __global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_grmhd_slow(const WaveDesc W) {

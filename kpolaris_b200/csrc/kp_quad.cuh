@@ -985,4 +985,22 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
     }
 }
 
+// The FP64 policy's far phase: quads as long as every ray of the launch gets
+// one of its own, one thread per ray beyond.  A quad's step is shorter (far
+// phase of a 16^2 to 96^2 image 19 to 25 -> 10 to 14 ms, of a 64^2 GRMHD
+// image 15 ms less), but its lanes repeat the connection: once the quads take
+// turns the SMs' FP64 units run more of it (128^2: 25.8 ms with threads, 29.5
+// with quads; 256^2: 50 and 116).  The two agree bit for bit, so a ray's
+// results do not depend on the choice.
+template<class P, int NF, class SC = SceneRiaf>
+__device__ __forceinline__ void far_phase(const WaveDesc& W) {
+    static_assert(!P::kMixed, "the forms agree bit for bit without contraction only");
+    const long long rays = W.fresh_end - W.fresh_begin + (long long)(W.in_ids ? *W.in_count : 0u);
+    if (rays <= (long long)gridDim.x * (blockDim.x >> 2)) {
+        quad_body<P, kPhaseFar, SC>(W);
+    } else {
+        far_body<P, NF, SC>(W);
+    }
+}
+
 }  // namespace kp

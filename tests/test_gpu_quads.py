@@ -9,6 +9,8 @@ and mixes at which four lanes per ray can go wrong.
 * Many small images of different spins and frequency counts in one batch, so
   that the quads of a warp trace different images: each is bit for bit the
   image traced alone, in either precision.
+* Just as many rays as a B200's resident quads (9,472) take the FP64 far phase
+  as quads, more as threads: both are the one-launch kernel's, bit for bit.
 * The mixed policy's far field takes many steps at once and counts them: on
   rays that miss the sphere, cameras near, inside the far boundary and far
   out, and large and small step caps, its reasons are those of the FP64 policy
@@ -62,6 +64,12 @@ def test_mixed_warps_match_images_alone(precision):
     for k, (p, m, f) in enumerate(jobs):
         alone = kp.image_riaf(p, m, f, precision=precision, schedule=_abi.SCHEDULE_PERSISTENT)
         assert_bitwise(outs[k], alone, k)
+
+
+@pytest.mark.parametrize("nx,ny", [(97, 97), (98, 97)])
+def test_far_phase_forms_agree(nx, ny):
+    p, m, f = job(nx, ny, 1, inclination=17.0)
+    assert_bitwise(kp.image_riaf(p, m, f, schedule=_abi.SCHEDULE_PERSISTENT), kp.image_riaf(p, m, f), (nx, ny))
 
 
 @pytest.mark.parametrize("radius,fov,max_step", [(1000.0, 0.5, 2.0), (300.0, 1.2, 2.0), (121.0, 0.6, 2.0),

@@ -284,27 +284,31 @@ __device__ __forceinline__ void quad_job(int kind, const ImageConsts& c, const D
     const bool sd = kind == kRkSD, single = kind == kRkRK4;
     const int nchain = __any_sync(kFullWarp, sd && !sure) ? 3 : (__any_sync(kFullWarp, sd || kind == kRkRK4x2) ? 2 : 1);
     D4 B = S;             // chain base
-    D4 K1, R2, end, A, X, k;
+    D4 K1, R2, end, A, X = S, k;
     double hc = single ? h : h * 0.5;
 #pragma unroll 1
     for (int chain = 0; chain < nchain; ++chain) {
-        // acc = ((k1 + 2 k2) + 2 k3) + k4
+        // acc = ((k1 + 2 k2) + 2 k3) + k4, around one right-hand side: three
+        // copies of it outgrow the innermost instruction cache
         const double hh = 0.5 * hc;
-        if (chain < 2) A = quad_rhs<P, SC>(geo, B, role);
-        if (chain == 0) K1 = A;
-        d4_axpy(X, B, hh, A);
 #pragma unroll 1
-        for (int st = 1; st < 3; ++st) {
+        for (int st = chain < 2 ? 0 : 1;; ++st) {
             k = quad_rhs<P, SC>(geo, X, role);
-            d4_acc(A, k, 2.0);
-            d4_axpy(X, B, st == 1 ? hh : hc, k);
+            if (st == 3) break;
+            if (st == 0) {
+                A = k;
+                if (chain == 0) K1 = k;
+            } else {
+                d4_acc(A, k, 2.0);
+            }
+            d4_axpy(X, B, st == 2 ? hc : hh, k);
         }
-        k = quad_rhs<P, SC>(geo, X, role);
         d4_add(A, k);
         d4_axpy(end, B, hc / 6.0, A);
         if (chain == 0) {
             R2 = end;
             B = end;
+            X = end;
         } else if (chain == 1) {
             if (nchain == 2) break;
             // the full chain from S, its first derivative known
@@ -312,6 +316,7 @@ __device__ __forceinline__ void quad_job(int kind, const ImageConsts& c, const D
             K1 = end;  // the two-half endpoint
             B = S;
             hc = h;
+            d4_axpy(X, S, 0.5 * h, A);
         }
     }
     if (nchain == 3) {

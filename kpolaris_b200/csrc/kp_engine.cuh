@@ -78,6 +78,10 @@ struct RadTraits<PolicyFP64, SceneRiaf> {
     __device__ static Co coeffs_ctl(const ImageConsts& c, const Sample& p, int g) {
         return riaf_coefficients(c, p, c.ctl_freq[g]);
     }
+    // step() with coefficients of zero
+    __device__ static void add_zero(Stokes& s) {
+        s = Stokes{s.I + 0.0, s.Q + 0.0, s.U + 0.0, s.V + 0.0};
+    }
     __device__ static void step(Stokes& s, const Co& co, double h, const ImageConsts& c, int f) {
         stokes_apply(s, stokes_op(co, abs_val(h) * c.dlambda_scale[f]), co.jI, co.jQ, co.jU, co.jV);
     }

@@ -843,6 +843,9 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
                 // lane takes one frequency, lanes past the image's last repeat it
                 const ImageConsts& c = J->c;
                 bool stopped = false;
+                // a step without plasma: its coefficients are zero, its
+                // transfer adds zero (the plain kernel's far field)
+                bool empty = false;
                 int required = 1, pred = 1;
                 double local_max_rs = 0.0;
                 typename RT::Co co;
@@ -870,7 +873,12 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
                             }
                         }
                         if (radiating && !stopped) ps = RT::sample(c, sample);
-                        if (!stopped) {
+                        empty = kAll && !radiating;
+                        if (empty) {
+                            const RadDepths none = {0.0, 0.0, 0.0};
+                            required = substeps_for(none, h, local_max_rs, c);
+                            pred = substeps_for(none, st.h_current, local_max_rs, c);
+                        } else if (!stopped) {
                             co = RT::coeffs(c, ps, f);
                             if (!c.faraday_rotation) co.rV = 0.0;
                             // Substep counts at h (required) and at h_current
@@ -914,7 +922,11 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
                              c.max_faraday_depth > 0.0))
                             st.cap = max_val(c.min_step_abs, over_pow2(st.h_current, pred));
                         if constexpr (kRad) {
-                            if (h > 0.0) RT::step(stokes, co, h, c, f);
+                            if (empty) {
+                                if constexpr (kAll) RT::add_zero(stokes);
+                            } else if (h > 0.0) {
+                                RT::step(stokes, co, h, c, f);
+                            }
                         }
                         V = next;
                         r_top = next_r;

@@ -11,8 +11,9 @@ at r = 1000 M, inclination 17 deg.  Inputs are the analytic plasma model
 (synthetic by construction).
 
 Headline (`--path mixed`, default): one step traces `--batch` images through
-kp_batch_riaf, the mixed-precision wavefront engine (FP64 geodesic state and
-step control, FP32 far-field contraction and FP32 transfer).  The plain FP64
+kp_batch_riaf, the wavefront engine with the mixed policy (FP64 in factored
+forms that round differently from the reference, many far-field steps bridged
+at once).  The plain FP64
 one-image-per-launch kernel is timed in the same run (`plain_fp64`), and the
 first image of the batch is compared with it (`accuracy_vs_fp64`: total flux
 and image-integrated EVPA per frequency).  `--path plain` makes the plain
@@ -536,17 +537,13 @@ PHASES = ("far", "near_a", "near_b")
 
 
 def phase_ops(flops, phase, mixed):
-    """(fp64_ops, fp32_ops) of one image in one engine phase.  Mixed policy:
-    the far phase contracts the connection in FP32 and near-B evaluates the
-    plasma and the thermal fits in FP32; the rest is FP64."""
+    """(fp64_ops, fp32_ops) of one image in one engine phase: FP64 throughout
+    in either policy.  The mixed policy's far phase bridges most of its steps,
+    so its algorithmic rate can pass the pipe's peak."""
     ph = flops[f"phase_{phase}"]
     rhs, other = ph["rhs_ops"], ph["other_ops"]
     rad = flops["plasma_ops"] + flops["thermal_ops"] if phase == "near_b" else 0
-    if not mixed:
-        return rhs + other + rad, 0
-    if phase == "far":
-        return other, rhs
-    return rhs + other, rad
+    return rhs + other + rad, 0
 
 
 def integrated_stokes(i, q, u):

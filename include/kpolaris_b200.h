@@ -91,15 +91,15 @@ typedef enum kp_precision {
     /* FP64 everywhere, IEEE operation order of the reference (bit-exact
      * termination status and fixed-step counts). */
     KP_PRECISION_FP64 = 0,
-    /* FP64 geodesic state, step control and near-hole geometry; FP32
-     * coefficients and Stokes transfer with a per-job 2^E scale and
-     * compensated accumulation. */
+    /* FP64 in factored, contracted forms that round differently from the
+     * reference; runs of far-field steps are bridged by one high-order step.
+     * Held to 1e-4 in flux and 0.1 degrees in EVPA against KP_PRECISION_FP64. */
     KP_PRECISION_MIXED = 1
 } kp_precision;
 
 /* How rays are scheduled on the device. */
 typedef enum kp_schedule {
-    /* One thread per pixel, one launch per image: the plain form. */
+    /* Four lanes per pixel, one launch per image: the plain form. */
     KP_SCHEDULE_PER_PIXEL = 0,
     /* Persistent kernel draining a global ray queue with per-lane refill. */
     KP_SCHEDULE_PERSISTENT = 1,
@@ -625,7 +625,7 @@ int kp_kharma_dump_time(const char* path, double* t);
 /*
  * One GRMHD image in FMKS coordinates, 1..KP_MAX_FREQUENCIES frequencies on
  * one geodesic, through the wavefront engine (options->precision FP64, or
- * MIXED: FP64 geodesic and grid sample, FP32 fits and transfer).  Replaces
+ * MIXED: the same in factored forms that round differently).  Replaces
  * run_grmhd_image (src/image/grmhd.hpp:12-32, src/image/grmhd.cpp:22-59) for
  * the FMKS backend; params->coordinate_system must be KP_COORD_FMKS and the
  * grid's spin must be params->spin.

@@ -297,9 +297,9 @@ double isco_radius(double spin) {
     return 3.0 + z2 - sign * std::sqrt((3.0 - z1) * (3.0 + z1 + 2.0 * z2));
 }
 
-// Exponent E of the FP32 emission scale 2^E of one frequency (mixed path).
+// Exponent E of the emission scale 2^E of one frequency (mixed path).
 // The invariant emissivity j ~ n_e e^2 nu_c / (c nu^2) is 1e-38..1e-48 in CGS,
-// below FP32 range; E is chosen so that the emission of one radiation step
+// far from 1; E is chosen so that the emission of one radiation step
 // at a reference plasma point (r = max(r_min, 3), equator, unit shape
 // factor bound 30) is 2^-6.  The transfer equation is linear in (j, S), so
 // the image is exactly rescaled by 2^-E in FP64 at the end.
@@ -526,7 +526,7 @@ bool separate_control(const double* freqs, int nfreq, double single_freq, const 
 }
 
 // The control list's frequencies, dlambda scales (length unit / frequency)
-// and, for the FP32 fits, 2^E emission scales.
+// and, for the mixed policy's fits, 2^E emission scales.
 void apply_control_riaf(ImageConsts& c, const kp_pass_a_params* p, const kp_riaf_model* m, const double* ctl,
                         int nctl) {
     const double length_unit = riaf_length_unit(m);

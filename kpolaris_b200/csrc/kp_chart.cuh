@@ -1,7 +1,7 @@
 // kp_chart.cuh -- the change of chart between the FMKS coordinates of the
 // GRMHD scene and Cartesian Kerr-Schild, for the mixed policy's far phase:
 // beyond the radiating sphere a GRMHD ray carries no plasma, so the far
-// kernel integrates it in CKS with the FP32 stage chains of the RIAF scene
+// kernel integrates it in CKS with the bridged runs of the RIAF scene
 // and converts at the phase boundary.  Records always hold FMKS states.
 //
 //   FMKS (x0, x1, x2, x3) -> spherical KS (t, r, theta, phi):

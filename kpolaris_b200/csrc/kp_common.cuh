@@ -113,7 +113,7 @@ struct ImageConsts {
     double thetae_unit;  // te_unit * k_B / (m_e c^2)
     double log_te0;      // log(Te0 thetae_unit)
     double isco;         // isco_radius(spin), riaf.hpp:166-174
-    // boundary of the far phase (FP32 contraction under the mixed policy):
+    // boundary of the far phase (bridged runs of steps under the mixed policy):
     // outside the radiating sphere by two of the longest steps
     double fp32_radius;
     int fit;             // 1 Pandya, 4 Dexter

@@ -1,10 +1,11 @@
-// kp_engine.cuh -- persistent ray engine: every lane of a warp holds one ray
-// and advances it through a resumable state machine whose loop iteration is
-// one RK job (a step-doubling attempt, an RK4 step, a composed pair of RK4
+// kp_engine.cuh -- the ray engine's policies, control modes and one-lane RK
+// jobs.  A quad (kp_quad.cuh) or a lane (kp_persistent.cuh) holds one ray and
+// advances it through a resumable state machine whose loop iteration is one RK
+// job (a step-doubling attempt, an RK4 step, a composed pair of RK4
 // half steps or a Cash-Karp attempt) started from the lane's current state.
 // Jobs run as a stage loop around ONE right-hand-side site, so lanes of a warp
 // evaluate the RHS together whatever their phase (pass A, surface refinement,
-// pass B, camera crossing).  Finished lanes refill from a global ray queue
+// pass B, camera crossing).  Finished rays are replaced from a global ray queue
 // shared by every image of the launch (warp-aggregated atomics), which removes
 // both the tail of uneven rays and the launch-per-image cost.
 //

@@ -183,7 +183,7 @@ KP_HD KSConn ks_conn_plain(double mass, double spin, const D4& X) {
 // The same with the exact quotients and roots of kp_exact.cuh: every result
 // has ks_conn_plain's bits.  A point for which an operand could leave their
 // range (never one of a ray that is still traced in earnest) takes the plain
-// form.  7 reciprocals and 19 quotients: 3225 -> KP_RHS_CYCLES cycles per
+// form.  7 reciprocals and 19 quotients: 3225 -> 1341 cycles per
 // right-hand side of a lone ray.
 static __device__ __noinline__ void ks_conn_far_out(double mass, double spin, const D4& X, KSConn& c) {
     c = ks_conn_plain(mass, spin, X);

@@ -1,6 +1,6 @@
 // kp_geometry_f32.cuh -- the Kerr-Schild transport right-hand side of the
 // mixed-precision policy, in a factored form templated on the arithmetic
-// type: FP32 in the far field, FP64 inside the radiating sphere.  The core
+// type; the kernels use it in FP64.  The core
 // (ks_transport_factored) works on T values; ks_rhs_factored wraps it for
 // FP64 Rays.
 //
@@ -29,7 +29,7 @@ namespace kp {
 // Newton's iteration (e = 1 - v y^2, y' = y + y e (1/2 + 3 e / 8); e = 1 - v y,
 // y' = y + y (e + e^2)), a few ulp, without the range checks and branches of
 // the IEEE forms: sqsum and r of a ray are far from the ends of the range.
-// FP32 (the far field, where the contraction's own cancellation already
+// FP32 (where the contraction's own cancellation already
 // limits it to ~3e-5): one hardware reciprocal square root or reciprocal.
 template<class T>
 KP_HD void kp_sqrt_pair(T v, T& sq, T& inv) {

@@ -131,9 +131,9 @@ inline ImageConsts image_consts_fmks(const kp_pass_a_params* p, const kp_grmhd_m
     return c;
 }
 
-// FP32 emission scales 2^E of a mixed-precision GRMHD image, one per
-// frequency.  The invariant emissivity j ~ n_e e^2 nu_c / (c nu^2) lies far
-// below FP32 range in CGS; E puts the emission of one radiation step at a
+// Emission scales 2^E of a mixed-precision GRMHD image, one per
+// frequency.  The invariant emissivity j ~ n_e e^2 nu_c / (c nu^2) is tiny
+// in CGS; E puts the emission of one radiation step at a
 // reference plasma point (code density 1, code field 0.05, shape factor bound
 // 30) at 2^-6.  The transfer is linear in the emission, so the image is
 // rescaled by 2^-E in FP64 at the end and E changes only rounding.
@@ -162,7 +162,7 @@ inline void grmhd_emission_scale(const kp_pass_a_params* p, const kp_grmhd_model
 }
 
 // A separate step-control list of a GRMHD image (the control frequencies,
-// their dlambda scales and FP32 emission scales).
+// their dlambda scales and emission scales).
 inline void grmhd_apply_control(const kp_pass_a_params* p, const kp_grmhd_model& m, ImageConsts& c,
                                 const double* ctl, int nctl) {
     const double length_unit = grmhd_length_unit_cgs(m);

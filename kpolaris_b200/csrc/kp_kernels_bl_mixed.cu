@@ -1,5 +1,5 @@
 // kp_kernels_bl_mixed.cu -- the RIAF in Boyer-Lindquist coordinates (SceneRiafBL)
-// on the wavefront engine with the mixed policy (FP64 BL geodesic, FP32 fits, FP64 transfer), compiled with FMA contraction.
+// on the wavefront engine with the mixed policy (FP64 BL geodesic, factored fits), compiled with FMA contraction.
 #include <cuda_runtime.h>
 
 #include "kp_launch.h"

@@ -1,6 +1,6 @@
 // kp_kernels_grmhd_mixed.cu -- the GRMHD scene (FMKS metric, grid plasma) of
-// the wavefront engine with the mixed policy: FP64 geodesic and grid sample,
-// FP32 thermal fits, FP64 Stokes transfer.
+// the wavefront engine with the mixed policy: factored geodesic,
+// fits and transfer, all of it FP64.
 // Compiled with FMA contraction (the mixed path is held to a flux/EVPA
 // budget, not to the reference's rounding).
 #include <cuda_runtime.h>

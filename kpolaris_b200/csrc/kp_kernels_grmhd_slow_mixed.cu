@@ -1,6 +1,6 @@
 // kp_kernels_grmhd_slow_mixed.cu -- slow-light GRMHD images (FMKS metric, grid plasma interpolated
 // in time between resident snapshots) on the wavefront engine with
-// the mixed policy (FP64 geodesic and grid sample, FP32 fits, FP64 transfer).  Compiled with FMA contraction.
+// the mixed policy (factored geodesic, fits and transfer, all of it FP64).  Compiled with FMA contraction.
 #include <cuda_runtime.h>
 
 #include "kp_launch.h"

@@ -1,6 +1,6 @@
-// kp_kernels_mixed.cu -- the mixed-precision wavefront kernels: FP64 ray
-// state, transport, step control and Stokes transfer, many far-field steps at
-// once, FP32 transfer coefficients.  Compiled with FMA contraction enabled.
+// kp_kernels_mixed.cu -- the mixed policy's wavefront kernels: FP64 in
+// factored, contracted forms that round differently from the reference, and
+// many far-field steps at once.  Compiled with FMA contraction enabled.
 #include <cuda_runtime.h>
 
 #include "kp_launch.h"

@@ -412,7 +412,7 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
         if constexpr (!kAll) {
             // ------------------------------------------------------------ claim
             // The far phase refills a warp as a whole: its rays then stay in
-            // step, all in a bridged run or all in an ordinary step (79 -> KP_FAR ms
+            // step, all in a bridged run or all in an ordinary step (79 -> 30 ms
             // per 8 x 256^2 step against refilling quad by quad).
             const bool busy = kMacro && __any_sync(kFullWarp, st.mode != kIdle);
             const bool want = claims && !exhausted && st.mode == kIdle && !busy;

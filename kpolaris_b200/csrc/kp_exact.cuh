@@ -9,13 +9,17 @@
 // System/6000 processor", IBM J. Res. Dev. 34 (1990) 111-119 (also Muller et
 // al., Handbook of Floating-Point Arithmetic, ch. 4).  With fused
 // multiply-adds, a reciprocal y of b within one ulp becomes the correctly
-// rounded one by y + y (1 - b y) (but for a divisor whose significand is all
-// ones); with it, a quotient q of a / b within one ulp becomes the correctly
-// rounded one by q - y (b q - a).  The residuals are formed as b q - a so that
-// a zero numerator keeps its sign.  A square root g of v within one ulp
-// becomes the rounded one by g + (v - g g) h with h = 1 / (2 sqrt(v)).  The
+// rounded one by y + y (1 - b y), but for a divisor whose significand is all
+// ones (exact_recip sees to it); with it, a quotient q of a / b within one ulp
+// becomes the correctly rounded one by q - y (b q - a).  The residuals are
+// formed as b q - a so that a zero numerator keeps its sign.  A square root g
+// of v within one ulp becomes the rounded one by g + (v - g g) h with h =
+// 1 / (2 sqrt(v)), but for one significand (exact_sqrt sees to it).  The
 // starting values are the hardware's approximate reciprocal and reciprocal
-// square root, taken to one ulp by a third-order Newton step.
+// square root, of 20 bits, taken to one ulp by the geometric series of
+// 1 / b = y / (1 - e), e = 1 - b y, and the binomial series of
+// v^-1/2 = y (1 - e)^-1/2, e = 1 - v y y, each to its term in e^2: what is
+// left out is below e^3 = 2^-57.
 #pragma once
 
 #include <cmath>
@@ -24,7 +28,21 @@
 
 namespace kp {
 
+#if defined(__CUDACC__) || defined(KP_EXACT_METHOD)  // the latter: a host test of the method
+
 #ifdef __CUDACC__
+__device__ __forceinline__ double recip_start(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    return y;
+}
+
+__device__ __forceinline__ double rsqrt_start(double v) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+    return y;
+}
+#endif
 
 struct ExactRecip {
     double b, y;
@@ -32,12 +50,16 @@ struct ExactRecip {
 
 // The correctly rounded reciprocal of b, 1e-150 < |b| < 1e150.
 __device__ __forceinline__ ExactRecip exact_recip(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    double y = recip_start(b);
     double e = __fma_rn(-b, y, 1.0);
     y = __fma_rn(y, __fma_rn(e, e, e), y);
     e = __fma_rn(-b, y, 1.0);
-    return ExactRecip{b, __fma_rn(y, e, y)};
+    y = __fma_rn(y, e, y);
+    // For b = 2^n (2 - 2^-52) that ends at 2^-(n + 1), and the reciprocal is
+    // the next number, 2^-(n + 1) (1 + 2^-52): its last bit is set.
+    const unsigned hi = unsigned(__double2hiint(b)) | 0xfff00000u, lo = unsigned(__double2loint(b));
+    const int last = (hi & lo) == 0xffffffffu ? 1 : 0;
+    return ExactRecip{b, __hiloint2double(__double2hiint(y), __double2loint(y) | last)};
 }
 
 // RN(a / b) for a zero or 1e-200 < |a| < 1e150 with 1e-250 < |a / b| < 1e150.
@@ -49,14 +71,18 @@ __device__ __forceinline__ double exact_quot(double a, const ExactRecip& r) {
 
 // RN(sqrt(v)), 1e-290 < v < 1e290.
 __device__ __forceinline__ double exact_sqrt(double v) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+    double y = rsqrt_start(v);
     const double e = __fma_rn(-__dmul_rn(v, y), y, 1.0);
     y = __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
     const double h = __dmul_rn(0.5, y);
     double g = __dmul_rn(v, y);
     g = __fma_rn(__fma_rn(-g, g, v), h, g);
-    return __fma_rn(__fma_rn(-g, g, v), h, g);
+    g = __fma_rn(__fma_rn(-g, g, v), h, g);
+    // For v = 4^n (1 - 2^-53), a hair under the middle between 2^n and the
+    // number below it, that can end at 2^n, and the root is the number below.
+    const unsigned hi = unsigned(__double2hiint(v)) | 0xfff00000u, lo = unsigned(__double2loint(v));
+    const int above = (hi & lo) == 0xffffffffu && __double2loint(g) == 0 ? 1 : 0;
+    return __longlong_as_double(__double_as_longlong(g) - above);
 }
 
 // A numerator's factor for which products of a few of its like stay clear of
@@ -100,7 +126,7 @@ __device__ __forceinline__ double exact_over(double a, double b, double inv) {
     if (exact_numerator(a)) return exact_quot(a, ExactRecip{b, inv});
     return plain_quot(a, b);
 }
-#define KP_OVER(a, b) exact_over((a), (b), 1.0 / (b))
+#define KP_OVER(a, b) ::kp::exact_over((a), (b), 1.0 / (b))
 
 #else  // host builds of the device code: the compiler's own
 

@@ -1,0 +1,47 @@
+"""The FP64 policy's quotients and square roots (kpolaris_b200/csrc/kp_exact.cuh)
+are IEEE's, bit for bit: exact_quots and KP_OVER for any operands, exact_recip,
+exact_quot and exact_sqrt within the ranges they state.
+
+The operands (tests/native/exact_quotients.h) cover both signs, zeros of both
+signs, subnormal numbers, infinities and NaN, the ends of the admitted ranges
+and just beyond them, and significands of all ones, nearly so, and powers of
+two.
+
+* CPU: tests/native/exact_quotients.cpp, the method with C's fma and
+  approximate starting values of 20 bits, good and at the hardware's stated
+  accuracy.
+* GPU: tests/native/exact_quotients.cu, against CUDA's own operators."""
+from __future__ import annotations
+
+import ctypes as C
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+NATIVE = ROOT / "tests" / "native"
+CSRC = ROOT / "kpolaris_b200" / "csrc"
+
+
+@pytest.mark.parametrize("err", [0.0, 1e-6])
+def test_host_emulation(tmp_path, err):
+    exe = tmp_path / "exact_quotients"
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", f"-I{CSRC}", f"-I{ROOT / 'include'}", f"-I{NATIVE}",
+                    "-o", str(exe), str(NATIVE / "exact_quotients.cpp")], check=True)
+    out = subprocess.run([str(exe), "2000000", repr(err)], capture_output=True, text=True, check=True).stdout.split()
+    assert [int(x) for x in out] == [0] * 5, dict(zip(("quots", "over", "quot", "recip", "root"), out))
+
+
+@pytest.mark.gpu
+def test_device_operators(tmp_path):
+    so = tmp_path / "exact_quotients.so"
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3", "--fmad=false",
+                    "-Xcompiler", "-fPIC,-ffp-contract=off", f"-I{CSRC}", f"-I{ROOT / 'include'}", f"-I{NATIVE}",
+                    "-shared", "-o", str(so), str(NATIVE / "exact_quotients.cu")], check=True)
+    counts = (C.c_ulonglong * 5)()
+    rc = C.CDLL(str(so)).kp_probe_exact_quotients(400, counts)
+    assert rc == 0, f"cudaError {rc}"
+    assert list(counts) == [0] * 5, dict(zip(("quots", "over", "quot", "recip", "root"), counts))

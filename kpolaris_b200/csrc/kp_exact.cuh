@@ -12,10 +12,10 @@
 // rounded one by y + y (1 - b y), but for a divisor whose significand is all
 // ones (exact_recip sees to it); with it, a quotient q of a / b within one ulp
 // becomes the correctly rounded one by q - y (b q - a).  The residuals are
-// formed as b q - a so that a zero numerator keeps its sign.  A square root g
-// of v within one ulp becomes the rounded one by g + (v - g g) h with h =
-// 1 / (2 sqrt(v)), but for one significand (exact_sqrt sees to it).  The
-// starting values are the hardware's approximate reciprocal and reciprocal
+// formed as b q - a so that a zero numerator over a positive divisor keeps its
+// sign.  A square root g of v within one ulp becomes the rounded one by
+// g + (v - g g) h with h = 1 / (2 sqrt(v)), but for one significand
+// (exact_sqrt sees to it).  The starting values are the hardware's approximate reciprocal and reciprocal
 // square root, of 20 bits, taken to one ulp by the geometric series of
 // 1 / b = y / (1 - e), e = 1 - b y, and the binomial series of
 // v^-1/2 = y (1 - e)^-1/2, e = 1 - v y y, each to its term in e^2: what is
@@ -48,7 +48,7 @@ struct ExactRecip {
     double b, y;
 };
 
-// The correctly rounded reciprocal of b, 1e-150 < |b| < 1e150.
+// The correctly rounded reciprocal of b, 1e-150 < b < 1e150.
 __device__ __forceinline__ ExactRecip exact_recip(double b) {
     double y = recip_start(b);
     double e = __fma_rn(-b, y, 1.0);
@@ -95,9 +95,10 @@ __device__ __forceinline__ bool exact_numerator(double v) {
     return (unsigned(__double2hiint(v) >> 20) & 0x7ffu) - 523u < 1000u || v == 0.0;
 }
 
-// 2^-200 < |b| < 2^200.
+// 2^-200 < b < 2^200.  A negative divisor would give a zero numerator's
+// quotient the wrong sign.
 __device__ __forceinline__ bool exact_divisor(double b) {
-    return (unsigned(__double2hiint(b) >> 20) & 0x7ffu) - 823u < 400u;
+    return (unsigned(__double2hiint(b)) >> 20) - 823u < 400u;
 }
 
 // The rare operands out of range.

@@ -81,7 +81,7 @@ struct Counts {
 // One draw of every kind.
 XQ_FN void check(uint64_t& s, Counts& n) {
     {
-        const double b = value(bits(anything(s)) & ~(uint64_t(1) << 63));
+        const double b = anything(s);
         double v[3] = {anything(s), anything(s), anything(s)}, q[3] = {v[0], v[1], v[2]};
         kp::exact_quots(q, b);
         for (int i = 0; i < 3; ++i) n.quots += !same(q[i], v[i] / b);

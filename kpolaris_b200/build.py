@@ -31,8 +31,17 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off",
           f"-I{INCLUDE}", f"-I{CSRC}", "-Xptxas", "-warn-spills"]
 
-# translation unit -> extra flags
+def _lanes(policy, scene, *more):
+    fp = ["--fmad=false"] if policy == "FP64" else ["--fmad=true", "--use_fast_math"]
+    return [*fp, f"-DKP_LANES_POLICY=Policy{policy}", f"-DKP_LANES_SCENE=Scene{scene}", *more]
+
+
+# translation unit, with the name of its build where it has several -> extra flags
 UNITS = {
+    "kp_lanes.cu fp64": _lanes("FP64", "Riaf", "-DKP_LANES_IMAGE"),
+    "kp_lanes.cu grmhd": _lanes("FP64", "Grmhd"),
+    "kp_lanes.cu grmhd_slow": _lanes("FP64", "GrmhdSlow"),
+    "kp_lanes.cu bl": _lanes("FP64", "RiafBL"),
     "kp_kernels_fp64.cu": ["--fmad=false"],
     "kp_kernels_mixed.cu": ["--fmad=true", "--use_fast_math"],
     "kp_kernels_grmhd.cu": ["--fmad=false"],
@@ -67,9 +76,13 @@ def _stale(target: Path, deps) -> bool:
     return any(Path(d).stat().st_mtime > t for d in deps)
 
 
+def _object(unit: str) -> Path:
+    return BUILD / (unit.replace(" ", ".") + ".o")
+
+
 def _compile(unit: str, flags, verbose: bool) -> Path:
-    src = CSRC / unit
-    obj = BUILD / (unit + ".o")
+    src = CSRC / unit.split()[0]
+    obj = _object(unit)
     cmd = [nvcc(), *ARCH, *COMMON, *flags, "-c", str(src), "-o", str(obj)]
     if verbose:
         print(" ".join(cmd), flush=True)
@@ -87,10 +100,10 @@ def build(force: bool = False, jobs: int = 4, verbose: bool = False) -> Path:
     todo = []
     objs = []
     for unit, flags in UNITS.items():
-        src = CSRC / unit
+        src = CSRC / unit.split()[0]
         if not src.exists():
             continue
-        obj = BUILD / (unit + ".o")
+        obj = _object(unit)
         objs.append(obj)
         if force or _stale(obj, [src, *headers, Path(__file__)]):
             todo.append((unit, flags))

@@ -645,6 +645,7 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         W.fresh_end = cycle == 0 && phase == kPhaseFar ? total : 0;
         W.in_ids = dev->d_ids[phase][cycle % 2];
         W.in_count = &ctrl->counts[cycle][phase];
+        W.rays_max = total;
         W.in_head = &ctrl->heads[cycle * kPhases + phase];
         for (int q = 0; q < kPhases; ++q) {
             const int gen = q > phase ? cycle : cycle + 1;

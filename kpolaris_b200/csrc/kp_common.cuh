@@ -216,6 +216,7 @@ struct WaveDesc {
     long long fresh_begin, fresh_end;
     const unsigned* in_ids;
     const unsigned* in_count;
+    long long rays_max;            // rays there can be at most (host)
     unsigned long long* in_head;   // pop counter, zero before the launch
     // queue of the next launch of each phase (this phase's own entry takes
     // the rays parked by the iteration budget)

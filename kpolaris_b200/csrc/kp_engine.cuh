@@ -306,8 +306,9 @@ __device__ __noinline__ void ck_job(const ImageConsts& c, const Ray& S, double h
 // one RHS site.  Out of line: the caller's control state is saved once per
 // job and the stage loop has the register file to itself.  `sure`: a
 // step-doubling attempt that is certain to be accepted with the growth of err
-// = 0 (certain_step) leaves its full chain out.
-template<class P, class SC>
+// = 0 (certain_step) leaves its full chain out.  PAIRS: composed pairs occur
+// (the surface-crossing search's trials).
+template<class P, class SC, bool PAIRS>
 __device__ __noinline__ void rk_job(int kind, const ImageConsts& c, const Ray& S, double h, bool sure,
                                     Ray& next, Ray& mid, double& err) {
     if (kind == kRkCK) {
@@ -316,8 +317,9 @@ __device__ __noinline__ void rk_job(int kind, const ImageConsts& c, const Ray& S
     }
     // Stage schedule (see file header): SD = half chain (4), second half
     // chain (4), full chain (3); RK4 = 4; RK4x2 = 4 + 4.
+    const bool pair = PAIRS && kind == kRkRK4x2;
     const int nstage = kind == kRkSD && !sure ? 11 : (kind == kRkRK4 ? 4 : 8);
-    const double hs = kind == kRkSD ? h * 0.5 : (kind == kRkRK4x2 ? h * 0.5 : h);  // step of the first chain
+    const double hs = kind == kRkSD || pair ? h * 0.5 : h;  // step of the first chain
     const double hh_s = 0.5 * hs;
     const double h6_s = hs / 6.0;
     const double hh_f = 0.5 * h;
@@ -357,7 +359,7 @@ __device__ __noinline__ void rk_job(int kind, const ImageConsts& c, const Ray& S
                     X = R2;
                 }
             } else if (st == 7) {
-                if (kind == kRkRK4x2 || sure) {
+                if (pair || sure) {
                     ray_axpy(next, R2, h6, A);
                     mid = R2;
                 } else {
@@ -379,7 +381,7 @@ __device__ __noinline__ void rk_job(int kind, const ImageConsts& c, const Ray& S
             }
         }
     }
-    if (kind == kRkRK4 || kind == kRkRK4x2) mid = next;
+    if (kind == kRkRK4 || pair) mid = next;
     if (nstage < 11) err = 0.0;
 }
 

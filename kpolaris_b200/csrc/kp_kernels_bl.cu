@@ -8,36 +8,31 @@
 
 namespace kp {
 
-template<int NF>
-__global__ void __launch_bounds__(kFarThreads, 2) wave_bl_far(const WaveDesc W) {
-    far_phase<PolicyFP64, NF, SceneRiafBL>(W);
+__global__ void __launch_bounds__(kFarThreads, kFarBlocks) wave_bl_far(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseFar, SceneRiafBL>(W);
 }
 
-__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_bl_near_a(const WaveDesc W) {
-    quad_body<PolicyFP64, kPhaseNearA, SceneRiafBL>(W);
+__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_bl_near_a(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseNearA, SceneRiafBL>(W);
 }
 
-__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_bl_near_b(const WaveDesc W) {
-    quad_body<PolicyFP64, kPhaseNearB, SceneRiafBL>(W);
+__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_bl_near_b(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseNearB, SceneRiafBL>(W);
 }
 
-template<int NF>
 static const void* wave_bl_kernel(int phase) {
-    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_bl_far<NF>);
+    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_bl_far);
     if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_bl_near_a);
     return reinterpret_cast<const void*>(wave_bl_near_b);
 }
 
 cudaError_t launch_wave_bl(int phase, const WaveDesc& W, int nf_max, int blocks, int threads, cudaStream_t stream) {
-    if (nf_max < 1 || nf_max > kMaxFreq || phase < 0 || phase >= kPhases) return cudaErrorInvalidValue;
-    const void* fn = nf_max == 1 ? wave_bl_kernel<1>(phase) : wave_bl_kernel<kMaxFreq>(phase);
-    void* args[] = {const_cast<WaveDesc*>(&W)};
-    return cudaLaunchKernel(fn, dim3(blocks), dim3(threads), args, 0, stream);
+    return launch_wave<PolicyFP64, SceneRiafBL>(wave_bl_kernel(phase), phase, W, nf_max, false, blocks, threads, stream);
 }
 
 int wave_occupancy_bl(int phase, int nf_max, int threads) {
     if (phase < 0 || phase >= kPhases) return 0;
-    const void* fn = nf_max == 1 ? wave_bl_kernel<1>(phase) : wave_bl_kernel<kMaxFreq>(phase);
+    const void* fn = wave_bl_kernel(phase);
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, 0);
     return n;

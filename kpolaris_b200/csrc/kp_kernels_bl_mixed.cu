@@ -9,7 +9,7 @@ namespace kp {
 
 template<int NF>
 __global__ void __launch_bounds__(kFarThreads, 2) wave_bl_mixed_far(const WaveDesc W) {
-    far_body<PolicyMixed, NF, SceneRiafBL>(W);
+    lane_body<PolicyMixed, NF, kPhaseFar, SceneRiafBL>(W);
 }
 
 __global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_bl_mixed_near_a(const WaveDesc W) {

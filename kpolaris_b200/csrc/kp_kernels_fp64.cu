@@ -159,6 +159,7 @@ cudaError_t launch_image_fp64(const ImageConsts& c, const ImageOutPtrs& out, int
     job.frame = camera_frame(c);
     job.out = out;
     job.npix = c.nx * c.ny;
+    if (job.npix > image_quad_pixels(c.nfreq, c.adaptive, std::max(1, sms))) return launch_image_lanes(job, stream);
     // As many warps as the SMs hold at once before a warp gets a second ray:
     // a small image is as slow as its longest ray, and a warp's rays share
     // its issue slots.
@@ -169,36 +170,28 @@ cudaError_t launch_image_fp64(const ImageConsts& c, const ImageOutPtrs& out, int
     return cudaGetLastError();
 }
 
-// The wavefront kernels of the FP64 policy.  NF is 1 for single-frequency
-// launches and 4 otherwise: the per-frequency arithmetic does not depend on
-// NF (the unit is compiled without FMA contraction), so every instantiation
-// traces a ray bit-identically to the plain kernel.
-template<int NF>
-__global__ void __launch_bounds__(kFarThreads, kFarBlocks) wave_far_fp64(const WaveDesc W) {
-    far_phase<PolicyFP64, NF>(W);
+// The wavefront kernels of the FP64 policy on quads.
+__global__ void __launch_bounds__(kFarThreads, kFarBlocks) wave_far_fp64(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseFar>(W);
 }
 
-__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_fp64(const WaveDesc W) {
-    quad_body<PolicyFP64, kPhaseNearA>(W);
+__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_fp64(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseNearA>(W);
 }
 
-__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_fp64(const WaveDesc W) {
-    quad_body<PolicyFP64, kPhaseNearB>(W);
+__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_fp64(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseNearB>(W);
 }
 
-template<int NF>
 static const void* wave_kernel_fp64(int phase) {
-    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_fp64<NF>);
+    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_fp64);
     if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_fp64);
     return reinterpret_cast<const void*>(wave_near_b_fp64);
 }
 
 cudaError_t launch_wave_fp64(int phase, const WaveDesc& W, int nf_max, int blocks, int threads,
                              cudaStream_t stream) {
-    if (nf_max < 1 || nf_max > kMaxFreq || phase < 0 || phase >= kPhases) return cudaErrorInvalidValue;
-    const void* fn = nf_max == 1 ? wave_kernel_fp64<1>(phase) : wave_kernel_fp64<kMaxFreq>(phase);
-    void* args[] = {const_cast<WaveDesc*>(&W)};
-    return cudaLaunchKernel(fn, dim3(blocks), dim3(threads), args, 0, stream);
+    return launch_wave<PolicyFP64, SceneRiaf>(wave_kernel_fp64(phase), phase, W, nf_max, false, blocks, threads, stream);
 }
 
 __global__ void __launch_bounds__(128) seed_fp64(const JobDesc* jobs, const SeedEntry* entries,
@@ -218,7 +211,7 @@ cudaError_t launch_seed_fp64(const JobDesc* jobs, const SeedEntry* entries, cons
 
 int wave_occupancy_fp64(int phase, int nf_max, int threads) {
     if (phase < 0 || phase >= kPhases) return 0;
-    const void* fn = nf_max == 1 ? wave_kernel_fp64<1>(phase) : wave_kernel_fp64<kMaxFreq>(phase);
+    const void* fn = wave_kernel_fp64(phase);
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, 0);
     return n;

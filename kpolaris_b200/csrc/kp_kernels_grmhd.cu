@@ -10,37 +10,32 @@
 
 namespace kp {
 
-template<int NF>
-__global__ void __launch_bounds__(kFarThreads, 2) wave_far_grmhd(const WaveDesc W) {
-    far_phase<PolicyFP64, NF, SceneGrmhd>(W);
+__global__ void __launch_bounds__(kFarThreads, kFarBlocks) wave_far_grmhd(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseFar, SceneGrmhd>(W);
 }
 
-__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_grmhd(const WaveDesc W) {
-    quad_body<PolicyFP64, kPhaseNearA, SceneGrmhd>(W);
+__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_grmhd(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseNearA, SceneGrmhd>(W);
 }
 
-__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_grmhd(const WaveDesc W) {
-    quad_body<PolicyFP64, kPhaseNearB, SceneGrmhd>(W);
+__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_grmhd(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseNearB, SceneGrmhd>(W);
 }
 
-template<int NF>
 static const void* wave_kernel_grmhd(int phase) {
-    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_grmhd<NF>);
+    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_grmhd);
     if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_grmhd);
     return reinterpret_cast<const void*>(wave_near_b_grmhd);
 }
 
 cudaError_t launch_wave_grmhd(int phase, const WaveDesc& W, int nf_max, int blocks, int threads,
                               cudaStream_t stream) {
-    if (nf_max < 1 || nf_max > kMaxFreq || phase < 0 || phase >= kPhases) return cudaErrorInvalidValue;
-    const void* fn = nf_max == 1 ? wave_kernel_grmhd<1>(phase) : wave_kernel_grmhd<kMaxFreq>(phase);
-    void* args[] = {const_cast<WaveDesc*>(&W)};
-    return cudaLaunchKernel(fn, dim3(blocks), dim3(threads), args, 0, stream);
+    return launch_wave<PolicyFP64, SceneGrmhd>(wave_kernel_grmhd(phase), phase, W, nf_max, true, blocks, threads, stream);
 }
 
 int wave_occupancy_grmhd(int phase, int nf_max, int threads) {
     if (phase < 0 || phase >= kPhases) return 0;
-    const void* fn = nf_max == 1 ? wave_kernel_grmhd<1>(phase) : wave_kernel_grmhd<kMaxFreq>(phase);
+    const void* fn = wave_kernel_grmhd(phase);
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, 0);
     return n;

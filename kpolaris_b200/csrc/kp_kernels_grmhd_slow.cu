@@ -9,37 +9,32 @@
 
 namespace kp {
 
-template<int NF>
-__global__ void __launch_bounds__(kFarThreads, 2) wave_far_grmhd_slow(const WaveDesc W) {
-    far_phase<PolicyFP64, NF, SceneGrmhdSlow>(W);
+__global__ void __launch_bounds__(kFarThreads, kFarBlocks) wave_far_grmhd_slow(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseFar, SceneGrmhdSlow>(W);
 }
 
-__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_grmhd_slow(const WaveDesc W) {
-    quad_body<PolicyFP64, kPhaseNearA, SceneGrmhdSlow>(W);
+__global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_grmhd_slow(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseNearA, SceneGrmhdSlow>(W);
 }
 
-__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_grmhd_slow(const WaveDesc W) {
-    quad_body<PolicyFP64, kPhaseNearB, SceneGrmhdSlow>(W);
+__global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_grmhd_slow(const WaveDesc W, long long quad_rays) {
+    if (wave_rays(W) <= quad_rays) quad_body<PolicyFP64, kPhaseNearB, SceneGrmhdSlow>(W);
 }
 
-template<int NF>
 static const void* wave_kernel_grmhd_slow(int phase) {
-    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_grmhd_slow<NF>);
+    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_grmhd_slow);
     if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_grmhd_slow);
     return reinterpret_cast<const void*>(wave_near_b_grmhd_slow);
 }
 
 cudaError_t launch_wave_grmhd_slow(int phase, const WaveDesc& W, int nf_max, int blocks, int threads,
                               cudaStream_t stream) {
-    if (nf_max < 1 || nf_max > kMaxFreq || phase < 0 || phase >= kPhases) return cudaErrorInvalidValue;
-    const void* fn = nf_max == 1 ? wave_kernel_grmhd_slow<1>(phase) : wave_kernel_grmhd_slow<kMaxFreq>(phase);
-    void* args[] = {const_cast<WaveDesc*>(&W)};
-    return cudaLaunchKernel(fn, dim3(blocks), dim3(threads), args, 0, stream);
+    return launch_wave<PolicyFP64, SceneGrmhdSlow>(wave_kernel_grmhd_slow(phase), phase, W, nf_max, true, blocks, threads, stream);
 }
 
 int wave_occupancy_grmhd_slow(int phase, int nf_max, int threads) {
     if (phase < 0 || phase >= kPhases) return 0;
-    const void* fn = nf_max == 1 ? wave_kernel_grmhd_slow<1>(phase) : wave_kernel_grmhd_slow<kMaxFreq>(phase);
+    const void* fn = wave_kernel_grmhd_slow(phase);
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, 0);
     return n;

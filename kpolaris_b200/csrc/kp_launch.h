@@ -8,8 +8,10 @@
 
 namespace kp {
 
-// Plain FP64 kernel, one quad per pixel, one image (kp_kernels_fp64.cu).
+// Plain FP64 kernel, one image: one quad per pixel (kp_kernels_fp64.cu), or
+// one thread (kp_lanes.cu).
 cudaError_t launch_image_fp64(const ImageConsts& c, const ImageOutPtrs& out, int sms, cudaStream_t stream);
+cudaError_t launch_image_lanes(const JobDesc& job, cudaStream_t stream);
 // Analysis mode: the per-pixel FP64 image with the line-of-sight
 // diagnostics (one frequency; radial_bins in 1..24).
 constexpr int kMaxRadialBins = 24;  // KPOLARIS_MAX_ANALYSIS_RADIAL_BINS
@@ -159,6 +161,7 @@ constexpr int kFarThreads = 128, kFarBlocks = 2;
 constexpr int kNearAThreads = 128, kNearABlocks = 2;
 constexpr int kNearBThreads = 256, kNearBBlocks = 1;
 constexpr int kImageThreads = 32, kImageBlocks = 8;  // the plain FP64 kernel: a warp's slot is free when its own rays end
+constexpr int kLaneNearThreads = 256;  // near-A and near-B with one ray per lane
 inline int wave_threads(int phase) {
     return phase == kPhaseFar ? kFarThreads : (phase == kPhaseNearA ? kNearAThreads : kNearBThreads);
 }
@@ -166,6 +169,65 @@ inline int wave_threads(int phase) {
 inline long long wave_blocks_needed(int phase, long long rays) {
     const int warps = wave_threads(phase) / 32;
     return (rays + warps - 1) / warps;
+}
+
+// Rays up to which a phase of the FP64 policy runs on quads; beyond, on lanes
+// (kp_lanes.cu).  `quads`: those of the phase's grid (9,472 on a B200).  The
+// lanes of a quad repeat the connection, so where rays fill the device lanes
+// are faster; near-B's quads share out the frequencies, which moves the line
+// up with their number unless FMKS makes the connection the larger part.
+// Measured, quads / lanes (ms), which agree bit for bit:
+//   far     128^2 26 / 26, 256^2 116 / 50
+//   near-A  256^2 16.6 / 17.7, 320^2 24.2 / 22.7, 512^2 61 / 37, 8 x 256^2 124 / 82
+//   near-B  1 frequency: 256^2 at 60 degrees 70 / 71, 512^2 166 / 72, 8 x 256^2 331 / 137
+//           2: 320^2 161 / 168, 512^2 338 / 282, 8 x 256^2 670 / 330
+//           4: 384^2 202 / 217, 512^2 344 / 343, 4 x 320^2 at 10 to 70 degrees 1655 / 1870,
+//              8 x 256^2 678 / 472
+//   GRMHD   256^2 177 / 185, 320^2 266 / 263, 512^2 628 / 474; four frequencies 720 / 582
+// (near-B: lanes until its input runs out, the rest on quads.  Without that
+// 4 x 320^2 took 3243, 8 x 256^2 492.)
+inline long long quad_rays(int phase, int nf_max, bool fmks, long long quads) {
+#ifdef KP_ROUNDS
+    return phase == kPhaseFar ? quads : KP_ROUNDS * quads;
+#endif
+    if (phase == kPhaseFar) return quads;
+    if (phase == kPhaseNearA || nf_max == 1 || fmks) return 8 * quads;
+    return (nf_max == 2 ? 24 : 48) * quads;
+}
+
+// Pixels up to which the plain FP64 kernel gives each a quad: with fixed
+// steps, whose rays are much of a length, while every ray gets one of its own
+// (128^2: 64 / 48 ms); with adaptive steps until the longest rays no longer
+// set the time (quads / lanes: one frequency 192^2 122 / 131, 256^2 217 / 165,
+// 1024^2 3205 / 1873; two 256^2 378 / 381, 512^2 1313 / 1075; four 512^2 1336
+// / 1439, 768^2 2900 / 2510).
+inline long long image_quad_pixels(int nfreq, bool adaptive, int sms) {
+#ifdef KP_ROUNDS
+    return KP_ROUNDS * 64ll * sms;
+#endif
+    return (!adaptive ? 1 : (nfreq == 1 ? 5 : (nfreq == 2 ? 24 : 48))) * 64ll * sms;
+}
+
+// One launch of a phase: the quad kernel and, where there can be more rays
+// than it takes, the lane kernel; whichever the launch's ray count is not for
+// returns at once.  The lane kernel of near-B hands at most its `lanes` rays
+// on, which the next launch takes on quads.
+template<class P, class SC>
+cudaError_t launch_lanes(int phase, const WaveDesc& W, int nf_max, long long lanes, long long quad_rays,
+                         cudaStream_t stream);
+
+template<class P, class SC>
+inline cudaError_t launch_wave(const void* quad_kernel, int phase, const WaveDesc& W, int nf_max, bool fmks,
+                               int blocks, int threads, cudaStream_t stream) {
+    if (nf_max < 1 || nf_max > kMaxFreq || phase < 0 || phase >= kPhases) return cudaErrorInvalidValue;
+    const long long lanes = (long long)blocks * threads;
+    long long rays = quad_rays(phase, nf_max, fmks, lanes / 4);
+    if (W.fresh_end - W.fresh_begin <= rays) {
+        void* args[] = {const_cast<WaveDesc*>(&W), &rays};
+        const cudaError_t e = cudaLaunchKernel(quad_kernel, dim3(blocks), dim3(threads), args, 0, stream);
+        if (e != cudaSuccess || W.rays_max <= rays) return e;
+    }
+    return launch_lanes<P, SC>(phase, W, nf_max, lanes, rays, stream);
 }
 
 }  // namespace kp

@@ -175,6 +175,7 @@ extern "C" int kp_batch_riaf_noalloc(const kp_riaf_job* jobs, int njobs, const k
             W.fresh_end = cycle == 0 && phase == kPhaseFar ? total : 0;
             W.in_ids = S->ids[phase][cycle % 2];
             W.in_count = &S->ctrl.counts[cycle][phase];
+            W.rays_max = total;
             W.in_head = &S->ctrl.heads[cycle * kPhases + phase];
             for (int q = 0; q < kPhases; ++q) {
                 const int gen = q > phase ? cycle : cycle + 1;

@@ -7,8 +7,8 @@
 //
 // Three phases, one kernel each, so that the lanes of a warp run the same
 // code and each kernel's instruction working set stays small (this file: what
-// they share, and the far phase with one ray per lane; kp_quad.cuh: four lanes
-// per ray):
+// they share, and their form with one ray per lane; kp_quad.cuh: four lanes per
+// ray):
 //   far     rays beyond ImageConsts::fp32_radius, pass A and pass B: pure
 //           transport (no surface lies within a step, no plasma is sampled);
 //   near-A  pass A inside: the surface-crossing search, no radiation;
@@ -223,6 +223,20 @@ __device__ __forceinline__ int phase_of(const ImageConsts& c, int in_b, double r
     return in_b ? kPhaseNearB : kPhaseNearA;
 }
 
+// The next trial of the surface-crossing search: the secant inside the
+// bracket's middle, else its half (pass_a_core.hpp:156-176).
+__device__ __forceinline__ double crossing_trial(const LaneState& b) {
+    const double width = b.hi - b.lo;
+    double trial = (b.lo + b.hi) * 0.5;
+    const double denom = b.flo - b.fhi;
+    if (b.use_secant && abs_val(denom) > kTiny) {
+        const double secant = b.lo + width * b.flo / denom;
+        const double g = width * 0.1;
+        if (secant > b.lo + g && secant < b.hi - g) trial = secant;
+    }
+    return trial;
+}
+
 // The scene a ray is finished in: a far-phase chart scene hands the ray
 // back to the scene its records use.
 template<class SC>
@@ -234,14 +248,29 @@ struct RecordScene<SceneFarCks<B>> {
     using type = B;
 };
 
-// The far phase with one ray per lane, for the scenes and policies that take
-// its steps one by one (FP64, and Boyer-Lindquist under either policy).  Pure
-// transport: every lane runs the same instructions, and with tens of
-// thousands of rays a lane per ray needs half the operations of a quad
-// (kp_quad.cuh), which evaluates a point's connection four times.
-template<class P, int NF, class SC = SceneRiaf>
-__device__ __forceinline__ void far_body(const WaveDesc& W) {
-    constexpr int PHASE = kPhaseFar;
+// Rays a launch starts with.
+__device__ __forceinline__ long long wave_rays(const WaveDesc& W) {
+    return W.fresh_end - W.fresh_begin + (long long)(W.in_ids ? *W.in_count : 0u);
+}
+
+// How a phase takes its rays: kPhaseAll is the whole life of a ray in one
+// kernel, besides the wavefront's phases (a ray is never parked and needs no
+// record, queue or counter).
+constexpr int kPhaseAll = kPhases;
+
+// The far phase, near-A, near-B or a ray's whole life with one ray per lane.
+// A lane contracts a point's connection with all three vectors, where the
+// four lanes of a quad (kp_quad.cuh) each evaluate it: with rays enough to
+// fill the device a lane per ray does less than half the operations.
+// Arithmetic and decisions are those of quad_body.  kPhaseAll: the rays
+// [fresh_begin, fresh_end) of job 0, one to each thread of the grid.
+template<class P, int NF, int PHASE, class SC = SceneRiaf>
+__device__ __forceinline__ void lane_body(const WaveDesc& W) {
+    constexpr bool kAll = PHASE == kPhaseAll;
+    constexpr bool kPassA = PHASE != kPhaseNearB;   // pass-A steps run here
+    constexpr bool kPassB = PHASE != kPhaseNearA;   // pass-B steps run here
+    constexpr bool kCross = kAll || PHASE == kPhaseNearA;  // surface-crossing search
+    constexpr bool kRad = kAll || PHASE == kPhaseNearB;    // radiative transfer
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     using RT = RadTraits<P, SC>;
@@ -249,56 +278,86 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
     st.mode = kIdle;
     st.job = -1;
     st.rk_kind = -1;
-    Ray S;
+    Ray S, kept;
     typename RT::Stokes stokes[NF];
     unsigned my_id = 0;
     int exhausted = 0;
     long long lane_jobs = 0;
     const JobDesc* J = nullptr;
+    // Near-A keeps the crossing search's best state in the record's Stokes
+    // slot, which pass A leaves unused, and its bracket in the record's
+    // control state: they hold no registers between the search's iterations.
+    static_assert(sizeof(((RayRecord*)nullptr)->stokes) >= sizeof(Ray), "the Stokes slot holds a ray");
+    auto best = [&]() -> Ray& {
+        if constexpr (kAll) return kept;
+        else return *reinterpret_cast<Ray*>(W.pool[my_id].stokes);
+    };
+    auto cs = [&]() -> LaneState& {
+        if constexpr (kAll) return st;
+        else return *reinterpret_cast<LaneState*>(W.pool[my_id].st);
+    };
     const long long nfresh = W.fresh_end - W.fresh_begin;
-    const long long total_in = nfresh + (long long)(W.in_ids ? *W.in_count : 0u);
+    long long total_in = 0;
+    if constexpr (kAll) {
+        const long long pixel = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+        if (pixel < nfresh) {
+            J = W.jobs;
+            start_ray<SC>(st, S, J, 0, int(pixel));
+        }
+    } else {
+        total_in = wave_rays(W);
+    }
 
 #pragma unroll 1
     while (true) {
-        // ------------------------------------------------------------ claim
-        const bool want = !exhausted && st.mode == kIdle;
         bool forward = false;
-        const unsigned need = __ballot_sync(FULL, want);
-        if (need) {
-            unsigned long long base = 0;
-            const int leader = __ffs(need) - 1;
-            if (lane == leader) base = atomicAdd(W.in_head, (unsigned long long)__popc(need));
-            base = __shfl_sync(FULL, base, leader);
-            if (want) {
-                const long long k = (long long)(base + __popc(need & ((1u << lane) - 1u)));
-                if (k >= total_in) {
-                    exhausted = 1;
-                } else if (k < nfresh) {
-                    // a fresh camera ray: locate its job and start pass A
-                    const long long id = W.fresh_begin + k;
-                    int lo = 0, hi = W.njobs - 1;
-                    while (lo < hi) {
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (W.jobs[mid].ray_begin <= id) lo = mid; else hi = mid - 1;
+        if constexpr (!kAll) {
+            // ------------------------------------------------------------ claim
+            const bool want = !exhausted && st.mode == kIdle;
+            const unsigned need = __ballot_sync(FULL, want);
+            if (need) {
+                unsigned long long base = 0;
+                const int leader = __ffs(need) - 1;
+                if (lane == leader) base = atomicAdd(W.in_head, (unsigned long long)__popc(need));
+                base = __shfl_sync(FULL, base, leader);
+                if (want) {
+                    const long long k = (long long)(base + __popc(need & ((1u << lane) - 1u)));
+                    if (k >= total_in) {
+                        exhausted = 1;
+                    } else if (k < nfresh) {
+                        // a fresh camera ray: locate its job and start pass A
+                        const long long id = W.fresh_begin + k;
+                        int lo = 0, hi = W.njobs - 1;
+                        while (lo < hi) {
+                            const int mid = (lo + hi + 1) >> 1;
+                            if (W.jobs[mid].ray_begin <= id) lo = mid; else hi = mid - 1;
+                        }
+                        my_id = unsigned(id);
+                        J = &W.jobs[lo];
+                        start_ray<SC>(st, S, J, lo, int(id - J->ray_begin));
+                    } else if (W.budget > 0 && lane_jobs >= W.budget) {
+                        // past the budget: hand the id on untouched (below)
+                        my_id = W.in_ids[k - nfresh];
+                        forward = true;
+                    } else {
+                        // a parked ray: resume from its record
+                        my_id = W.in_ids[k - nfresh];
+                        const RayRecord& rec = W.pool[my_id];
+                        S = rec.S;
+                        memcpy(&st, rec.st, kLaneStateBytes<PHASE>);
+                        J = &W.jobs[st.job];
+                        if constexpr (kRad) memcpy(&stokes[0], rec.stokes, sizeof(stokes));
                     }
-                    my_id = unsigned(id);
-                    J = &W.jobs[lo];
-                    start_ray<SC>(st, S, J, lo, int(id - J->ray_begin));
-                } else if (W.budget > 0 && lane_jobs >= W.budget) {
-                    // past the budget: hand the id on untouched (below)
-                    my_id = W.in_ids[k - nfresh];
-                    forward = true;
-                } else {
-                    // a parked ray: resume from its record
-                    my_id = W.in_ids[k - nfresh];
-                    const RayRecord& rec = W.pool[my_id];
-                    S = rec.S;
-                    memcpy(&st, rec.st, kLaneStateBytes<PHASE>);
-                    J = &W.jobs[st.job];
                 }
             }
+            queue_push(W.out_ids[PHASE], W.out_count[PHASE], forward, my_id);
         }
-        queue_push(W.out_ids[PHASE], W.out_count[PHASE], forward, my_id);
+        // Near-B hands the rays left when its input runs out to the quads of
+        // its next launch: the longest rays, of which few are left then, take
+        // a step in half to a quarter of a lane's time.
+        bool hand_over = false;
+        if constexpr (PHASE == kPhaseNearB)
+            hand_over = (long long)*(const volatile unsigned long long*)W.in_head >= total_in;
         const bool active = st.mode != kIdle;
         // The block leaves the loop together, so the barrier below is
         // reached by every thread of the block in every iteration.  A lane
@@ -308,33 +367,33 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
 
         // ---------------------------------------------- control before the job
         int dest = -1;  // phase the ray is handed to (PHASE itself: its next launch)
-        {
+        if constexpr (kPassA) {
             if (active && st.mode == kAStep && st.rk_kind < 0) {
                 const ImageConsts& c = J->c;
-                const double r_bl = SC::radius(c, S.x);
-                const int want_phase = phase_of(c, 0, r_bl);
+                const double r_top = SC::template top_radius<P::kMixed>(c, S.x);
+                const int want_phase = kAll ? PHASE : phase_of(c, 0, r_top);
                 if (want_phase != PHASE) {
                     dest = want_phase;
-                } else if (W.budget > 0 && lane_jobs >= W.budget) {
+                } else if (!kAll && W.budget > 0 && lane_jobs >= W.budget) {
                     dest = PHASE;
                 } else if (st.n >= c.max_steps) {
                     // pass-A loop top (pass_b.hpp:793-838)
                     st.mode = kEndA;
                 } else {
                     if (!st.entered) {
-                        if (r_bl <= c.outer_radius) {
+                        if (r_top <= c.outer_radius) {
                             st.entered = 1;
                             st.inside = 0;
                         }
-                    } else if (r_bl - c.inner_radius <= 0.0) {
+                    } else if (r_top - c.inner_radius <= 0.0) {
                         st.reason = kReachedInner;
                         st.mode = kEndA;
-                    } else if (st.inside > 0 && r_bl >= c.outer_radius) {
+                    } else if (st.inside > 0 && r_top >= c.outer_radius) {
                         st.reason = kEscaped;
                         st.mode = kEndA;
                     }
                     if (st.mode == kAStep) {
-                        st.old_r = r_bl;
+                        st.old_r = r_top;
                         double mn = c.min_step_abs;
                         if (abs_val(st.h_current) < mn) mn = abs_val(st.h_current);
                         issue_step(st, c, st.h_current, mn, c.max_step);
@@ -356,7 +415,7 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
                     // the ray reaches the radiating phase
 #pragma unroll
                     for (int f = 0; f < NF; ++f) RT::zero(stokes[f]);
-                    memcpy(W.pool[my_id].stokes, &stokes[0], sizeof(stokes));
+                    if constexpr (!kAll) memcpy(W.pool[my_id].stokes, &stokes[0], sizeof(stokes));
                 } else {
                     st.mode = kDone;
                 }
@@ -367,42 +426,49 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
             if (st.reached || st.steps >= c.max_steps) {
                 st.mode = kDone;
             } else {
-                const double r_bl = SC::radius(c, S.x);
-                const int want_phase = phase_of(c, 1, r_bl);
+                const double r_top = SC::template top_radius<P::kMixed>(c, S.x);
+                const int want_phase = kAll ? PHASE : phase_of(c, 1, r_top);
                 if (want_phase != PHASE) {
                     dest = want_phase;
-                } else if (W.budget > 0 && lane_jobs >= W.budget) {
+                } else if (hand_over || (!kAll && W.budget > 0 && lane_jobs >= W.budget)) {
                     dest = PHASE;
                 } else {
                     // pass-B loop top (pass_b.hpp:966-981)
                     double h = st.h_current;
-                    st.start_r = r_bl;
+                    st.start_r = r_top;
                     if (st.start_r <= c.outer_radius && st.cap > 0.0) h = min_val(h, st.cap);
                     st.hB = h;
                     issue_step(st, c, h, c.min_step_abs, c.max_step);
                 }
             }
         }
-        const bool park = dest >= 0;
-        if (park) {
-            RayRecord& rec = W.pool[my_id];
-            rec.S = S;
-            memcpy(rec.st, &st, kLaneStateBytes<PHASE>);
-        }
-        // A lane past its budget keeps claiming and parks each claimed ray at
-        // once, so every input ends the launch finished or in a queue.
+        const bool park = !kAll && dest >= 0;
+        if constexpr (!kAll) {
+            if (park) {
+                RayRecord& rec = W.pool[my_id];
+                rec.S = S;
+                memcpy(rec.st, &st, kLaneStateBytes<PHASE>);
+                if constexpr (kRad) memcpy(rec.stokes, &stokes[0], sizeof(stokes));
+            }
+            // A lane past its budget keeps claiming and parks each claimed ray at
+            // once, so every input ends the launch finished or in a queue.
 #pragma unroll
-        for (int d = 0; d < kPhases; ++d) queue_push(W.out_ids[d], W.out_count[d], dest == d, my_id);
-        if (park) st.mode = kIdle;
+            for (int d = 0; d < kPhases; ++d) queue_push(W.out_ids[d], W.out_count[d], dest == d, my_id);
+            if (park) st.mode = kIdle;
+        }
 
         // ------------------------------------------------------------ RK job
-        const bool run = !park && (st.mode == kAStep || st.mode == kBStep || st.mode == kBCamCross);
+        const bool crossing_job = kCross && (st.mode == kACrossHi || st.mode == kACrossTrial);
+        const bool run = !park && (st.mode == kAStep || crossing_job || st.mode == kBStep || st.mode == kBCamCross);
         Ray next, mid;
         double err = 0.0;
         if (run) {
+            const int kind = crossing_job ? (J->c.adaptive ? kRkRK4x2 : kRkRK4) : st.rk_kind;
+            const double hj =
+                crossing_job ? (st.mode == kACrossHi ? cs().full_h : cs().full_h * cs().trial) : st.h_try;
             bool sure = false;
             if constexpr (SC::kCksRhs) {
-                if (st.rk_kind == kRkSD) {
+                if (kind == kRkSD) {
                     double km = 0.0, w = 0.0, z = 0.0;
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
@@ -416,8 +482,8 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
                                         (abs_val(st.h_try) == st.ctl_max ? 0.25 : 1.0 / 64.0) * tol);
                 }
             }
-            rk_job<P, SC>(st.rk_kind, J->c, S, st.h_try, sure, next, mid, err);
-            if (++lane_jobs > (1LL << 30)) {
+            rk_job<P, SC, kCross>(kind, J->c, S, hj, sure, next, mid, err);
+            if (!kAll && ++lane_jobs > (1LL << 30)) {
                 st.reason = kInvalidState;
                 st.mode = kDone;
                 st.in_b = 0;
@@ -431,9 +497,10 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
         __syncthreads();
 
         // ----------------------------------------------- control after the job
-        if (run && st.mode == kAStep) {
+        if (kPassA && run && st.mode == kAStep) {
             const ImageConsts& c = J->c;
             bool accepted = true;
+            const double used_h = st.h_try;
             if (st.rk_kind != kRkRK4) {
                 const double tol = max_val(c.tolerance, kTolFloor);
                 if (err <= tol) {
@@ -454,7 +521,7 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
             if (accepted) {
                 // pass_b.hpp:864-937
                 st.rk_kind = -1;
-                const double next_r = SC::radius(c, next.x);
+                const double next_r = SC::template top_radius<P::kMixed>(c, next.x);
                 const double old_r = st.old_r;
                 if (!st.entered && next_r <= c.outer_radius) {
                     st.entered = 1;
@@ -473,9 +540,26 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
                         crossing = kEscaped;
                     }
                     if (crossing != kNone) {
-                        atomicExch(W.status, 3);  // surfaces lie inside the near phase
-                        st.reason = kInvalidState;
-                        st.mode = kDone;
+                        if constexpr (kCross) {
+                            cs().cross_reason = crossing;
+                            cs().surf = crossing == kReachedInner ? c.inner_radius : c.outer_radius;
+                            cs().full_h = used_h;
+                            best() = S;
+                            cs().lo = 0.0;
+                            cs().hi = 1.0;
+                            cs().flo = old_r - cs().surf;
+                            if (cs().flo == 0.0 || !finite_ray(next)) {
+                                st.pa_steps += 1;  // the event keeps the first state
+                                st.reason = crossing;
+                                st.mode = kEndA;
+                            } else {
+                                st.mode = kACrossHi;
+                            }
+                        } else {
+                            atomicExch(W.status, 3);  // surfaces lie inside the near phase
+                            st.reason = kInvalidState;
+                            st.mode = kDone;
+                        }
                     } else {
                         S = next;
                         st.pa_steps += 1;
@@ -484,7 +568,58 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
                     }
                 }
             }
-        } else if (run && (st.mode == kBStep || st.mode == kBCamCross)) {
+        } else if (kCross && run && (st.mode == kACrossHi || st.mode == kACrossTrial)) {
+            const ImageConsts& c = J->c;
+            const int next_finite = finite_ray(next);
+            const double next_r = SC::template top_radius<P::kMixed>(c, next.x);
+            bool finish = false;
+            if (st.mode == kACrossHi) {
+                if (!next_finite) {
+                    finish = true;
+                } else {
+                    const double fhi = next_r - cs().surf;
+                    if (!(fhi == fhi) || abs_val(fhi) >= kLarge) {
+                        finish = true;
+                    } else if (fhi == 0.0) {
+                        best() = next;
+                        finish = true;
+                    } else if ((cs().flo > 0.0) == (fhi > 0.0)) {
+                        finish = true;
+                    } else {
+                        cs().fhi = fhi;
+                        cs().iter = 0;
+                        cs().use_secant = 1;
+                    }
+                }
+            } else {
+                const double ft = next_finite ? next_r - cs().surf : 0.0;
+                if (!next_finite || !(ft == ft) || abs_val(ft) >= kLarge) {
+                    cs().hi = cs().trial;
+                    cs().use_secant = 0;
+                } else if (ft == 0.0) {
+                    best() = next;
+                    finish = true;
+                } else if ((cs().flo > 0.0) == (ft > 0.0)) {
+                    cs().lo = cs().trial;
+                    cs().flo = ft;
+                    best() = next;
+                } else {
+                    cs().hi = cs().trial;
+                    cs().fhi = ft;
+                }
+                cs().iter += 1;
+            }
+            if (!finish && cs().iter >= 12) finish = true;
+            if (finish) {
+                S = best();
+                st.pa_steps += 1;
+                st.reason = cs().cross_reason;
+                st.mode = kEndA;
+            } else {
+                cs().trial = crossing_trial(cs());
+                st.mode = kACrossTrial;
+            }
+        } else if (kPassB && run && (st.mode == kBStep || st.mode == kBCamCross)) {
             const ImageConsts& c = J->c;
             const bool cam = st.mode == kBCamCross;
             bool proceed = true;
@@ -511,11 +646,12 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
             }
             if (proceed) {
                 Ray sample = st.rk_kind == kRkSD ? mid : next;
+                double next_r = SC::template top_radius<P::kMixed>(c, next.x);
                 int crosses = 1;
                 if (!cam) {
                     // camera surface (pass_b.hpp:999-1028)
                     const double s0 = st.start_r - c.cam_radius;
-                    const double s1 = SC::radius(c, next.x) - c.cam_radius;
+                    const double s1 = next_r - c.cam_radius;
                     crosses = (s0 == 0.0 || s1 == 0.0) ? 1 : ((s0 < 0.0 && s1 > 0.0) || (s0 > 0.0 && s1 < 0.0));
                     if (crosses) {
                         const double denom = s0 - s1;
@@ -525,6 +661,7 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
                             h = 0.0;
                             next = S;
                             sample = S;
+                            next_r = st.start_r;
                         } else if (frac < 0.999999999999) {
                             h = h_cross;
                             const double mn = min_val(c.min_step_abs, abs_val(h));
@@ -536,22 +673,100 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
                     }
                 }
                 if (proceed) {
-                    // The sample lies outside the radiating sphere: every
-                    // coefficient is zero, the transfer step leaves the Stokes
-                    // vector unchanged and the step cap resolves to max_step
-                    // (pass_b.hpp:1414-1496).
-                    const double sample_r = SC::radius(c, sample.x);
-                    const double next_r = SC::radius(c, next.x);
-                    if ((c.max_radiation_step > 0.0 &&
-                         (st.start_r <= c.outer_radius || sample_r <= c.outer_radius || next_r <= c.outer_radius)) ||
-                        (sample_r - c.inner_radius > 0.0 && sample_r < c.outer_radius))
+                    // radiation at the sample point (pass_b.hpp:1414-1496)
+                    const double sample_r = SC::template top_radius<P::kMixed>(c, sample.x);
+                    const double local_max_rs =
+                        (c.max_radiation_step > 0.0 &&
+                         (st.start_r <= c.outer_radius || sample_r <= c.outer_radius || next_r <= c.outer_radius))
+                            ? c.max_radiation_step : 0.0;
+                    bool radiating = sample_r - c.inner_radius > 0.0 && sample_r < c.outer_radius;
+                    bool stopped = false;
+                    int required = 1, pred = 1;
+                    typename RT::Co co[NF];
+                    // a step without plasma: its coefficients are zero, its
+                    // transfer adds zero
+                    const bool empty = kAll && !radiating;
+                    const int nf = c.nfreq < NF ? c.nfreq : NF;
+                    if constexpr (kRad) {
+                        typename RT::Sample ps = RT::none();
+                        if constexpr (SC::kSlowLight) {
+                            // slow_light_driver.hpp:1295-1304: a radiating sample
+                            // needs its fluid time among the resident snapshots;
+                            // otherwise the ray ends where it stands
+                            radiating = sample_r >= c.inner_radius && sample_r < c.outer_radius;
+                            if (radiating && !SC::time_resident(c, sample)) {
+                                st.reason = kSlowLightTimeExhausted;
+                                st.mode = kDone;
+                                stopped = true;
+                            }
+                        }
+                        if (radiating && !stopped) ps = RT::sample(c, sample);
+                        if (empty) {
+                            const RadDepths none = {0.0, 0.0, 0.0};
+                            required = substeps_for(none, h, local_max_rs, c);
+                            pred = substeps_for(none, st.h_current, local_max_rs, c);
+                        } else if (!stopped) {
+                            // The frequency loops stay rolled: one copy of the
+                            // coefficient and transfer code keeps the kernel's
+                            // instruction working set small.
+#pragma unroll 1
+                            for (int f = 0; f < nf; ++f) {
+                                co[f] = RT::coeffs(c, ps, f);
+                                if (!c.faraday_rotation) co[f].rV = 0.0;
+                            }
+                            // Substep counts at h (required) and at h_current
+                            // (predictive) in one pass: neither test changes h or
+                            // h_current.  Over the image's frequencies, or over a
+                            // separate step-control list (pass_b.hpp:1787-1833).
+                            const bool fused = c.nctl == 0;
+#pragma unroll 1
+                            for (int g = 0; g < (fused ? nf : c.nctl); ++g) {
+                                typename RT::Co cg = co[fused ? g : 0];
+                                double dls = c.dlambda_scale[fused ? g : 0];
+                                if (!fused) {
+                                    cg = RT::coeffs_ctl(c, ps, g);
+                                    if (!c.faraday_rotation) cg.rV = 0.0;
+                                    dls = c.ctl_dlambda_scale[g];
+                                }
+                                const RadDepths depth = RT::depths(cg, dls);
+                                const int cand = substeps_for(depth, h, local_max_rs, c);
+                                required = cand > required ? cand : required;
+                                const int pc = substeps_for(depth, st.h_current, local_max_rs, c);
+                                pred = pc > pred ? pc : pred;
+                            }
+                        }
+                    } else if (local_max_rs > 0.0 || radiating) {
+                        // far phase: every sample lies outside the radiating sphere
                         atomicExch(W.status, 3);
-                    st.cap = c.max_step;
-                    S = next;
-                    st.steps += 1;
-                    if (crosses) st.reached = 1;
-                    st.mode = kBStep;
-                    st.rk_kind = -1;
+                    }
+                    if (!stopped) {
+                        if (kRad && required > 1 && h > c.min_step_abs * 1.0001) {
+                            st.h_current = max_val(c.min_step_abs, over_pow2(h, required));
+                            st.cap = st.h_current;
+                        } else {
+                            st.cap = c.max_step;
+                            if (kRad && pred > 1 &&
+                                (local_max_rs > 0.0 || c.max_radiation_depth > 0.0 || c.max_absorption_depth > 0.0 ||
+                                 c.max_faraday_depth > 0.0))
+                                st.cap = max_val(c.min_step_abs, over_pow2(st.h_current, pred));
+                            if constexpr (kRad) {
+                                if (empty) {
+                                    if constexpr (kAll) {
+#pragma unroll
+                                        for (int f = 0; f < NF; ++f) RT::add_zero(stokes[f]);
+                                    }
+                                } else if (h > 0.0) {
+#pragma unroll 1
+                                    for (int f = 0; f < nf; ++f) RT::step(stokes[f], co[f], h, c, f);
+                                }
+                            }
+                            S = next;
+                            st.steps += 1;
+                            if (crosses) st.reached = 1;
+                        }
+                        st.mode = kBStep;
+                        st.rk_kind = -1;
+                    }
                 }
             }
         }
@@ -575,7 +790,9 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
             double obs[NF][4];
             Stokes4<double> sd[NF];
             // only the radiating phase carries the Stokes vector: it is in the record
-            if (st.in_b) memcpy(&stokes[0], W.pool[my_id].stokes, sizeof(stokes));
+            if constexpr (!kRad) {
+                if (st.in_b) memcpy(&stokes[0], W.pool[my_id].stokes, sizeof(stokes));
+            }
 #pragma unroll
             for (int f = 0; f < NF; ++f)
                 sd[f] = st.in_b ? RT::result(stokes[f], c, f) : Stokes4<double>{0.0, 0.0, 0.0, 0.0};
@@ -585,7 +802,7 @@ __device__ __forceinline__ void far_body(const WaveDesc& W) {
             if constexpr (SC::kSlowLight) {
                 if (!st.in_b) J->out.basis_identity_error[st.pixel] = 0.0;
             }
-            if (W.job_done) atomicAdd(&W.job_done[st.job], 1u);
+            if (!kAll && W.job_done) atomicAdd(&W.job_done[st.job], 1u);
             st.mode = kIdle;
         }
     }

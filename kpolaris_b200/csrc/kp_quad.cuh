@@ -329,10 +329,6 @@ __device__ __forceinline__ void quad_job(int kind, const ImageConsts& c, const D
     mid = sd ? R2 : next;
 }
 
-// The whole life of a ray in one kernel, besides the wavefront's phases: a
-// ray is never parked and needs no record, queue or counter.
-constexpr int kPhaseAll = kPhases;
-
 // The run of steps to bridge from a step just issued (count 0: take the
 // step): a step-doubling or a fixed step, in Cartesian Kerr-Schild.
 template<class SC, class LS>
@@ -399,7 +395,7 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
             r_top = SC::template top_radius<P::kMixed>(J->c, S.x);
         }
     } else {
-        total_in = nfresh + (long long)(W.in_ids ? *W.in_count : 0u);
+        total_in = wave_rays(W);
         // With fewer rays than quads the rays spread over the warps: a warp's
         // issue slots then serve fewer rays.
         const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
@@ -774,15 +770,7 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
                 st.reason = st.cross_reason;
                 st.mode = kEndA;
             } else {
-                const double width = st.hi - st.lo;
-                double trial = (st.lo + st.hi) * 0.5;
-                const double denom = st.flo - st.fhi;
-                if (st.use_secant && abs_val(denom) > kTiny) {
-                    const double secant = st.lo + width * st.flo / denom;
-                    const double g = width * 0.1;
-                    if (secant > st.lo + g && secant < st.hi - g) trial = secant;
-                }
-                st.trial = trial;
+                st.trial = crossing_trial(st);
                 st.mode = kACrossTrial;
             }
         } else if (kPassB && run && (st.mode == kBStep || st.mode == kBCamCross)) {
@@ -999,24 +987,6 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
                 st.mode = kIdle;
             }
         }
-    }
-}
-
-// The FP64 policy's far phase: quads as long as every ray of the launch gets
-// one of its own, one thread per ray beyond.  A quad's step is shorter (far
-// phase of a 16^2 to 96^2 image 19 to 25 -> 10 to 14 ms, of a 64^2 GRMHD
-// image 15 ms less), but its lanes repeat the connection: once the quads take
-// turns the SMs' FP64 units run more of it (128^2: 25.8 ms with threads, 29.5
-// with quads; 256^2: 50 and 116).  The two agree bit for bit, so a ray's
-// results do not depend on the choice.
-template<class P, int NF, class SC = SceneRiaf>
-__device__ __forceinline__ void far_phase(const WaveDesc& W) {
-    static_assert(!P::kMixed, "the forms agree bit for bit without contraction only");
-    const long long rays = W.fresh_end - W.fresh_begin + (long long)(W.in_ids ? *W.in_count : 0u);
-    if (rays <= (long long)gridDim.x * (blockDim.x >> 2)) {
-        quad_body<P, kPhaseFar, SC>(W);
-    } else {
-        far_body<P, NF, SC>(W);
     }
 }
 

@@ -285,6 +285,7 @@ void worker_main(kp_server* s) {
     while (true) {
         // ---- admission (FIFO; the head of the queue waits for room)
         std::vector<std::shared_ptr<ServerJob>> admitted;
+        long long inflight_rays = 0;
         bool any_inflight = false;
         {
             std::unique_lock<std::mutex> lock(s->mu);
@@ -339,7 +340,6 @@ void worker_main(kp_server* s) {
                 admitted.push_back(j);
                 s->pending.pop_front();
             }
-            long long inflight_rays = 0;
             int inflight_jobs = 0;
             for (const auto& j : s->slots)
                 if (j) {
@@ -420,6 +420,7 @@ void worker_main(kp_server* s) {
                 W.fresh_end = 0;
                 W.in_ids = s->ids[sc][p][cur];
                 W.in_count = cnt + cur * kPhases + p;
+                W.rays_max = inflight_rays;
                 W.in_head = s->heads[sc] + p;
                 for (int q = 0; q < kPhases; ++q) {
                     const int g = q > p ? cur : nxt;

@@ -10,7 +10,11 @@ and mixes at which four lanes per ray can go wrong.
   that the quads of a warp trace different images: each is bit for bit the
   image traced alone, in either precision.
 * Just as many rays as a B200's resident quads (9,472) take the FP64 far phase
-  as quads, more as threads: both are the one-launch kernel's, bit for bit.
+  as quads, more as lanes (one ray per thread): both are the one-launch
+  kernel's, bit for bit.
+* The near phases and the one-launch kernel take lanes from a number of rays
+  on: the smallest launches that do, of one image or several, one to four
+  frequencies, every scene, are those of the quads, bit for bit.
 * The mixed policy's far field takes many steps at once and counts them: on
   rays that miss the sphere, cameras near, inside the far boundary and far
   out, and large and small step caps, its reasons are those of the FP64 policy
@@ -23,7 +27,7 @@ import pytest
 
 import kpolaris_b200 as kp
 import oracle
-from kpolaris_b200 import _abi, configs
+from kpolaris_b200 import _abi, configs, synthetic
 
 pytestmark = pytest.mark.gpu
 
@@ -84,3 +88,51 @@ def test_far_field_runs_keep_the_step_counts(radius, fov, max_step):
     for key in ("pass_a_steps", "steps"):
         d = mixed.arrays[key] != fp64.arrays[key]
         assert np.mean(d) <= 0.005, (key, int(d.sum()))
+
+
+def forms(image, **options):
+    """An image with the launch's own choice of quads and lanes, and with
+    quads in every near phase: the line is a number of rays per quad of the
+    grid, which blocks_per_sm enlarges."""
+    return image(**options), image(blocks_per_sm=16, **options)
+
+
+# The smallest launches that take lanes on a B200 (148 SMs): 75,776 rays in
+# near-A and at one frequency, 227,328 at two, 454,656 at three or four.
+@pytest.mark.parametrize("sizes,nf", [([(279, 272)], 1), ([(478, 476)], 2), ([(477, 477), (97, 9), (1, 1)], 4),
+                                      ([(256, 256)] * 7, 3)])
+def test_near_phase_forms_agree(sizes, nf):
+    jobs = [job(nx, ny, 1 + (k + nf - 1) % nf, inclination=17.0 + 9.0 * k, spin=0.9375 - 0.1 * k)
+            for k, (nx, ny) in enumerate(sizes)]
+    a, b = forms(lambda **o: kp.batch_riaf(jobs, precision=_abi.PRECISION_FP64, **o))
+    for k in range(len(jobs)):
+        assert_bitwise(a[k], b[k], k)
+
+
+@pytest.mark.parametrize("coordinates", ["fmks", "slow", "bl"])
+def test_near_phase_forms_agree_in_other_scenes(coordinates):
+    options = dict(precision=_abi.PRECISION_FP64, schedule=_abi.SCHEDULE_PERSISTENT)
+    if coordinates == "bl":
+        p, m, f = job(280, 271, 1)
+        p.coordinate_system = _abi.COORD_BOYER_LINDQUIST
+        a, b = forms(lambda **o: kp.image_riaf(p, m, f, **o), **options)
+    else:
+        grids = []
+        for t in (0.0, 60.0):
+            prims, model = synthetic.fm_torus(96, 48, 48, time=t)
+            grids.append(kp.Grid(model, prims))
+        p = synthetic.fmks_pass_a_params(model, 280, 271)
+        if coordinates == "fmks":
+            a, b = forms(lambda **o: kp.image_grmhd(p, grids[0], [230e9, 345e9], **o), **options)
+        else:
+            a, b = forms(lambda **o: kp.image_grmhd_slow_light(p, grids, [0.0, 60.0], 1040.0, [230e9], **o), **options)
+    assert_bitwise(a, b, coordinates)
+
+
+# One pixel above the line of the one-launch kernel (9,472 pixels of fixed
+# steps, 47,360 at one frequency, 227,328 at two) against the wavefront.
+@pytest.mark.parametrize("nx,ny,nf,adaptive", [(43, 221, 1, False), (43, 221, 4, False), (11, 4306, 1, True),
+                                               (478, 476, 2, True)])
+def test_plain_kernel_forms_agree(nx, ny, nf, adaptive):
+    p, m, f = job(nx, ny, nf, adaptive=adaptive)
+    assert_bitwise(kp.image_riaf(p, m, f), kp.image_riaf(p, m, f, schedule=_abi.SCHEDULE_PERSISTENT), (nx, ny))

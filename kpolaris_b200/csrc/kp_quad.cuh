@@ -448,9 +448,10 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
                         J = &W.jobs[st.job];
                         if constexpr (SC::kFarChart) {
                             Ray S = rec.S;
+                            const bool paused = st.chart;
                             enter_chart<SC>(st, J->c, S);
                             V = role == 0 ? S.x : (role == 1 ? S.k : (role == 2 ? S.e1 : S.e2));
-                            r_top = SC::template top_radius<P::kMixed>(J->c, S.x);
+                            r_top = paused ? st.start_r : SC::template top_radius<P::kMixed>(J->c, S.x);
                         } else {
                             V = reinterpret_cast<const D4*>(&rec.S)[role];
                             r_top = SC::template top_radius<P::kMixed>(J->c, rec.S.x);
@@ -573,6 +574,10 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
             }
             if (park) {
                 RayRecord& rec = W.pool[my_id];
+                // a pause keeps the chart's radius too (start_r is unused
+                // here): evaluated again at another call site, its fused
+                // operations may differ
+                if constexpr (SC::kFarChart) st.start_r = r_top;
                 reinterpret_cast<D4*>(&rec.S)[role] = V;
                 if (role == 0) memcpy(rec.st, &st, kLaneStateBytes<PHASE>);
                 if constexpr (kRad) memcpy(rec.stokes + 4 * role, &stokes, sizeof(stokes));

@@ -92,3 +92,21 @@ def test_grmhd_job_validation(tori):
         big = synthetic.fmks_pass_a_params(model, 128, 128)
         with pytest.raises(kp.KPolarisError):
             srv.submit_grmhd(big, g, [230e9])
+
+
+@pytest.mark.parametrize("tick", [16, 20, 24, 28, 33, 40, 50, 64])
+def test_mixed_grmhd_rays_resume_bit_for_bit(tori, tick):
+    """Ticks of so few RK jobs park a mixed GRMHD ray many times in the far
+    phase, which holds it in another chart than its record; the image is the
+    one traced without a pause.  (Which rays pause where differs from run to
+    run, so one tick length alone may miss a pause that matters.)"""
+    (p0, m0), _ = tori
+    with kp.Grid(m0, p0) as g:
+        p = synthetic.fmks_pass_a_params(m0, 150, 150)
+        alone = kp.image_grmhd(p, g, [230e9], precision=_abi.PRECISION_MIXED)
+        with kp.Server(precision=_abi.PRECISION_MIXED, tick_budget=tick) as srv:
+            tickets = [srv.submit_grmhd(p, g, [230e9]) for _ in range(2)]
+            for t in tickets:
+                srv.wait(t, timeout=300.0)
+            for t in tickets:
+                assert_bitwise(srv.result(t), alone, tick)

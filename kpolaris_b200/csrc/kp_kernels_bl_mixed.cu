@@ -7,9 +7,10 @@
 
 namespace kp {
 
-template<int NF>
+// one form whatever shares the launch: compiled for one frequency, the end of
+// a ray rounds differently
 __global__ void __launch_bounds__(kFarThreads, 2) wave_bl_mixed_far(const WaveDesc W) {
-    lane_body<PolicyMixed, NF, kPhaseFar, SceneRiafBL>(W);
+    lane_body<PolicyMixed, kMaxFreq, kPhaseFar, SceneRiafBL>(W);
 }
 
 __global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_bl_mixed_near_a(const WaveDesc W) {
@@ -20,23 +21,22 @@ __global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_bl_mixed_nea
     quad_body<PolicyMixed, kPhaseNearB, SceneRiafBL>(W);
 }
 
-template<int NF>
 static const void* wave_bl_mixed_kernel(int phase) {
-    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_bl_mixed_far<NF>);
+    if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_bl_mixed_far);
     if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_bl_mixed_near_a);
     return reinterpret_cast<const void*>(wave_bl_mixed_near_b);
 }
 
 cudaError_t launch_wave_bl_mixed(int phase, const WaveDesc& W, int nf_max, int blocks, int threads, cudaStream_t stream) {
     if (nf_max < 1 || nf_max > kMaxFreq || phase < 0 || phase >= kPhases) return cudaErrorInvalidValue;
-    const void* fn = nf_max == 1 ? wave_bl_mixed_kernel<1>(phase) : wave_bl_mixed_kernel<kMaxFreq>(phase);
+    const void* fn = wave_bl_mixed_kernel(phase);
     void* args[] = {const_cast<WaveDesc*>(&W)};
     return cudaLaunchKernel(fn, dim3(blocks), dim3(threads), args, 0, stream);
 }
 
 int wave_occupancy_bl_mixed(int phase, int nf_max, int threads) {
     if (phase < 0 || phase >= kPhases) return 0;
-    const void* fn = nf_max == 1 ? wave_bl_mixed_kernel<1>(phase) : wave_bl_mixed_kernel<kMaxFreq>(phase);
+    const void* fn = wave_bl_mixed_kernel(phase);
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, 0);
     return n;

@@ -31,7 +31,7 @@ import pytest
 
 import kpolaris_b200 as kp
 from golden_cases import BL_CASES, build_bl_case
-from kpolaris_b200 import _abi
+from kpolaris_b200 import _abi, configs
 from test_gpu_batch import EVPA_TOL_DEG, FLUX_RTOL_MIXED, evpa_diff, integrated
 from test_gpu_parity import check_fp64
 
@@ -78,3 +78,20 @@ def test_bl_alone_equals_in_batch(precision):
     mix = kp.batch_riaf([b, a, b], precision=precision)
     for key in alone.arrays:
         assert np.array_equal(mix[1].arrays[key], alone.arrays[key], equal_nan=True), key
+
+
+@pytest.mark.parametrize("precision", [_abi.PRECISION_FP64, _abi.PRECISION_MIXED])
+def test_bl_one_frequency_alone_equals_beside_four(precision):
+    jobs = []
+    for nx, ny, nf, spin, inclination in ((61, 44, 1, 0.15, 31.0), (97, 61, 4, 0.75, 75.0), (32, 37, 1, 0.6, 64.0)):
+        p = configs.config2(nx, ny)[0]
+        p.spin = spin
+        p.inner_radius = configs.reference_horizon(spin) * 1.05
+        p.camera.inclination = configs.inclination_from_degrees(inclination)
+        p.coordinate_system = _abi.COORD_BOYER_LINDQUIST
+        jobs.append((p, configs.riaf_model(), configs.CONFIG2_FREQS[:nf]))
+    mix = kp.batch_riaf(jobs, precision=precision)
+    for k, (p, m, f) in enumerate(jobs):
+        alone = kp.image_riaf(p, m, f, precision=precision, schedule=_abi.SCHEDULE_PERSISTENT)
+        for key in alone.arrays:
+            assert np.array_equal(mix[k].arrays[key], alone.arrays[key], equal_nan=True), (k, key)

@@ -31,17 +31,12 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off",
           f"-I{INCLUDE}", f"-I{CSRC}", "-Xptxas", "-warn-spills"]
 
-def _lanes(policy, scene, *more):
-    fp = ["--fmad=false"] if policy == "FP64" else ["--fmad=true", "--use_fast_math"]
-    return [*fp, f"-DKP_LANES_POLICY=Policy{policy}", f"-DKP_LANES_SCENE=Scene{scene}", *more]
-
-
 # translation unit, with the name of its build where it has several -> extra flags
 UNITS = {
-    "kp_lanes.cu fp64": _lanes("FP64", "Riaf", "-DKP_LANES_IMAGE"),
-    "kp_lanes.cu grmhd": _lanes("FP64", "Grmhd"),
-    "kp_lanes.cu grmhd_slow": _lanes("FP64", "GrmhdSlow"),
-    "kp_lanes.cu bl": _lanes("FP64", "RiafBL"),
+    "kp_lanes.cu fp64": ["--fmad=false", "-DKP_LANES_SCENE=SceneRiaf", "-DKP_LANES_IMAGE"],
+    "kp_lanes.cu grmhd": ["--fmad=false", "-DKP_LANES_SCENE=SceneGrmhd"],
+    "kp_lanes.cu grmhd_slow": ["--fmad=false", "-DKP_LANES_SCENE=SceneGrmhdSlow"],
+    "kp_lanes.cu bl": ["--fmad=false", "-DKP_LANES_SCENE=SceneRiafBL"],
     "kp_kernels_fp64.cu": ["--fmad=false"],
     "kp_kernels_mixed.cu": ["--fmad=true", "--use_fast_math"],
     "kp_kernels_grmhd.cu": ["--fmad=false"],

@@ -69,7 +69,7 @@ constexpr size_t kGraphCacheSize = 8;
 // a ray for a phase that comes later in the cycle into generation c, for its
 // own or an earlier phase into generation c + 1.
 struct WaveCtrl {
-    unsigned long long heads[kMaxWaveCycles * kPhases];
+    unsigned long long heads[kMaxWaveCycles * kPhases], lane_heads[kMaxWaveCycles * kPhases];
     unsigned counts[kMaxWaveCycles + 1][kPhases];
     int status;
 };
@@ -104,7 +104,7 @@ struct DeviceState {
     // instantiated launch graphs (KP_SCHEDULE_GRAPH), keyed by everything
     // they bake in; the oldest is dropped beyond kGraphCacheSize
     struct GraphEntry {
-        int family, nf_max, njobs, cycles;
+        int family, nf_max, njobs, cycles, forms;
         long long total;
         int blocks[kPhases];
         const void* jobs;
@@ -635,6 +635,8 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         const long long needed = wave_blocks_needed(phase, total);
         if (blocks[phase] > needed) blocks[phase] = int(needed);
     }
+    int forms = 0;
+    for (int i = 0; i < njobs; ++i) forms |= dev->h_jobs[i].lanes ? kFormLanes : kFormQuads;
     WaveCtrl* ctrl = dev->d_ctrl;
     auto launch = [&](int cycle, int phase) -> cudaError_t {
         WaveDesc W;
@@ -647,6 +649,8 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         W.in_count = &ctrl->counts[cycle][phase];
         W.rays_max = total;
         W.in_head = &ctrl->heads[cycle * kPhases + phase];
+        W.lane_head = &ctrl->lane_heads[cycle * kPhases + phase];
+        W.forms = forms;
         for (int q = 0; q < kPhases; ++q) {
             const int gen = q > phase ? cycle : cycle + 1;
             W.out_ids[q] = dev->d_ids[q][gen % 2];
@@ -693,6 +697,7 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         key.nf_max = nf_max;
         key.njobs = njobs;
         key.cycles = cycles;
+        key.forms = forms;
         key.total = total;
         for (int p = 0; p < kPhases; ++p) {
             key.blocks[p] = blocks[p];
@@ -706,7 +711,7 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         key.lpt = dev->d_lpt;
         cudaGraphExec_t exec = nullptr;
         for (const auto& g : dev->graphs) {
-            if (g.family == key.family && g.nf_max == key.nf_max && g.njobs == key.njobs && g.cycles == key.cycles &&
+            if (g.family == key.family && g.nf_max == key.nf_max && g.njobs == key.njobs && g.cycles == key.cycles && g.forms == key.forms &&
                 g.total == key.total && std::memcmp(g.blocks, key.blocks, sizeof(key.blocks)) == 0 &&
                 g.jobs == key.jobs && g.pool == key.pool && g.ctrl == key.ctrl && g.sorted == key.sorted &&
                 g.lpt == key.lpt && std::memcmp(g.ids, key.ids, sizeof(key.ids)) == 0) {
@@ -1325,6 +1330,7 @@ static int batch_riaf_impl(const kp_riaf_job* jobs, int njobs, const kp_run_opti
         d.ray_begin = ray;
         d.npix = npix;
         d.precision = opt.precision;
+        d.lanes = opt.precision == KP_PRECISION_MIXED && lane_image(d.c, npix);
         ray += npix;
     }
     st = run_wave_jobs(dev, stream, njobs, total, family, nf_max, opt, stats);
@@ -1709,6 +1715,7 @@ int grmhd_image(const kp_pass_a_params* params, const kp_grid* const* grids, con
     d.ray_begin = 0;
     d.npix = npix;
     d.precision = opt.precision;
+    d.lanes = opt.precision == KP_PRECISION_MIXED && lane_image(d.c, npix);
     const bool mixed = opt.precision == KP_PRECISION_MIXED;
     if (mixed) grmhd_emission_scale(params, grid->model, d.c);
     if (nctl > 0) grmhd_apply_control(params, grid->model, d.c, ctl, nctl);

@@ -180,6 +180,7 @@ struct JobDesc {
     long long ray_begin;  // first global ray index of this job
     int npix;
     int precision;        // kp_precision of this job
+    int lanes;            // mixed policy: near phases with one ray per lane (lane_image)
 };
 
 // Resumable state of one ray between launches (lives in HBM, 464 bytes):
@@ -207,6 +208,8 @@ struct SeedEntry {
     long long ray_base;
 };
 
+enum Form : int { kFormQuads = 1, kFormLanes = 2 };
+
 // Device-side launch description (kernel parameter).
 struct WaveDesc {
     const JobDesc* jobs;           // device array, ordered by ray_begin
@@ -217,7 +220,9 @@ struct WaveDesc {
     const unsigned* in_ids;
     const unsigned* in_count;
     long long rays_max;            // rays there can be at most (host)
+    int forms;                     // mixed policy: kForm bits of the forms the rays' images take
     unsigned long long* in_head;   // pop counter, zero before the launch
+    unsigned long long* lane_head; // the lane kernel's, where both forms have rays
     // queue of the next launch of each phase (this phase's own entry takes
     // the rays parked by the iteration budget)
     unsigned* out_ids[kPhases];

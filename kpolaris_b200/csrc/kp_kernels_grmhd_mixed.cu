@@ -5,7 +5,7 @@
 // budget, not to the reference's rounding).
 #include <cuda_runtime.h>
 
-#include "kp_launch.h"
+#include "kp_lanes.cuh"
 #include "kp_quad.cuh"
 
 namespace kp {
@@ -14,31 +14,32 @@ __global__ void __launch_bounds__(kFarThreads, kFarBlocks) wave_far_grmhd_mixed(
     quad_body<PolicyMixed, kPhaseFar, SceneFarCks<SceneGrmhd>>(W);
 }
 
+template<bool SHARED>
 __global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_grmhd_mixed(const WaveDesc W) {
-    quad_body<PolicyMixed, kPhaseNearA, SceneGrmhd>(W);
+    quad_body<PolicyMixed, kPhaseNearA, SceneGrmhd, SHARED>(W);
 }
 
+template<bool SHARED>
 __global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_grmhd_mixed(const WaveDesc W) {
-    quad_body<PolicyMixed, kPhaseNearB, SceneGrmhd>(W);
+    quad_body<PolicyMixed, kPhaseNearB, SceneGrmhd, SHARED>(W);
 }
 
+template<bool SHARED>
 static const void* wave_kernel_grmhd_mixed(int phase) {
     if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_grmhd_mixed);
-    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_grmhd_mixed);
-    return reinterpret_cast<const void*>(wave_near_b_grmhd_mixed);
+    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_grmhd_mixed<SHARED>);
+    return reinterpret_cast<const void*>(wave_near_b_grmhd_mixed<SHARED>);
 }
 
 cudaError_t launch_wave_grmhd_mixed(int phase, const WaveDesc& W, int nf_max, int blocks, int threads,
                                     cudaStream_t stream) {
-    if (nf_max < 1 || nf_max > kMaxFreq || phase < 0 || phase >= kPhases) return cudaErrorInvalidValue;
-    const void* fn = wave_kernel_grmhd_mixed(phase);
-    void* args[] = {const_cast<WaveDesc*>(&W)};
-    return cudaLaunchKernel(fn, dim3(blocks), dim3(threads), args, 0, stream);
+    const void* const fn[2] = {wave_kernel_grmhd_mixed<false>(phase), wave_kernel_grmhd_mixed<true>(phase)};
+    return launch_forms<PolicyMixed, SceneGrmhd>(fn, phase, W, nf_max, blocks, threads, stream);
 }
 
 int wave_occupancy_grmhd_mixed(int phase, int nf_max, int threads) {
     if (phase < 0 || phase >= kPhases) return 0;
-    const void* fn = wave_kernel_grmhd_mixed(phase);
+    const void* fn = wave_kernel_grmhd_mixed<false>(phase);
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, 0);
     return n;

@@ -176,7 +176,8 @@ extern "C" int kp_batch_riaf_noalloc(const kp_riaf_job* jobs, int njobs, const k
             W.in_ids = S->ids[phase][cycle % 2];
             W.in_count = &S->ctrl.counts[cycle][phase];
             W.rays_max = total;
-            W.in_head = &S->ctrl.heads[cycle * kPhases + phase];
+            W.in_head = W.lane_head = &S->ctrl.heads[cycle * kPhases + phase];
+            W.forms = kFormQuads;
             for (int q = 0; q < kPhases; ++q) {
                 const int gen = q > phase ? cycle : cycle + 1;
                 W.out_ids[q] = S->ids[q][gen % 2];

@@ -253,6 +253,13 @@ __device__ __forceinline__ long long wave_rays(const WaveDesc& W) {
     return W.fresh_end - W.fresh_begin + (long long)(W.in_ids ? *W.in_count : 0u);
 }
 
+// Under the mixed policy quads and lanes round differently, so an image's form
+// depends on the image alone.  A launch with rays of both is run by both
+// kernels, each of which passes the other's rays over.
+__device__ __forceinline__ bool of_form(const WaveDesc& W, unsigned id, int lanes) {
+    return W.jobs[reinterpret_cast<const LaneState*>(W.pool[id].st)->job].lanes == lanes;
+}
+
 // How a phase takes its rays: kPhaseAll is the whole life of a ray in one
 // kernel, besides the wavefront's phases (a ray is never parked and needs no
 // record, queue or counter).
@@ -267,6 +274,7 @@ constexpr int kPhaseAll = kPhases;
 template<class P, int NF, int PHASE, class SC = SceneRiaf>
 __device__ __forceinline__ void lane_body(const WaveDesc& W) {
     constexpr bool kAll = PHASE == kPhaseAll;
+    constexpr bool kShared = P::kMixed && (PHASE == kPhaseNearA || PHASE == kPhaseNearB);  // may share a launch
     constexpr bool kPassA = PHASE != kPhaseNearB;   // pass-A steps run here
     constexpr bool kPassB = PHASE != kPhaseNearA;   // pass-B steps run here
     constexpr bool kCross = kAll || PHASE == kPhaseNearA;  // surface-crossing search
@@ -298,6 +306,7 @@ __device__ __forceinline__ void lane_body(const WaveDesc& W) {
     };
     const long long nfresh = W.fresh_end - W.fresh_begin;
     long long total_in = 0;
+    unsigned long long* const head = kShared ? W.lane_head : W.in_head;
     if constexpr (kAll) {
         const long long pixel = (long long)blockIdx.x * blockDim.x + threadIdx.x;
         if (pixel < nfresh) {
@@ -313,50 +322,58 @@ __device__ __forceinline__ void lane_body(const WaveDesc& W) {
         bool forward = false;
         if constexpr (!kAll) {
             // ------------------------------------------------------------ claim
-            const bool want = !exhausted && st.mode == kIdle;
-            const unsigned need = __ballot_sync(FULL, want);
-            if (need) {
-                unsigned long long base = 0;
-                const int leader = __ffs(need) - 1;
-                if (lane == leader) base = atomicAdd(W.in_head, (unsigned long long)__popc(need));
-                base = __shfl_sync(FULL, base, leader);
-                if (want) {
-                    const long long k = (long long)(base + __popc(need & ((1u << lane) - 1u)));
-                    if (k >= total_in) {
-                        exhausted = 1;
-                    } else if (k < nfresh) {
-                        // a fresh camera ray: locate its job and start pass A
-                        const long long id = W.fresh_begin + k;
-                        int lo = 0, hi = W.njobs - 1;
-                        while (lo < hi) {
-                            const int mid = (lo + hi + 1) >> 1;
-                            if (W.jobs[mid].ray_begin <= id) lo = mid; else hi = mid - 1;
+            bool foreign = false;
+#pragma unroll 1
+            do {
+                foreign = false;
+                const bool want = !exhausted && st.mode == kIdle && !forward;
+                const unsigned need = __ballot_sync(FULL, want);
+                if (need) {
+                    unsigned long long base = 0;
+                    const int leader = __ffs(need) - 1;
+                    if (lane == leader) base = atomicAdd(head, (unsigned long long)__popc(need));
+                    base = __shfl_sync(FULL, base, leader);
+                    if (want) {
+                        const long long k = (long long)(base + __popc(need & ((1u << lane) - 1u)));
+                        if (k >= total_in) {
+                            exhausted = 1;
+                        } else if (k < nfresh) {
+                            // a fresh camera ray: locate its job and start pass A
+                            const long long id = W.fresh_begin + k;
+                            int lo = 0, hi = W.njobs - 1;
+                            while (lo < hi) {
+                                const int mid = (lo + hi + 1) >> 1;
+                                if (W.jobs[mid].ray_begin <= id) lo = mid; else hi = mid - 1;
+                            }
+                            my_id = unsigned(id);
+                            J = &W.jobs[lo];
+                            start_ray<SC>(st, S, J, lo, int(id - J->ray_begin));
+                        } else if (kShared && W.forms == (kFormQuads | kFormLanes) &&
+                               !of_form(W, W.in_ids[k - nfresh], 1)) {
+                            foreign = true;
+                        } else if (W.budget > 0 && lane_jobs >= W.budget) {
+                            // past the budget: hand the id on untouched (below)
+                            my_id = W.in_ids[k - nfresh];
+                            forward = true;
+                        } else {
+                            // a parked ray: resume from its record
+                            my_id = W.in_ids[k - nfresh];
+                            const RayRecord& rec = W.pool[my_id];
+                            S = rec.S;
+                            memcpy(&st, rec.st, kLaneStateBytes<PHASE>);
+                            J = &W.jobs[st.job];
+                            if constexpr (kRad) memcpy(&stokes[0], rec.stokes, sizeof(stokes));
                         }
-                        my_id = unsigned(id);
-                        J = &W.jobs[lo];
-                        start_ray<SC>(st, S, J, lo, int(id - J->ray_begin));
-                    } else if (W.budget > 0 && lane_jobs >= W.budget) {
-                        // past the budget: hand the id on untouched (below)
-                        my_id = W.in_ids[k - nfresh];
-                        forward = true;
-                    } else {
-                        // a parked ray: resume from its record
-                        my_id = W.in_ids[k - nfresh];
-                        const RayRecord& rec = W.pool[my_id];
-                        S = rec.S;
-                        memcpy(&st, rec.st, kLaneStateBytes<PHASE>);
-                        J = &W.jobs[st.job];
-                        if constexpr (kRad) memcpy(&stokes[0], rec.stokes, sizeof(stokes));
                     }
                 }
-            }
+            } while (kShared && __any_sync(FULL, foreign));
             queue_push(W.out_ids[PHASE], W.out_count[PHASE], forward, my_id);
         }
         // Near-B hands the rays left when its input runs out to the quads of
         // its next launch: the longest rays, of which few are left then, take
         // a step in half to a quarter of a lane's time.
         bool hand_over = false;
-        if constexpr (PHASE == kPhaseNearB)
+        if constexpr (PHASE == kPhaseNearB && !P::kMixed)
             hand_over = (long long)*(const volatile unsigned long long*)W.in_head >= total_in;
         const bool active = st.mode != kIdle;
         // The block leaves the loop together, so the barrier below is
@@ -504,7 +521,7 @@ __device__ __forceinline__ void lane_body(const WaveDesc& W) {
             if (st.rk_kind != kRkRK4) {
                 const double tol = max_val(c.tolerance, kTolFloor);
                 if (err <= tol) {
-                    st.h_current = accepted_next_h(st.h_try, err, tol, st.ctl_min, st.ctl_max, st.req_h);
+                    st.h_current = accepted_next_h<P::kMixed && PHASE != kPhaseFar>(st.h_try, err, tol, st.ctl_min, st.ctl_max, st.req_h);
                 } else {
                     accepted = false;
                     if (rejected_attempt(st, err, tol)) {
@@ -628,7 +645,7 @@ __device__ __forceinline__ void lane_body(const WaveDesc& W) {
                 const double tol = max_val(c.tolerance, kTolFloor);
                 if (err <= tol) {
                     h = abs_val(st.h_try);
-                    if (!cam) st.h_current = abs_val(accepted_next_h(st.h_try, err, tol, st.ctl_min, st.ctl_max, st.req_h));
+                    if (!cam) st.h_current = abs_val(accepted_next_h<P::kMixed && PHASE != kPhaseFar>(st.h_try, err, tol, st.ctl_min, st.ctl_max, st.req_h));
                 } else {
                     proceed = false;
                     if (rejected_attempt(st, err, tol)) {

@@ -357,8 +357,9 @@ __device__ __forceinline__ void enter_chart(LS& st, const ImageConsts& c, Ray& S
 
 // A phase kernel of the wavefront engine on quads: persistent_body's control
 // machine, one ray per quad.  With kPhaseAll: the rays [fresh_begin,
-// fresh_end) of job 0, `per_warp` of them to each warp of the grid.
-template<class P, int PHASE, class SC = SceneRiaf>
+// fresh_end) of job 0, `per_warp` of them to each warp of the grid.  SHARED: the
+// launch has rays of lane images too, which a lane kernel takes.
+template<class P, int PHASE, class SC = SceneRiaf, bool SHARED = false>
 __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
     constexpr bool kAll = PHASE == kPhaseAll;
     constexpr bool kPassA = PHASE != kPhaseNearB;   // pass-A steps run here
@@ -411,56 +412,64 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
             // step, all in a bridged run or all in an ordinary step (79 -> 30 ms
             // per 8 x 256^2 step against refilling quad by quad).
             const bool busy = kMacro && __any_sync(kFullWarp, st.mode != kIdle);
-            const bool want = claims && !exhausted && st.mode == kIdle && !busy;
-            const unsigned need = __ballot_sync(kFullWarp, want && role == 0);
-            if (need) {
-                unsigned long long base = 0;
-                if (lane == 0) base = atomicAdd(W.in_head, (unsigned long long)__popc(need));
-                base = __shfl_sync(kFullWarp, base, 0);
-                if (want) {
-                    const long long k = (long long)(base + __popc(need & ((1u << (quad * 4)) - 1u)));
-                    if (k >= total_in) {
-                        exhausted = 1;
-                    } else if (k < nfresh) {
-                        // a fresh camera ray: locate its job and start pass A
-                        const long long id = W.fresh_begin + k;
-                        int lo = 0, hi = W.njobs - 1;
-                        while (lo < hi) {
-                            const int mid = (lo + hi + 1) >> 1;
-                            if (W.jobs[mid].ray_begin <= id) lo = mid; else hi = mid - 1;
-                        }
-                        my_id = unsigned(id);
-                        J = &W.jobs[lo];
-                        Ray S;
-                        start_ray<SC>(st, S, J, lo, int(id - J->ray_begin));
-                        enter_chart<SC>(st, J->c, S);
-                        V = role == 0 ? S.x : (role == 1 ? S.k : (role == 2 ? S.e1 : S.e2));
-                        r_top = SC::template top_radius<P::kMixed>(J->c, S.x);
-                    } else if (W.budget > 0 && quad_jobs >= W.budget) {
-                        // past the budget: hand the id on untouched (below)
-                        my_id = W.in_ids[k - nfresh];
-                        forward = true;
-                    } else {
-                        // a parked ray: resume from its record
-                        my_id = W.in_ids[k - nfresh];
-                        const RayRecord& rec = W.pool[my_id];
-                        memcpy(&st, rec.st, kLaneStateBytes<PHASE>);
-                        J = &W.jobs[st.job];
-                        if constexpr (SC::kFarChart) {
-                            Ray S = rec.S;
-                            const bool paused = st.chart;
+            bool foreign = false, pushing = false;
+#pragma unroll 1
+            do {
+                foreign = false;
+                const bool want = claims && !exhausted && st.mode == kIdle && !busy && !forward;
+                const unsigned need = __ballot_sync(kFullWarp, want && role == 0);
+                if (need) {
+                    unsigned long long base = 0;
+                    if (lane == 0) base = atomicAdd(W.in_head, (unsigned long long)__popc(need));
+                    base = __shfl_sync(kFullWarp, base, 0);
+                    if (want) {
+                        const long long k = (long long)(base + __popc(need & ((1u << (quad * 4)) - 1u)));
+                        if (k >= total_in) {
+                            exhausted = 1;
+                        } else if (k < nfresh) {
+                            // a fresh camera ray: locate its job and start pass A
+                            const long long id = W.fresh_begin + k;
+                            int lo = 0, hi = W.njobs - 1;
+                            while (lo < hi) {
+                                const int mid = (lo + hi + 1) >> 1;
+                                if (W.jobs[mid].ray_begin <= id) lo = mid; else hi = mid - 1;
+                            }
+                            my_id = unsigned(id);
+                            J = &W.jobs[lo];
+                            Ray S;
+                            start_ray<SC>(st, S, J, lo, int(id - J->ray_begin));
                             enter_chart<SC>(st, J->c, S);
                             V = role == 0 ? S.x : (role == 1 ? S.k : (role == 2 ? S.e1 : S.e2));
-                            r_top = paused ? st.start_r : SC::template top_radius<P::kMixed>(J->c, S.x);
+                            r_top = SC::template top_radius<P::kMixed>(J->c, S.x);
+                        } else if (SHARED && !of_form(W, W.in_ids[k - nfresh], 0)) {
+                            foreign = true;
+                        } else if (W.budget > 0 && quad_jobs >= W.budget) {
+                            // past the budget: hand the id on untouched (below)
+                            my_id = W.in_ids[k - nfresh];
+                            forward = true;
                         } else {
-                            V = reinterpret_cast<const D4*>(&rec.S)[role];
-                            r_top = SC::template top_radius<P::kMixed>(J->c, rec.S.x);
+                            // a parked ray: resume from its record
+                            my_id = W.in_ids[k - nfresh];
+                            const RayRecord& rec = W.pool[my_id];
+                            memcpy(&st, rec.st, kLaneStateBytes<PHASE>);
+                            J = &W.jobs[st.job];
+                            if constexpr (SC::kFarChart) {
+                                Ray S = rec.S;
+                                const bool paused = st.chart;
+                                enter_chart<SC>(st, J->c, S);
+                                V = role == 0 ? S.x : (role == 1 ? S.k : (role == 2 ? S.e1 : S.e2));
+                                r_top = paused ? st.start_r : SC::template top_radius<P::kMixed>(J->c, S.x);
+                            } else {
+                                V = reinterpret_cast<const D4*>(&rec.S)[role];
+                                r_top = SC::template top_radius<P::kMixed>(J->c, rec.S.x);
+                            }
+                            if constexpr (kRad) memcpy(&stokes, rec.stokes + 4 * role, sizeof(stokes));
                         }
-                        if constexpr (kRad) memcpy(&stokes, rec.stokes + 4 * role, sizeof(stokes));
                     }
                 }
-            }
-            if (need) queue_push(W.out_ids[PHASE], W.out_count[PHASE], forward && role == 0, my_id);
+                pushing = pushing || need;
+            } while (SHARED && __any_sync(kFullWarp, foreign));
+            if (pushing) queue_push(W.out_ids[PHASE], W.out_count[PHASE], forward && role == 0, my_id);
         }
         const bool active = st.mode != kIdle;
         // The block's warps leave the loop together: the barriers are reached by

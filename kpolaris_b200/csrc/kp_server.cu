@@ -108,7 +108,7 @@ struct kp_server {
     RayRecord* pool = nullptr;
     unsigned* ids[kServeScenes][kPhases][2] = {};
     unsigned* counts[kServeScenes] = {};           // per scene [2][kPhases]
-    unsigned long long* heads[kServeScenes] = {};  // per scene [kPhases]
+    unsigned long long* heads[kServeScenes] = {};  // per scene [2][kPhases]
     long long scene_cycle[kServeScenes] = {};      // generation parity of each scene's queues
     unsigned* sorted = nullptr;                    // near-B queue in longest-first order (max_rays)
     unsigned* lpt = nullptr;                       // its bucket counters (512)
@@ -187,7 +187,7 @@ int allocate_device(kp_server* s) {
         for (auto& q : s->ids[sc])
             for (auto& b : q) dev((void**)&b, sizeof(unsigned) * size_t(c.max_rays));
         dev((void**)&s->counts[sc], sizeof(unsigned) * 2 * kPhases);
-        dev((void**)&s->heads[sc], sizeof(unsigned long long) * kPhases);
+        dev((void**)&s->heads[sc], sizeof(unsigned long long) * 2 * kPhases);
     }
     dev((void**)&s->status, sizeof(int));
     dev((void**)&s->done, sizeof(unsigned) * size_t(c.max_jobs));
@@ -243,6 +243,7 @@ JobDesc job_desc(const kp_server* s, const ServerJob& j) {
     d.ray_begin = j.ray_base;
     d.npix = int(j.npix);
     d.precision = s->cfg.precision;
+    d.lanes = d.precision == KP_PRECISION_MIXED && lane_image(d.c, d.npix);
     return d;
 }
 
@@ -388,6 +389,12 @@ void worker_main(kp_server* s) {
                 e = cudaMemcpyAsync(s->d_prefix, s->h_prefix, sizeof(long long) * size_t(nseed + kServeScenes),
                                     cudaMemcpyHostToDevice, s->stream);
         }
+        int forms[kServeScenes] = {0, 0};  // of the images in flight
+        {
+            std::lock_guard<std::mutex> lock(s->mu);
+            for (const auto& j : s->slots)
+                if (j) forms[j->scene] |= s->h_jobs[j->slot].lanes ? kFormLanes : kFormQuads;
+        }
         // ---- one cycle of the three phases for each scene with jobs in flight;
         // each scene's queues alternate with its own tick count
         for (int sc = 0; sc < kServeScenes && e == cudaSuccess; ++sc) {
@@ -396,7 +403,7 @@ void worker_main(kp_server* s) {
             const int cur = int(cycle % 2), nxt = int((cycle + 1) % 2);
             unsigned* cnt = s->counts[sc];
             if (e == cudaSuccess) e = cudaMemsetAsync(cnt + nxt * kPhases, 0, sizeof(unsigned) * kPhases, s->stream);
-            if (e == cudaSuccess) e = cudaMemsetAsync(s->heads[sc], 0, sizeof(unsigned long long) * kPhases, s->stream);
+            if (e == cudaSuccess) e = cudaMemsetAsync(s->heads[sc], 0, sizeof(unsigned long long) * 2 * kPhases, s->stream);
             if (seed_count[sc] > 0 && e == cudaSuccess) {
                 const SeedEntry* ents = s->d_seed + seed_first[sc];
                 const long long* pre = s->d_prefix + seed_first[sc] + sc;
@@ -422,6 +429,8 @@ void worker_main(kp_server* s) {
                 W.in_count = cnt + cur * kPhases + p;
                 W.rays_max = inflight_rays;
                 W.in_head = s->heads[sc] + p;
+                W.lane_head = s->heads[sc] + kPhases + p;
+                W.forms = forms[sc];
                 for (int q = 0; q < kPhases; ++q) {
                     const int g = q > p ? cur : nxt;
                     W.out_ids[q] = s->ids[sc][q][g];

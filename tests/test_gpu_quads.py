@@ -15,6 +15,9 @@ and mixes at which four lanes per ray can go wrong.
 * The near phases and the one-launch kernel take lanes from a number of rays
   on: the smallest launches that do, of one image or several, one to four
   frequencies, every scene, are those of the quads, bit for bit.
+* The mixed policy chooses quads or lanes by the image: the smallest images on
+  lanes against the FP64 policy, and both kinds in one launch or one server,
+  each bit for bit the image traced alone.
 * The mixed policy's far field takes many steps at once and counts them: on
   rays that miss the sphere, cameras near, inside the far boundary and far
   out, and large and small step caps, its reasons are those of the FP64 policy
@@ -109,24 +112,35 @@ def test_near_phase_forms_agree(sizes, nf):
         assert_bitwise(a[k], b[k], k)
 
 
-@pytest.mark.parametrize("coordinates", ["fmks", "slow", "bl"])
-def test_near_phase_forms_agree_in_other_scenes(coordinates):
-    options = dict(precision=_abi.PRECISION_FP64, schedule=_abi.SCHEDULE_PERSISTENT)
-    if coordinates == "bl":
-        p, m, f = job(280, 271, 1)
-        p.coordinate_system = _abi.COORD_BOYER_LINDQUIST
-        a, b = forms(lambda **o: kp.image_riaf(p, m, f, **o), **options)
-    else:
-        grids = []
-        for t in (0.0, 60.0):
-            prims, model = synthetic.fm_torus(96, 48, 48, time=t)
-            grids.append(kp.Grid(model, prims))
-        p = synthetic.fmks_pass_a_params(model, 280, 271)
-        if coordinates == "fmks":
-            a, b = forms(lambda **o: kp.image_grmhd(p, grids[0], [230e9, 345e9], **o), **options)
-        else:
-            a, b = forms(lambda **o: kp.image_grmhd_slow_light(p, grids, [0.0, 60.0], 1040.0, [230e9], **o), **options)
-    assert_bitwise(a, b, coordinates)
+@pytest.fixture(scope="module")
+def tori():
+    grids = []
+    for t in (0.0, 400.0):
+        prims, model = synthetic.fm_torus(96, 48, 48, time=t)
+        grids.append(kp.Grid(model, prims))
+    yield grids
+    for g in grids:
+        g.release()
+
+
+def scene_call(scene, nx, ny, tori):
+    """The parameters of an image of a scene, and the call that traces it."""
+    wave = dict(schedule=_abi.SCHEDULE_PERSISTENT)
+    if scene in ("cks", "bl"):
+        p, m, f = job(nx, ny, 1)
+        if scene == "bl":
+            p.coordinate_system = _abi.COORD_BOYER_LINDQUIST
+        return p, lambda **o: kp.image_riaf(p, m, f, **wave, **o)
+    p = synthetic.fmks_pass_a_params(tori[0].model, nx, ny)
+    if scene == "fmks":
+        return p, lambda **o: kp.image_grmhd(p, tori[0], [230e9], **wave, **o)
+    return p, lambda **o: kp.image_grmhd_slow_light(p, tori, [0.0, 400.0], 1213.0, [230e9], **wave, **o)
+
+
+@pytest.mark.parametrize("scene", ["fmks", "slow", "bl"])
+def test_near_phase_forms_agree_in_other_scenes(scene, tori):
+    call = scene_call(scene, 280, 271, tori)[1]
+    assert_bitwise(*forms(lambda **o: call(precision=_abi.PRECISION_FP64, **o)), scene)
 
 
 # One pixel above the line of the one-launch kernel (9,472 pixels of fixed
@@ -136,3 +150,60 @@ def test_near_phase_forms_agree_in_other_scenes(coordinates):
 def test_plain_kernel_forms_agree(nx, ny, nf, adaptive):
     p, m, f = job(nx, ny, nf, adaptive=adaptive)
     assert_bitwise(kp.image_riaf(p, m, f), kp.image_riaf(p, m, f, schedule=_abi.SCHEDULE_PERSISTENT), (nx, ny))
+
+
+# The smallest images of one frequency that the mixed policy traces with one
+# ray per lane (above 120,000 pixels, 80,000 in Boyer-Lindquist), against the
+# FP64 policy.  A rounding moves the substeps or the end of a few rays -- some
+# tens of these, on quads or lanes alike -- so reasons are held to the bar of
+# the small images (99%, tests/test_gpu_grmhd.py), all but one pixel in a
+# thousand to 1e-4 of the brightest, and the sums over those to the policy's
+# flux and EVPA budget.
+@pytest.mark.parametrize("scene,nx,ny", [("cks", 347, 346), ("bl", 283, 283), ("fmks", 347, 346), ("slow", 347, 346)])
+def test_mixed_lane_images_within_budget(scene, nx, ny, tori):
+    p, call = scene_call(scene, nx, ny, tori)
+    mixed, fp64 = (call(precision=x) for x in (_abi.PRECISION_MIXED, _abi.PRECISION_FP64))
+    assert np.mean(mixed.reason == fp64.reason) >= 0.99
+    peak = np.nanmax(fp64.arrays["image_i"])
+    assert peak > 0.0
+    on = np.abs(mixed.arrays["image_i"] - fp64.arrays["image_i"]) <= 1e-4 * peak
+    assert np.mean(on) >= 0.999, int((~on).sum())
+    i, q, u = ([r.arrays[k][on].sum() for r in (mixed, fp64)] for k in ("image_i", "image_q", "image_u"))
+    assert abs(i[0] / i[1] - 1.0) <= 1e-4, i
+    d = 0.5 * np.degrees(np.arctan2(u[0], q[0]) - np.arctan2(u[1], q[1]))
+    assert abs((d + 90.0) % 180.0 - 90.0) <= 0.1, d
+
+
+# Images on either side of that line in one launch: each kernel passes the
+# other's rays over, and every image is the one traced alone.
+@pytest.mark.parametrize("coordinates", ["cks", "bl"])
+@pytest.mark.parametrize("schedule", [_abi.SCHEDULE_PERSISTENT, _abi.SCHEDULE_GRAPH])
+def test_mixed_forms_share_a_launch(coordinates, schedule):
+    sizes = [(31, 7, 3), (347, 346, 1), (200, 90, 2), (1, 1, 1), (320, 377, 1), (97, 61, 4)]
+    jobs = [job(nx, ny, nf, inclination=20.0 + 11.0 * k, spin=0.15 * k) for k, (nx, ny, nf) in enumerate(sizes)]
+    for p, _, _ in jobs:
+        if coordinates == "bl":
+            p.coordinate_system = _abi.COORD_BOYER_LINDQUIST
+    outs = kp.batch_riaf(jobs, precision=_abi.PRECISION_MIXED, schedule=schedule)
+    for k, (p, m, f) in enumerate(jobs):
+        alone = kp.image_riaf(p, m, f, precision=_abi.PRECISION_MIXED, schedule=_abi.SCHEDULE_PERSISTENT)
+        assert_bitwise(outs[k], alone, k)
+
+
+# In a server's ticks, of a few RK jobs each, too.
+@pytest.mark.parametrize("budget", [64, 0])
+def test_mixed_forms_share_a_server(tori, budget):
+    cfg = kp.default_server_config()
+    if budget:
+        cfg.tick_budget = budget
+    images = [scene_call("fmks", nx, ny, tori)[0] for nx, ny in ((23, 19), (347, 346), (40, 64))]
+    riaf = [job(347, 346, 1), job(50, 40, 2)]
+    with kp.Server(cfg) as srv:
+        tickets = [srv.submit_grmhd(p, tori[0], [230e9]) for p in images] + [srv.submit(*j) for j in riaf]
+        for t in tickets:
+            srv.wait(t, timeout=300.0)
+        got = [srv.result(t) for t in tickets]
+    for k, p in enumerate(images):
+        assert_bitwise(got[k], kp.image_grmhd(p, tori[0], [230e9], precision=_abi.PRECISION_MIXED), k)
+    for k, (p, m, f) in enumerate(riaf):
+        assert_bitwise(got[len(images) + k], kp.image_riaf(p, m, f, precision=_abi.PRECISION_MIXED), k)

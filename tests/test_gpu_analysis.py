@@ -24,6 +24,8 @@ from kpolaris_b200 import _abi, configs
 
 INT_FIELDS = ("reason", "steps", "pass_a_steps")
 
+needs_reference = pytest.mark.skipif(not oracle.ref_available(), reason="reference oracle not built")
+
 
 def _maxdiff(a, b):
     d = np.abs(np.asarray(a, dtype=np.float64) - np.asarray(b, dtype=np.float64))
@@ -58,6 +60,7 @@ def _compare(got, ref, got_an, ref_an, cond):
         assert _maxdiff(g, v) <= bar, (k, _maxdiff(g, v), bar, scale)
 
 
+@needs_reference
 @pytest.mark.gpu
 @pytest.mark.parametrize("controls", ["config2", "config1"])
 def test_analysis_matches_reference(controls):
@@ -94,6 +97,7 @@ RESPONSE_CASES = [("density_scale", "radial"), ("none", "region"), ("coefficient
                   ("temperature_scale", "thetae"), ("magnetic_scale", "plasma_region"), ("none", "ne_cgs")]
 
 
+@needs_reference
 @pytest.mark.gpu
 @pytest.mark.parametrize("response,partition", RESPONSE_CASES)
 def test_analysis_response_channels_match_reference(response, partition):

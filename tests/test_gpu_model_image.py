@@ -109,17 +109,19 @@ def test_tool_csv_equals_library(tmp_path):
             assert np.array_equal(rows[:, col["total_steps"]], pk["total_steps"])
             assert fluxes[fi] == pk["flux_jy"][0] or (np.isnan(fluxes[fi]) and np.isnan(pk["flux_jy"][0]))
             fi += 1
-    # one geodesic per pixel: every chunk's steps and reasons equal, and
-    # equal to the reference's control variant (adaptive: within +-2 steps)
-    ref = oracle.image_riaf_control(params, configs.riaf_model(freq=FREQS[0]), FREQS[:4], FREQS, threads=0)
+    # one geodesic per pixel: every chunk's steps and reasons equal, and,
+    # where the reference oracle is built, equal to the reference's control
+    # variant (adaptive: within +-2 steps)
     first = data[data[:, col["freq_index"]] == 0]
     for fi in range(len(FREQS)):
         rows = data[data[:, col["freq_index"]] == fi]
         for c in ("reason", "pass_a_steps", "pass_b_steps"):
             assert np.array_equal(rows[:, col[c]], first[:, col[c]]), (fi, c)
-    assert np.array_equal(first[:, col["reason"]], ref.reason)
-    assert np.abs(first[:, col["pass_a_steps"]] - ref.pass_a_steps).max() <= 2
-    assert np.abs(first[:, col["pass_b_steps"]] - ref.steps).max() <= 2
+    if oracle.ref_available():
+        ref = oracle.image_riaf_control(params, configs.riaf_model(freq=FREQS[0]), FREQS[:4], FREQS, threads=0)
+        assert np.array_equal(first[:, col["reason"]], ref.reason)
+        assert np.abs(first[:, col["pass_a_steps"]] - ref.pass_a_steps).max() <= 2
+        assert np.abs(first[:, col["pass_b_steps"]] - ref.steps).max() <= 2
     params_file = Path(str(out) + ".params")
     assert params_file.exists() and "derived_freq_list=86000000000,230000000000" in params_file.read_text()
 

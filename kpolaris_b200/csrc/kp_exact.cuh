@@ -52,14 +52,14 @@ struct ExactRecip {
 __device__ __forceinline__ ExactRecip exact_recip(double b) {
     double y = recip_start(b);
     double e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, __fma_rn(e, e, e), y);
+    // Rounded up: from the number above its reciprocal the last step finds that
+    // of b = 2^n (2 - 2^-52) too, 2^-(n + 1) (1 + 2^-52).  From below, at
+    // 2^-(n + 1), it lands halfway between the two and stays.  (Elsewhere the
+    // step is off by e e / b, and a reciprocal within that of a halfway point,
+    // which is 2^-106 / b from the nearest, is half an ulp from the number above.)
+    y = __fma_ru(y, __fma_rn(e, e, e), y);
     e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, e, y);
-    // For b = 2^n (2 - 2^-52) that ends at 2^-(n + 1), and the reciprocal is
-    // the next number, 2^-(n + 1) (1 + 2^-52): its last bit is set.
-    const unsigned hi = unsigned(__double2hiint(b)) | 0xfff00000u, lo = unsigned(__double2loint(b));
-    const int last = (hi & lo) == 0xffffffffu ? 1 : 0;
-    return ExactRecip{b, __hiloint2double(__double2hiint(y), __double2loint(y) | last)};
+    return ExactRecip{b, __fma_rn(y, e, y)};
 }
 
 // RN(a / b) for a zero or 1e-200 < |a| < 1e150 with 1e-250 < |a / b| < 1e150.
@@ -73,16 +73,14 @@ __device__ __forceinline__ double exact_quot(double a, const ExactRecip& r) {
 __device__ __forceinline__ double exact_sqrt(double v) {
     double y = rsqrt_start(v);
     const double e = __fma_rn(-__dmul_rn(v, y), y, 1.0);
-    y = __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
-    const double h = __dmul_rn(0.5, y);
-    double g = __dmul_rn(v, y);
+    const double ye = __dmul_rn(y, e), c = __fma_rn(0.375, e, 0.5);
+    const double h = __dmul_rn(0.5, __fma_rn(ye, c, y));
+    // Rounded down: the root of v = 4^n (1 - 2^-53) lies a hair under the middle
+    // between 2^n and the number below it.  The steps reach that number from
+    // below; from 2^n they would stay there.
+    double g = __dmul_rd(v, __fma_rd(ye, c, y));
     g = __fma_rn(__fma_rn(-g, g, v), h, g);
-    g = __fma_rn(__fma_rn(-g, g, v), h, g);
-    // For v = 4^n (1 - 2^-53), a hair under the middle between 2^n and the
-    // number below it, that can end at 2^n, and the root is the number below.
-    const unsigned hi = unsigned(__double2hiint(v)) | 0xfff00000u, lo = unsigned(__double2loint(v));
-    const int above = (hi & lo) == 0xffffffffu && __double2loint(g) == 0 ? 1 : 0;
-    return __longlong_as_double(__double_as_longlong(g) - above);
+    return __fma_rn(__fma_rn(-g, g, v), h, g);
 }
 
 // A numerator's factor for which products of a few of its like stay clear of

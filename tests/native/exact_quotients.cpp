@@ -5,6 +5,7 @@
 // the accuracy is known, are the correct values off by up to `err` relative
 // (argument 2), at random.  argv: draws, err.  Prints the mismatches of each
 // kind (xq::Counts).
+#include <cfenv>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -23,6 +24,16 @@ inline double off() {
     return 1.0 + start_err * (double(start_state >> 11) * 0x1p-52 - 1.0);
 }
 inline double __fma_rn(double a, double b, double c) { return std::fma(a, b, c); }
+inline double rounded(int mode, double a, double b, double c) {
+    volatile double x = a, y = b, z = c;
+    std::fesetround(mode);
+    volatile double r = std::fma(x, y, z);
+    std::fesetround(FE_TONEAREST);
+    return r;
+}
+inline double __fma_ru(double a, double b, double c) { return rounded(FE_UPWARD, a, b, c); }
+inline double __fma_rd(double a, double b, double c) { return rounded(FE_DOWNWARD, a, b, c); }
+inline double __dmul_rd(double a, double b) { return rounded(FE_DOWNWARD, a, b, 0.0); }
 inline double __dmul_rn(double a, double b) { return a * b; }
 inline long long __double_as_longlong(double v) {
     long long u;

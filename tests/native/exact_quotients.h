@@ -35,9 +35,17 @@ XQ_FN uint64_t next(uint64_t& s) {
 }
 
 // Significands: random, all ones, within 256 of all ones, a power of two, few
-// leading bits, few trailing bits.
+// leading bits, few trailing bits, and those of reciprocals and roots closest
+// to halfway between two numbers: B with B M = 2^106 - 1, - 2 or - 4 for an M
+// of 54 bits, V with M M = 2^54 V + 1, 9, -7, -15, 17 or 25.
 XQ_FN uint64_t significand(uint64_t& s) {
     const uint64_t full = (uint64_t(1) << 52) - 1, m = next(s) & full;
+    const uint64_t close[20] = {0x1e756f08df1792, 0x1e20adbc4078a2, 0x1ef7930608393e, 0x1de441d5331432, 0x1da210daeb138e,
+                                0x1bea3278b789d2, 0x1ffb8a8b628dbc, 0x1fe24bffeb8794, 0x1c928b5b9dc714, 0x15555555555554,
+                                0x10000000000001, 0x10000000000003, 0x10000000000005, 0x1fffffffffffff, 0x1ffffffffffffd,
+                                0x1ffffffffffffb, 0x1d407bb3641da5, 0x15b95344972fe2, 0x12b035c1197f48,
+                                0x1256565cadcbf4};
+    if ((next(s) & 7) == 0) return close[next(s) % 20] & full;
     switch (next(s) >> 61) {
     case 0: return full;
     case 1: return full - (m & 255);

@@ -8,8 +8,7 @@ and just beyond them, and significands of all ones, nearly so, and powers of
 two.
 
 * CPU: tests/native/exact_quotients.cpp, the method with C's fma and
-  approximate starting values of 20 bits, good and at the hardware's stated
-  accuracy.
+  starting values of 20 bits, exact but for them and off by twice as much.
 * GPU: tests/native/exact_quotients.cu, against CUDA's own operators."""
 from __future__ import annotations
 
@@ -25,7 +24,7 @@ NATIVE = ROOT / "tests" / "native"
 CSRC = ROOT / "kpolaris_b200" / "csrc"
 
 
-@pytest.mark.parametrize("err", [0.0, 1e-6])
+@pytest.mark.parametrize("err", [0.0, 2e-6])
 def test_host_emulation(tmp_path, err):
     exe = tmp_path / "exact_quotients"
     subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", f"-I{CSRC}", f"-I{ROOT / 'include'}", f"-I{NATIVE}",

@@ -230,20 +230,9 @@ __device__ __forceinline__ D4 quad_macro_step(const ImageConsts& c, const D4& S,
             z0 = z1;
             d4_axpy(z1, z2, 2.0 * hs, f);
         }
-        // Neville's scheme in the step squared: column k of this row from
-        // column k - 1 and the row before, q = 1 / ((n_j / n_(j-k))^2 - 1)
-        const double q[3] = {j == 1 ? 1.0 / 3.0 : (j == 2 ? 0.8 : 9.0 / 7.0), j == 2 ? 0.125 : 1.0 / 3.0, 1.0 / 15.0};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            double v = 0.5 * (z1.v[i] + (z0.v[i] + hs * f.v[i]));
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const double w = v + (v - C[k].v[i]) * q[k];
-                if (k <= j) C[k].v[i] = v;
-                if (k < j) v = w;
-            }
-            t.v[i] = v;
-        }
+        for (int i = 0; i < 4; ++i)
+            t.v[i] = macro_row(j, 0.5 * (z1.v[i] + (z0.v[i] + hs * f.v[i])), C[0].v[i], C[1].v[i], C[2].v[i]);
     }
     return t;
 }

@@ -10,7 +10,9 @@
 //   the largest distance (over max(1, |.|)) between the extrapolated midpoint
 //   rule over a run and the steps themselves,
 //   how many steps certain_step promised, and the largest error of one of
-//   them over the error it was promised to stay under.
+//   them over the error it was promised to stay under,
+//   the largest distance between a run bridged at once and in eight parts,
+//   and the largest such error of random vectors.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -49,10 +51,14 @@ static double distance(const Ray& a, const Ray& b) {
     return d;
 }
 
-// Gragg's midpoint rule with 2, 4, 6, 8 substeps, extrapolated.
+// Gragg's midpoint rule with 2, 4, 6, 8 substeps, extrapolated by the
+// library's macro_row.
 static Ray midpoint(double M, double a, const Ray& s, double H) {
     const Ray f0 = ks_rhs(M, a, s);
-    Ray T[4], P[4];
+    Ray t, C[3];
+    double* const v = reinterpret_cast<double*>(&t);
+    double* const c[3] = {reinterpret_cast<double*>(&C[0]), reinterpret_cast<double*>(&C[1]),
+                          reinterpret_cast<double*>(&C[2])};
     for (int j = 0; j < 4; ++j) {
         const int n = 2 * j + 2;
         const double h = H / n;
@@ -62,25 +68,18 @@ static Ray midpoint(double M, double a, const Ray& s, double H) {
             z0 = z1;
             z1 = z2;
         }
-        Ray t = axpy(axpy(axpy(z1, h, ks_rhs(M, a, z1)), 1.0, z0), 0.0, z0);
-        double* v = reinterpret_cast<double*>(&t);
-        for (int i = 0; i < 16; ++i) v[i] *= 0.5;
-        T[0] = t;
-        for (int k = 1; k <= j; ++k) {
-            const double q = double(n) / (2.0 * (j - k) + 2.0);
-            T[k] = axpy(axpy(T[k - 1], 1.0 / (q * q - 1.0), T[k - 1]), -1.0 / (q * q - 1.0), P[k - 1]);
-        }
-        for (int k = 0; k <= j; ++k) P[k] = T[k];
+        t = axpy(axpy(z1, h, ks_rhs(M, a, z1)), 1.0, z0);
+        for (int i = 0; i < 16; ++i) v[i] = macro_row(j, 0.5 * v[i], c[0][i], c[1][i], c[2][i]);
     }
-    return P[3];
+    return t;
 }
 
 int main() {
     std::mt19937_64 rng(20260101);
     std::uniform_real_distribution<double> u(0.0, 1.0);
-    double worst_const = 0.0, worst_dist = 0.0;
+    double worst_const = 0.0, worst_dist = 0.0, worst_rule = 0.0;
     int runs = 0, wrong = 0;
-    for (int ray = 0; ray < 400; ++ray) {
+    for (int ray = 0; ray < 600; ++ray) {
         ImageConsts c;
         std::memset(&c, 0, sizeof(c));
         c.mass = 1.0;
@@ -90,11 +89,15 @@ int main() {
         c.step = ray % 4 == 3 ? 1.0 : 0.025;
         c.tolerance = ray % 4 == 2 ? 1e-6 : 1e-8;
         c.outer_radius = 50.0 + 65.0 * u(rng);
+        if (ray >= 400) {  // small spheres, short steps, near cameras
+            c.max_step = 0.025 + 0.475 * u(rng);
+            c.outer_radius = 4.0 + 46.0 * u(rng);
+        }
         c.fp32_radius = c.outer_radius + 2.0 * std::fmax(c.max_step, c.step);
-        c.cam_radius = 200.0 + 1800.0 * u(rng);
+        c.cam_radius = ray < 400 ? 200.0 + 1800.0 * u(rng) : 60.0 + 300.0 * u(rng);
         // a ray through the camera's radius at some impact parameter, its
         // wavevector null in the Kerr-Schild metric to first order
-        const double r = c.cam_radius, b = 400.0 * (u(rng) - 0.5), th = std::acos(2.0 * u(rng) - 1.0), ph = 6.28 * u(rng);
+        const double r = c.cam_radius, b = (ray < 400 ? 400.0 : 0.8 * c.cam_radius) * (u(rng) - 0.5), th = std::acos(2.0 * u(rng) - 1.0), ph = 6.28 * u(rng);
         const double n[3] = {std::sin(th) * std::cos(ph), std::sin(th) * std::sin(ph), std::cos(th)};
         double e[3] = {n[1], -n[0], 0.0};
         const double en = std::sqrt(e[0] * e[0] + e[1] * e[1]) + 1e-300;
@@ -132,6 +135,9 @@ int main() {
                 if (run.count < 3) break;
                 ++runs;
                 const Ray far = midpoint(c.mass, c.spin, s, dir * run.length);
+                Ray parts = s;
+                for (int k = 0; k < 8; ++k) parts = midpoint(c.mass, c.spin, parts, 0.125 * dir * run.length);
+                worst_rule = std::fmax(worst_rule, distance(far, parts));
                 double len = 0.0, hh = h, old = r0;
                 bool ok = true;
                 for (int k = 0; k < run.count; ++k) {
@@ -172,7 +178,7 @@ int main() {
         ImageConsts c;
         std::memset(&c, 0, sizeof(c));
         c.mass = 1.0;
-        c.spin = 0.99 * u(rng);
+        c.spin = 0.998 * u(rng);
         c.nx = c.ny = 64;
         c.cam_radius = u(rng) < 0.5 ? 1000.0 : 50.0 + 1000.0 * u(rng);
         const double inc = 0.1 + 2.9 * u(rng);
@@ -195,8 +201,8 @@ int main() {
                 w = std::fmax(w, std::fmax(std::fabs(s.e1.v[i]), std::fabs(s.e2.v[i])));
             }
             w = std::fmax(km, w);
-            for (const double h : {4.0, 2.0, 0.7, 0.2, 0.03}) {
-                for (const double lim : {2.5e-9, 1e-8 / 64.0, 1e-6 / 64.0}) {
+            for (const double h : {8.0, 4.0, 2.0, 0.7, 0.2, 0.03}) {
+                for (const double lim : {2.5e-9, 2.5e-11, 1e-8 / 64.0, 1e-6 / 64.0}) {
                     if (!certain_step(c.mass, r, km, w, h, lim)) continue;
                     ++certain;
                     const Ray half = rk4(c.mass, c.spin, s, 0.5 * dir * h);
@@ -208,6 +214,45 @@ int main() {
             if (!(std::fabs(s.x.v[1]) < 1e9)) break;
         }
     }
-    std::printf("%.3f %d %d %.3e %ld %.3f\n", worst_const, runs, wrong, worst_dist, certain, worst_certain);
+    // and of random vectors: k on the null cone with its spatial part up to half
+    // as long again, of any size and direction, e1 and e2 of any
+    double worst_random = 0.0;
+    for (int i = 0; i < 30000; ++i) {
+        const double spin = 0.998 * u(rng), r = 2.2 * std::pow(700.0, u(rng)), size = std::pow(3.0, 2.0 * u(rng) - 1.0);
+        Ray s;
+        double n[3], d[3];
+        for (double* v : {n, d}) {
+            const double th = std::acos(2.0 * u(rng) - 1.0), ph = 6.283185307 * u(rng);
+            v[0] = std::sin(th) * std::cos(ph);
+            v[1] = std::sin(th) * std::sin(ph);
+            v[2] = std::cos(th);
+        }
+        s.x.v[0] = 0.0;
+        for (int k = 0; k < 3; ++k) s.x.v[k + 1] = std::sqrt(r * r + spin * spin) * n[k];
+        const KSMetricPoint g = ks_point(1.0, spin, s.x);
+        const double ld = g.l[1] * d[0] + g.l[2] * d[1] + g.l[3] * d[2];
+        const double qa = g.amp - 1.0, qb = 2.0 * g.amp * ld, qc = 1.0 + g.amp * ld * ld, disc = qb * qb - 4.0 * qa * qc;
+        if (!(disc > 0.0) || !(qa < 0.0)) continue;
+        s.k.v[0] = size * std::fmax((-qb - std::sqrt(disc)) / (2.0 * qa), (-qb + std::sqrt(disc)) / (2.0 * qa));
+        const double off = size * (0.8 + 0.7 * u(rng));
+        double km = std::fabs(s.k.v[0]), w = 0.0;
+        for (int k = 0; k < 3; ++k) km = std::fmax(km, std::fabs(s.k.v[k + 1] = off * d[k]));
+        for (int k = 0; k < 4; ++k) {
+            s.e1.v[k] = 2.0 * u(rng) - 1.0;
+            s.e2.v[k] = 2.0 * u(rng) - 1.0;
+            w = std::fmax(w, std::fmax(std::fabs(s.e1.v[k]), std::fabs(s.e2.v[k])));
+        }
+        w = std::fmax(km, w);
+        const double rb = ks_radius(spin, s.x);
+        for (const double h : {16.0, 8.0, 4.0, 2.0, 0.7, 0.2, 0.03}) {
+            for (const double lim : {2.5e-9, 2.5e-11, 1e-8 / 64.0, 1e-6 / 64.0, 2.5e-7}) {
+                if (!certain_step(1.0, rb, km, w, h, lim)) continue;
+                const Ray half = rk4(1.0, spin, s, 0.5 * h);
+                worst_random = std::fmax(worst_random, distance(rk4(1.0, spin, s, h), rk4(1.0, spin, half, 0.5 * h)) / lim);
+            }
+        }
+    }
+    std::printf("%.3f %d %d %.3e %ld %.3f %.3e %.3f\n", worst_const, runs, wrong, worst_dist, certain, worst_certain,
+                worst_rule, worst_random);
     return 0;
 }

@@ -99,9 +99,9 @@ typedef enum kp_precision {
 
 /* How rays are scheduled on the device. */
 typedef enum kp_schedule {
-    /* Four lanes per pixel, one launch per image: the plain form. */
+    /* One launch per image, four lanes or one per pixel: the plain form. */
     KP_SCHEDULE_PER_PIXEL = 0,
-    /* Persistent kernel draining a global ray queue with per-lane refill. */
+    /* Persistent kernels draining a global ray queue, refilled ray by ray. */
     KP_SCHEDULE_PERSISTENT = 1,
     /* The persistent engine with its launch loop captured in a CUDA graph:
      * a fixed number of (far, near-A, near-B) cycles, the counter reset and
@@ -238,7 +238,7 @@ typedef struct kp_run_options {
     int timing;          /* 1: print "timing <name> <seconds> s" lines like the reference */
     /* Persistent-schedule tunables.  blocks_per_sm: 0 selects the
      * occupancy-derived CTA count.  threads_per_block must be 0: the kernels
-     * fix it (128 far, 256 near). */
+     * fix it (128 far and near-A, 256 near-B). */
     int blocks_per_sm;
     int threads_per_block;
 } kp_run_options;

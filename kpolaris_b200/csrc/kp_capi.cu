@@ -423,7 +423,7 @@ ImageConsts make_consts(const kp_pass_a_params* p, const kp_riaf_model* m, const
     // Boundary of the far phase: two of the longest steps either pass can
     // take (adaptive steps are clamped to max_step, fixed steps are `step`)
     // beyond the radiating sphere, so no far-phase step reaches the sphere.
-    c.fp32_radius = p->outer_radius + 2.0 * std::max(std::fabs(p->max_step), std::fabs(p->step));
+    c.far_radius = p->outer_radius + 2.0 * std::max(std::fabs(p->max_step), std::fabs(p->step));
     c.fit = m->emission_type == KP_FIT_DEXTER ? 4 : 1;
     c.nfreq = nfreq;
     const double length_unit = riaf_length_unit(m);
@@ -612,8 +612,8 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         if (e != cudaSuccess) return cuda_error(e, "cudaMemsetAsync(wave counters)");
     }
     if (opt.threads_per_block != 0)
-        return set_error(KP_ERR_INVALID, "threads_per_block is fixed by the wavefront kernels (%d far, %d near): pass 0",
-                         kFarThreads, kNearBThreads);
+        return set_error(KP_ERR_INVALID, "threads_per_block is fixed by the wavefront kernels (%d far, %d near-A, %d near-B): pass 0",
+                         kFarThreads, kNearAThreads, kNearBThreads);
     const bool mixed = family == kFamilyRiafMixed;
     int blocks[kPhases];
     for (int phase = 0; phase < kPhases; ++phase) {

@@ -1,7 +1,6 @@
 // kp_common.cuh -- shared device types and per-image launch constants for the
-// B200 GRRT kernels.  Geometry types are FP64; radiation types are templated
-// on the transfer precision R (double for the FP64 path, float for the mixed
-// path).
+// B200 GRRT kernels.  All arithmetic is FP64; the FP64 policy keeps the
+// reference's operation order, the mixed policy uses factored, fused forms.
 #pragma once
 
 #include <cstdint>
@@ -115,7 +114,7 @@ struct ImageConsts {
     double isco;         // isco_radius(spin), riaf.hpp:166-174
     // boundary of the far phase (bridged runs of steps under the mixed policy):
     // outside the radiating sphere by two of the longest steps
-    double fp32_radius;
+    double far_radius;
     int fit;             // 1 Pandya, 4 Dexter
     // frequencies sharing one geodesic
     int nfreq;
@@ -194,7 +193,7 @@ struct alignas(16) RayRecord {
 };
 
 // Phases of the wavefront engine (one kernel each).  Far: rays whose loop
-// tops lie beyond ImageConsts::fp32_radius (camera to radiating sphere and
+// tops lie beyond ImageConsts::far_radius (camera to radiating sphere and
 // back: pure transport).  Near-A: pass A inside (surface-crossing search).
 // Near-B: pass B inside (radiative transfer).  Rays migrate between the
 // phases through id queues.

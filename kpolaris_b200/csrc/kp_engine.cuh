@@ -22,8 +22,8 @@
 #include "kp_integrate.cuh"
 #include "kp_radiation.cuh"
 #include "kp_trace_fp64.cuh"
-#include "kp_geometry_f32.cuh"
-#include "kp_radiation_f32.cuh"
+#include "kp_geometry_mixed.cuh"
+#include "kp_radiation_mixed.cuh"
 #include "kp_scene.cuh"
 
 namespace kp {
@@ -56,7 +56,7 @@ struct PolicyMixed {
 
 // Radiation side of a policy and scene: FP64 (the reference's arithmetic) or
 // the factored form with the per-frequency 2^E emission scale
-// (kp_radiation_f32.cuh).
+// (kp_radiation_mixed.cuh).
 template<class P, class S = SceneRiaf>
 struct RadTraits;
 
@@ -93,27 +93,27 @@ __device__ __forceinline__ double norm_refined(double x, double y, double z) {
     const double n2 = x * x + y * y + z * z;
     if (!(n2 > 1e-280 && n2 < 1e280)) return sqrt(n2);
     double n, inv;
-    kp_sqrt_pair<double>(n2, n, inv);
+    kp_sqrt_pair(n2, n, inv);
     return n;
 }
 
 template<>
 struct RadTraits<PolicyMixed, SceneRiaf> {
     using Stokes = StokesM;
-    using Co = CoeffsF;
-    using Sample = RiafSampleF;
+    using Co = CoeffsM;
+    using Sample = RiafSampleM;
     __device__ static void zero(Stokes& s) { s = StokesM{0.0, 0.0, 0.0, 0.0}; }
-    __device__ static Sample sample(const ImageConsts& c, const Ray& r) { return riaf_sample_f(c, r); }
+    __device__ static Sample sample(const ImageConsts& c, const Ray& r) { return riaf_sample_m(c, r); }
     __device__ static Sample none() {
         Sample s;
         s.emitting = 0;
         return s;
     }
     __device__ static Co coeffs(const ImageConsts& c, const Sample& p, int f) {
-        return riaf_coefficients_f(c, p, c.freq[f] * 1e-9, c.emission_scale_pow2[f]);
+        return riaf_coefficients_m(c, p, c.freq[f] * 1e-9, c.emission_scale_pow2[f]);
     }
     __device__ static Co coeffs_ctl(const ImageConsts& c, const Sample& p, int g) {
-        return riaf_coefficients_f(c, p, c.ctl_freq[g] * 1e-9, c.ctl_emission_scale_pow2[g]);
+        return riaf_coefficients_m(c, p, c.ctl_freq[g] * 1e-9, c.ctl_emission_scale_pow2[g]);
     }
     __device__ static RadDepths depths(const Co& co, double dls) {
         return RadDepths{abs_val(co.aI) + norm_refined(co.aQ, co.aU, co.aV), norm_refined(co.rQ, co.rU, co.rV),
@@ -158,8 +158,8 @@ struct RadTraits<PolicyFP64, SceneGrmhd> {
 // field four-vectors and the screen angle stay FP64 (grmhd_sample, the
 // reference's fluid_state); the thermal fit per frequency and the transfer
 // are the mixed RIAF scene's.
-__device__ __forceinline__ RiafSampleF grmhd_sample_to_f(const ImageConsts& c, const GrmhdSample& p) {
-    RiafSampleF o;
+__device__ __forceinline__ RiafSampleM grmhd_sample_to_m(const ImageConsts& c, const GrmhdSample& p) {
+    RiafSampleM o;
     o.emitting = p.emitting && p.ne > 0.0;
     o.on_axis = 0;
     o.has_chi = p.has_chi;
@@ -172,17 +172,17 @@ __device__ __forceinline__ RiafSampleF grmhd_sample_to_f(const ImageConsts& c, c
     o.sin_theta = p.st;
     o.cos2chi = p.cos2chi;
     o.sin2chi = p.sin2chi;
-    riaf_sample_thermal_f(c, o);
+    riaf_sample_thermal_m(c, o);
     return o;
 }
 
-__device__ __forceinline__ RiafSampleF grmhd_sample_f(const ImageConsts& c, const Ray& r) {
-    return grmhd_sample_to_f(c, grmhd_sample(c, r));
+__device__ __forceinline__ RiafSampleM grmhd_sample_m(const ImageConsts& c, const Ray& r) {
+    return grmhd_sample_to_m(c, grmhd_sample(c, r));
 }
 
 template<>
 struct RadTraits<PolicyMixed, SceneGrmhd> : RadTraits<PolicyMixed, SceneRiaf> {
-    __device__ static Sample sample(const ImageConsts& c, const Ray& r) { return grmhd_sample_f(c, r); }
+    __device__ static Sample sample(const ImageConsts& c, const Ray& r) { return grmhd_sample_m(c, r); }
 };
 
 // Slow light: the grid plasma interpolated in time between the resident
@@ -192,13 +192,13 @@ struct RadTraits<PolicyFP64, SceneGrmhdSlow> : RadTraits<PolicyFP64, SceneGrmhd>
     __device__ static Sample sample(const ImageConsts& c, const Ray& r) { return grmhd_sample_series(c, r); }
 };
 
-__device__ __forceinline__ RiafSampleF grmhd_series_sample_f(const ImageConsts& c, const Ray& r) {
-    return grmhd_sample_to_f(c, grmhd_sample_series(c, r));
+__device__ __forceinline__ RiafSampleM grmhd_series_sample_m(const ImageConsts& c, const Ray& r) {
+    return grmhd_sample_to_m(c, grmhd_sample_series(c, r));
 }
 
 template<>
 struct RadTraits<PolicyMixed, SceneGrmhdSlow> : RadTraits<PolicyMixed, SceneRiaf> {
-    __device__ static Sample sample(const ImageConsts& c, const Ray& r) { return grmhd_series_sample_f(c, r); }
+    __device__ static Sample sample(const ImageConsts& c, const Ray& r) { return grmhd_series_sample_m(c, r); }
 };
 
 // The RIAF in Boyer-Lindquist coordinates: the same plasma model, sampled
@@ -209,8 +209,8 @@ struct RadTraits<PolicyFP64, SceneRiafBL> : RadTraits<PolicyFP64, SceneRiaf> {
     __device__ static Sample sample(const ImageConsts& c, const Ray& r) { return riaf_sample_t<true>(c, r); }
 };
 
-__device__ __forceinline__ RiafSampleF riaf_sample_to_f(const ImageConsts& c, const RiafSample& p) {
-    RiafSampleF o;
+__device__ __forceinline__ RiafSampleM riaf_sample_to_m(const ImageConsts& c, const RiafSample& p) {
+    RiafSampleM o;
     o.emitting = p.emitting;
     o.on_axis = p.on_axis;
     o.has_chi = p.has_chi;
@@ -223,14 +223,14 @@ __device__ __forceinline__ RiafSampleF riaf_sample_to_f(const ImageConsts& c, co
     o.sin_theta = p.sin_theta;
     o.cos2chi = p.cos2chi;
     o.sin2chi = p.sin2chi;
-    riaf_sample_thermal_f(c, o);
+    riaf_sample_thermal_m(c, o);
     return o;
 }
 
 template<>
 struct RadTraits<PolicyMixed, SceneRiafBL> : RadTraits<PolicyMixed, SceneRiaf> {
     __device__ static Sample sample(const ImageConsts& c, const Ray& r) {
-        return riaf_sample_to_f(c, riaf_sample_t<true>(c, r));
+        return riaf_sample_to_m(c, riaf_sample_t<true>(c, r));
     }
 };
 
@@ -241,7 +241,7 @@ struct RadTraits<P, SceneFarCks<B>> : RadTraits<P, B> {};
 
 // The scene's transport RHS under a policy.  The FP64 policy keeps the
 // reference's operation order; the mixed policy uses the factored form
-// (kp_geometry_f32.cuh).
+// (kp_geometry_mixed.cuh).
 template<class P, class S>
 __device__ __forceinline__ Ray policy_rhs(const ImageConsts& c, const Ray& X) {
     return S::template rhs<P::kMixed>(c, X);

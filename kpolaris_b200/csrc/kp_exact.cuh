@@ -15,10 +15,10 @@
 // formed as b q - a so that a zero numerator over a positive divisor keeps its
 // sign.  A square root g of v within one ulp becomes the rounded one by
 // g + (v - g g) h with h = 1 / (2 sqrt(v)), but for one significand
-// (exact_sqrt sees to it).  The starting values are the hardware's approximate reciprocal and reciprocal
-// square root, of 20 bits, taken to one ulp by the geometric series of
-// 1 / b = y / (1 - e), e = 1 - b y, and the binomial series of
-// v^-1/2 = y (1 - e)^-1/2, e = 1 - v y y, each to its term in e^2: what is
+// (exact_sqrt sees to it).  The starting values are the hardware's approximate
+// reciprocal and reciprocal square root, of 20 bits, taken to one ulp by the
+// geometric series of 1 / b = y / (1 - e), e = 1 - b y, and the binomial series
+// of v^-1/2 = y (1 - e)^-1/2, e = 1 - v y y, each to its term in e^2: what is
 // left out is below e^3 = 2^-57.
 #pragma once
 

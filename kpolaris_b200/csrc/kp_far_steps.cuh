@@ -69,7 +69,7 @@ KP_HD MacroRun macro_run(const ImageConsts& c, double r, double xk, double v, do
     } else {
         reach = min_val(reach, abs_val(r - c.cam_radius) - 1.1 * v * cap);
     }
-    if (!(along > 0.1 * r * v)) reach = min_val(reach, r - c.fp32_radius - 0.1 * v * cap);
+    if (!(along > 0.1 * r * v)) reach = min_val(reach, r - c.far_radius - 0.1 * v * cap);
     const double span = reach / (v * (1.0 + 4.0 * c.mass / rmin));
     if (!(span >= h) || !(span < 1e300) || left < 1) return none;
     MacroRun run = {0, 0.0, h};

@@ -13,7 +13,7 @@
 
 #include "kp_camera.cuh"
 #include "kp_exact.cuh"
-#include "kp_geometry_f32.cuh"
+#include "kp_geometry_mixed.cuh"
 
 namespace kp {
 
@@ -109,8 +109,8 @@ KP_HD FmksTheta fmks_theta(const FmksParams& m, double x1, double x2) {
     FmksMap q;
     if constexpr (MIXED) {
         // reciprocals of the map's constants, and its angle in half turns
-        const double inv_xt = kp_recip<double>(m.poly_xt);
-        const double inv_al1 = kp_recip<double>(m.poly_alpha + 1.0);
+        const double inv_xt = kp_recip(m.poly_xt);
+        const double inv_al1 = kp_recip(m.poly_alpha + 1.0);
         double za, za1, za2;
         fmks_powers(m, y * inv_xt, za, za1, za2);
         q.za_al = za * inv_al1;
@@ -380,14 +380,14 @@ KP_HD FmksFactored fmks_factored_conn(const FmksParams& m, const D4& x) {
     sincos(t.th, &sn, &cs);
     const double a2 = a * a, s2 = sn * sn, safe_s2 = max_val(s2, kTiny);
     const double rho2 = r * r + a2 * cs * cs;
-    const double inv_rho2 = kp_recip<double>(rho2);
+    const double inv_rho2 = kp_recip(rho2);
     const double inv_rho4 = inv_rho2 * inv_rho2;
     const double f = 2.0 * M * r * inv_rho2;
     const double delta = r * r - 2.0 * M * r + a2;
     FmksFactored o;
     o.r = r;
-    o.inv_r = kp_recip<double>(r);
-    o.inv_dth2 = kp_recip<double>(t.dth2);
+    o.inv_r = kp_recip(r);
+    o.inv_dth2 = kp_recip(t.dth2);
     o.dth1 = t.dth1;
     o.dth2 = t.dth2;
     o.d2th11 = t.d2th11;
@@ -398,7 +398,7 @@ KP_HD FmksFactored fmks_factored_conn(const FmksParams& m, const D4& x) {
     o.G11 = delta * inv_rho2;
     o.G13 = a * inv_rho2;
     o.G22 = inv_rho2;
-    o.G33 = inv_rho2 * kp_recip<double>(safe_s2);
+    o.G33 = inv_rho2 * kp_recip(safe_s2);
     const double drho_dth = -2.0 * a2 * sn * cs, ds2_dth = 2.0 * sn * cs;
     const double df_dr = 2.0 * M * (rho2 - 2.0 * r * r) * inv_rho4;
     const double df_dth = -2.0 * M * r * drho_dth * inv_rho4;

@@ -116,7 +116,7 @@ inline ImageConsts image_consts_fmks(const kp_pass_a_params* p, const kp_grmhd_m
     c.max_pol_frac = m.max_pol_frac;
     c.min_sin_theta = 1e-4;  // grmhd_grid.hpp:1149
     c.fit = m.emission_type == KP_FIT_DEXTER ? 4 : 1;
-    c.fp32_radius = p->outer_radius + 2.0 * std::max(std::fabs(p->max_step), std::fabs(p->step));
+    c.far_radius = p->outer_radius + 2.0 * std::max(std::fabs(p->max_step), std::fabs(p->step));
     c.nfreq = nfreq;
     const double length_unit = grmhd_length_unit_cgs(m);
     for (int f = 0; f < nfreq; ++f) {

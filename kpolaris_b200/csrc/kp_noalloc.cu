@@ -91,8 +91,8 @@ extern "C" int kp_batch_riaf_noalloc(const kp_riaf_job* jobs, int njobs, const k
     if (opt.integrator != KP_INTEGRATOR_STEP_DOUBLING_RK4 && opt.integrator != KP_INTEGRATOR_CASH_KARP)
         return set_error(KP_ERR_INVALID, "unknown integrator %d", opt.integrator);
     if (opt.threads_per_block != 0)
-        return set_error(KP_ERR_INVALID, "threads_per_block is fixed by the wavefront kernels (%d far, %d near): pass 0",
-                         kFarThreads, kNearBThreads);
+        return set_error(KP_ERR_INVALID, "threads_per_block is fixed by the wavefront kernels (%d far, %d near-A, %d near-B): pass 0",
+                         kFarThreads, kNearAThreads, kNearBThreads);
     long long total = 0;
     int nf_max = 1;
     for (int i = 0; i < njobs; ++i) {

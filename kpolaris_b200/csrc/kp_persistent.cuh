@@ -9,7 +9,7 @@
 // code and each kernel's instruction working set stays small (this file: what
 // they share, and their form with one ray per lane; kp_quad.cuh: four lanes per
 // ray):
-//   far     rays beyond ImageConsts::fp32_radius, pass A and pass B: pure
+//   far     rays beyond ImageConsts::far_radius, pass A and pass B: pure
 //           transport (no surface lies within a step, no plasma is sampled);
 //   near-A  pass A inside: the surface-crossing search, no radiation;
 //   near-B  pass B inside: radiative transfer.
@@ -89,7 +89,7 @@ __device__ __forceinline__ double fifth_root(double x) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const double y2 = y * y, y4 = y2 * y2;
-                y = y - (y4 * y - x) * kp_recip<double>(5.0 * y4);
+                y = y - (y4 * y - x) * kp_recip(5.0 * y4);
             }
             return y;
         }
@@ -105,7 +105,7 @@ __device__ __forceinline__ double accepted_next_h(double h, double err, double t
                                                   double max_step, double requested) {
     double factor = 2.0;
     if (err > 0.0 && !(tol >= 64.0 * err)) {
-        factor = 0.9 * fifth_root<MIXED>(MIXED ? tol * kp_recip<double>(err) : tol / err);
+        factor = 0.9 * fifth_root<MIXED>(MIXED ? tol * kp_recip(err) : tol / err);
         factor = min_val(2.0, max_val(0.2, factor));
     }
     double next_h = min_val(max_step, max_val(min_step, abs_val(h) * factor));
@@ -219,7 +219,7 @@ __device__ __forceinline__ void seed_body(const JobDesc* jobs, const SeedEntry* 
 
 // Phase that advances a ray from the top of its pass-A or pass-B loop.
 __device__ __forceinline__ int phase_of(const ImageConsts& c, int in_b, double r_bl) {
-    if (r_bl > c.fp32_radius) return kPhaseFar;
+    if (r_bl > c.far_radius) return kPhaseFar;
     return in_b ? kPhaseNearB : kPhaseNearA;
 }
 

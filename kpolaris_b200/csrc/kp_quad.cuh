@@ -136,7 +136,7 @@ __device__ __forceinline__ double quad_control_error(const D4& a, const D4& b, d
     for (int i = 0; i < 4; ++i) {
         const double s = max_val(1.0, max_val(abs_val(a.v[i]), abs_val(b.v[i])));
         const double d = abs_val(a.v[i] - b.v[i]);
-        e[i] = MIXED && s < 1e150 ? d * kp_recip<double>(s) : d / s;
+        e[i] = MIXED && s < 1e150 ? d * kp_recip(s) : d / s;
         nan = nan || !(e[i] == e[i]);
         n = max_val(n, e[i]);
     }
@@ -207,8 +207,7 @@ __device__ __noinline__ void quad_ck_job(const typename SC::Geo& c, double toler
 // extrapolated to zero step (W. Gragg, SIAM J. Numer. Anal. 2 (1965) 384;
 // Hairer, Norsett, Wanner, Solving ODEs I, II.9: order 8), 21 right-hand
 // sides in FP64 for up to hundreds of steps of 11.  A 256^2 image has 908 far
-// steps per ray; they were 45% of its time in FP32 stage chains, whose
-// rounding moved the step counts of a few rays in ten thousand.
+// steps per ray: 147 ms of an 8 x 256^2 step one by one, 45 ms bridged.
 constexpr int kRkMacro = 4;
 
 template<class P, class SC>
@@ -655,7 +654,7 @@ __device__ __forceinline__ void quad_body(const WaveDesc& W, int per_warp = 8) {
                 st.cap = J->c.max_step;
                 st.steps += run_of.count;
             }
-            if (!(next_r > J->c.fp32_radius)) atomicExch(W.status, 3);
+            if (!(next_r > J->c.far_radius)) atomicExch(W.status, 3);
         } else if (kPassA && run && st.mode == kAStep) {
             const ImageConsts& c = J->c;
             bool accepted = true;

@@ -1,4 +1,4 @@
-// kp_radiation_f32.cuh -- the radiation side of the mixed policy: RIAF plasma
+// kp_radiation_mixed.cuh -- the radiation side of the mixed policy: RIAF plasma
 // state, thermal synchrotron coefficients and the Strang transfer step, with
 // the formulas of kp_radiation.cuh (and the reference's
 // src/model/riaf.hpp:54-549, src/radiation/thermal_synchrotron.hpp:60-627,
@@ -18,11 +18,11 @@
 // (the transfer equation is linear in (j, S)); the image is unscaled at the end.
 #pragma once
 
-#include "kp_geometry_f32.cuh"
+#include "kp_geometry_mixed.cuh"
 
 namespace kp {
 
-namespace f32c {
+namespace mixc {
 constexpr double kPiD = 3.141592653589793;
 constexpr double kEE = 4.803204712570263e-10;
 constexpr double kME = 9.1093837015e-28;
@@ -48,75 +48,74 @@ constexpr double kRhoV = (4.0 * kPiD * kEE * kEE / kME) * (kEE / (kME * kCL)) / 
 // rho_Q nu = (4 pi e^2 / m_e) (e / (m_e c))^2 n_e B^2 sin^2(theta) / (2^4 pi^3 c nu^2) x fit
 constexpr double kRhoQ = (4.0 * kPiD * kEE * kEE / kME) * (kEE / (kME * kCL)) * (kEE / (kME * kCL)) * kPiD /
                          (16.0 * kPiD * kPiD * kPiD * kPiD * kCL);
-}  // namespace f32c
+}  // namespace mixc
 
-using CoeffsF = Coeffs<double>;
+using CoeffsM = Coeffs<double>;
 
 // K0/K2 and K1/K2 for x = 1/Theta_e with the polynomial fits of
 // thermal_synchrotron.hpp:108-158; for x > 2 the factor e^-x / sqrt(x) cancels.
-template<class T>
-KP_HD void bessel_ratios(T x, T lg, T& r0, T& r1) {  // lg = log(x / 2)
-    T p, q;
-    if (x <= T(2)) {
-        const T y = x * x * T(0.25);
-        const T t = y * T(4.0 / (3.75 * 3.75));
-        T i0 = T(0.0045813);
-        i0 = T(0.0360768) + t * i0;
-        i0 = T(0.2659732) + t * i0;
-        i0 = T(1.2067492) + t * i0;
-        i0 = T(3.0899424) + t * i0;
-        i0 = T(3.5156229) + t * i0;
-        i0 = T(1) + t * i0;
-        T i1 = T(0.00032411);
-        i1 = T(0.00301532) + t * i1;
-        i1 = T(0.02658733) + t * i1;
-        i1 = T(0.15084934) + t * i1;
-        i1 = T(0.51498869) + t * i1;
-        i1 = T(0.87890594) + t * i1;
-        i1 = x * (T(0.5) + t * i1);
-        T a = T(0.00000740);
-        a = T(0.00010750) + y * a;
-        a = T(0.00262698) + y * a;
-        a = T(0.03488590) + y * a;
-        a = T(0.23069756) + y * a;
-        a = T(0.42278420) + y * a;
-        a = T(-0.57721566) + y * a;
+KP_HD void bessel_ratios(double x, double lg, double& r0, double& r1) {  // lg = log(x / 2)
+    double p, q;
+    if (x <= 2.0) {
+        const double y = x * x * 0.25;
+        const double t = y * (4.0 / (3.75 * 3.75));
+        double i0 = 0.0045813;
+        i0 = 0.0360768 + t * i0;
+        i0 = 0.2659732 + t * i0;
+        i0 = 1.2067492 + t * i0;
+        i0 = 3.0899424 + t * i0;
+        i0 = 3.5156229 + t * i0;
+        i0 = 1.0 + t * i0;
+        double i1 = 0.00032411;
+        i1 = 0.00301532 + t * i1;
+        i1 = 0.02658733 + t * i1;
+        i1 = 0.15084934 + t * i1;
+        i1 = 0.51498869 + t * i1;
+        i1 = 0.87890594 + t * i1;
+        i1 = x * (0.5 + t * i1);
+        double a = 0.00000740;
+        a = 0.00010750 + y * a;
+        a = 0.00262698 + y * a;
+        a = 0.03488590 + y * a;
+        a = 0.23069756 + y * a;
+        a = 0.42278420 + y * a;
+        a = -0.57721566 + y * a;
         p = a - lg * i0;
-        T b = T(-0.00004686);
-        b = T(-0.00110404) + y * b;
-        b = T(-0.01919402) + y * b;
-        b = T(-0.18156897) + y * b;
-        b = T(-0.67278579) + y * b;
-        b = T(0.15443144) + y * b;
-        b = T(1) + y * b;
-        q = lg * i1 + b * kp_recip<T>(x);
+        double b = -0.00004686;
+        b = -0.00110404 + y * b;
+        b = -0.01919402 + y * b;
+        b = -0.18156897 + y * b;
+        b = -0.67278579 + y * b;
+        b = 0.15443144 + y * b;
+        b = 1.0 + y * b;
+        q = lg * i1 + b * kp_recip(x);
     } else {
-        const T y = T(2) * kp_recip<T>(x);
-        T a = T(0.00053208);
-        a = T(-0.00251540) + y * a;
-        a = T(0.00587872) + y * a;
-        a = T(-0.01062446) + y * a;
-        a = T(0.02189568) + y * a;
-        a = T(-0.07832358) + y * a;
-        p = T(1.25331414) + y * a;
-        T b = T(-0.00068245);
-        b = T(0.00325614) + y * b;
-        b = T(-0.00780353) + y * b;
-        b = T(0.01504268) + y * b;
-        b = T(-0.03655620) + y * b;
-        b = T(0.23498619) + y * b;
-        q = T(1.25331414) + y * b;
+        const double y = 2.0 * kp_recip(x);
+        double a = 0.00053208;
+        a = -0.00251540 + y * a;
+        a = 0.00587872 + y * a;
+        a = -0.01062446 + y * a;
+        a = 0.02189568 + y * a;
+        a = -0.07832358 + y * a;
+        p = 1.25331414 + y * a;
+        double b = -0.00068245;
+        b = 0.00325614 + y * b;
+        b = -0.00780353 + y * b;
+        b = 0.01504268 + y * b;
+        b = -0.03655620 + y * b;
+        b = 0.23498619 + y * b;
+        q = 1.25331414 + y * b;
     }
-    const T k2 = p + T(2) * q * kp_recip<T>(x);
-    const T inv = k2 > T(0) ? kp_recip<T>(k2) : T(0);
-    r0 = k2 > T(0) ? p * inv : T(1);
-    r1 = k2 > T(0) ? q * inv : T(1);
+    const double k2 = p + 2.0 * q * kp_recip(x);
+    const double inv = k2 > 0.0 ? kp_recip(k2) : 0.0;
+    r0 = k2 > 0.0 ? p * inv : 1.0;
+    r1 = k2 > 0.0 ? q * inv : 1.0;
 }
 
 // Plasma state at a sample point, with the frequency-independent factors of
-// the thermal fits (riaf_sample_thermal_f).
-struct RiafSampleF {
-    double ne, thetae, b, nu_fluid, cos_theta, sin_theta, theta, cos2chi, sin2chi;
+// the thermal fits (riaf_sample_thermal_m).
+struct RiafSampleM {
+    double ne, thetae, b, nu_fluid, cos_theta, sin_theta, cos2chi, sin2chi;
     double xs0;     // argument of the emission fit, over the frequency in hertz
     double xf0;     // argument of the Faraday fits times the root of the frequency
     double rv0;     // rho_V nu times the frequency, without the fit's logarithm
@@ -128,9 +127,10 @@ struct RiafSampleF {
     int emitting, on_axis, has_chi;
 };
 
-// Cube root of x > 0 to a few ulp: Newton's step in FP64 from a
-// single-precision start.  The fits take exp(-x^(1/3)): an error of the root
-// is multiplied by the root there.
+// Cube root of x > 0: Newton's step in FP64 from a single-precision start, whose
+// relative error it squares: 3e-13 for x in 1..1e7, 7e-12 over the whole range.
+// The fits take exp(-x^(1/3)): an error of the root is multiplied by the root
+// there.
 KP_HD double cube_root(double x) {
     if (!(x > 1e-30 && x < 1e30)) return cbrt(x);
 #ifdef __CUDA_ARCH__
@@ -139,40 +139,40 @@ KP_HD double cube_root(double x) {
     const double y = double(cbrtf(float(x)));
 #endif
     const double y2 = y * y;
-    return y - (y2 * y - x) * kp_recip<double>(3.0 * y2);
+    return y - (y2 * y - x) * kp_recip(3.0 * y2);
 }
 
 // Frequency-independent factors of the thermal fits at one sample
 // (thermal_synchrotron.hpp:312-395, 462-506), evaluated once per sample
 // instead of once per frequency.  lt = log(Theta_e).
-KP_HD void riaf_sample_thermal_f(const ImageConsts& c, RiafSampleF& p, double lt) {
+KP_HD void riaf_sample_thermal_m(const ImageConsts& c, RiafSampleM& p, double lt) {
     const double te = p.thetae, st = max_val(p.sin_theta, c.min_sin_theta);
-    const double inv_nu = kp_recip<double>(p.nu_fluid);
+    const double inv_nu = kp_recip(p.nu_fluid);
     double r0, r1;
-    bessel_ratios<double>(kp_recip<double>(te), -lt - 0.69314718055994530942, r0, r1);
-    p.rv0 = f32c::kRhoV * p.ne * p.b * r0 * p.cos_theta * inv_nu;
-    p.rq0 = f32c::kRhoQ * p.ne * (p.b * p.b) * (r1 + 6.0 * te) * (st * st) * (inv_nu * inv_nu);
+    bessel_ratios(kp_recip(te), -lt - 0.69314718055994530942, r0, r1);
+    p.rv0 = mixc::kRhoV * p.ne * p.b * r0 * p.cos_theta * inv_nu;
+    p.rq0 = mixc::kRhoQ * p.ne * (p.b * p.b) * (r1 + 6.0 * te) * (st * st) * (inv_nu * inv_nu);
     {
         double g, inv;
-        kp_sqrt_pair<double>(max_val(f32c::kFaradayX2 * st * p.b * inv_nu, 1e-200), g, inv);
+        kp_sqrt_pair(max_val(mixc::kFaradayX2 * st * p.b * inv_nu, 1e-200), g, inv);
         p.xf0 = te * g;
     }
-    const double nus = c.fit == 4 ? f32c::kDexNus * p.b * st * te * te + 1.0 : f32c::kPandyaNus * p.b * st * te * te;
-    p.xs0 = p.nu_fluid * kp_recip<double>(max_val(nus, 1e-200));
+    const double nus = c.fit == 4 ? mixc::kDexNus * p.b * st * te * te + 1.0 : mixc::kPandyaNus * p.b * st * te * te;
+    p.xs0 = p.nu_fluid * kp_recip(max_val(nus, 1e-200));
     p.qterm = p.vt1 = p.vt2a = 0.0;
     if (c.fit == 4) {
-        p.pref = p.ne * kp_recip<double>(te * te);
+        p.pref = p.ne * kp_recip(te * te);
         return;
     }
-    p.pref = f32c::kPandyaPref * p.ne * p.b;
+    p.pref = mixc::kPandyaPref * p.ne * p.b;
     const double t2425 = exp(0.96 * lt);
-    p.qterm = (7.0 * t2425 + 35.0) * kp_recip<double>(10.0 * t2425 + 75.0);
+    p.qterm = (7.0 * t2425 + 35.0) * kp_recip(10.0 * t2425 + 75.0);
     const double sin_shift = st * 0.4356824462767121 - p.cos_theta * 0.9001004421765051;
-    p.vt1 = (37.0 - 87.0 * sin_shift) * kp_recip<double>(100.0 * (te + 1.0));
+    p.vt1 = (37.0 - 87.0 * sin_shift) * kp_recip(100.0 * (te + 1.0));
     p.vt2a = exp(0.6 * lt) * 0.04 + 0.7;
 }
 
-KP_HD void riaf_sample_thermal_f(const ImageConsts& c, RiafSampleF& p) { riaf_sample_thermal_f(c, p, log(p.thetae)); }
+KP_HD void riaf_sample_thermal_m(const ImageConsts& c, RiafSampleM& p) { riaf_sample_thermal_m(c, p, log(p.thetae)); }
 
 // Boyer-Lindquist metric entries at (r, theta) with unit mass, FP64.
 struct BlEntries {
@@ -183,7 +183,7 @@ struct BlEntries {
 KP_HD BlEntries bl_entries(double r, double s2, double c2, double a) {
     const double a2 = a * a, ra = r * r + a2;
     const double sigma = r * r + a2 * c2, delta = ra - 2.0 * r;
-    const double i_s = kp_recip<double>(sigma), i_d = kp_recip<double>(max_val(delta, 1e-30));
+    const double i_s = kp_recip(sigma), i_d = kp_recip(max_val(delta, 1e-30));
     const double f = 2.0 * r * i_s, i_sd = i_s * i_d;
     BlEntries m;
     m.tt = f - 1.0;
@@ -192,7 +192,7 @@ KP_HD BlEntries bl_entries(double r, double s2, double c2, double a) {
     m.rr = sigma * i_d;
     m.itt = -(ra * ra - a2 * delta * s2) * i_sd;
     m.itp = -2.0 * a * r * i_sd;
-    m.ipp = (delta - a2 * s2) * i_sd * kp_recip<double>(s2);
+    m.ipp = (delta - a2 * s2) * i_sd * kp_recip(s2);
     m.irr = delta * i_s;
     return m;
 }
@@ -202,8 +202,8 @@ KP_HD BlEntries bl_entries(double r, double s2, double c2, double a) {
 // so a dot product is eta(u, v) + f (l.u)(l.v) with l.u formed once per
 // vector; (l1, l2) = sin(theta) (cos phi, sin phi) gives the BL angles, and
 // the azimuthal vector is (0, -y, x, 0).
-KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
-    RiafSampleF out;
+KP_HD RiafSampleM riaf_sample_m(const ImageConsts& c, const Ray& s) {
+    RiafSampleM out;
     out.emitting = 0;
     out.on_axis = 0;
     out.has_chi = 0;
@@ -211,14 +211,14 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
     const double x = s.x.v[1], y = s.x.v[2], z = s.x.v[3];
     const double sqsum = x * x + y * y + z * z - a2;
     double discr, inv_discr, r, inv_r;
-    kp_sqrt_pair<double>(sqsum * sqsum + 4.0 * a2 * z * z, discr, inv_discr);
-    kp_sqrt_pair<double>(max_val(0.5 * (sqsum + discr), 1e-30), r, inv_r);
+    kp_sqrt_pair(sqsum * sqsum + 4.0 * a2 * z * z, discr, inv_discr);
+    kp_sqrt_pair(max_val(0.5 * (sqsum + discr), 1e-30), r, inv_r);
     const double r_bl = max_val(r, c.min_radius);
     if (r_bl <= c.horizon + c.horizon_buffer || r_bl < c.r_min || r_bl > c.r_max) return out;
-    const double r2 = r * r, inv_rp = kp_recip<double>(r2 + a2);
+    const double r2 = r * r, inv_rp = kp_recip(r2 + a2);
     const double l1 = (r * x + a * y) * inv_rp, l2 = (r * y - a * x) * inv_rp, l3 = z * inv_r;
     const double c2 = min_val(l3 * l3, 1.0), s2 = max_val((x * x + y * y) * inv_rp, 1e-30);
-    const double amp = 2.0 * c.mass * r2 * r * kp_recip<double>(r2 * r2 + a2 * z * z);
+    const double amp = 2.0 * c.mass * r2 * r * kp_recip(r2 * r2 + a2 * z * z);
     // n_e, Theta_e and B (riaf.hpp:54-96)
     double ne, thetae, b, lt;
     {
@@ -226,7 +226,7 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
         const double h = max_val(c.disk_h, 1e-6);
         const double rcyl2 = max_val(r_bl * r_bl * s2, c.min_radius * c.min_radius);
         const double zc = r_bl * l3;
-        ne = c.nth0 * exp(c.pow_nth * lr - zc * zc * kp_recip<double>(2.0 * rcyl2 * h * h));
+        ne = c.nth0 * exp(c.pow_nth * lr - zc * zc * kp_recip(2.0 * rcyl2 * h * h));
         if (!(ne > 0.0)) return out;
         ne *= c.ne_unit;
         lt = c.log_te0 + c.pow_T * lr;
@@ -235,9 +235,9 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
             thetae = c.min_thetae;
             lt = log(thetae);
         }
-        const double kb = 8.0 * 3.141592653589793 * 0.1 * f32c::kMP * f32c::kCL * f32c::kCL / 6.0;
+        const double kb = 8.0 * 3.141592653589793 * 0.1 * mixc::kMP * mixc::kCL * mixc::kCL / 6.0;
         double inv;
-        kp_sqrt_pair<double>(max_val(kb * ne * kp_recip<double>(r_bl), 1e-24), b, inv);
+        kp_sqrt_pair(max_val(kb * ne * kp_recip(r_bl), 1e-24), b, inv);
     }
     out.emitting = 1;
     out.ne = ne;
@@ -250,28 +250,28 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
         const BlEntries m = bl_entries(rr, s2, c2, a);
         const double kf = c.keplerian_factor, inf = c.infall_factor;
         if (rr < c.horizon) {
-            vt = kp_recip<double>(sqrt(max_val(-m.itt, 1e-30)));
+            vt = kp_recip(sqrt(max_val(-m.itt, 1e-30)));
         } else {
             double omega;
             const bool plunge = rr < c.isco;
             if (plunge) {
                 const double ri = c.isco;
                 const BlEntries mi = bl_entries(ri, s2, c2, a);
-                const double oi = kp_recip<double>(ri * sqrt(ri) + a);
+                const double oi = kp_recip(ri * sqrt(ri) + a);
                 const double qi = mi.tt + 2.0 * oi * mi.tp + oi * oi * mi.pp;
-                const double ut = kp_recip<double>(sqrt(max_val(-qi, 1e-30)));
+                const double ut = kp_recip(sqrt(max_val(-qi, 1e-30)));
                 const double e = (mi.tt + mi.tp * oi) * ut, l = (mi.tp + mi.pp * oi) * ut;
                 const double kc = m.itt * e * e + 2.0 * m.itp * e * l + m.ipp * l * l;
-                vr = -m.irr * sqrt(max_val(-(1.0 + kc) * kp_recip<double>(max_val(m.irr, 1e-30)), 0.0));
-                omega = (m.itp * e + m.ipp * l) * kp_recip<double>(max_val(m.itt * e + m.itp * l, 1e-30));
+                vr = -m.irr * sqrt(max_val(-(1.0 + kc) * kp_recip(max_val(m.irr, 1e-30)), 0.0));
+                omega = (m.itp * e + m.ipp * l) * kp_recip(max_val(m.itt * e + m.itp * l, 1e-30));
             } else {
                 double sr, isr;
-                kp_sqrt_pair<double>(rr, sr, isr);
-                omega = kp_recip<double>(rr * sr + a);
+                kp_sqrt_pair(rr, sr, isr);
+                omega = kp_recip(rr * sr + a);
             }
             if (kf != 1.0) {
                 const double g = m.itt;
-                const double off = m.itp * kp_recip<double>(abs_val(g) > 1e-30 ? g : (g < 0.0 ? -1e-30 : 1e-30));
+                const double off = m.itp * kp_recip(abs_val(g) > 1e-30 ? g : (g < 0.0 ? -1e-30 : 1e-30));
                 omega = omega + (1.0 - kf) * (off - omega);
             }
             if (inf != 0.0) {
@@ -280,10 +280,10 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
             }
             const double q = m.tt + 2.0 * omega * m.tp + omega * omega * m.pp;
             double inv;
-            kp_sqrt_pair<double>(max_val(-(1.0 + vr * vr * m.rr) * kp_recip<double>(q), 1e-60), vt, inv);
+            kp_sqrt_pair(max_val(-(1.0 + vr * vr * m.rr) * kp_recip(q), 1e-60), vt, inv);
             vphi = omega * vt;
         }
-        const double i_d = kp_recip<double>(max_val(rr * rr - 2.0 * rr + a2, 1e-30));
+        const double i_d = kp_recip(max_val(rr * rr - 2.0 * rr + a2, 1e-30));
         vt += 2.0 * rr * i_d * vr;
         vphi += a * i_d * vr;
     }
@@ -301,7 +301,7 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
         const double n2 = dot(u, u);
         if (n2 < 0.0) {
             double n, inv;
-            kp_sqrt_pair<double>(max_val(-n2, 1e-30), n, inv);
+            kp_sqrt_pair(max_val(-n2, 1e-30), n, inv);
             u = Vec{u.t * inv, u.x * inv, u.y * inv, u.z * inv, u.l * inv};
         }
     }
@@ -321,19 +321,19 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
     if (!(bsq > 1e-30)) project(vec(0.0, 1.0, 0.0, 0.0));
     if (bsq > 1e-30) {
         double n, inv;
-        kp_sqrt_pair<double>(bsq, n, inv);
+        kp_sqrt_pair(bsq, n, inv);
         bv = Vec{bv.t * inv, bv.x * inv, bv.y * inv, bv.z * inv, bv.l * inv};
     }
     const double kb = dot(k, bv);
-    const double ct = min_val(max_val(kb * kp_recip<double>(max_val(nu_fluid, 1e-30)), -1.0), 1.0);
+    const double ct = min_val(max_val(kb * kp_recip(max_val(nu_fluid, 1e-30)), -1.0), 1.0);
     out.nu_fluid = nu_fluid;
     out.cos_theta = ct;
     {
         double st, inv;
-        kp_sqrt_pair<double>(max_val(1.0 - ct * ct, 1e-60), st, inv);
+        kp_sqrt_pair(max_val(1.0 - ct * ct, 1e-60), st, inv);
         out.sin_theta = max_val(st, c.min_sin_theta);
     }
-    riaf_sample_thermal_f(c, out, lt);
+    riaf_sample_thermal_m(c, out, lt);
     if (ct >= 1.0 || ct <= -1.0) {
         out.on_axis = 1;
         return out;
@@ -343,7 +343,7 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
     const Vec e2 = vec(s.e2.v[0], s.e2.v[1], s.e2.v[2], s.e2.v[3]);
     double b1 = dot(e1, bv), b2 = dot(e2, bv);
     if (abs_val(uk) > 1e-30) {
-        const double iu = -kp_recip<double>(uk);
+        const double iu = -kp_recip(uk);
         const double ub = dot(u, bv), Kb = kb * iu - ub;
         const double ue1 = dot(u, e1), ue2 = dot(u, e2);
         b1 += ue1 * ub - (dot(k, e1) * iu - ue1) * Kb;
@@ -351,7 +351,7 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
     }
     const double bproj2 = b1 * b1 + b2 * b2;
     if (bproj2 > 1e-30) {
-        const double inv = kp_recip<double>(bproj2);
+        const double inv = kp_recip(bproj2);
         out.has_chi = 1;
         out.cos2chi = (b2 * b2 - b1 * b1) * inv;
         out.sin2chi = -2.0 * b1 * b2 * inv;
@@ -361,12 +361,12 @@ KP_HD RiafSampleF riaf_sample_f(const ImageConsts& c, const Ray& s) {
 
 // Thermal coefficients at one frequency (in GHz), emission scaled by 2^E
 // (`escale`).
-KP_HD CoeffsF riaf_coefficients_f(const ImageConsts& c, const RiafSampleF& p, double freq_ghz, double escale) {
-    CoeffsF o = {};
+KP_HD CoeffsM riaf_coefficients_m(const ImageConsts& c, const RiafSampleM& p, double freq_ghz, double escale) {
+    CoeffsM o = {};
     if (!p.emitting) return o;
     const double freq = freq_ghz * 1e9;
     double sf, isf;
-    kp_sqrt_pair<double>(freq, sf, isf);
+    kp_sqrt_pair(freq, sf, isf);
     const double inv_freq = isf * isf;
     // Faraday rotation and conversion (symphony_rho_QV), invariant rho nu
     const double x = max_val(p.xf0 * isf, 1e-12);
@@ -385,31 +385,31 @@ KP_HD CoeffsF riaf_coefficients_f(const ImageConsts& c, const RiafSampleF& p, do
         j -= e47;
         // 0.5 + 0.5 tanh(z) = 1 / (1 + e^-2z); below z = -20 it is under 1e-17
         const double z2 = 20.0 * (lx - 4.787491742782046);
-        if (z2 > -40.0) j += (e47 - 369.69342869090815 * exp((-8.0 / 3.0) * lx)) * kp_recip<double>(1.0 + exp(-z2));
+        if (z2 > -40.0) j += (e47 - 369.69342869090815 * exp((-8.0 / 3.0) * lx)) * kp_recip(1.0 + exp(-z2));
         rQ = p.rq0 * j * (inv_freq * inv_freq);
     }
     // emissivities j / nu^2, scaled by 2^E
     const double nu = max_val(freq * p.nu_fluid, 1.0);
-    const double inv_nu2 = escale * kp_recip<double>(nu * nu);
+    const double inv_nu2 = escale * kp_recip(nu * nu);
     const double xs = max_val(p.xs0 * freq, 1e-200), root = cube_root(xs);
     double jI, jQ, jV;
     if (c.fit == 4) {
-        const double inv_root = kp_recip<double>(root), inv2 = inv_root * inv_root;
+        const double inv_root = kp_recip(root), inv2 = inv_root * inv_root;
         const double shape = exp(-1.8899 * root);
-        const double pref = f32c::kDexPref * p.pref * nu * shape * inv_nu2;
+        const double pref = mixc::kDexPref * p.pref * nu * shape * inv_nu2;
         jI = pref * (2.5651 * (1.0 + 1.92 * inv_root + 0.9977 * inv2));
         jQ = pref * (2.5651 * (1.0 + 0.93193 * inv_root + 0.499873 * inv2));
         const double iv = 1.81384 * (inv2 * inv_root) + 3.42319 * inv2 + 0.0292545 * sqrt(inv2 * inv_root) + 2.03773 * inv_root;
         double cft = p.cos_theta;
         if (abs_val(cft) < 1e-10) cft = cft >= 0.0 ? 1e-10 : -1e-10;
         const double st = max_val(p.sin_theta, c.min_sin_theta);
-        jV = f32c::kDexPrefV * p.pref * nu * cft * kp_recip<double>(st * p.thetae) * iv * shape * inv_nu2;
+        jV = mixc::kDexPrefV * p.pref * nu * cft * kp_recip(st * p.thetae) * iv * shape * inv_nu2;
     } else {
         double sx, isx, sr, isr;
-        kp_sqrt_pair<double>(xs, sx, isx);
-        kp_sqrt_pair<double>(root, sr, isr);
+        kp_sqrt_pair(xs, sx, isx);
+        kp_sqrt_pair(root, sr, isr);
         const double st = max_val(p.sin_theta, c.min_sin_theta);
-        const double pref = p.pref * exp(-root) * inv_nu2, lin = pref * f32c::kTerm1 * st;
+        const double pref = p.pref * exp(-root) * inv_nu2, lin = pref * mixc::kTerm1 * st;
         const double bend = 1.8877486253633869933 * sr;
         const double hi = sx + bend, hq = sx + p.qterm * bend;
         jI = lin * (hi * hi);
@@ -426,9 +426,9 @@ KP_HD CoeffsF riaf_coefficients_f(const ImageConsts& c, const RiafSampleF& p, do
     }
     // Kirchhoff: a = j / B_nu, with B_nu = 2 h nu^3 / (c^2 (e^x - 1)) and the
     // reference's series for small x
-    const double xb = f32c::kHOverMc2 * nu * kp_recip<double>(p.thetae);
+    const double xb = mixc::kHOverMc2 * nu * kp_recip(p.thetae);
     const double em1 = xb < 2e-3 ? xb * (1.0 / 24.0) * (24.0 + xb * (12.0 + xb * (4.0 + xb))) : exp(xb) - 1.0;
-    const double fac = f32c::kC2Over2h * em1 * kp_recip<double>(escale) * c.absorption_scale;
+    const double fac = mixc::kC2Over2h * em1 * kp_recip(escale) * c.absorption_scale;
     const double es = c.emission_scale, fs = c.faraday_scale;
     o.jI = es * jI;
     o.jV = es * jV;
@@ -489,7 +489,7 @@ KP_HD void kp_sincospi(double u, double* s, double* c) {
 #endif
 }
 
-KP_HD RotationM faraday_rotation(const CoeffsF& c, double dl) {
+KP_HD RotationM faraday_rotation(const CoeffsM& c, double dl) {
     RotationM r;
     const double rq = c.rQ, ru = c.rU, rv = c.rV;
     const double n2 = rq * rq + ru * ru + rv * rv;
@@ -497,7 +497,7 @@ KP_HD RotationM faraday_rotation(const CoeffsF& c, double dl) {
     if (r.none) return r;
     double n, inv;
     if (n2 > 1e-280 && n2 < 1e280) {
-        kp_sqrt_pair<double>(n2, n, inv);
+        kp_sqrt_pair(n2, n, inv);
     } else {
         n = sqrt(n2);
         inv = 1.0 / n;
@@ -522,7 +522,7 @@ KP_HD void faraday_rotate(StokesM& s, const RotationM& r) {
     s.V = pz + ((r.nx * py - r.ny * px) * r.st + (r.nz * f - pz) * r.omc);
 }
 
-KP_HD void absorb_emit(StokesM& s, const CoeffsF& c, double dl) {
+KP_HD void absorb_emit(StokesM& s, const CoeffsM& c, double dl) {
     const double aq = c.aQ, au = c.aU, av = c.aV, ai = c.aI;
     const double jq = c.jQ, ju = c.jU, jv = c.jV, ji = c.jI;
     const double n2 = aq * aq + au * au + av * av;
@@ -536,7 +536,7 @@ KP_HD void absorb_emit(StokesM& s, const CoeffsF& c, double dl) {
         return;
     }
     double an, inv;
-    kp_sqrt_pair<double>(n2, an, inv);
+    kp_sqrt_pair(n2, an, inv);
     const double nx = aq * inv, ny = au * inv, nz = av * inv;
     const double par = nx * s.Q + ny * s.U + nz * s.V;
     const double jpar = nx * jq + ny * ju + nz * jv;
@@ -553,7 +553,7 @@ KP_HD void absorb_emit(StokesM& s, const CoeffsF& c, double dl) {
     s.V += nz * dpar + (em * (s.V - nz * par) + src * (jv - nz * jpar));
 }
 
-KP_HD void stokes_step_m(StokesM& s, const CoeffsF& c, double dl) {
+KP_HD void stokes_step_m(StokesM& s, const CoeffsM& c, double dl) {
     const RotationM r = faraday_rotation(c, dl);
     faraday_rotate(s, r);
     absorb_emit(s, c, dl);

@@ -13,7 +13,7 @@
 #include "kp_camera.cuh"
 #include "kp_chart.cuh"
 #include "kp_fmks.cuh"
-#include "kp_geometry_f32.cuh"
+#include "kp_geometry_mixed.cuh"
 #include "kp_grmhd.cuh"
 #include "kp_trace_fp64.cuh"
 
@@ -25,7 +25,7 @@ namespace kp {
 // know whether the mixed policy's form was requested.
 template<bool MIXED>
 __device__ __forceinline__ Ray riaf_rhs(double mass, double spin, const Ray& X) {
-    if constexpr (MIXED) return ks_rhs_factored<double>(mass, spin, X);
+    if constexpr (MIXED) return ks_rhs_factored(mass, spin, X);
     else return ks_rhs(mass, spin, X);
 }
 
@@ -60,10 +60,10 @@ struct SceneRiaf {
     template<bool MIXED>
     __device__ static D4 transport(const Geo& c, const D4& x, const D4& k, const D4& q) {
         if constexpr (MIXED) {
-            const KsFactored<double> w = ks_factored_conn<double>(c.mass, c.spin, x.v[1], x.v[2], x.v[3]);
-            const KsFactoredK<double> p = ks_factored_k<double>(w, k.v);
+            const KsFactored w = ks_factored_conn(c.mass, c.spin, x.v[1], x.v[2], x.v[3]);
+            const KsFactoredK p = ks_factored_k(w, k.v);
             D4 d;
-            ks_factored_contract<double>(w, p, q.v, d.v);
+            ks_factored_contract(w, p, q.v, d.v);
             return d;
         } else {
             const KSConn w = ks_conn(c.mass, c.spin, x);
@@ -198,8 +198,7 @@ struct SceneGrmhd {
     __device__ static double radius(const ImageConsts&, const D4& X) { return fmks_radius(X); }
     template<bool MIXED>
     __device__ static double top_radius(const ImageConsts&, const D4& X) { return fmks_radius(X); }
-    // FP64 everywhere (an FP32 FMKS connection puts its rounding noise into
-    // the step-doubling error norm); the mixed policy uses the factored form
+    // the mixed policy uses the factored form
     template<bool MIXED>
     __device__ static Ray rhs(const ImageConsts& c, const Ray& X) {
         if constexpr (MIXED) {

@@ -93,7 +93,7 @@ int main() {
             c.max_step = 0.025 + 0.475 * u(rng);
             c.outer_radius = 4.0 + 46.0 * u(rng);
         }
-        c.fp32_radius = c.outer_radius + 2.0 * std::fmax(c.max_step, c.step);
+        c.far_radius = c.outer_radius + 2.0 * std::fmax(c.max_step, c.step);
         c.cam_radius = ray < 400 ? 200.0 + 1800.0 * u(rng) : 60.0 + 300.0 * u(rng);
         // a ray through the camera's radius at some impact parameter, its
         // wavevector null in the Kerr-Schild metric to first order
@@ -122,10 +122,10 @@ int main() {
             double h = c.step;
             if (pass == 1) h = cap;
             const double rr = ks_radius(c.spin, s.x);
-            if (pass == 1 && !(rr > c.fp32_radius)) break;
+            if (pass == 1 && !(rr > c.far_radius)) break;
             for (int guard = 0; guard < 60; ++guard) {
                 const double r0 = ks_radius(c.spin, s.x);
-                if (!(r0 > c.fp32_radius)) break;
+                if (!(r0 > c.far_radius)) break;
                 double xk = 0.0, kk = 0.0;
                 for (int i = 1; i < 4; ++i) {
                     xk += s.x.v[i] * s.k.v[i];
@@ -142,7 +142,7 @@ int main() {
                 bool ok = true;
                 for (int k = 0; k < run.count; ++k) {
                     const double rk = ks_radius(c.spin, s.x);
-                    ok = ok && rk > c.fp32_radius;
+                    ok = ok && rk > c.far_radius;
                     const Ray full = rk4(c.mass, c.spin, s, dir * hh);
                     const Ray half = rk4(c.mass, c.spin, s, 0.5 * dir * hh);
                     const Ray two = rk4(c.mass, c.spin, half, 0.5 * dir * hh);
@@ -162,7 +162,7 @@ int main() {
                     if (pass == 1) ok = ok && (old - c.cam_radius) * (r1 - c.cam_radius) > 0.0;
                     old = r1;
                 }
-                ok = ok && old > c.fp32_radius && std::fabs(len - run.length) <= 1e-9 * len &&
+                ok = ok && old > c.far_radius && std::fabs(len - run.length) <= 1e-9 * len &&
                      std::fabs(hh - run.next_h) <= 1e-12 * hh;
                 if (!ok) ++wrong;
                 worst_dist = std::fmax(worst_dist, distance(far, s));

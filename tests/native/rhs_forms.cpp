@@ -1,21 +1,38 @@
 // Host check of the mixed policy's factored transport RHS
-// (kpolaris_b200/csrc/kp_geometry_f32.cuh) against the reference-order FP64
-// RHS (kp_geometry.cuh) on seeded states around a Kerr black hole.  Prints
-// the largest normwise relative deviation of the FP64 form (all radii) and of
-// the FP32 form beyond r = 100 M (where the mixed policy uses it).
+// (kpolaris_b200/csrc/kp_geometry_mixed.cuh) against the reference-order FP64
+// RHS (kp_geometry.cuh) on seeded states around a Kerr black hole, and of the
+// FMKS one (fmks_rhs_factored against fmks_rhs in kp_fmks.cuh).  Prints the
+// largest normwise relative deviation of each.
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <random>
 #define __host__
 #define __device__
 #define __forceinline__ inline
 #define __noinline__
-#include "kp_geometry_f32.cuh"
+#include "kp_fmks.cuh"
+
+// The largest deviation of dk, de1 and de2, each against its own largest component.
+static double deviation(const kp::Ray& ref, const kp::Ray& got) {
+    const kp::D4* R[3] = {&ref.k, &ref.e1, &ref.e2};
+    const kp::D4* A[3] = {&got.k, &got.e1, &got.e2};
+    double worst = 0.0;
+    for (int w = 0; w < 3; ++w) {
+        double scale = 0.0, d = 0.0;
+        for (int k = 0; k < 4; ++k) {
+            scale = std::fmax(scale, std::fabs(R[w]->v[k]));
+            d = std::fmax(d, std::fabs(A[w]->v[k] - R[w]->v[k]));
+        }
+        if (scale > 0.0) worst = std::fmax(worst, d / scale);
+    }
+    return worst;
+}
 
 int main() {
     std::mt19937_64 rng(12345);
     std::uniform_real_distribution<double> u(-1.0, 1.0);
-    double worst64 = 0.0, far32 = 0.0;
+    double worst_ks = 0.0, worst_fmks = 0.0;
     for (int i = 0; i < 20000; ++i) {
         const double spin = 0.99 * std::fabs(u(rng));
         const double rad = 1.5 + std::pow(10.0, 3.0 * std::fabs(u(rng)));
@@ -30,25 +47,22 @@ int main() {
             s.e2.v[k] = u(rng);
         }
         s.k.v[0] = 1.0 + std::fabs(u(rng));
-        const kp::Ray ref = kp::ks_rhs(1.0, spin, s);
-        const kp::Ray f64 = kp::ks_rhs_factored<double>(1.0, spin, s);
-        const kp::Ray f32 = kp::ks_rhs_factored<float>(1.0, spin, s);
-        const kp::D4* R[3] = {&ref.k, &ref.e1, &ref.e2};
-        const kp::D4* A[3] = {&f64.k, &f64.e1, &f64.e2};
-        const kp::D4* B[3] = {&f32.k, &f32.e1, &f32.e2};
-        for (int w = 0; w < 3; ++w) {
-            double scale = 0.0, d64 = 0.0, d32 = 0.0;
-            for (int k = 0; k < 4; ++k) {
-                scale = std::fmax(scale, std::fabs(R[w]->v[k]));
-                d64 = std::fmax(d64, std::fabs(A[w]->v[k] - R[w]->v[k]));
-                d32 = std::fmax(d32, std::fabs(B[w]->v[k] - R[w]->v[k]));
-            }
-            if (scale > 0.0) {
-                worst64 = std::fmax(worst64, d64 / scale);
-                if (rad > 100.0) far32 = std::fmax(far32, d32 / scale);
-            }
-        }
+        worst_ks = std::fmax(worst_ks, deviation(kp::ks_rhs(1.0, spin, s), kp::ks_rhs_factored(1.0, spin, s)));
+        kp::FmksParams m;
+        std::memset(&m, 0, sizeof(m));
+        m.mass = 1.0;
+        m.spin = spin;
+        m.startx1 = std::log(1.2);
+        m.hslope = 0.3;
+        m.mks_smooth = 0.5;
+        m.poly_alpha = 14.0;
+        m.poly_xt = 0.82;
+        m.poly_norm = 0.5 * 3.141592653589793 / (1.0 + 1.0 / 15.0 / std::pow(0.82, 14.0));
+        s.x.v[1] = std::log(rad);
+        s.x.v[2] = 0.5 + 0.49 * u(rng);
+        s.x.v[3] = 3.0 * u(rng);
+        worst_fmks = std::fmax(worst_fmks, deviation(kp::fmks_rhs(m, s), kp::fmks_rhs_factored(m, s)));
     }
-    std::printf("%.3e %.3e\n", worst64, far32);
+    std::printf("%.3e %.3e\n", worst_ks, worst_fmks);
     return 0;
 }

@@ -9,7 +9,13 @@ two.
 
 * CPU: tests/native/exact_quotients.cpp, the method with C's fma and
   starting values of 20 bits, exact but for them and off by twice as much.
-* GPU: tests/native/exact_quotients.cu, against CUDA's own operators."""
+* GPU: tests/native/exact_quotients.cu, against CUDA's own operators.
+
+The mixed policy's reciprocals and roots (kp_geometry_mixed.cuh,
+kp_radiation_mixed.cuh) are not exact.  On the GPU: kp_recip and kp_sqrt_pair
+within 4 ulp, cube_root within 1e-12 for x in 1..1e7 and 1e-11 beyond -- a
+single-precision root is off by at most log(x) 2^-23 / 3, and Newton's step
+squares that."""
 from __future__ import annotations
 
 import ctypes as C
@@ -33,14 +39,28 @@ def test_host_emulation(tmp_path, err):
     assert [int(x) for x in out] == [0] * 5, dict(zip(("quots", "over", "quot", "recip", "root"), out))
 
 
-@pytest.mark.gpu
-def test_device_operators(tmp_path):
-    so = tmp_path / "exact_quotients.so"
+@pytest.fixture(scope="module")
+def device(tmp_path_factory):
+    so = tmp_path_factory.mktemp("exact") / "exact_quotients.so"
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3", "--fmad=false",
                     "-Xcompiler", "-fPIC,-ffp-contract=off", f"-I{CSRC}", f"-I{ROOT / 'include'}", f"-I{NATIVE}",
                     "-shared", "-o", str(so), str(NATIVE / "exact_quotients.cu")], check=True)
+    return C.CDLL(str(so))
+
+
+@pytest.mark.gpu
+def test_device_operators(device):
     counts = (C.c_ulonglong * 5)()
-    rc = C.CDLL(str(so)).kp_probe_exact_quotients(400, counts)
+    rc = device.kp_probe_exact_quotients(400, counts)
     assert rc == 0, f"cudaError {rc}"
     assert list(counts) == [0] * 5, dict(zip(("quots", "over", "quot", "recip", "root"), counts))
+
+
+@pytest.mark.gpu
+def test_device_mixed_roots(device):
+    errors = (C.c_double * 5)()
+    rc = device.kp_probe_mixed_roots(400, errors)
+    assert rc == 0, f"cudaError {rc}"
+    ulp = 2.0 ** -52
+    assert all(e <= bar for e, bar in zip(errors, (4 * ulp, 4 * ulp, 4 * ulp, 1e-12, 1e-11))), list(errors)

@@ -152,7 +152,7 @@ def integrated_pol(arrays, f):
 
 @pytest.mark.parametrize("name", ["grmhd_adaptive_16", "grmhd_multifreq_12x10", "grmhd_fixed_16"])
 def test_grmhd_mixed_within_budget_of_reference(name):
-    """Mixed policy (FP64 geodesic and grid sample, FP32 fits and transfer)
+    """Mixed policy (factored geodesic, fits and transfer, all of it FP64)
     against the reference's FP64 image: total flux within 1e-4, EVPA within
     0.1 deg, polarisation fractions within 1e-4, reasons 99% identical."""
     fx, prims, model, params, freqs, _ = load_case(name)

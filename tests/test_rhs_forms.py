@@ -1,8 +1,8 @@
-"""CPU check of the mixed policy's factored transport RHS
-(kpolaris_b200/csrc/kp_geometry_f32.cuh, host build of tests/native/rhs_forms.cpp)
-against the reference-order FP64 RHS on 20000 seeded states: the FP64 form
-within 1e-12 normwise (it regroups the same algebra), the FP32 form within
-1e-4 beyond r = 100 M (the far field, where the mixed policy uses it)."""
+"""CPU check of the mixed policy's factored transport right-hand sides (host
+build of tests/native/rhs_forms.cpp) against the reference-order FP64 ones on
+20000 seeded states: Kerr-Schild (kpolaris_b200/csrc/kp_geometry_mixed.cuh) and
+FMKS (kpolaris_b200/csrc/kp_fmks.cuh) within 1e-12 normwise (they regroup the
+same algebra)."""
 from __future__ import annotations
 
 import subprocess
@@ -17,6 +17,5 @@ def test_factored_rhs_matches_reference_order(tmp_path):
                     f"-I{ROOT / 'include'}", "-o", str(exe), str(ROOT / "tests" / "native" / "rhs_forms.cpp")],
                    check=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split()
-    worst64, far32 = float(out[0]), float(out[1])
-    assert worst64 <= 1e-12, worst64
-    assert far32 <= 1e-4, far32
+    for form, worst in zip(("Kerr-Schild", "FMKS"), out):
+        assert float(worst) <= 1e-12, (form, worst)

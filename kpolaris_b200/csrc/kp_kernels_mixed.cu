@@ -3,7 +3,7 @@
 // many far-field steps at once.  Compiled with FMA contraction enabled.
 #include <cuda_runtime.h>
 
-#include "kp_lanes.cuh"
+#include "kp_launch.h"
 #include "kp_quad.cuh"
 
 namespace kp {
@@ -12,26 +12,24 @@ __global__ void __launch_bounds__(kFarThreads, kFarBlocks) wave_far_mixed(const 
     quad_body<PolicyMixed, kPhaseFar>(W);
 }
 
-template<bool SHARED>
 __global__ void __launch_bounds__(kNearAThreads, kNearABlocks) wave_near_a_mixed(const WaveDesc W) {
-    quad_body<PolicyMixed, kPhaseNearA, SceneRiaf, SHARED>(W);
+    quad_body<PolicyMixed, kPhaseNearA>(W);
 }
 
-template<bool SHARED>
 __global__ void __launch_bounds__(kNearBThreads, kNearBBlocks) wave_near_b_mixed(const WaveDesc W) {
-    quad_body<PolicyMixed, kPhaseNearB, SceneRiaf, SHARED>(W);
+    quad_body<PolicyMixed, kPhaseNearB>(W);
 }
 
-template<bool SHARED>
 static const void* wave_kernel_mixed(int phase) {
     if (phase == kPhaseFar) return reinterpret_cast<const void*>(wave_far_mixed);
-    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_mixed<SHARED>);
-    return reinterpret_cast<const void*>(wave_near_b_mixed<SHARED>);
+    if (phase == kPhaseNearA) return reinterpret_cast<const void*>(wave_near_a_mixed);
+    return reinterpret_cast<const void*>(wave_near_b_mixed);
 }
 
 cudaError_t launch_wave_mixed(int phase, const WaveDesc& W, int blocks, int threads, cudaStream_t stream) {
-    const void* const fn[2] = {wave_kernel_mixed<false>(phase), wave_kernel_mixed<true>(phase)};
-    return launch_forms<PolicyMixed, SceneRiaf>(fn, phase, W, kMaxFreq, blocks, threads, stream);
+    if (phase < 0 || phase >= kPhases) return cudaErrorInvalidValue;
+    void* args[] = {const_cast<WaveDesc*>(&W)};
+    return cudaLaunchKernel(wave_kernel_mixed(phase), dim3(blocks), dim3(threads), args, 0, stream);
 }
 
 __global__ void __launch_bounds__(128) seed_mixed(const JobDesc* jobs, const SeedEntry* entries,
@@ -52,7 +50,7 @@ cudaError_t launch_seed_mixed(const JobDesc* jobs, const SeedEntry* entries, con
 int wave_occupancy_mixed(int phase, int threads) {
     if (phase < 0 || phase >= kPhases) return 0;
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wave_kernel_mixed<false>(phase), threads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wave_kernel_mixed(phase), threads, 0);
     return n;
 }
 

@@ -232,31 +232,31 @@ inline cudaError_t launch_wave(const void* quad_kernel, int phase, const WaveDes
 
 // Whether an image's near phases run with one ray per lane under the mixed
 // policy.  The forms round differently, so the line is drawn by the image
-// alone: an image is the same in a batch, in a server and by itself.  At
-// several frequencies the longest rays of a Faraday-thick image, which a quad
-// steps faster, set the time up to much larger images.  Measured, quads / lanes
-// (ms per image):
-//   RIAF, one frequency    256^2 27 / 30, 320^2 41 / 36, 512^2 103 / 71, 1024^2 407 / 276;
-//                          at 60 degrees 320^2 47 / 57, 512^2 114 / 107
-//   RIAF, two or four      512^2 155 / 218, at 60 degrees 392 / 890; 768^2 at 60 degrees
-//                          580 / 721 and 585 / 978; 1024^2 603 / 415 and 604 / 479
-//   Boyer-Lindquist        one: 256^2 102 / 104, 320^2 152 / 136, 512^2 356 / 287; four: 512^2 482 / 537
-//   GRMHD                  256^2 69 / 89, 320^2 108 / 130, 384^2 152 / 142, 512^2 270 / 206;
-//                          four frequencies 384^2 184 / 180, 512^2 322 / 263
-//   slow light             320^2 106 / 106, 512^2 262 / 169
+// alone: an image is the same in a batch, in a server and by itself.  Measured,
+// quads / lanes (ms per image):
+//   GRMHD           256^2 69 / 89, 320^2 108 / 130, 384^2 152 / 142, 512^2 270 / 206;
+//                   four frequencies 384^2 184 / 180, 512^2 322 / 263
+//   slow light      320^2 106 / 106, 512^2 262 / 169
+//   Boyer-Lindquist one frequency 256^2 102 / 104, 320^2 152 / 136, 512^2 356 / 287; four
+//                   512^2 482 / 537 (the longest rays of a Faraday-thick image set the time,
+//                   and a quad steps them faster)
+// Cartesian Kerr-Schild images keep the quads: one of 512^2 at one frequency takes
+// 103 / 71, but images of many sizes share launches there, and 64 of 32^2 to
+// 512^2 take 2.62 s on quads, 2.78 s with the larger ones on lanes, whose
+// kernels end with their own longest rays after those of the quads.
 inline int lane_image(const ImageConsts& c, int npix) {
 #ifdef KP_LANE_PIXELS
     return npix > KP_LANE_PIXELS;
 #endif
-    const bool riaf = c.scene == kSceneRiafCks || c.scene == kSceneRiafBL;
-    if (riaf && c.nfreq > 1) return npix > 800000;
-    return npix > (c.scene == kSceneRiafBL ? 80000 : 120000);
+    if (c.scene == kSceneRiafCks) return 0;
+    if (c.scene == kSceneRiafBL) return npix > (c.nfreq == 1 ? 80000 : 800000);
+    return npix > 120000;
 }
 
 // A launch of a phase under the mixed policy: one kernel for each form that
 // its images take.  `quad_kernel`: of the phase, and of the phase where it
-// shares its launch with lanes (the test of every ray's form costs a RIAF
-// image 2% of its time).
+// shares its launch with lanes (the test of every ray's form costs an
+// image alone 2% of its time).
 template<class P, class SC>
 inline cudaError_t launch_forms(const void* const (&quad_kernel)[2], int phase, const WaveDesc& W, int nf_max,
                                 int blocks, int threads, cudaStream_t stream) {

@@ -31,24 +31,35 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off",
           f"-I{INCLUDE}", f"-I{CSRC}", "-Xptxas", "-warn-spills"]
 
+FP64 = ["--fmad=false"]
+MIXED = ["--fmad=true", "--use_fast_math"]
+
+
+def _lanes(policy: str, scene: str, *more: str):
+    return [*(FP64 if policy == "FP64" else MIXED), f"-DKP_LANES_POLICY=Policy{policy}", f"-DKP_LANES_SCENE=Scene{scene}", *more]
+
+
 # translation unit, with the name of its build where it has several -> extra flags
 UNITS = {
-    "kp_lanes.cu fp64": ["--fmad=false", "-DKP_LANES_SCENE=SceneRiaf", "-DKP_LANES_IMAGE"],
-    "kp_lanes.cu grmhd": ["--fmad=false", "-DKP_LANES_SCENE=SceneGrmhd"],
-    "kp_lanes.cu grmhd_slow": ["--fmad=false", "-DKP_LANES_SCENE=SceneGrmhdSlow"],
-    "kp_lanes.cu bl": ["--fmad=false", "-DKP_LANES_SCENE=SceneRiafBL"],
-    "kp_kernels_fp64.cu": ["--fmad=false"],
-    "kp_kernels_mixed.cu": ["--fmad=true", "--use_fast_math"],
-    "kp_kernels_grmhd.cu": ["--fmad=false"],
-    "kp_kernels_grmhd_mixed.cu": ["--fmad=true", "--use_fast_math"],
-    "kp_kernels_grmhd_slow.cu": ["--fmad=false"],
-    "kp_kernels_bl.cu": ["--fmad=false"],
-    "kp_kernels_bl_mixed.cu": ["--fmad=true", "--use_fast_math"],
-    "kp_kernels_grmhd_slow_mixed.cu": ["--fmad=true", "--use_fast_math"],
-    "kp_capi.cu": ["--fmad=false"],
-    "kp_reorder.cu": ["--fmad=false"],
-    "kp_noalloc.cu": ["--fmad=false"],
-    "kp_server.cu": ["--fmad=false"],
+    "kp_lanes.cu fp64": _lanes("FP64", "Riaf", "-DKP_LANES_IMAGE"),
+    "kp_lanes.cu grmhd": _lanes("FP64", "Grmhd"),
+    "kp_lanes.cu grmhd_slow": _lanes("FP64", "GrmhdSlow"),
+    "kp_lanes.cu bl": _lanes("FP64", "RiafBL"),
+    "kp_lanes.cu grmhd_mixed": _lanes("Mixed", "Grmhd"),
+    "kp_lanes.cu grmhd_slow_mixed": _lanes("Mixed", "GrmhdSlow"),
+    "kp_lanes.cu bl_mixed": _lanes("Mixed", "RiafBL"),
+    "kp_kernels_fp64.cu": FP64,
+    "kp_kernels_mixed.cu": MIXED,
+    "kp_kernels_grmhd.cu": FP64,
+    "kp_kernels_grmhd_mixed.cu": MIXED,
+    "kp_kernels_grmhd_slow.cu": FP64,
+    "kp_kernels_bl.cu": FP64,
+    "kp_kernels_bl_mixed.cu": MIXED,
+    "kp_kernels_grmhd_slow_mixed.cu": MIXED,
+    "kp_capi.cu": FP64,
+    "kp_reorder.cu": FP64,
+    "kp_noalloc.cu": FP64,
+    "kp_server.cu": FP64,
     "kp_peak.cu": [],
     "kp_io.cu": [f"-I{HOST}"],
 }

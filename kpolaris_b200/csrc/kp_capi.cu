@@ -104,7 +104,7 @@ struct DeviceState {
     // instantiated launch graphs (KP_SCHEDULE_GRAPH), keyed by everything
     // they bake in; the oldest is dropped beyond kGraphCacheSize
     struct GraphEntry {
-        int family, nf_max, njobs, cycles, forms;
+        int family, nf_max, njobs, cycles, forms, fixed_steps;
         long long total;
         int blocks[kPhases];
         const void* jobs;
@@ -612,8 +612,8 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         if (e != cudaSuccess) return cuda_error(e, "cudaMemsetAsync(wave counters)");
     }
     if (opt.threads_per_block != 0)
-        return set_error(KP_ERR_INVALID, "threads_per_block is fixed by the wavefront kernels (%d far, %d near-A, %d near-B): pass 0",
-                         kFarThreads, kNearAThreads, kNearBThreads);
+        return set_error(KP_ERR_INVALID, "threads_per_block is fixed by the wavefront kernels (%d far, %d near-A, %d near-B): pass 0", kFarThreads,
+                         kNearAThreads, kNearBThreads);
     const bool mixed = family == kFamilyRiafMixed;
     int blocks[kPhases];
     for (int phase = 0; phase < kPhases; ++phase) {
@@ -635,8 +635,11 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         const long long needed = wave_blocks_needed(phase, total);
         if (blocks[phase] > needed) blocks[phase] = int(needed);
     }
-    int forms = 0;
-    for (int i = 0; i < njobs; ++i) forms |= dev->h_jobs[i].lanes ? kFormLanes : kFormQuads;
+    int forms = 0, fixed_steps = 1;
+    for (int i = 0; i < njobs; ++i) {
+        forms |= dev->h_jobs[i].lanes ? kFormLanes : kFormQuads;
+        if (dev->h_jobs[i].c.adaptive) fixed_steps = 0;
+    }
     WaveCtrl* ctrl = dev->d_ctrl;
     auto launch = [&](int cycle, int phase) -> cudaError_t {
         WaveDesc W;
@@ -651,6 +654,7 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         W.in_head = &ctrl->heads[cycle * kPhases + phase];
         W.lane_head = &ctrl->lane_heads[cycle * kPhases + phase];
         W.forms = forms;
+        W.fixed_steps = fixed_steps;
         for (int q = 0; q < kPhases; ++q) {
             const int gen = q > phase ? cycle : cycle + 1;
             W.out_ids[q] = dev->d_ids[q][gen % 2];
@@ -698,6 +702,7 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         key.njobs = njobs;
         key.cycles = cycles;
         key.forms = forms;
+        key.fixed_steps = fixed_steps;
         key.total = total;
         for (int p = 0; p < kPhases; ++p) {
             key.blocks[p] = blocks[p];
@@ -711,10 +716,11 @@ int run_wave_jobs(DeviceState* dev, cudaStream_t stream, int njobs, long long to
         key.lpt = dev->d_lpt;
         cudaGraphExec_t exec = nullptr;
         for (const auto& g : dev->graphs) {
-            if (g.family == key.family && g.nf_max == key.nf_max && g.njobs == key.njobs && g.cycles == key.cycles && g.forms == key.forms &&
-                g.total == key.total && std::memcmp(g.blocks, key.blocks, sizeof(key.blocks)) == 0 &&
-                g.jobs == key.jobs && g.pool == key.pool && g.ctrl == key.ctrl && g.sorted == key.sorted &&
-                g.lpt == key.lpt && std::memcmp(g.ids, key.ids, sizeof(key.ids)) == 0) {
+            if (g.family == key.family && g.nf_max == key.nf_max && g.njobs == key.njobs && g.cycles == key.cycles &&
+                g.forms == key.forms && g.fixed_steps == key.fixed_steps && g.total == key.total &&
+                std::memcmp(g.blocks, key.blocks, sizeof(key.blocks)) == 0 && g.jobs == key.jobs && g.pool == key.pool &&
+                g.ctrl == key.ctrl && g.sorted == key.sorted && g.lpt == key.lpt &&
+                std::memcmp(g.ids, key.ids, sizeof(key.ids)) == 0) {
                 exec = g.exec;
                 break;
             }

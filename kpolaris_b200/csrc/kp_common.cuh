@@ -219,6 +219,7 @@ struct WaveDesc {
     const unsigned* in_ids;
     const unsigned* in_count;
     long long rays_max;            // rays there can be at most (host)
+    int fixed_steps;               // every image's steps are fixed (host)
     int forms;                     // mixed policy: kForm bits of the forms the rays' images take
     unsigned long long* in_head;   // pop counter, zero before the launch
     unsigned long long* lane_head; // the lane kernel's, where both forms have rays

@@ -2,7 +2,7 @@
 // on the wavefront engine with the mixed policy (FP64 BL geodesic, factored fits), compiled with FMA contraction.
 #include <cuda_runtime.h>
 
-#include "kp_lanes.cuh"
+#include "kp_launch.h"
 #include "kp_quad.cuh"
 
 namespace kp {

@@ -5,7 +5,7 @@
 // budget, not to the reference's rounding).
 #include <cuda_runtime.h>
 
-#include "kp_lanes.cuh"
+#include "kp_launch.h"
 #include "kp_quad.cuh"
 
 namespace kp {

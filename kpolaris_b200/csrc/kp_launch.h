@@ -183,35 +183,30 @@ inline long long wave_blocks_needed(int phase, long long rays) {
 //           2: 320^2 161 / 168, 512^2 338 / 282, 8 x 256^2 670 / 330
 //           4: 384^2 202 / 217, 512^2 344 / 343, 4 x 320^2 at 10 to 70 degrees 1655 / 1870,
 //              8 x 256^2 678 / 472
+//   fixed steps, which are much of a length: near-B 192^2 32 / 11
 //   GRMHD   256^2 177 / 185, 320^2 266 / 263, 512^2 628 / 474; four frequencies 720 / 582
 // (near-B: lanes until its input runs out, the rest on quads.  Without that
 // 4 x 320^2 took 3243, 8 x 256^2 492.)
-inline long long quad_rays(int phase, int nf_max, bool fmks, long long quads) {
-#ifdef KP_ROUNDS
-    return phase == kPhaseFar ? quads : KP_ROUNDS * quads;
-#endif
-    if (phase == kPhaseFar) return quads;
+inline long long quad_rays(int phase, int nf_max, bool fmks, bool fixed_steps, long long quads) {
+    if (phase == kPhaseFar || fixed_steps) return quads;
     if (phase == kPhaseNearA || nf_max == 1 || fmks) return 8 * quads;
     return (nf_max == 2 ? 24 : 48) * quads;
 }
 
 // Pixels up to which the plain FP64 kernel gives each a quad: with fixed
 // steps, whose rays are much of a length, while every ray gets one of its own
-// (128^2: 64 / 48 ms); with adaptive steps until the longest rays no longer
+// (96^2 32 / 31 ms, 128^2 56 / 31, 256^2 209 / 87); with adaptive steps until the longest rays no longer
 // set the time (quads / lanes: one frequency 192^2 122 / 131, 256^2 217 / 165,
 // 1024^2 3205 / 1873; two 256^2 378 / 381, 512^2 1313 / 1075; four 512^2 1336
 // / 1439, 768^2 2900 / 2510).
 inline long long image_quad_pixels(int nfreq, bool adaptive, int sms) {
-#ifdef KP_ROUNDS
-    return KP_ROUNDS * 64ll * sms;
-#endif
     return (!adaptive ? 1 : (nfreq == 1 ? 5 : (nfreq == 2 ? 24 : 48))) * 64ll * sms;
 }
 
 // One launch of a phase: the quad kernel and, where there can be more rays
 // than it takes, the lane kernel; whichever the launch's ray count is not for
 // returns at once.  The lane kernel of near-B hands at most its `lanes` rays
-// on, which the next launch takes on quads.
+// on, 4 per quad, which the next launch takes on quads (their line is above).
 template<class P, class SC>
 cudaError_t launch_lanes(int phase, const WaveDesc& W, int nf_max, long long lanes, long long quad_rays,
                          cudaStream_t stream);
@@ -221,7 +216,7 @@ inline cudaError_t launch_wave(const void* quad_kernel, int phase, const WaveDes
                                int blocks, int threads, cudaStream_t stream) {
     if (nf_max < 1 || nf_max > kMaxFreq || phase < 0 || phase >= kPhases) return cudaErrorInvalidValue;
     const long long lanes = (long long)blocks * threads;
-    long long rays = quad_rays(phase, nf_max, fmks, lanes / 4);
+    long long rays = quad_rays(phase, nf_max, fmks, W.fixed_steps, lanes / 4);
     if (W.fresh_end - W.fresh_begin <= rays) {
         void* args[] = {const_cast<WaveDesc*>(&W), &rays};
         const cudaError_t e = cudaLaunchKernel(quad_kernel, dim3(blocks), dim3(threads), args, 0, stream);
@@ -245,9 +240,6 @@ inline cudaError_t launch_wave(const void* quad_kernel, int phase, const WaveDes
 // 512^2 take 2.62 s on quads, 2.78 s with the larger ones on lanes, whose
 // kernels end with their own longest rays after those of the quads.
 inline int lane_image(const ImageConsts& c, int npix) {
-#ifdef KP_LANE_PIXELS
-    return npix > KP_LANE_PIXELS;
-#endif
     if (c.scene == kSceneRiafCks) return 0;
     if (c.scene == kSceneRiafBL) return npix > (c.nfreq == 1 ? 80000 : 800000);
     return npix > 120000;

@@ -124,6 +124,7 @@ extern "C" int kp_batch_riaf_noalloc(const kp_riaf_job* jobs, int njobs, const k
     // job table: built on the host stack, copied into the static scratch
     JobDesc table[KP_NOALLOC_MAX_JOBS];
     long long ray = 0;
+    int fixed_steps = 1;
     for (int i = 0; i < njobs; ++i) {
         const kp_riaf_job& jb = jobs[i];
         JobDesc& d = table[i];
@@ -138,6 +139,7 @@ extern "C" int kp_batch_riaf_noalloc(const kp_riaf_job* jobs, int njobs, const k
             d.frame.e2.v[mu] = fr[3][mu];
             d.frame.e3.v[mu] = fr[4][mu];
         }
+        if (d.c.adaptive) fixed_steps = 0;
         d.out = from_abi(&jb.out);
         d.ray_begin = ray;
         d.npix = jb.params.camera.nx * jb.params.camera.ny;
@@ -178,6 +180,7 @@ extern "C" int kp_batch_riaf_noalloc(const kp_riaf_job* jobs, int njobs, const k
             W.rays_max = total;
             W.in_head = W.lane_head = &S->ctrl.heads[cycle * kPhases + phase];
             W.forms = kFormQuads;
+            W.fixed_steps = fixed_steps;
             for (int q = 0; q < kPhases; ++q) {
                 const int gen = q > phase ? cycle : cycle + 1;
                 W.out_ids[q] = S->ids[q][gen % 2];

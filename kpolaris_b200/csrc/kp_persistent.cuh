@@ -371,10 +371,11 @@ __device__ __forceinline__ void lane_body(const WaveDesc& W) {
         }
         // Near-B hands the rays left when its input runs out to the quads of
         // its next launch: the longest rays, of which few are left then, take
-        // a step in half to a quarter of a lane's time.
+        // a step in half to a quarter of a lane's time.  (Rays of fixed steps
+        // end together.)
         bool hand_over = false;
         if constexpr (PHASE == kPhaseNearB && !P::kMixed)
-            hand_over = (long long)*(const volatile unsigned long long*)W.in_head >= total_in;
+            hand_over = !W.fixed_steps && (long long)*(const volatile unsigned long long*)W.in_head >= total_in;
         const bool active = st.mode != kIdle;
         // The block leaves the loop together, so the barrier below is
         // reached by every thread of the block in every iteration.  A lane

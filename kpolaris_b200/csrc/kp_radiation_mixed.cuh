@@ -115,7 +115,9 @@ KP_HD void bessel_ratios(double x, double lg, double& r0, double& r1) {  // lg =
 // Plasma state at a sample point, with the frequency-independent factors of
 // the thermal fits (riaf_sample_thermal_m).
 struct RiafSampleM {
-    double ne, thetae, b, nu_fluid, cos_theta, sin_theta, cos2chi, sin2chi;
+    double ne, thetae, b, nu_fluid, cos_theta, sin_theta;
+    double unused;  // without this slot near-B of slow light spills 440 instead of 332 B (72 x 50: 32.5 / 31.6 ms)
+    double cos2chi, sin2chi;
     double xs0;     // argument of the emission fit, over the frequency in hertz
     double xf0;     // argument of the Faraday fits times the root of the frequency
     double rv0;     // rho_V nu times the frequency, without the fit's logarithm

@@ -431,6 +431,7 @@ void worker_main(kp_server* s) {
                 W.in_head = s->heads[sc] + p;
                 W.lane_head = s->heads[sc] + kPhases + p;
                 W.forms = forms[sc];
+                W.fixed_steps = 0;  // of images in flight, some may be adaptive
                 for (int q = 0; q < kPhases; ++q) {
                     const int g = q > p ? cur : nxt;
                     W.out_ids[q] = s->ids[sc][q][g];
